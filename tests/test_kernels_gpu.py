@@ -132,6 +132,40 @@ def test_rope_kv_write(d, rot, neox, qk_norm):
     assert torch.equal(vc, vc_r)
 
 
+@pytest.mark.parametrize("t,hq,hkv", [(1, 5, 1), (3, 32, 8), (700, 19, 3), (2100, 32, 8)])   # one head per lane, or four
+@pytest.mark.parametrize("d,rot,neox", [(64, 32, True), (64, 0, True), (128, 96, True), (128, 24, False), (256, 256, True)])
+@pytest.mark.parametrize("shift", [0, 1])     # 1: rows off the 16-byte boundary (the 4-byte kernel)
+def test_rope_kv_write_edges(t, hq, hkv, d, rot, neox, shift):
+    """Head counts that leave lane groups empty, partly rotated heads, skipped slots, both access widths; against fp32
+    formulas at bf16 rounding (2^-9 relative per step, two steps)."""
+    from gllm_b200.ops import sm100
+    if (rot // 2) % (d // 32):
+        pytest.skip("rotated halves must hold whole lanes")
+    torch.manual_seed(t + d)
+    page, pages = 16, (t + 15) // 16 + 2
+    width = (hq + 2 * hkv) * d
+    buf = torch.randn(t, width + 8, device=_dev()).bfloat16()
+    ref_buf = buf.clone()
+    pos = torch.randint(0, 4000, (t,), device=_dev(), dtype=torch.int32)
+    slots = torch.randperm(pages * page, device=_dev())[:t].to(torch.int32)
+    slots[t // 2] = -1
+    cs = ref.build_cos_sin_cache(rot, 4096, 10000.0).to(_dev()) if rot else None
+    qn = (1 + 0.1 * torch.randn(d, device=_dev())).bfloat16()
+    kn = (1 + 0.1 * torch.randn(d, device=_dev())).bfloat16()
+    shape = ref.kv_cache_shape(pages, hkv, d, page)
+    caches = [torch.zeros(shape, device=_dev(), dtype=torch.bfloat16) for _ in range(4)]
+
+    def views(b):
+        b = b[:, 2 * shift:2 * shift + width]
+        return (b[:, : hq * d].unflatten(1, (hq, d)), b[:, hq * d: (hq + hkv) * d].unflatten(1, (hkv, d)),
+                b[:, (hq + hkv) * d:].unflatten(1, (hkv, d)))
+
+    sm100.rope_kv_write(*views(buf), pos, cs, rot, neox, qn, kn, 1e-6, caches[0], caches[1], slots)
+    ref.rope_kv_write(*views(ref_buf), pos, cs, rot, neox, qn, kn, 1e-6, caches[2], caches[3], slots)
+    assert _rel_err(buf, ref_buf) < 8e-3 and _rel_err(caches[0], caches[2]) < 8e-3
+    assert torch.equal(caches[1], caches[3])
+
+
 @pytest.mark.parametrize("sec", [[16, 24, 24], [24, 20, 20, 1]])   # chunked (Qwen2.5-VL) / interleaved (Qwen3-VL)
 @pytest.mark.parametrize("strided", [False, True])
 def test_rope_mrope(sec, strided):
