@@ -28,7 +28,14 @@ def linear(x, w, bias=None, out=None):
 
 
 def linear_silu_mul(x, w_interleaved, out=None, act="silu"):
-    """act(gate) * up of one gate / up projection (rows interleaved per 128); `act`: "silu" | "gelu" (tanh form)."""
+    """act(gate) * up of one gate / up projection (rows interleaved per 128); `act`: "silu" | "gelu" (tanh form).
+    An fp8 weight is the pair (e4m3 [gate rows ; up rows], scale_inv), not interleaved; silu only."""
+    if isinstance(w_interleaved, tuple):
+        assert act == "silu" and out is None
+        w8, ws = w_interleaved
+        if x.is_cuda and w8.shape[0] % 256 == 0:
+            return _sm().linear_fp8_block(x, w8, ws, silu=True)
+        return silu_and_mul(linear(x, w_interleaved))
     if x.is_cuda:
         return _sm().linear_silu_mul(x, w_interleaved, out, act=act)
     y = ref.linear_silu_mul(x, w_interleaved, act=act)

@@ -216,6 +216,8 @@ class DenseMLP(nn.Module):
     def act(self, h: torch.Tensor, tpc: TPComm) -> torch.Tensor:
         if self.fused_act:
             return tpc.col_linear_silu_mul(h, self.gate_up_w)
+        if self.gate_up_ws is not None:
+            return tpc.col_linear_silu_mul(h, _qw(self.gate_up_w, self.gate_up_ws))
         return Fn.silu_and_mul(tpc.col_linear(h, _qw(self.gate_up_w, self.gate_up_ws)))
 
 

@@ -35,6 +35,15 @@ def _count(n=1):
     _launch_count += n
 
 
+def waits_given_up() -> int:
+    """Bounded waits that ran out in this process's kernels (csrc/common/bounded.cuh); 0 in a healthy run."""
+    L = _lib.load()
+    return sum(getattr(L, f"gllm_waits_given_up_{f}")() for f in _WAIT_FAMILIES)
+
+
+_WAIT_FAMILIES = ("fp8",)
+
+
 # ----------------------------------------------------------------------------------------------
 # GEMM
 # ----------------------------------------------------------------------------------------------
@@ -438,26 +447,28 @@ def fp8_quant_group(x: torch.Tensor):
     q = torch.empty(m, k, dtype=torch.float8_e4m3fn, device=x.device)
     s = torch.empty(k // 128, m, dtype=torch.float32, device=x.device)
     L = _lib.load()
-    check(L.gllm_fp8_quant_group(_p(x), x.stride(0), _p(q), _p(s), m, k, stream_ptr()), "fp8_quant_group")
+    check(L.gllm_fp8_quant_group(_p(x), x.stride(0), _p(q), _p(s), m, k, None, stream_ptr()), "fp8_quant_group")
     _count()
     return q, s
 
 
 def linear_fp8_block(x: torch.Tensor, w8: torch.Tensor, w_scale_inv: torch.Tensor,
-                     bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """x bf16 [M,K]; w8 e4m3 [N,K]; w_scale_inv fp32 [ceil(N/128), K/128] -> bf16 [M,N]."""
+                     bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
+                     silu: bool = False) -> torch.Tensor:
+    """x bf16 [M,K]; w8 e4m3 [N,K]; w_scale_inv fp32 [ceil(N/128), K/128] -> bf16 [M,N]. `silu`: w8 is [gate rows ; up
+    rows] and the result silu(gate) * up [M, N/2] (N/2 % 128 == 0)."""
     assert w8.dtype == torch.float8_e4m3fn and w8.is_contiguous() and w_scale_inv.dtype == torch.float32
     assert w_scale_inv.is_contiguous()
     m, k = x.shape
     n = w8.shape[0]
     if out is None:
-        out = torch.empty(m, n, dtype=_BF16, device=x.device)
+        out = torch.empty(m, n // 2 if silu else n, dtype=_BF16, device=x.device)
     if m == 0:
         return out
     xq, xs = fp8_quant_group(x)
     L = _lib.load()
     check(L.gllm_gemm_fp8_block(_p(xq), _p(xs), _p(w8), _p(w_scale_inv), _p(out), out.stride(0), m, n, k, _p(bias),
-                                stream_ptr()), "gemm_fp8_block")
+                                int(silu), stream_ptr()), "gemm_fp8_block")
     _count()
     return out
 

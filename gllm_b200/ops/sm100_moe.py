@@ -158,10 +158,10 @@ def fused_experts_fp8(x: torch.Tensor, w13: torch.Tensor, w13_s: torch.Tensor, w
     st = stream_ptr()
     check(L.gllm_moe_align_gather(_p(topk_ids), _p(expert_map), t, k, e_local, _p(meta), _p(tile_expert), max_tiles,
                                   _p(slot_pos), _p(x), x.stride(0), _p(xs), h, None, st), "moe_align_gather")
-    check(L.gllm_fp8_quant_group(_p(xs), h, _p(xs8), _p(xs_s), rows, h, st), "fp8_quant(xs)")
+    check(L.gllm_fp8_quant_group(_p(xs), h, _p(xs8), _p(xs_s), rows, h, _p(meta), st), "fp8_quant(xs)")   # meta[0]: live tiles
     check(L.gllm_moe_grouped_gemm_fp8(_p(xs8), _p(xs_s), _p(w13), _p(w13_s), _p(hbuf), inter, max_tiles, two_i, h,
                                       e_local, _p(tile_expert), _p(meta), 1, st), "moe_grouped_gemm_fp8(1)")
-    check(L.gllm_fp8_quant_group(_p(hbuf), inter, _p(h8), _p(h_s), rows, inter, st), "fp8_quant(h)")
+    check(L.gllm_fp8_quant_group(_p(hbuf), inter, _p(h8), _p(h_s), rows, inter, _p(meta), st), "fp8_quant(h)")
     check(L.gllm_moe_grouped_gemm_fp8(_p(h8), _p(h_s), _p(w2), _p(w2_s), _p(ybuf), h, max_tiles, h, inter, e_local,
                                       _p(tile_expert), _p(meta), 0, st), "moe_grouped_gemm_fp8(2)")
     check(L.gllm_moe_combine(_p(ybuf), _p(slot_pos), _p(topk_w), _p(out), t, k, h, st), "moe_combine")

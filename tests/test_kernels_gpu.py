@@ -469,7 +469,8 @@ def test_moe_fused_experts(t, e, k, h, i, ep):
 
 
 @pytest.mark.parametrize("m,n,k", [(1, 256, 128), (77, 1536, 512), (300, 4096, 7168), (1024, 2048, 2048),
-                                   (64, 576, 7168)])      # 576 = kv_a_proj_with_mqa (MLA): N not a multiple of 128
+                                   (64, 576, 7168),       # 576 = kv_a_proj_with_mqa (MLA): N not a multiple of 128
+                                   (129, 8200, 640), (3000, 1032, 384), (2500, 4352, 1152)])   # tiles of 64, 128, 256
 def test_gemm_fp8_block(m, n, k):
     from gllm_b200.ops import sm100
     torch.manual_seed(m)
@@ -486,6 +487,13 @@ def test_gemm_fp8_block(m, n, k):
     y = sm100.linear_fp8_block(x, w8, s_inv.contiguous(), b)
     y_ref = ref.linear_fp8_block(x, w8, s_inv, b)
     assert _rel_err(y, y_ref) < 1e-2, _rel_err(y, y_ref)
+    assert sm100.waits_given_up() == 0
+    if n % 256 == 0:      # [gate ; up] weight with the gated epilogue: the activation leaves the fp32 sums, no bf16 between
+        y = sm100.linear_fp8_block(x, w8, s_inv.contiguous(), silu=True)
+        xq, xs = ref.fp8_quant_group(x)
+        wide = w8.float() * s_inv.repeat_interleave(128, 0)[:n].repeat_interleave(128, 1)
+        g, u = ((xq.float() * xs.repeat_interleave(128, 1)) @ wide.t()).chunk(2, -1)
+        assert _rel_err(y, torch.nn.functional.silu(g) * u) < 1e-2
     # and the quantiser alone
     q, s = sm100.fp8_quant_group(x)
     q_r, s_r = ref.fp8_quant_group(x)
