@@ -271,7 +271,8 @@ __global__ void __launch_bounds__(256) rope_kv_write_vec_kernel(
 // in shared memory by the whole block (SiLU, unit length and the q scale applied there). With KD the decay is one
 // value per key channel, gk[t, h * D + d] in fp32 (`key_decay_kernel`), acting on row d; it is staged beside the key as
 // (k, decay) pairs, so the update still costs two shared loads per state entry. `step`: the softplus that forms the
-// decay is also the write strength (u = softplus(a + dt_bias) v); dskip (per head): o += dskip v.
+// decay is also the write strength (u = softplus(a + dt_bias) v); dskip (per head): o += dskip v. max_len > 0: longer
+// sequences are another kernel's (the chunked delta rule, delta_ops.cu).
 template <typename T, int NS, int PARTS, bool KD>
 __global__ void __launch_bounds__(32 * PARTS) linear_state_kernel(
     const T* __restrict__ q, long ldq, const T* __restrict__ k, long ldk, const T* __restrict__ v, long ldv,
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(32 * PARTS) linear_state_kernel(
     const float* __restrict__ dt_bias, const float* __restrict__ decay, float* __restrict__ state,
     const int* __restrict__ rec_slots, const int* __restrict__ seq_lens, const int* __restrict__ qsl, int H, int G,
     int D, int V, int silu_in, int unit_qk, float q_scale, int delta, float* __restrict__ out,
-    const float* __restrict__ gk, long ldgk, int step, const float* __restrict__ dskip) {
+    const float* __restrict__ gk, long ldgk, int step, const float* __restrict__ dskip, int max_len) {
   constexpr int TCH = 8;               // tokens staged per round (16 measured 2.4x slower: registers)
   constexpr int ROWS = KD ? 3 : 2;
   extern __shared__ float sm[];
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(32 * PARTS) linear_state_kernel(
   const bool active = vcol < V;
   const int vc = active ? vcol : V - 1;          // idle lanes mirror the last column (loads only)
   const int q0 = qsl[s], q1 = qsl[s + 1];
-  if (q1 <= q0) return;                          // uniform over the block
+  if (q1 <= q0 || (max_len > 0 && q1 - q0 > max_len)) return;      // uniform over the block
   const bool carried = state != nullptr && (seq_lens[s] - (q1 - q0)) > 0;
   float* st = state != nullptr ? state + ((size_t)rec_slots[s] * H + h) * (size_t)D * V : nullptr;
   float S[NS];
@@ -733,12 +734,12 @@ int state_dispatch(dim3 grid, size_t smem, cudaStream_t st, const void* q, long 
                    const void* v, long ldv, const void* beta, long ldb, const void* a, long lda, const float* neg_a,
                    const float* dt_bias, const float* decay, float* state, const int* rec_slots, const int* seq_lens,
                    const int* qsl, int H, int G, int D, int V, int silu_in, int unit_qk, float q_scale, int delta,
-                   float* out, int parts, const float* zk, long ldz, int step, const float* dskip) {
+                   float* out, int parts, const float* zk, long ldz, int step, const float* dskip, int max_len) {
 #define GLLM_STATE_KD(NS, PARTS, KD)                                                                                \
   linear_state_kernel<T, NS, PARTS, KD><<<grid, 32 * PARTS, smem, st>>>(                                            \
       (const T*)q, ldq, (const T*)k, ldk, (const T*)v, ldv, (const T*)beta, ldb, (const T*)a, lda, neg_a, dt_bias,  \
       decay, state, rec_slots, seq_lens, qsl, H, G, D, V, silu_in, unit_qk, q_scale, delta, out, zk, ldz, \
-      step, dskip)
+      step, dskip, max_len)
 #define GLLM_STATE(NS, PARTS)                                               \
   do {                                                                      \
     if (zk != nullptr) GLLM_STATE_KD(NS, PARTS, true);                      \
@@ -830,7 +831,7 @@ GLLM_EXPORT int gllm_seq_linear_state(const void* q, long ldq, const void* k, lo
                                       const void* seq_lens, const void* qsl, int nseq, int H, int G, int D, int V,
                                       int silu_in, int unit_qk, float q_scale, int delta, void* out, int is_f32,
                                       int parts, const void* gk, long ldgk, int step, const void* dskip,
-                                      void* stream) {
+                                      int max_len, void* stream) {
   if (nseq <= 0) return 0;
   if (step && (delta || a == nullptr)) return 2;                       // the step is the decay's own softplus
   if (gk != nullptr && (delta || G != H)) return 2;                    // key-channel decay: plain update, own keys
@@ -843,12 +844,12 @@ GLLM_EXPORT int gllm_seq_linear_state(const void* q, long ldq, const void* k, lo
     rc = state_dispatch<float>(grid, smem, st, q, ldq, k, ldk, v, ldv, beta, ldb, a, lda, (const float*)neg_a,
                                (const float*)dt_bias, (const float*)decay, (float*)state, (const int*)rec_slots,
                                (const int*)seq_lens, (const int*)qsl, H, G, D, V, silu_in, unit_qk, q_scale, delta,
-                               (float*)out, parts, (const float*)gk, ldgk, step, (const float*)dskip);
+                               (float*)out, parts, (const float*)gk, ldgk, step, (const float*)dskip, max_len);
   else
     rc = state_dispatch<bf16_t>(grid, smem, st, q, ldq, k, ldk, v, ldv, beta, ldb, a, lda, (const float*)neg_a,
                                 (const float*)dt_bias, (const float*)decay, (float*)state, (const int*)rec_slots,
                                 (const int*)seq_lens, (const int*)qsl, H, G, D, V, silu_in, unit_qk, q_scale, delta,
-                                (float*)out, parts, (const float*)gk, ldgk, step, (const float*)dskip);
+                                (float*)out, parts, (const float*)gk, ldgk, step, (const float*)dskip, max_len);
   if (rc) return rc;
   CUDA_CHECK_RET(cudaGetLastError());
   return 0;

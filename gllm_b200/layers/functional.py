@@ -229,9 +229,11 @@ def masked_attention(q, k_cache, v_cache, inp, scale, num_q_heads, head_dim, v_d
 def linear_state_scan(q, k, v, beta, a, neg_a, dt_bias, decay, state, inp, heads, qk_heads, dim, v_dim, silu_in,
                       unit_qk, q_scale, delta, zk=None, zk_bias=None, inv_tau=1.0):
     slots = inp.rec_slots if state is not None else None
-    fn = _seq().linear_state_scan if q.is_cuda else ref.linear_state_scan
-    return fn(q, k, v, beta, a, neg_a, dt_bias, decay, state, slots, inp.seq_lens, inp.query_start_loc, heads,
-              qk_heads, dim, v_dim, silu_in, unit_qk, q_scale, delta, zk, zk_bias, inv_tau)
+    args = (q, k, v, beta, a, neg_a, dt_bias, decay, state, slots, inp.seq_lens, inp.query_start_loc, heads, qk_heads,
+            dim, v_dim, silu_in, unit_qk, q_scale, delta, zk, zk_bias, inv_tau)
+    if q.is_cuda:
+        return _seq().linear_state_scan(*args, max_q_len=getattr(inp, "max_q_len", None))
+    return ref.linear_state_scan(*args)
 
 
 def gated_group_norm(o, gate, w, group, eps, act, out_scale=1.0, out=None, out_dtype=None):

@@ -34,7 +34,9 @@ def _L():
             "gllm_seq_qk_norm_rope_kv_write": [P, G, I, I, I, I, I, P, P, F, P, I, ctypes.c_double, P, P, P, P, I, I, I,
                                                I, P, F, I, P, P, I, F, I, P, G, P, P],
             "gllm_seq_linear_state": [P, G, P, G, P, G, P, G, P, G, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I, P,
-                                      I, I, P, G, I, P, P],
+                                      I, I, P, G, I, P, I, P],
+            "gllm_delta_unit_bytes": [],
+            "gllm_delta_chunk": [P, G, P, G, P, G, P, G, P, G] + [P] * 6 + [I] * 7 + [F, I, I, P, P, P],
             "gllm_seq_key_decay": [P, G, P, F, P, I, I, I, P],
             "gllm_seq_gemm_mma_f32out": [P, G, G, P, G, G, P, G, G, I, I, I, I, P],
             "gllm_seq_gated_group_norm": [P, I, P, G, P, I, I, F, I, F, P, G, I, I, P],
@@ -304,10 +306,38 @@ def qk_norm_rope_kv_write(qkv, num_heads, num_kv_heads, dim, v_dim, q_norm_w, k_
     return q
 
 
+# Where the chunked delta rule starts to pay (32 heads of 128 x 128, chunked against serial): 4 portions of 8 tokens 57 / 26 us,
+# of 16 tokens 60 / 42 us, one of 64 tokens 29 / 76 us.
+_DELTA_MIN_TOKENS = 32
+_DELTA_WORK_BYTES = 256 << 20       # its workspace (31 KB per chunk and head) at a time; more heads take another round
+
+
+def _delta_chunked(q, k, v, beta, a, neg_a, dt_bias, state, rec_slots, seq_lens, query_start_loc, heads, qk_heads, dim,
+                   v_dim, unit_qk, q_scale, out) -> bool:
+    """The sequences with at least _DELTA_MIN_TOKENS new tokens on csrc/seq/delta_ops.cu; False: sizes or alignment outside
+    its envelope."""
+    L = _L()
+    t, nseq, unit = q.shape[0], seq_lens.shape[0], L.gllm_delta_unit_bytes()
+    slots = t // 64 + nseq
+    at_once = max(1, min(heads, _DELTA_WORK_BYTES // (slots * unit)))
+    work = torch.empty(slots * at_once * unit, dtype=torch.uint8, device=q.device)
+    rc = L.gllm_delta_chunk(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(beta), beta.stride(0), _p(a),
+                            a.stride(0), _p(neg_a), _p(dt_bias), _p(state), _p(rec_slots), _p(seq_lens),
+                            _p(query_start_loc), t, nseq, heads, qk_heads, dim, v_dim, int(unit_qk), float(q_scale),
+                            _DELTA_MIN_TOKENS, at_once, _p(work), _p(out), stream_ptr())
+    if rc == 2:
+        return False
+    check(rc, "delta_chunk")
+    sm100._count(2 * -(-heads // at_once))
+    return True
+
+
 def linear_state_scan(q, k, v, beta, a, neg_a, dt_bias, decay, state, rec_slots, seq_lens, query_start_loc, heads,
                       qk_heads, dim, v_dim, silu_in, unit_qk, q_scale, delta, zk=None, zk_bias=None, inv_tau=1.0,
-                      step=False, d_skip=None, out=None):
-    """`step`: the softplus behind the decay is also the write strength; `d_skip` [heads] fp32: o += d_skip v."""
+                      step=False, d_skip=None, out=None, max_q_len: Optional[int] = None):
+    """`step`: the softplus behind the decay is also the write strength; `d_skip` [heads] fp32: o += d_skip v.
+    With `max_q_len` (the longest portion of the batch), the delta rule runs in the chunked form on portions of
+    `_DELTA_MIN_TOKENS` tokens and more; the length of a sequence's own portion decides, not what else is in the batch."""
     t = q.shape[0]
     for x in (q, k, v, beta, a, zk):
         assert x is None or (x.stride(1) == 1 and x.dtype == q.dtype)
@@ -327,13 +357,22 @@ def linear_state_scan(q, k, v, beta, a, neg_a, dt_bias, decay, state, rec_slots,
     # 4 x 2048 tokens, head size 128: 8 heads 1.9x faster, 32 heads 1.4x slower than 4 lanes). Otherwise 4: decode-like
     # batches want the wider contiguous runs of the state rows, whose read + write is all that a single token costs
     nseq = seq_lens.shape[0]
+    max_len = 0
+    if delta and max_q_len is not None and max_q_len >= _DELTA_MIN_TOKENS and not silu_in and a is not None and \
+            not step and d_skip is None and q.dtype == torch.bfloat16 and _delta_chunked(
+                q, k, v, beta, a, neg_a, dt_bias, state, rec_slots, seq_lens, query_start_loc, heads, qk_heads, dim, v_dim,
+                unit_qk, q_scale, out):
+        if nseq == 1:
+            return out
+        max_len = _DELTA_MIN_TOKENS - 1
     blocks = nseq * heads * ((v_dim + 31) // 32)
     parts = 8 if (dim > 64 and t >= 16 * nseq and blocks <= 2 * _NUM_SMS) else 4
     check(_L().gllm_seq_linear_state(_p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0), _p(beta), ld(beta),
                                      _p(a), ld(a), _p(neg_a), _p(dt_bias), _p(decay), _p(state), _p(rec_slots),
                                      _p(seq_lens), _p(query_start_loc), seq_lens.shape[0], heads, qk_heads, dim, v_dim,
                                      int(silu_in), int(unit_qk), float(q_scale), int(delta), _p(out), _f32(q),
-                                     parts, _p(gk), ld(gk), int(step), _p(d_skip), stream_ptr()), "seq_linear_state")
+                                     parts, _p(gk), ld(gk), int(step), _p(d_skip), max_len, stream_ptr()),
+          "seq_linear_state")
     sm100._count()
     return out
 

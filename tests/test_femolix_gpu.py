@@ -292,3 +292,56 @@ def test_greedy_generation_with_cuda_graphs(models):
         for _ in range(n):
             cur.append(int(oracle.forward(cfg, w, cur, torch.float64)[-1].argmax()))
         assert s.token_ids == cur
+
+
+def _delta_exact(q, k, v, beta, a, neg_a, dt_bias, st, qsl, sl, H, G, D, V):
+    """The delta rule token by token in float64."""
+    f = lambda x: x.double().cpu()   # noqa: E731
+    q, k, v, beta, a, neg_a, dt_bias, st = (f(x) for x in (q, k, v, beta, a, neg_a, dt_bias, st))
+    out, ends = torch.empty(q.shape[0], H * V, dtype=torch.float64), st.clone()
+    for s in range(len(sl)):
+        q0, q1 = int(qsl[s]), int(qsl[s + 1])
+        S = st[s].clone() if int(sl[s]) > q1 - q0 else torch.zeros(H, D, V, dtype=torch.float64)
+        for t in range(q0, q1):
+            qq, kk = (x[t].view(G, D) / torch.sqrt((x[t].view(G, D) ** 2).sum(-1, keepdim=True) + 1e-6) for x in (q, k))
+            qq, kk = (qq * D ** -0.5).repeat_interleave(H // G, 0), kk.repeat_interleave(H // G, 0)
+            S = S * torch.exp(neg_a * torch.nn.functional.softplus(a[t] + dt_bias)).view(H, 1, 1)
+            u = torch.sigmoid(beta[t]).view(H, 1) * (v[t].view(H, V) - torch.einsum("hdv,hd->hv", S, kk))
+            S = S + kk.unsqueeze(-1) * u.unsqueeze(1)
+            out[t] = torch.einsum("hdv,hd->hv", S, qq).reshape(-1)
+        if q1 > q0:
+            ends[s] = S
+    return out, ends
+
+
+@pytest.mark.parametrize("H,G,D,V", [(4, 2, 128, 128), (3, 3, 64, 72), (2, 1, 40, 8), (2, 2, 120, 136)])
+@pytest.mark.parametrize("lens,ctx", [([1, 32, 31, 64, 65, 200], [5, 0, 9, 0, 70, 0]), ([130], [0]), ([33, 3], [1, 0])])
+@pytest.mark.parametrize("decay", ["slow", "fast"])
+def test_chunked_delta_rule(H, G, D, V, lens, ctx, decay):
+    """Chunked against token-serial, both against float64 from the same bf16 inputs: tile edges, ragged and short portions
+    (below 32 tokens the serial kernel takes them), carried state, decays that wipe the state. The chunked form keeps the
+    serial one's accuracy (a fixed 2e-6 covers the few-token cases, where either is a handful of fp32 roundings)."""
+    from gllm_b200.ops import sm100_seq as S
+    torch.manual_seed(D + len(lens))
+    dev, t, n = "cuda", sum(lens), len(lens)
+    qkv = torch.randn(t, 2 * G * D + H * V, device=dev).bfloat16()
+    q, k, v = qkv[:, :G * D], qkv[:, G * D:2 * G * D], qkv[:, 2 * G * D:]
+    ba = torch.randn(t, 2 * H, device=dev).bfloat16()
+    beta, a = ba[:, :H], ba[:, H:]
+    if decay == "fast":
+        a[t // 2] = 300.0                       # one token whose decay is an exact zero
+    neg_a = -torch.rand(H, device=dev) * (1.0 if decay == "slow" else 16.0)
+    dt_bias = torch.full((H,), -4.0 if decay == "slow" else 0.5, device=dev)
+    st0 = torch.randn(n, H, D, V, device=dev)
+    qsl = torch.tensor([0] + lens, device=dev).cumsum(0).to(torch.int32)
+    sl = torch.tensor([x + c for x, c in zip(lens, ctx)], device=dev, dtype=torch.int32)
+    rs = torch.arange(n, device=dev, dtype=torch.int32)
+    exact = _delta_exact(q, k, v, beta, a, neg_a, dt_bias, st0, qsl, sl, H, G, D, V)
+    err = {}
+    for name, mx in (("chunk", max(lens)), ("serial", None)):
+        st = st0.clone()
+        o = S.linear_state_scan(q, k, v, beta, a, neg_a, dt_bias, None, st, rs, sl, qsl, H, G, D, V, False, True, D ** -0.5,
+                                True, max_q_len=mx)
+        err[name] = [float((x.double().cpu() - e).norm() / e.norm()) for x, e in ((o, exact[0]), (st, exact[1]))]
+    for c, s in zip(err["chunk"], err["serial"]):
+        assert c <= max(1.2 * s, 2e-6), err
