@@ -170,9 +170,11 @@ def causal_conv_silu(xz, channels, w, b, conv_state, inp, act="silu", in_bias=No
 
 def selective_scan(xc, dt_raw, proj, xz, a, d_skip, dt_bias, ssm_state, inp, channels, nstate, dt_rank):
     slots = inp.rec_slots if ssm_state is not None else None
-    fn = _seq().selective_scan if xc.is_cuda else ref.selective_scan
-    return fn(xc, dt_raw, proj, xz, a, d_skip, dt_bias, ssm_state, slots, inp.seq_lens, inp.query_start_loc,
-              channels, nstate, dt_rank)
+    args = (xc, dt_raw, proj, xz, a, d_skip, dt_bias, ssm_state, slots, inp.seq_lens, inp.query_start_loc, channels,
+            nstate, dt_rank)
+    if xc.is_cuda:
+        return _seq().selective_scan(*args, max_q_len=getattr(inp, "max_q_len", None))
+    return ref.selective_scan(*args)
 
 
 def relu2(x):
