@@ -8,7 +8,9 @@
 // What bounds it: issue slots, about 11 per (token, channel, state) and pass, most of them the accurate expf. The serial kernel
 // does the exponentials once, but its longest sequence is one chain of tokens on a part of the machine, and the four threads of
 // a channel each form the same steps and gates.
-// SCAN_MEASURED
+// 8192 ragged tokens in 4 sequences, 8192 channels, 16 states: 527 + 29 + 740 us, token-serial 2999 us (B200); one sequence of
+// 8192 tokens: 1.28 ms / 8.5 ms. The hardware's 2^x on an exponent in two parts would take 250 us off, but its error is up to
+// 1.8 times that of expf (state of 2048 tokens against float64: 3.1e-7 / 1.8e-7).
 #include <cuda_bf16.h>
 
 #include "common/host_utils.h"
