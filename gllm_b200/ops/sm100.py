@@ -41,7 +41,7 @@ def waits_given_up() -> int:
     return sum(getattr(L, f"gllm_waits_given_up_{f}")() for f in _WAIT_FAMILIES)
 
 
-_WAIT_FAMILIES = ("fp8",)
+_WAIT_FAMILIES = ("fp8", "attn")
 
 
 # ----------------------------------------------------------------------------------------------
@@ -246,7 +246,7 @@ _attn_ws = {}
 _FUSED_MERGE = os.environ.get("GLLM_ATTN_FUSED_MERGE", "0") == "1"
 # tcgen05 / TMEM prefill attention (csrc/attn/prefill_attention_tc.cu) is the default prefill kernel (validated on
 # B200: profiles/attn_prefill_tc.md; 1.3-2.1x the mma.sync kernel); GLLM_ATTN_TC=0 selects the mma.sync kernel, which
-# also serves the shapes outside the tcgen05 kernel's envelope. ATTN_TC_KV = keys per pipeline stage (64 or 128;
+# also serves the shapes outside the tcgen05 kernel's envelope. ATTN_TC_KV bounds its page size (64 or 128;
 # 64 measured faster at every shape). Module attributes so tests / benches can flip them.
 ATTN_TC = os.environ.get("GLLM_ATTN_TC", "1") == "1"
 ATTN_TC_KV = int(os.environ.get("GLLM_ATTN_TC_KV", "64"))
@@ -335,7 +335,7 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
         rc = 2
         if ATTN_TC:
             rc = L.gllm_attn_prefill_tc(_p(q), q.stride(0), _p(out), _p(k_cache), _p(v_cache), pages, _p(block_table),
-                                        _p(seq_lens), _p(query_start_loc), n_prefill, num_decode_seqs, max_q_len,
+                                        _p(seq_lens), _p(query_start_loc), t, n_prefill, num_decode_seqs, max_q_len,
                                         max_blocks, hq, hkv, d, page_size, float(scale), ATTN_TC_KV, st)
             if rc != 2:                     # 2 = shape outside the tcgen05 kernel's envelope -> mma.sync kernel
                 check(rc, "attn_prefill_tc")

@@ -54,7 +54,7 @@ def _L():
             "gllm_seq_gemm_simt": [P, G, P, G, P, G, I, I, I, I, P, P],
             "gllm_attn_decode_win": [P, G, P, P, P, G, P, P, I, I, I, I, I, I, I, F, I, P, P],
             "gllm_attn_prefill_win": [P, G, P, P, P, G, P, P, P, I, I, I, I, I, I, I, I, F, I, P, P],
-            "gllm_attn_prefill_tc_cap": [P, G, P, P, P, G, P, P, P, I, I, I, I, I, I, I, I, F, I, P, F, I, G, P, P, P, G, P,
+            "gllm_attn_prefill_tc_cap": [P, G, P, P, P, G, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P, F, I, G, P, P, P, G, P,
                                          P, I, P],
             "gllm_attn_decode_mask": [P, G, P, G, P, P, G, P, P, I, I, I, I, I, I, I, F, I, I, P, F, F, P, P, P, G, P, P,
                                       I, P],
@@ -201,7 +201,7 @@ def window_attention(q, k_cache, v_cache, block_table, seq_lens, query_start_loc
         if rest and not chunk and sm100.ATTN_TC and out_scale == 1.0 and vec16 and tc is not False and \
                 head_dim in (64, 128) and sm100.ATTN_TC_KV % ps == 0:
             rc = L.gllm_attn_prefill_tc_cap(_p(q), q.stride(0), _p(out), _p(k_cache), _p(v_cache), pages,
-                                            _p(block_table), _p(seq_lens), _p(query_start_loc), nseq - num_decode_seqs,
+                                            _p(block_table), _p(seq_lens), _p(query_start_loc), t, nseq - num_decode_seqs,
                                             num_decode_seqs, max_q_len, block_table.stride(0), num_q_heads, hkv,
                                             head_dim, ps, float(scale), sm100.ATTN_TC_KV, _p(sink), float(softcap),
                                             int(window or 0), out.stride(0), *extras, st)

@@ -257,6 +257,33 @@ def test_prefill_attention_tc(hq, hkv, d, kv_tile, monkeypatch):
     assert _rel_err(o, o_ref) < 1e-2, _rel_err(o, o_ref)
 
 
+@pytest.mark.parametrize("hq,hkv,d", [(8, 1, 128), (4, 4, 128), (6, 2, 64)])
+@pytest.mark.parametrize("page", [8, 16, 64])
+@pytest.mark.parametrize("many", [False, True])       # few CTAs: one query tile each; many: two
+def test_prefill_attention_tc_edges(hq, hkv, d, page, many, monkeypatch):
+    """Chunks and contexts at the edges of the 128-row query tiles (16, 128 and 42 tokens), of their pairs and of the 128-key
+    tiles; scores that grow along the keys so that the running reference of the exponentials moves; the same bits again."""
+    from gllm_b200.ops import sm100
+    monkeypatch.setattr(sm100, "ATTN_TC", True)
+    q_lens = [1, 15, 16, 17, 32, 33, 127, 128, 129, 255, 256, 257, 5, 300]
+    ctx = [0, 1, 127, 128, 129, 0, 1, 500, 0, 1, 0, 255, 1000, 84]
+    if many:
+        q_lens, ctx = q_lens * 3, ctx * 3
+    seq_lens = [a + b for a, b in zip(q_lens, ctx)]
+    q, kc, vc, bt, sl, qsl = _make_paged(seq_lens, q_lens, hq, hkv, d, page, _dev(), seed=3)
+    for i, n in enumerate(seq_lens):                  # scores rise by some 40 over a sequence
+        for b in range((n + page - 1) // page):
+            kc[bt[i, b].long()] *= 1 + 6.0 * b * page / 1024
+    scale = 1.0 / math.sqrt(d)
+    args = (q, kc, vc, bt, sl, qsl, scale, hq, d, 0, len(seq_lens), max(q_lens), max(seq_lens))
+    o = sm100.paged_attention(*args)
+    again = sm100.paged_attention(*args)
+    o_ref = ref.paged_attention(q, kc, vc, bt, sl, qsl, scale, hq, d)
+    assert torch.isfinite(o.float()).all() and torch.equal(o, again)
+    assert _rel_err(o, o_ref) < 1e-2, _rel_err(o, o_ref)
+    assert sm100.waits_given_up() == 0
+
+
 def test_sampler_greedy_and_filter():
     from gllm_b200.ops import sm100
     torch.manual_seed(6)
