@@ -60,32 +60,34 @@ struct AttnSmem {
 };
 
 // ---------------------------------------------------------------------------------------------
-// producer: stream the KV tiles [tile_begin, tile_end) of one sequence / kv head
+// producer: stream the KV tiles [tile_begin, tile_end) of one sequence / kv head. Called by a whole warp: one lane per box
+// (a page of K or of V), whose block-table entry was fetched while the tile before was on its way. One lane that read the
+// entries where it used them spent some 470 cycles on each. 256 sequences of up to 2048 keys, 32 / 8 heads of 128: 129 -> 124 us.
 // ---------------------------------------------------------------------------------------------
 template <int D>
 __device__ __forceinline__ void kv_producer(const CUtensorMap* tk, const CUtensorMap* tv, uint8_t* smem,
                                             uint64_t* full_bar, uint64_t* empty_bar, const int32_t* bt, int kvh,
-                                            int Hkv, int page_size, int seq_len, int tile_begin, int tile_end) {
+                                            int Hkv, int page_size, int seq_len, int tile_begin, int tile_end, int lane) {
   using SM = AttnSmem<D>;
-  const int pages_per_tile = kTileN / page_size;
+  if (tile_begin >= tile_end) return;
+  const int pages_per_tile = kTileN / page_size;       // at most 8
   const int page_bytes = page_size * D * 2;
   const int last_page = (seq_len - 1) / page_size;
+  const int j = lane % pages_per_tile, which = lane / pages_per_tile;      // which: 0 K, 1 V
+  auto page_of = [&](int tile) { return bt[min(tile * pages_per_tile + j, last_page)]; };   // masked columns: finite data
+  int page = which < 2 ? page_of(tile_begin) : 0;
   uint32_t it = 0;
   for (int tile = tile_begin; tile < tile_end; ++tile, ++it) {
     const int s = it % SM::kStages;
     const uint32_t ph = (it / SM::kStages) & 1;
+    const int next = which < 2 && tile + 1 < tile_end ? page_of(tile + 1) : 0;
     mbar_wait(&empty_bar[s], ph ^ 1);
-    uint8_t* sk = smem + s * SM::kStageBytes;
-    uint8_t* sv = sk + SM::kTileBytes;
-    mbar_expect_tx(&full_bar[s], SM::kStageBytes);
-    for (int j = 0; j < pages_per_tile; ++j) {
-      int pi = tile * pages_per_tile + j;
-      if (pi > last_page) pi = last_page;  // keep smem finite for masked columns
-      const int page = bt[pi];
-      const int slab = (page * Hkv + kvh) * (D / 64);
-      tma_load_3d(sk + j * page_bytes, tk, &full_bar[s], 0, 0, slab);
-      tma_load_3d(sv + j * page_bytes, tv, &full_bar[s], 0, 0, slab);
-    }
+    if (lane == 0) mbar_expect_tx(&full_bar[s], SM::kStageBytes);
+    __syncwarp();
+    if (which < 2)
+      tma_load_3d(smem + s * SM::kStageBytes + which * SM::kTileBytes + j * page_bytes, which == 0 ? tk : tv, &full_bar[s], 0, 0,
+                  (page * Hkv + kvh) * (D / 64));
+    page = next;
   }
 }
 
@@ -130,10 +132,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   __syncthreads();
 
   if (warp == kMathWarps) {
-    if (lane == 0 && tile_end > tile_begin) {
-      kv_producer<D>(&tmap_k, &tmap_v, smem, full_bar, empty_bar, p.block_table + (size_t)seq * p.max_blocks, kvh,
-                     p.Hkv, p.page_size, seq_len, tile_begin, tile_end);
-    }
+    kv_producer<D>(&tmap_k, &tmap_v, smem, full_bar, empty_bar, p.block_table + (size_t)seq * p.max_blocks, kvh,
+                   p.Hkv, p.page_size, seq_len, tile_begin, tile_end, lane);
     return;
   }
 
@@ -459,10 +459,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
   __syncthreads();
 
   if (warp == kMathWarps) {
-    if (lane == 0) {
-      kv_producer<D>(&tmap_k, &tmap_v, smem, full_bar, empty_bar, p.block_table + (size_t)seq * p.max_blocks, kvh,
-                     p.Hkv, p.page_size, seq_len, tile_lo, n_tiles);
-    }
+    kv_producer<D>(&tmap_k, &tmap_v, smem, full_bar, empty_bar, p.block_table + (size_t)seq * p.max_blocks, kvh,
+                   p.Hkv, p.page_size, seq_len, tile_lo, n_tiles, lane);
     return;
   }
 
@@ -764,9 +762,9 @@ static int attn_decode_impl(const void* q, int64_t q_ts, void* out, const void* 
   if (p.num_splits > 1 && p.split_cnt == nullptr) {
     // merge covers sequences [seq_offset, seq_offset + num_seqs)
     const size_t off = (size_t)seq_offset * Hq;
-    CUDA_CHECK_RET(launch_pdl(attn_merge_kernel, dim3(num_seqs * Hq), dim3(D < 128 ? D : 128), 0, st,
-                              p.part_o + off * p.num_splits * D, p.part_lse + off * p.num_splits,
-                              p.out + off * D, p.num_splits, D));
+    if (launch_attn_merge(p.part_o + off * p.num_splits * D, p.part_lse + off * p.num_splits, p.out + off * D, num_seqs * Hq,
+                          p.num_splits, D, st))
+      return 1;
   }
   return 0;
 }
