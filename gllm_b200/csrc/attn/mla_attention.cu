@@ -266,11 +266,11 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
   }
 }
 
-// Per token: interleaved-pair RoPE on the rope dims of every query head (written into q_full[:, :, 512:576]) and
-// of the shared key, then the latent row [c_kv (512) | rope(k_pe) (64)] goes into its paged-cache slot.
+// Per token: interleaved-pair RoPE on the rope dims of every query head (written to q_out: the last 64 columns of the
+// absorbed queries, or q_pe itself) and of the shared key, then the latent row [c_kv (512) | rope(k_pe) (64)] goes into its paged-cache slot.
 // (reference: rotary_embedding + concat_and_cache_mla, gllm/layers/attention.py:443-451)
-__global__ void mla_rope_cache_kernel(const __nv_bfloat16* __restrict__ q_pe, int64_t q_ts, int64_t q_hs, int H,
-                                      __nv_bfloat16* __restrict__ q_full, const __nv_bfloat16* __restrict__ k_pe,
+__global__ void mla_rope_cache_kernel(const __nv_bfloat16* q_pe, int64_t q_ts, int64_t q_hs, int H,
+                                      __nv_bfloat16* q_out, int64_t o_ts, int64_t o_hs, const __nv_bfloat16* __restrict__ k_pe,
                                       int64_t k_ts, const __nv_bfloat16* __restrict__ kv_c, int64_t c_ts,
                                       const float* __restrict__ cos_sin, const int32_t* __restrict__ positions,
                                       const int32_t* __restrict__ slots, __nv_bfloat16* __restrict__ cache,
@@ -285,7 +285,7 @@ __global__ void mla_rope_cache_kernel(const __nv_bfloat16* __restrict__ q_pe, in
     const uint32_t raw = *reinterpret_cast<const uint32_t*>(q_pe + tok * q_ts + h * q_hs + 2 * pr);
     const float2 x = unpack_bf16(raw);
     const float c = cs[pr], sn = cs[32 + pr];
-    *reinterpret_cast<uint32_t*>(q_full + (static_cast<size_t>(tok) * H + h) * kLat + kLatV + 2 * pr) =
+    *reinterpret_cast<uint32_t*>(q_out + tok * o_ts + h * o_hs + 2 * pr) =
         pack_bf16(x.x * c - x.y * sn, x.y * c + x.x * sn);
   }
   const int slot = slots != nullptr ? slots[tok] : -1;
@@ -302,6 +302,65 @@ __global__ void mla_rope_cache_kernel(const __nv_bfloat16* __restrict__ q_pe, in
     const float2 x = unpack_bf16(*reinterpret_cast<const uint32_t*>(k_pe + tok * k_ts + 2 * pr));
     const float c = cs[pr], sn = cs[32 + pr];
     *reinterpret_cast<uint32_t*>(dst + 8 * slab_stride + 2 * pr) = pack_bf16(x.x * c - x.y * sn, x.y * c + x.x * sn);
+  }
+}
+
+// First row of every sequence in the gathered latents (each takes whole 64-row tiles): rows[s] = sum of the lengths before it,
+// rounded up to 64.
+__global__ void mla_rows_kernel(const int32_t* __restrict__ seq_lens, int nseq, int32_t* __restrict__ rows) {
+  __shared__ int32_t part[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int base = 0;
+  for (int s0 = 0; s0 <= nseq; s0 += blockDim.x) {
+    const int s = s0 + threadIdx.x;
+    const int n = s < nseq ? (seq_lens[s] + 63) / 64 * 64 : 0;
+    int sum = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += up;
+    }
+    if (lane == 31) part[warp] = sum;
+    __syncthreads();
+    int before = base, all = base;
+    for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) {
+      if (w < warp) before += part[w];
+      all += part[w];
+    }
+    if (s <= nseq) rows[s] = before + sum - n;
+    base = all;
+    __syncthreads();
+  }
+}
+
+// Latent rows of whole sequences out of their pages: lat [rows, 512] and the rotated key part pe [rows, 64], zeros behind a
+// sequence's end. One warp per row, 16-byte accesses; memory-bound.
+__global__ void __launch_bounds__(256) mla_gather_kernel(const __nv_bfloat16* __restrict__ cache,
+                                                         const int32_t* __restrict__ block_table, int max_blocks,
+                                                         const int32_t* __restrict__ seq_lens,
+                                                         const int32_t* __restrict__ rows, int nseq, int total, int page_size,
+                                                         __nv_bfloat16* __restrict__ lat, __nv_bfloat16* __restrict__ pe) {
+  const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= total) return;
+  int lo = 0, hi = nseq - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (rows[mid] <= r) lo = mid; else hi = mid - 1;
+  }
+  const int i = r - rows[lo];
+  const bool ok = i < seq_lens[lo];
+  const int page = ok ? block_table[static_cast<size_t>(lo) * max_blocks + i / page_size] : 0;
+  const __nv_bfloat16* src = cache + (static_cast<size_t>(page) * (kLat / 64) * page_size + i % page_size) * 64;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int c = k * 32 + lane;                         // 16-byte chunk: 64 of the latent, 8 of the rotated part
+    if (c < kLat / 8) {
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (ok) v = *reinterpret_cast<const uint4*>(src + static_cast<size_t>(c >> 3) * page_size * 64 + (c & 7) * 8);
+      __nv_bfloat16* dst = c < kLatV / 8 ? lat + static_cast<size_t>(r) * kLatV + c * 8
+                                         : pe + static_cast<size_t>(r) * 64 + (c - kLatV / 8) * 8;
+      *reinterpret_cast<uint4*>(dst) = v;
+    }
   }
 }
 
@@ -354,16 +413,31 @@ GLLM_EXPORT int gllm_mla_attention(const void* q, void* out, const void* cache, 
   return 0;
 }
 
+// rows [nseq + 1] int32 (written), lat [total, 512], pe [total, 64]; total = the sequences' lengths, each rounded up to 64
+GLLM_EXPORT int gllm_mla_gather(const void* cache, const void* block_table, int max_blocks, const void* seq_lens, int nseq,
+                                int total, int page_size, void* rows, void* lat, void* pe, void* stream) {
+  if (nseq <= 0 || total <= 0) return 0;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  mla_rows_kernel<<<1, 256, 0, st>>>(reinterpret_cast<const int32_t*>(seq_lens), nseq, reinterpret_cast<int32_t*>(rows));
+  mla_gather_kernel<<<(total + 7) / 8, 256, 0, st>>>(
+      reinterpret_cast<const __nv_bfloat16*>(cache), reinterpret_cast<const int32_t*>(block_table), max_blocks,
+      reinterpret_cast<const int32_t*>(seq_lens), reinterpret_cast<const int32_t*>(rows), nseq, total, page_size,
+      reinterpret_cast<__nv_bfloat16*>(lat), reinterpret_cast<__nv_bfloat16*>(pe));
+  CUDA_CHECK_RET(cudaGetLastError());
+  return 0;
+}
+
 // q_pe: strided view [T, H, 64] of the projected queries; k_pe [T, 64]; kv_c [T, 512] (normalised latent);
-// cos_sin fp32 [max_pos, 64]; writes q_full[:, :, 512:] and the cache rows at `slots`.
-GLLM_EXPORT int gllm_mla_rope_cache(const void* q_pe, int64_t q_ts, int64_t q_hs, int H, void* q_full,
-                                    const void* k_pe, int64_t k_ts, const void* kv_c, int64_t c_ts,
+// cos_sin fp32 [max_pos, 64]; writes the rotated queries to q_out (token and head strides o_ts, o_hs; may be q_pe itself) and the
+// cache rows at `slots`.
+GLLM_EXPORT int gllm_mla_rope_cache(const void* q_pe, int64_t q_ts, int64_t q_hs, int H, void* q_out, int64_t o_ts,
+                                    int64_t o_hs, const void* k_pe, int64_t k_ts, const void* kv_c, int64_t c_ts,
                                     const void* cos_sin, const void* positions, const void* slots, void* cache,
                                     int page_size, int tokens, void* stream) {
   if (tokens <= 0) return 0;
   CUDA_CHECK_RET(launch_pdl(mla_rope_cache_kernel, dim3(tokens), dim3(128), 0, reinterpret_cast<cudaStream_t>(stream),
                             reinterpret_cast<const __nv_bfloat16*>(q_pe), q_ts, q_hs, H,
-                            reinterpret_cast<__nv_bfloat16*>(q_full), reinterpret_cast<const __nv_bfloat16*>(k_pe), k_ts,
+                            reinterpret_cast<__nv_bfloat16*>(q_out), o_ts, o_hs, reinterpret_cast<const __nv_bfloat16*>(k_pe), k_ts,
                             reinterpret_cast<const __nv_bfloat16*>(kv_c), c_ts, reinterpret_cast<const float*>(cos_sin),
                             reinterpret_cast<const int32_t*>(positions), reinterpret_cast<const int32_t*>(slots),
                             reinterpret_cast<__nv_bfloat16*>(cache), page_size));

@@ -68,7 +68,7 @@ struct TcAttnParams {
   int window;         // sliding window: a query at i sees keys j with i - j < window (0 = the whole past)
   AttnExtras ex;      // distance bias or table (kernel template BIAS), turned values, output gate
   int q_tiles;        // query tiles per CTA (2, or 1 where that gives every SM at most one CTA)
-  const int32_t* kv_row;   // DENSE: first row of each sequence in the expanded keys and values
+  const int32_t* kv_row;   // DENSE: first row of each sequence of this launch in the expanded keys and values
 };
 
 // BIAS of the kernel: none, the logarithmic distance bias, the distance table
@@ -220,7 +220,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       const bool has_k = sl < DK / 64, has_v = sl < DV / 64;
       const int32_t* bt = p.block_table + static_cast<size_t>(seq) * p.max_blocks;
       const int last_page = (seq_len - 1) / p.page_size;
-      const int row0 = DENSE ? p.kv_row[seq] : 0;
+      const int row0 = DENSE ? p.kv_row[blockIdx.y] : 0;
       auto page_of = [&](int tile) {                       // masked columns read the last page: keep the data finite
         return DENSE ? 0 : bt[min(((tile0 + tile) * KV + j * box) / p.page_size, last_page)];
       };
@@ -694,4 +694,31 @@ GLLM_EXPORT int gllm_attn_prefill_tc_cap(const void* q, int64_t q_ts, void* out,
   return attn_prefill_tc_impl(q, q_ts, out, k_cache, v_cache, num_pages, block_table, seq_lens, q_start, num_tokens, num_seqs,
                               seq_offset, max_q_len, max_blocks, Hq, Hkv, D, page_size, scale, kv_tile, sink, softcap,
                               stream, window, out_ts, make_extras(r1, r2, gate, ldg, v_turn, dtab, dtab_n));
+}
+
+// Causal attention of expanded latent heads: q [tokens, H, 192] (token stride q_ts), kv [rows, H, 256] = [128 key | 128 value
+// columns], pe [rows, 64] = the key columns shared by all heads, both from kv_row[s] on for sequence s of this launch (64-row
+// tiles); out [tokens, H, 128]. Sequences seq_offset .. + num_seqs of seq_lens / q_start. Returns 2 for unaligned queries.
+GLLM_EXPORT int gllm_attn_prefill_expanded(const void* q, int64_t q_ts, void* out, const void* kv, const void* pe, int64_t rows,
+                                           const void* kv_row, const void* seq_lens, const void* q_start, int num_tokens,
+                                           int num_seqs, int seq_offset, int max_q_len, int H, float scale, void* stream) {
+  if (num_seqs <= 0 || max_q_len <= 0) return 0;
+  if (q_ts % 8 != 0 || (reinterpret_cast<uintptr_t>(q) & 15) != 0) return 2;
+  CUtensorMap tkv, tpe;
+  if (make_tmap_2d(&tkv, kv, rows, static_cast<uint64_t>(H) * 256, static_cast<uint64_t>(H) * 512, 64, 64,
+                   CU_TENSOR_MAP_DATA_TYPE_BFLOAT16))
+    return 1;
+  if (make_tmap_2d(&tpe, pe, rows, 64, 128, 64, 64, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)) return 1;
+  TcAttnParams p = {};
+  p.q = reinterpret_cast<const __nv_bfloat16*>(q); p.q_ts = q_ts;
+  p.out = reinterpret_cast<__nv_bfloat16*>(out);
+  p.seq_lens = reinterpret_cast<const int32_t*>(seq_lens);
+  p.q_start = reinterpret_cast<const int32_t*>(q_start);
+  p.Hq = H; p.Hkv = H; p.G = 1; p.GP = 1;
+  p.page_size = 64; p.seq_offset = seq_offset;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  p.out_ts = static_cast<int64_t>(H) * 128;
+  p.kv_row = reinterpret_cast<const int32_t*>(kv_row);
+  return launch_prefill_tc<192, 128, true>(tkv, tkv, tpe, p, num_seqs, num_tokens, max_q_len,
+                                           reinterpret_cast<cudaStream_t>(stream));
 }

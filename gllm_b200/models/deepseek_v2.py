@@ -11,13 +11,16 @@ On sm_100a the attention runs in the *absorbed* form: q_nope·W_UK per head (bat
 views, written straight into the 576-wide query), fused RoPE + latent-cache write, split-KV multi-query attention
 over the paged latent cache (csrc/attn/mla_attention.cu), then out_lat·W_UV per head (the same batched GEMM,
 written in the [T, heads·v] layout o_proj reads). No cuBLAS and no host synchronisation on that path, so decode
-batches run inside CUDA graphs. The CPU / odd-shape path below evaluates the *expanded* form
-with PyTorch ops per sequence (the numerical oracle of the GPU path).
+batches run inside CUDA graphs. Prompt portions of 32 tokens and more (on average) take the
+*expanded* form instead: the cached latents are gathered, one GEMM makes every head's keys and values, and the tcgen05
+prefill attention runs on them. The CPU / odd-shape path below evaluates the expanded form with PyTorch ops per sequence
+(the numerical oracle of the GPU path).
 """
 from __future__ import annotations
 
 from typing import Optional
 
+import numpy as np
 import torch
 import torch.nn.functional as F
 from torch import nn
@@ -79,7 +82,8 @@ class MLAAttention(nn.Module):
             q = Fn.linear(h, _qw(self.q_w, self.q_ws))
         q = q.view(t, hl, self.qk_dim)
         kv_a = Fn.linear(h, _qw(self.kv_a_w, self.kv_a_ws))
-        kv_c, _ = Fn.rmsnorm(kv_a[:, : self.kv_lora].contiguous(), self.kv_a_norm_w, self.eps)
+        lat = kv_a[:, : self.kv_lora]
+        kv_c, _ = Fn.rmsnorm(lat if lat.is_cuda and kv_a.shape[1] % 8 == 0 else lat.contiguous(), self.kv_a_norm_w, self.eps)
         if kv_cache is None:
             return q[:, :, : self.v_dim].reshape(t, hl * self.v_dim).contiguous()
         cache = kv_cache.k_cache[self.layer_id]
@@ -137,21 +141,50 @@ class MLAAttention(nn.Module):
             self.process_weights()
         return self._w_abs
 
+    # Expanded heads cost a GEMM of 2 * 256 * 512 operations per cached row and head, and then 640 per (query, key) pair
+    # instead of 2176 on a kernel eight times as fast: they win from some twenty new tokens per sequence on; below that a portion
+    # is a few rows of one 128-row tile. 5 prompts of 4096 tokens together, 16 heads: 2459 -> 479 us. Their keys and values stay
+    # below this many bytes.
+    _EXPAND_MIN_TOKENS = 32
+    _EXPAND_MAX_BYTES = 1 << 30
+
+    def _expanded_rows(self, inp) -> int:
+        """Rows of latents to expand for this batch's prompt portions (each sequence rounded up to 64), or 0: attend in
+        the absorbed form."""
+        n0, b = inp.num_decode_seqs, getattr(inp, "batch", None)
+        if b is None or inp.padded_tokens or n0 == inp.num_seqs or (self.nope, self.v_dim) != (128, 128):
+            return 0
+        seq_lens = b.seq_lens[n0:inp.num_seqs].astype(np.int64)
+        new = int(b.query_start_loc[inp.num_seqs]) - int(b.query_start_loc[n0])
+        rows = int(((seq_lens + 63) // 64 * 64).sum())
+        if new < self._EXPAND_MIN_TOKENS * len(seq_lens) or rows * self.num_heads * 512 > self._EXPAND_MAX_BYTES:
+            return 0
+        return rows
+
     def _forward_absorbed(self, inp, q, kv_c, k_pe, cache):
-        """sm_100a path: multi-query attention over the latent cache (csrc/attn/mla_attention.cu). No host
-        synchronisation, so decode batches run inside CUDA graphs."""
+        """sm_100a path: multi-query attention over the latent cache (csrc/attn/mla_attention.cu) for decoding sequences and
+        short portions, expanded heads on the tcgen05 prefill kernel for prompts. No host synchronisation, so decode batches
+        run inside CUDA graphs."""
         from gllm_b200.ops import sm100
         t, hl = q.shape[0], self.num_heads
-        w_uk, w_uv = self._absorbed_weights()
-        q_full = torch.empty(t, hl, 576, dtype=q.dtype, device=q.device)
-        sm100.gemm_batched(q[:, :, : self.nope], w_uk, q_full[:, :, :512])   # per head: q_nope · W_UK
-        sm100.mla_rope_cache(q[:, :, self.nope:], q_full, k_pe, kv_c, self.rope.cos_sin, inp.positions,
-                             inp.slot_mapping, cache)
-        splits = sm100.mla_splits(t, hl)
-        out_lat = sm100.mla_attention(q_full, cache, inp.block_table, inp.tok_seq, inp.positions, self.scaling,
-                                      splits=splits)
         out = torch.empty(t, hl, self.v_dim, dtype=q.dtype, device=q.device)
-        sm100.gemm_batched(out_lat, w_uv, out)                                # per head: out_lat · W_UV
+        rows = self._expanded_rows(inp)
+        n = inp.num_decode_seqs if rows else t           # leading rows in the absorbed form
+        pos = inp.positions if inp.positions.dim() == 1 else inp.positions[0]
+        if n:
+            w_uk, w_uv = self._absorbed_weights()
+            q_full = torch.empty(n, hl, 576, dtype=q.dtype, device=q.device)
+            sm100.gemm_batched(q[:n, :, : self.nope], w_uk, q_full[:, :, :512])   # per head: q_nope · W_UK
+            sm100.mla_rope_cache(q[:n, :, self.nope:], q_full, k_pe[:n], kv_c[:n], self.rope.cos_sin, pos[:n],
+                                 inp.slot_mapping[:n], cache)
+            out_lat = sm100.mla_attention(q_full, cache, inp.block_table, None if rows else inp.tok_seq, pos[:n],
+                                          self.scaling, splits=sm100.mla_splits(n, hl))
+            sm100.gemm_batched(out_lat, w_uv, out[:n])                            # per head: out_lat · W_UV
+        if rows:
+            sm100.mla_rope_cache(q[n:, :, self.nope:], None, k_pe[n:], kv_c[n:], self.rope.cos_sin, pos[n:],
+                                 inp.slot_mapping[n:], cache)
+            sm100.mla_expanded_attention(q, cache, inp.block_table, inp.seq_lens, inp.query_start_loc, self.kv_b_w, rows,
+                                         inp.num_decode_seqs, inp.max_q_len, self.scaling, out)
         return out.view(t, hl * self.v_dim)
 
 

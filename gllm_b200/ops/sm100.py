@@ -499,20 +499,48 @@ def _mla_workspace(device, heads: int):
     return ws
 
 
-def mla_rope_cache(q_pe: torch.Tensor, q_full: torch.Tensor, k_pe: torch.Tensor, kv_c: torch.Tensor,
+def mla_rope_cache(q_pe: torch.Tensor, q_full: Optional[torch.Tensor], k_pe: torch.Tensor, kv_c: torch.Tensor,
                    cos_sin: torch.Tensor, positions: torch.Tensor, slots: torch.Tensor, cache: torch.Tensor):
-    """q_pe [T,H,64] (strided view), q_full [T,H,576] (rope part written), k_pe [T,64], kv_c [T,512];
-    latent row -> cache [pages,1,9,page,64] at `slots`."""
+    """q_pe [T,H,64] (strided view), q_full [T,H,576] (rope part written; None: q_pe is rotated in place), k_pe [T,64],
+    kv_c [T,512]; latent row -> cache [pages,1,9,page,64] at `slots`."""
     t, h, r = q_pe.shape
     assert r == 64 and q_pe.stride(2) == 1 and k_pe.stride(-1) == 1 and kv_c.stride(1) == 1 and kv_c.shape[1] == 512
-    assert q_full.is_contiguous() and q_full.shape == (t, h, 576) and cos_sin.dtype == torch.float32
+    assert cos_sin.dtype == torch.float32
+    if q_full is not None:
+        assert q_full.is_contiguous() and q_full.shape == (t, h, 576)
+    dst = q_pe if q_full is None else q_full[:, :, 512:]
     if positions.dim() == 2:
         positions = positions[0]
     L = _lib.load()
-    check(L.gllm_mla_rope_cache(_p(q_pe), q_pe.stride(0), q_pe.stride(1), h, _p(q_full), _p(k_pe), k_pe.stride(0),
-                                _p(kv_c), kv_c.stride(0), _p(cos_sin), _p(positions), _p(slots), _p(cache),
+    check(L.gllm_mla_rope_cache(_p(q_pe), q_pe.stride(0), q_pe.stride(1), h, _p(dst), dst.stride(0), dst.stride(1), _p(k_pe),
+                                k_pe.stride(0), _p(kv_c), kv_c.stride(0), _p(cos_sin), _p(positions), _p(slots), _p(cache),
                                 cache.shape[3], t, stream_ptr()), "mla_rope_cache")
     _count()
+
+
+def mla_expanded_attention(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, seq_lens: torch.Tensor,
+                           query_start_loc: torch.Tensor, kv_b_w: torch.Tensor, rows: int, first_seq: int, max_q_len: int,
+                           scale: float, out: torch.Tensor) -> torch.Tensor:
+    """Causal attention of the sequences from `first_seq` on in the expanded form: their cached latents are gathered
+    (`rows` of them, every sequence rounded up to 64), kv_b_w [H * 256, 512] makes each head's 128 key and 128 value columns
+    from them in one GEMM, and the tcgen05 prefill kernel runs on keys [128 | 64 shared] and values 128 wide.
+    q [T, H, 192] rotated; out [T, H, 128]: the rows of those sequences are written."""
+    t, h, d = q.shape
+    n = seq_lens.shape[0] - first_seq
+    assert d == 192 and q.stride(2) == 1 and q.stride(1) == d and out.is_contiguous() and out.shape == (t, h, 128)
+    assert kv_b_w.shape == (h * 256, 512) and block_table.stride(1) == 1
+    dev, L, st = q.device, _lib.load(), stream_ptr()
+    start = torch.empty(n + 1, dtype=torch.int32, device=dev)
+    lat = torch.empty(rows, 512, dtype=_BF16, device=dev)
+    pe = torch.empty(rows, 64, dtype=_BF16, device=dev)
+    check(L.gllm_mla_gather(_p(cache), _p(block_table[first_seq:]), block_table.stride(0), _p(seq_lens[first_seq:]), n, rows,
+                            cache.shape[3], _p(start), _p(lat), _p(pe), st), "mla_gather")
+    kv = linear(lat, kv_b_w)
+    check(L.gllm_attn_prefill_expanded(_p(q), q.stride(0), _p(out), _p(kv), _p(pe), rows, _p(start), _p(seq_lens),
+                                       _p(query_start_loc), t, n, first_seq, max_q_len, h, float(scale), st),
+          "attn_prefill_expanded")
+    _count(3)
+    return out
 
 
 def mla_attention(q_full: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor,

@@ -687,3 +687,42 @@ def test_moe_fused_experts_fp8(t, e, k):
     assert _rel_err(out, want) < 2.5e-2, _rel_err(out, want)
     # and within quantisation noise of the un-quantised-activation oracle
     assert _rel_err(out, ref.fused_experts(x, torch.stack(d13), torch.stack(d2), tw, ids)) < 8e-2
+
+
+@pytest.mark.parametrize("heads,page", [(3, 16), (16, 64), (8, 8)])
+@pytest.mark.parametrize("n_dec", [0, 2])
+def test_mla_expanded_attention(heads, page, n_dec):
+    """Expanded heads (128 key columns of their own + 64 shared, values 128 wide) over gathered latents: chunks and contexts at
+    the edges of the 64-row gather tiles, 64-key and 128-query tiles; decoding sequences in front are left alone. Against fp32
+    over the same bf16 latents and weights; keys and values are rounded once to bf16 (2^-9), like P."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(9)
+    q_lens, ctx = [1] * n_dec + [1, 63, 64, 65, 128, 129, 40, 300], [7, 90][:n_dec] + [0, 1, 64, 0, 127, 0, 500, 3]
+    lens = [a + b for a, b in zip(q_lens, ctx)]
+    need = [-(-n // page) for n in lens]
+    perm = torch.randperm(sum(need), device=_dev()).to(torch.int32)
+    bt, at = torch.zeros(len(lens), max(need), dtype=torch.int32, device=_dev()), 0
+    for i, k in enumerate(need):
+        bt[i, :k] = perm[at:at + k]
+        at += k
+    cache = torch.randn(sum(need), 1, 9, page, 64, device=_dev()).bfloat16()
+    w = (torch.randn(heads * 256, 512, device=_dev()) * 512 ** -0.5).bfloat16()
+    t = sum(q_lens)
+    q = torch.randn(t, heads, 192, device=_dev()).bfloat16()
+    qsl = torch.tensor([0] + q_lens, device=_dev()).cumsum(0).to(torch.int32)
+    sl = torch.tensor(lens, dtype=torch.int32, device=_dev())
+    rows = sum(-(-n // 64) * 64 for n in lens[n_dec:])
+    out = torch.full((t, heads, 128), 7.0, device=_dev()).bfloat16()
+    scale = 192 ** -0.5
+    sm100.mla_expanded_attention(q, cache, bt, sl, qsl, w, rows, n_dec, max(q_lens), scale, out)
+    assert bool((out[:n_dec] == 7.0).all()) and sm100.waits_given_up() == 0
+    want = torch.empty(t, heads, 128, device=_dev())
+    for i, n in enumerate(lens):
+        a, b = int(qsl[i]), int(qsl[i + 1])
+        row = ref.gather_kv(cache, bt[i], n)[:, 0].float()
+        kv = (row[:, :512] @ w.float().t()).view(n, heads, 256)
+        k = torch.cat([kv[..., :128], row[:, None, 512:].expand(n, heads, 64)], -1)
+        s = torch.einsum("qhd,khd->hqk", q[a:b].float(), k) * scale
+        s.masked_fill_(torch.arange(n, device=_dev())[None] > torch.arange(n - (b - a), n, device=_dev())[:, None], float("-inf"))
+        want[a:b] = torch.einsum("hqk,khd->qhd", s.softmax(-1), kv[..., 128:])
+    assert _rel_err(out[n_dec:], want[n_dec:]) < 1.2e-2, _rel_err(out[n_dec:], want[n_dec:])
