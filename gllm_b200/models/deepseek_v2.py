@@ -178,7 +178,7 @@ class MLAAttention(nn.Module):
             sm100.mla_rope_cache(q[:n, :, self.nope:], q_full, k_pe[:n], kv_c[:n], self.rope.cos_sin, pos[:n],
                                  inp.slot_mapping[:n], cache)
             out_lat = sm100.mla_attention(q_full, cache, inp.block_table, None if rows else inp.tok_seq, pos[:n],
-                                          self.scaling, splits=sm100.mla_splits(n, hl))
+                                          self.scaling)
             sm100.gemm_batched(out_lat, w_uv, out[:n])                            # per head: out_lat · W_UV
         if rows:
             sm100.mla_rope_cache(q[n:, :, self.nope:], None, k_pe[n:], kv_c[n:], self.rope.cos_sin, pos[n:],

@@ -64,7 +64,7 @@ def _declare(lib):
     sig("gllm_attn_decode", [P, L, P, P, P, L, P, P, P, P, I, I, I, I, I, I, I, I, F, P, P])
     sig("gllm_attn_prefill", [P, L, P, P, P, L, P, P, P, I, I, I, I, I, I, I, I, F, P])
     sig("gllm_attn_prefill_tc", [P, L, P, P, P, L, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P])
-    sig("gllm_mla_attention", [P, P, P, L, P, P, P, P, P, I, I, I, I, I, F, I, P, P])
+    sig("gllm_mla_attention", [P, P, P, L, P, P, P, P, P, P, I, I, I, I, I, F, I, P, P])
     sig("gllm_mla_rope_cache", [P, L, L, I, P, L, L, P, L, P, L, P, P, P, P, I, I, P])
     sig("gllm_mla_gather", [P, P, I, P, I, I, I, P, P, P, P])
     sig("gllm_attn_prefill_expanded", [P, L, P, P, P, L, P, P, P, I, I, I, I, I, F, P])

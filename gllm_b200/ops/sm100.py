@@ -41,7 +41,7 @@ def waits_given_up() -> int:
     return sum(getattr(L, f"gllm_waits_given_up_{f}")() for f in _WAIT_FAMILIES)
 
 
-_WAIT_FAMILIES = ("fp8", "attn")
+_WAIT_FAMILIES = ("fp8", "attn", "mla")
 
 
 # ----------------------------------------------------------------------------------------------
@@ -293,8 +293,6 @@ def reserve_attn_workspace(device, max_seqs: int, num_q_heads: int, head_dim: in
     _workspace(device, max_seqs * num_q_heads * max_splits * head_dim, "part_o")
     _workspace(device, max_seqs * num_q_heads * max_splits, "part_lse")
     _split_counters(device, max_seqs * num_q_heads)
-    if head_dim == 576:      # MLA latent attention: its own split-KV partials
-        _mla_workspace(device, num_q_heads)
 
 
 def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
@@ -476,29 +474,6 @@ def linear_fp8_block(x: torch.Tensor, w8: torch.Tensor, w_scale_inv: torch.Tenso
 # ----------------------------------------------------------------------------------------------
 # multi-head latent attention (DeepSeek): absorbed MQA over the paged latent cache
 # ----------------------------------------------------------------------------------------------
-def mla_splits(tokens: int, heads: int) -> int:
-    """KV splits so that a decode batch still fills the machine (one CTA = 16 heads of one token)."""
-    ctas = max(1, tokens * ((heads + 15) // 16))
-    return max(1, min(16, 296 // ctas))
-
-
-def _mla_workspace(device, heads: int):
-    """Split-KV partials of the MLA kernel, allocated ONCE per device (never re-allocated: CUDA graphs captured
-    earlier keep writing to it — a lazily grown buffer was freed under them and a later replay faulted). Capacity:
-    a forward splits only while tokens * ceil(heads/16) * splits <= 296 CTAs (`mla_splits`), i.e. at most
-    296 * 16 (token, head, split) rows, or 16 splits of one token's heads."""
-    key = ("mla_ws", torch.device(device))
-    ws = _attn_ws.get(key)
-    rows = max(296 * 16, 16 * heads)
-    if ws is None or ws[1].numel() < rows:
-        assert not (torch.cuda.is_available() and torch.cuda.is_current_stream_capturing()), \
-            "reserve_attn_workspace() must run before CUDA-graph capture"
-        ws = (torch.empty(rows * 512, dtype=torch.float32, device=device),
-              torch.empty(rows, dtype=torch.float32, device=device))
-        _attn_ws[key] = ws
-    return ws
-
-
 def mla_rope_cache(q_pe: torch.Tensor, q_full: Optional[torch.Tensor], k_pe: torch.Tensor, kv_c: torch.Tensor,
                    cos_sin: torch.Tensor, positions: torch.Tensor, slots: torch.Tensor, cache: torch.Tensor):
     """q_pe [T,H,64] (strided view), q_full [T,H,576] (rope part written; None: q_pe is rotated in place), k_pe [T,64],
@@ -556,21 +531,14 @@ def mla_attention(q_full: torch.Tensor, cache: torch.Tensor, block_table: torch.
     if positions.dim() == 2:
         positions = positions[0]
     assert sink is None or (sink.dtype == torch.float32 and sink.is_contiguous())
-    if splits is None:
-        splits = mla_splits(t, h)
-        if window:
-            splits = max(1, min(splits, (window + 63) // 64))
+    # one CTA per SM, each with an equal share of all key tiles (fewer if the caller bounds the CTAs per token and 16 heads)
+    ctas = NUM_SMS if splits is None else min(NUM_SMS, t * ((h + 15) // 16) * max(1, splits))
     out = torch.empty(t, h, 512, dtype=_BF16, device=q_full.device)
-    part_o = part_lse = None
-    if splits > 1:
-        if t * h * splits > max(296 * 16, 16 * h):
-            splits = max(1, max(296 * 16, 16 * h) // (t * h))      # caller-forced split beyond the workspace
-    if splits > 1:
-        part_o, part_lse = _mla_workspace(q_full.device, h)
-        assert t * h * splits <= part_lse.numel()
+    part_o = torch.empty(ctas * 2 * 16 * 512, dtype=torch.float32, device=q_full.device)
+    part_lse = torch.empty(ctas * (2 * 16 + 4), dtype=torch.float32, device=q_full.device)   # and 16 bytes per CTA
     L = _lib.load()
     check(L.gllm_mla_attention(_p(q_full), _p(out), _p(cache), pages, _p(block_table), _p(tok_seq), _p(positions),
-                               _p(part_o), _p(part_lse), t, block_table.shape[1], h, page_size, splits, float(scale),
-                               int(window or 0), _p(sink), stream_ptr()), "mla_attention")
-    _count(2 if splits > 1 else 1)
+                               _p(part_o), _p(part_lse), _p(part_lse[ctas * 32:]), t, block_table.shape[1], h, page_size, ctas,
+                               float(scale), int(window or 0), _p(sink), stream_ptr()), "mla_attention")
+    _count(2)
     return out

@@ -598,6 +598,35 @@ def test_mla_attention_decode(heads, splits):
     assert _rel_err(out, want) < 1.5e-2, _rel_err(out, want)
 
 
+@pytest.mark.parametrize("heads", [16, 40])
+@pytest.mark.parametrize("tokens,longest", [(1, 5000), (3, 700), (149, 130), (300, 64)])
+@pytest.mark.parametrize("page", [8, 64])
+def test_mla_attention_shares(heads, tokens, longest, page):
+    """Key tiles cut into one share per SM: shares with many tokens, tokens over many shares, more tokens than threads, lengths at
+    the edges of a 64-key tile; a window and a sink in the first part. Probabilities are rounded once to bf16."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(tokens + page)
+    lens = [longest] + [(1, 63, 64, 65, 128)[i % 5] for i in range(tokens - 1)]
+    need = [-(-n // page) for n in lens]
+    perm = torch.randperm(sum(need), device=_dev()).to(torch.int32)
+    bt, at = torch.zeros(tokens, max(need), dtype=torch.int32, device=_dev()), 0
+    for i, k in enumerate(need):
+        bt[i, :k] = perm[at:at + k]
+        at += k
+    cache = (torch.randn(sum(need), 1, 9, page, 64, device=_dev()) * 0.5).bfloat16()
+    q = (torch.randn(tokens, heads, 576, device=_dev()) * 0.3).bfloat16()
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=_dev())
+    sink = torch.randn(heads, device=_dev())
+    out = sm100.mla_attention(q, cache, bt, None, pos, 192 ** -0.5)
+    win = sm100.mla_attention(q, cache, bt, None, pos, 192 ** -0.5, window=100, sink=sink)
+    assert sm100.waits_given_up() == 0
+    assert _rel_err(out, _mla_ref(q, cache, bt, None, pos, 192 ** -0.5)) < 1.5e-2
+    for i, n in enumerate(lens):
+        lat = ref.gather_kv(cache, bt[i], n)[-100:, 0].float()
+        att = torch.softmax(torch.cat([q[i].float() @ lat.t() * 192 ** -0.5, sink[:, None]], -1), -1)[:, :-1]
+        assert _rel_err(win[i], att @ lat[:, :512]) < 1.5e-2, i
+
+
 def test_mla_attention_prefill_tokens_and_rope_cache():
     """Mixed batch: every token attends to its own causal prefix (tok_seq / positions); plus the fused
     rope + latent-cache write against the PyTorch oracle ops."""
