@@ -312,6 +312,24 @@ def test_sampler_greedy_and_filter():
     assert (probs.gather(1, tok.long().view(-1, 1)) > 0).all()
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("v", [1, 7, 8, 9, 8 * 1024 * 4 + 5, 50001])
+def test_sampler_greedy_edges(v, dt):
+    """The first largest element whatever the row's length and alignment: whole 16-byte chunks, remainders, unaligned rows, ties
+    inside a chunk and across threads, a penalty on the winner."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(v)
+    base = torch.randn(3, v + 3, device=_dev()).to(dt)
+    for off in (0, 1, 3):
+        z = base[:, off:off + v]
+        z[1, :] = z[1].clamp(max=z[1].float().median().item())         # many ties at the top
+        assert sm100.sample(z).tolist() == [int((r == r.max()).nonzero()[0, 0]) for r in z]
+    seen = torch.full((3, (v + 31) // 32), -1, dtype=torch.int32, device=_dev())
+    pen = torch.full((3,), 1.5, device=_dev())
+    want = torch.where(z.float() > 0, z.float() / 1.5, z.float() * 1.5)
+    assert sm100.sample(z, rep_penalty=pen, seen_bits=seen).tolist() == [int((r == r.max()).nonzero()[0, 0]) for r in want]
+
+
 def test_sampler_distribution():
     from gllm_b200.ops import sm100
     torch.manual_seed(7)
