@@ -290,6 +290,10 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   }
 }
 
+// defined in gemv_bf16.cu
+int gemv_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int M, int N, int K, const void* bias,
+              int act, cudaStream_t st);
+
 }  // namespace b200
 
 using namespace b200;
@@ -303,6 +307,10 @@ GLLM_EXPORT int gllm_gemm_smallm(const void* A, int64_t lda, const void* W, int6
   if (M > 256 || (K % 8) != 0 || (lda % 8) != 0 || (ldw % 8) != 0) {
     fprintf(stderr, "[gllm_b200] gemm_smallm: unsupported shape M=%d K=%d\n", M, K);
     return 1;
+  }
+  if (force_split <= 0) {
+    const int rc = gemv_bf16(A, lda, W, ldw, C, ldc, M, N, K, bias, silu, reinterpret_cast<cudaStream_t>(stream));
+    if (rc >= 0) return rc;
   }
   SmallMParams p;
   memset(&p, 0, sizeof(p));

@@ -773,3 +773,27 @@ def test_mla_expanded_attention(heads, page, n_dec):
         s.masked_fill_(torch.arange(n, device=_dev())[None] > torch.arange(n - (b - a), n, device=_dev())[:, None], float("-inf"))
         want[a:b] = torch.einsum("hqk,khd->qhd", s.softmax(-1), kv[..., 128:])
     assert _rel_err(out[n_dec:], want[n_dec:]) < 1.2e-2, _rel_err(out[n_dec:], want[n_dec:])
+
+
+@pytest.mark.parametrize("m", [1, 2])
+@pytest.mark.parametrize("n,k", [(1, 8), (5, 264), (130, 1024), (4097, 1024), (4100, 2056), (257, 6144), (640, 8192)])
+def test_linear_few_rows(m, n, k):
+    """One and two rows: a warp per weight row with the whole of K. Rows and columns beyond the last block, K below one 16-byte
+    load per lane, K over several chunks, strided input and output, a bias. fp32 sums of bf16 products, one rounding to bf16."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(n + k)
+    x = torch.randn(m, k + 16, device=_dev()).bfloat16()[:, 8:8 + k]
+    w = torch.randn(n, k + 8, device=_dev()).bfloat16()[:, :k]
+    b = torch.randn(n, device=_dev()).bfloat16()
+    out = torch.full((m + 1, n + 8), 7.0, device=_dev()).bfloat16()
+    sm100.linear(x, w, b, out=out[:m, :n])
+    want = x.double() @ w.double().t() + b.double()
+    assert bool((out[m] == 7.0).all()) and bool((out[:, n:] == 7.0).all())
+    tol = want.abs() * 2.0 ** -8 + (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24
+    assert bool(((out[:m, :n].double() - want).abs() <= tol).all())
+    if k >= 1024:
+        gu = torch.randn(512, k, device=_dev()).bfloat16() * k ** -0.5
+        inter = ref.interleave_gate_up(gu)
+        for act, f in (("silu", torch.nn.functional.silu), ("gelu", lambda z: torch.nn.functional.gelu(z, approximate="tanh"))):
+            g, u = (x.float() @ gu.float().t()).chunk(2, -1)
+            assert _rel_err(sm100.linear_silu_mul(x, inter, act=act), f(g) * u) < 6e-3      # one bf16 rounding and fast exp
