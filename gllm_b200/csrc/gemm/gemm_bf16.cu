@@ -50,6 +50,7 @@ struct GemmParams {
   // grouped (MoE) mode: M tile t multiplies the weight slab of expert tile_expert[t]
   const int32_t* tile_expert;
   const int32_t* num_m_tiles_ptr;  // device scalar: number of live M tiles
+  int moe_experts;                 // > 0: num_m_tiles_ptr points to moe_align's whole block (counts and offsets of that many experts)
   int n_per_expert;
   // per-row destination table (EP combine push): row r of C is stored at row_dest[r] (any rank's memory
   // mapped over NVLink); 0 = padding row, not stored. comm/ep_a2a.cu builds the table.
@@ -91,6 +92,7 @@ struct GemmCfg {
 template <int BN, int EPI>
 __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                 const __grid_constant__ CUtensorMap tmap_a16,   // A in boxes of 16 rows (grouped mode with moe_experts)
                  const GemmParams p) {
   using Cfg = GemmCfg<BN>;
   constexpr int S = Cfg::kStages;
@@ -114,6 +116,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const bool grouped = p.tile_expert != nullptr || p.num_m_tiles_ptr != nullptr || p.batch > 0;
   if (grouped) griddep_wait();
 
+  // Rows that exist in expert tile mt. A decode batch leaves a few in each tile of 128: only they are loaded (in 16-row boxes up to
+  // 64) and stored, what the rest of the tile holds is multiplied and dropped. 48 tokens x 8 of 128 experts (2048 -> 2 x 768
+  // -> 2048): first product 152 -> 102 us, second 65 -> 55 us.
+  auto tile_rows = [&](int mt) {
+    if (p.moe_experts <= 0) return kBlockM;
+    const int e = p.tile_expert[mt];
+    const int end = p.num_m_tiles_ptr[2 + 2 * p.moe_experts + e] + p.num_m_tiles_ptr[2 + e];
+    return min(kBlockM, end - mt * kBlockM);
+  };
   const int tpb = p.batch > 0 ? (p.rows_per_batch + kBlockM - 1) / kBlockM : 0;   // M tiles per batch entry
   const int num_m = p.batch > 0 ? p.batch * tpb
                     : p.num_m_tiles_ptr != nullptr ? min(*p.num_m_tiles_ptr, (p.M + kBlockM - 1) / kBlockM)
@@ -187,6 +198,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           while (static_cast<int32_t>(ld_acquire_sys(p.a_ready + mt) - want) < 0) guard.poll();
           asm volatile("fence.proxy.async;" ::: "memory");
         }
+        const int boxes = (tile_rows(mt) + 15) / 16;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % S;
           const uint32_t ph = (it / S) & 1;
@@ -197,6 +209,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             continue;
           }
           mbar_wait(&empty_bar[s], ph ^ 1);
+          if (boxes <= 4) {
+            mbar_expect_tx(&full_bar[s], Cfg::kStageBytes - Cfg::kABytes + boxes * (16 * kBlockK * 2));
+            tma_load_2d(sb, &tmap_b, &full_bar[s], kb * kBlockK, n0 + b_row_off, kEvictNormal);
+            for (int i = 0; i < boxes; ++i)
+              tma_load_2d(sa + i * (16 * kBlockK * 2), &tmap_a16, &full_bar[s], kb * kBlockK, m0 + i * 16, kEvictNormal);
+            continue;
+          }
           mbar_expect_tx(&full_bar[s], Cfg::kStageBytes);
           if (p.batch > 0) tma_load_3d(sa, &tmap_a, &full_bar[s], kb * kBlockK, (mt - bidx * tpb) * kBlockM, bidx);
           else tma_load_2d(sa, &tmap_a, &full_bar[s], kb * kBlockK, m0, kEvictNormal);
@@ -260,6 +279,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         row_in = row < p.rows_per_batch;
         c_off = static_cast<int64_t>(bidx) * p.c_batch_stride;
       }
+      if (p.moe_experts > 0) row_in = row_in && q * 32 + lane < tile_rows(m0 / kBlockM);
       const uint32_t t_row = tmem_base + buf * BN + (static_cast<uint32_t>(q * 32) << 16);
 
       // destination row pointer (local C, or the owner rank's staging buffer for RS)
@@ -488,7 +508,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
 template <int BN, int EPI>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
-                       cudaStream_t stream) {
+                       cudaStream_t stream, const CUtensorMap* ta16 = nullptr) {
   using Cfg = GemmCfg<BN>;
   static PerDeviceOnce configured;
   auto kern = gemm_bf16_kernel<BN, EPI>;
@@ -503,7 +523,8 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
   const int tiles = num_m * num_n * split;
   const int sms = (num_sms() / split) * split;  // split-K slices of a tile must run in the same round
   const int grid = tiles < sms ? tiles : sms;
-  CUDA_CHECK_RET(launch_pdl(kern, dim3(grid), dim3(kNumThreads), Cfg::kSmemBytes, stream, ta, tb, p));
+  CUDA_CHECK_RET(launch_pdl(kern, dim3(grid), dim3(kNumThreads), Cfg::kSmemBytes, stream, ta, tb,
+                            ta16 != nullptr ? *ta16 : ta, p));
   return 0;
 }
 
@@ -748,7 +769,8 @@ GLLM_EXPORT int gllm_gemm_bf16_batched(const void* A, int64_t lda_t, int64_t lda
 }
 
 // Grouped (MoE) GEMM: rows of A are expert-sorted and padded to 128-row tiles; tile t uses the weight
-// slab W[tile_expert[t]] ([E, N, K] contiguous). The live tile count is read on the device.
+// slab W[tile_expert[t]] ([E, N, K] contiguous). num_tiles_ptr is the block that gllm_moe_align_gather filled: the live tile count
+// and the experts' row counts and offsets are read on the device. Rows beyond an expert's count are neither read nor written.
 // epi: 0 store, 1 SiLU-gate (slab rows interleaved per 64 like the dense gate/up weight).
 static int moe_grouped_gemm_impl(const void* A, int64_t lda, const void* W, void* C, int64_t ldc, int max_tiles, int N,
                                  int K, int E, const void* tile_expert, const void* num_tiles_ptr, int epi,
@@ -756,9 +778,10 @@ static int moe_grouped_gemm_impl(const void* A, int64_t lda, const void* W, void
   if (max_tiles <= 0) return 0;
   if ((K % 8) != 0 || (N % 8) != 0 || (lda % 8) != 0 || (ldc % 8) != 0) return 1;
   const int bn = 128;  // 64|64 gate/up interleave for the SiLU epilogue; good balance for expert tiles
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb, ta16;
   const int M = max_tiles * kBlockM;
   if (make_tmap_2d(&ta, A, M, K, lda * 2, kBlockM, kBlockK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)) return 1;
+  if (make_tmap_2d(&ta16, A, M, K, lda * 2, 16, kBlockK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)) return 1;
   if (make_tmap_2d(&tb, W, static_cast<uint64_t>(E) * N, K, static_cast<uint64_t>(K) * 2, bn, kBlockK,
                    CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)) return 1;
   GemmParams p;
@@ -768,13 +791,15 @@ static int moe_grouped_gemm_impl(const void* A, int64_t lda, const void* W, void
   p.ldc = static_cast<int>(ldc);
   p.tile_expert = reinterpret_cast<const int32_t*>(tile_expert);
   p.num_m_tiles_ptr = reinterpret_cast<const int32_t*>(num_tiles_ptr);
+  p.moe_experts = E;
   p.n_per_expert = N;
   p.row_dest = reinterpret_cast<const int64_t*>(row_dest);
   p.glu_limit = glu_limit;
   p.glu_alpha = glu_alpha;
   p.act = act;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  return epi == kEpiSiluMul ? launch_gemm<128, kEpiSiluMul>(ta, tb, p, st) : launch_gemm<128, kEpiStore>(ta, tb, p, st);
+  return epi == kEpiSiluMul ? launch_gemm<128, kEpiSiluMul>(ta, tb, p, st, &ta16)
+                            : launch_gemm<128, kEpiStore>(ta, tb, p, st, &ta16);
 }
 
 GLLM_EXPORT int gllm_moe_grouped_gemm(const void* A, int64_t lda, const void* W, void* C, int64_t ldc,

@@ -513,6 +513,29 @@ def test_moe_fused_experts(t, e, k, h, i, ep):
     assert _rel_err(y, y_ref) < 2e-2, _rel_err(y, y_ref)
 
 
+@pytest.mark.parametrize("counts", [(1, 15, 16, 17), (63, 0, 64, 65), (127, 128, 129, 300)])
+def test_moe_expert_tiles_partly_filled(counts):
+    """Only the rows that an expert has are loaded and stored: counts at the edges of the 16-row boxes and of the 128-row tiles,
+    with a workspace full of NaN around them. Two bf16 roundings (the gated product, the result) of products of bf16 factors."""
+    from gllm_b200.ops import sm100_moe
+    torch.manual_seed(sum(counts))
+    e, h, i, t = len(counts), 192, 256, sum(counts)
+    x = torch.randn(t, h, device=_dev()).bfloat16()
+    w13 = (torch.randn(e, 2 * i, h, device=_dev()) * h ** -0.5).bfloat16()
+    w2 = (torch.randn(e, h, i, device=_dev()) * i ** -0.5).bfloat16()
+    ids = torch.repeat_interleave(torch.arange(e), torch.tensor(counts))[torch.randperm(t)].to(torch.int32).to(_dev())[:, None]
+    w13_il = torch.stack([ref.interleave_gate_up(w13[j], 64) for j in range(e)])
+    one = torch.ones(t, 1, device=_dev())
+    sm100_moe.fused_experts(x, w13_il, w2, one, ids)
+    for b in sm100_moe._ws.values():
+        if b.dtype == torch.bfloat16:
+            b.fill_(float("nan"))
+    y = sm100_moe.fused_experts(x, w13_il, w2, one, ids)
+    g, u = torch.einsum("th,tnh->tn", x.float(), w13.float()[ids[:, 0].long()]).chunk(2, -1)
+    want = torch.einsum("ti,thi->th", torch.nn.functional.silu(g) * u, w2.float()[ids[:, 0].long()])
+    assert _rel_err(y, want) < 6e-3, _rel_err(y, want)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 256, 128), (77, 1536, 512), (300, 4096, 7168), (1024, 2048, 2048),
                                    (64, 576, 7168),       # 576 = kv_a_proj_with_mqa (MLA): N not a multiple of 128
                                    (129, 8200, 640), (3000, 1032, 384), (2500, 4352, 1152)])   # tiles of 64, 128, 256
