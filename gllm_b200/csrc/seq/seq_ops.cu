@@ -363,8 +363,9 @@ __global__ void conv_silu_kernel(const T* __restrict__ xz, long ldxz, int C, con
 
 // The same convolution for bf16 rows whose channels come in aligned groups of 4: a thread owns 4 channels (8-byte loads
 // and stores, weights in registers: 8 channels would halve the occupancy) and walks `rows` consecutive batch rows with
-// the last TAPS - 1 inputs in registers, so every input row is read once per block instead of TAPS times. The next
-// row's load is in flight while the current one is computed. Sequences of one token also update their carried inputs here (longer ones: the kernel
+// the last TAPS - 1 inputs in registers, so every input row is read once per block instead of TAPS times. The next four
+// rows' loads are in flight while four are computed (6000 rows of 8192 channels: 105 -> 86 us against one row ahead).
+// Sequences of one token also update their carried inputs here (longer ones: the kernel
 // below, after every block has read them).
 template <int TAPS>
 __global__ void __launch_bounds__(128) conv_silu_vec_kernel(
@@ -393,51 +394,65 @@ __global__ void __launch_bounds__(128) conv_silu_vec_kernel(
   };
   float win[TAPS][4];                            // win[0 .. TAPS-2]: inputs before the row; win[TAPS-1]: the row's own
   int s = find_seq(qsl, nseq, t0), q0 = 0, q1 = -1;
-  uint2 cur = *reinterpret_cast<const uint2*>(xz + (size_t)t0 * ldxz + c);
-  for (int t = t0; t < t1; ++t) {
-    const uint2 nxt = t + 1 < t1 ? *reinterpret_cast<const uint2*>(xz + (size_t)(t + 1) * ldxz + c) : cur;
-    if (t >= q1) {                               // first row of the block or of a sequence: gather its past
-      while (s + 1 < nseq && qsl[s + 1] <= t) ++s;
-      q0 = qsl[s];
-      q1 = qsl[s + 1];
-      const int li = t - q0, pos0 = seq_lens[s] - (q1 - q0);
-      const bool carried = state != nullptr && pos0 > 0;
+  constexpr int kAhead = 4;
+  uint2 q[kAhead], q2[kAhead];
+  auto fetch = [&](int tb, uint2 (&v)[kAhead]) {
 #pragma unroll
-      for (int j = 0; j < TAPS - 1; ++j) {
-        const int src = li - (TAPS - 1) + j;
-        const bool own = src >= 0, have = own || (carried && pos0 + src >= 0);
-        float f[4];
-        if (own) unpack(*reinterpret_cast<const uint2*>(xz + (size_t)(q0 + src) * ldxz + c), f);
-        else if (have)
-          unpack(*reinterpret_cast<const uint2*>(state + ((size_t)rec_slots[s] * (TAPS - 1) + TAPS - 1 + src) * C + c), f);
+    for (int i = 0; i < kAhead; ++i)
+      if (tb + i < t1) v[i] = *reinterpret_cast<const uint2*>(xz + (size_t)(tb + i) * ldxz + c);
+  };
+  fetch(t0, q);
+  for (int tb = t0; tb < t1; tb += kAhead) {
+    fetch(tb + kAhead, q2);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) win[j][e] = have ? f[e] + ib[e] : 0.f;
+    for (int i = 0; i < kAhead; ++i) {
+      const int t = tb + i;
+      if (t >= t1) break;
+      const uint2 cur = q[i];
+      if (t >= q1) {                               // first row of the block or of a sequence: gather its past
+        while (s + 1 < nseq && qsl[s + 1] <= t) ++s;
+        q0 = qsl[s];
+        q1 = qsl[s + 1];
+        const int li = t - q0, pos0 = seq_lens[s] - (q1 - q0);
+        const bool carried = state != nullptr && pos0 > 0;
+#pragma unroll
+        for (int j = 0; j < TAPS - 1; ++j) {
+          const int src = li - (TAPS - 1) + j;
+          const bool own = src >= 0, have = own || (carried && pos0 + src >= 0);
+          float f[4];
+          if (own) unpack(*reinterpret_cast<const uint2*>(xz + (size_t)(q0 + src) * ldxz + c), f);
+          else if (have)
+            unpack(*reinterpret_cast<const uint2*>(state + ((size_t)rec_slots[s] * (TAPS - 1) + TAPS - 1 + src) * C + c), f);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) win[j][e] = have ? f[e] + ib[e] : 0.f;
+        }
+      }
+      unpack(cur, win[TAPS - 1]);
+      __align__(16) __nv_bfloat16 o[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        win[TAPS - 1][e] += ib[e];
+        float acc = br[e];
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) acc = fmaf(wr[e * TAPS + j], win[j][e], acc);
+        o[e] = __float2bfloat16_rn(act == 0 ? acc * __fdividef(1.0f, 1.0f + __expf(-acc)) : acc);
+#pragma unroll
+        for (int j = 0; j + 1 < TAPS; ++j) win[j][e] = win[j + 1][e];
+      }
+      *reinterpret_cast<uint2*>(out + (size_t)t * C + c) = *reinterpret_cast<const uint2*>(o);
+      if (TAPS > 1 && state != nullptr && q1 - q0 == 1) {
+        // a single token's sequence: nobody else reads its slot, so the carried inputs move up here
+        __nv_bfloat16* st = state + (size_t)rec_slots[s] * (TAPS - 1) * C + c;
+        const bool carried = seq_lens[s] > 1;
+#pragma unroll
+        for (int j = 0; j + 1 < TAPS - 1; ++j)
+          *reinterpret_cast<uint2*>(st + (size_t)j * C) =
+              carried ? *reinterpret_cast<const uint2*>(st + (size_t)(j + 1) * C) : make_uint2(0u, 0u);
+        *reinterpret_cast<uint2*>(st + (size_t)(TAPS - 2) * C) = cur;
       }
     }
-    unpack(cur, win[TAPS - 1]);
-    __align__(16) __nv_bfloat16 o[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      win[TAPS - 1][e] += ib[e];
-      float acc = br[e];
-#pragma unroll
-      for (int j = 0; j < TAPS; ++j) acc = fmaf(wr[e * TAPS + j], win[j][e], acc);
-      o[e] = __float2bfloat16_rn(act == 0 ? acc * __fdividef(1.0f, 1.0f + __expf(-acc)) : acc);
-#pragma unroll
-      for (int j = 0; j + 1 < TAPS; ++j) win[j][e] = win[j + 1][e];
-    }
-    *reinterpret_cast<uint2*>(out + (size_t)t * C + c) = *reinterpret_cast<const uint2*>(o);
-    if (TAPS > 1 && state != nullptr && q1 - q0 == 1) {
-      // a single token's sequence: nobody else reads its slot, so the carried inputs move up here
-      __nv_bfloat16* st = state + (size_t)rec_slots[s] * (TAPS - 1) * C + c;
-      const bool carried = seq_lens[s] > 1;
-#pragma unroll
-      for (int j = 0; j + 1 < TAPS - 1; ++j)
-        *reinterpret_cast<uint2*>(st + (size_t)j * C) =
-            carried ? *reinterpret_cast<const uint2*>(st + (size_t)(j + 1) * C) : make_uint2(0u, 0u);
-      *reinterpret_cast<uint2*>(st + (size_t)(TAPS - 2) * C) = cur;
-    }
-    cur = nxt;
+    for (int i = 0; i < kAhead; ++i) q[i] = q2[i];
   }
 }
 

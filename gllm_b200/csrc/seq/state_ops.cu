@@ -11,6 +11,7 @@
 #include <cuda_bf16.h>
 
 #include "common/host_utils.h"
+#include "common/ptx.cuh"
 #include "seq/seq_common.cuh"
 
 namespace {
@@ -433,6 +434,57 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ o, int n, cons
     const float gt = to_f(gate[(size_t)t * ldg + col]);
     const float ga = act ? sigmoid_f(gt) : silu_f(gt);
     out[(size_t)t * ldo + col] = from_f<T>(src[d] * r * to_f(w[col % wlen]) * ga * out_scale);
+  }
+}
+
+// The same for bf16 rows whose groups are 128 or 256 wide and lie on 8-byte boundaries (o: 16): 16- and 8-byte accesses, and a
+// warp has the loads of 4 x 128 columns in flight, where 4-byte loads of one group at a time were bound by their latency.
+// 6000 tokens x 32 groups of 128: 97 -> 58 us.
+template <int NCH>
+__global__ void __launch_bounds__(128) gated_group_norm_vec_kernel(
+    const float* __restrict__ o, int n, const __nv_bfloat16* __restrict__ gate, long ldg, const __nv_bfloat16* __restrict__ w,
+    int wlen, float eps, int act, float out_scale, __nv_bfloat16* __restrict__ out, long ldo, int ntok) {
+  constexpr int kGroup = 128 * NCH, kRows = 4 / NCH;
+  const int lane = threadIdx.x & 31, ngroups = n / kGroup;
+  const long g0 = ((long)blockIdx.x * 4 + (threadIdx.x >> 5)) * kRows, total = (long)ntok * ngroups;
+  if (g0 >= total) return;
+  const int count = (int)min((long)kRows, total - g0);
+  int t = (int)(g0 / ngroups), gi = (int)(g0 % ngroups);
+  float4 v[kRows][NCH];
+  uint2 gt[kRows][NCH];
+  int tok[kRows], col[kRows];
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    tok[i] = t;
+    col[i] = gi * kGroup + lane * 4;
+    if (++gi == ngroups) { gi = 0; ++t; }
+    if (i < count) {
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) {
+        v[i][c] = *reinterpret_cast<const float4*>(o + (size_t)tok[i] * n + col[i] + c * 128);
+        gt[i][c] = *reinterpret_cast<const uint2*>(gate + (size_t)tok[i] * ldg + col[i] + c * 128);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    if (i >= count) break;
+    float ss = 0.f;
+#pragma unroll
+    for (int c = 0; c < NCH; ++c)
+      ss += v[i][c].x * v[i][c].x + v[i][c].y * v[i][c].y + v[i][c].z * v[i][c].z + v[i][c].w * v[i][c].w;
+    ss = warp_sum(ss);
+    const float r = 1.0f / sqrtf(ss / (float)kGroup + eps);
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) {
+      const float2 g01 = b200::unpack_bf16(gt[i][c].x), g23 = b200::unpack_bf16(gt[i][c].y);
+      const uint2 wr = *reinterpret_cast<const uint2*>(w + (col[i] + c * 128) % wlen);
+      const float2 w01 = b200::unpack_bf16(wr.x), w23 = b200::unpack_bf16(wr.y);
+      auto one = [&](float x, float wt, float g) { return x * r * wt * (act ? sigmoid_f(g) : silu_f(g)) * out_scale; };
+      *reinterpret_cast<uint2*>(out + (size_t)tok[i] * ldo + col[i] + c * 128) =
+          make_uint2(b200::pack_bf16(one(v[i][c].x, w01.x, g01.x), one(v[i][c].y, w01.y, g01.y)),
+                     b200::pack_bf16(one(v[i][c].z, w23.x, g23.x), one(v[i][c].w, w23.y, g23.y)));
+    }
   }
 }
 
@@ -862,6 +914,15 @@ GLLM_EXPORT int gllm_seq_gated_group_norm(const void* o, int n, const void* gate
   if (group <= 0 || n % group != 0) return 2;
   cudaStream_t st = (cudaStream_t)stream;
   const long warps = (long)ntok * (n / group);
+  if (!is_f32 && (group == 128 || group == 256) && ((uintptr_t)o & 15) == 0 && wlen % 4 == 0 && ldg % 4 == 0 && ldo % 4 == 0 &&
+      (((uintptr_t)gate | (uintptr_t)w | (uintptr_t)out) & 7) == 0) {
+    const unsigned vblocks = (unsigned)((warps * (group / 128) + 15) / 16);
+    auto run = group == 128 ? gated_group_norm_vec_kernel<1> : gated_group_norm_vec_kernel<2>;
+    run<<<vblocks, 128, 0, st>>>((const float*)o, n, (const __nv_bfloat16*)gate, ldg, (const __nv_bfloat16*)w, wlen, eps, act,
+                                 out_scale, (__nv_bfloat16*)out, ldo, ntok);
+    CUDA_CHECK_RET(cudaGetLastError());
+    return 0;
+  }
   const unsigned blocks = (unsigned)((warps + 3) / 4);
   GLLM_BY_DTYPE(is_f32,
                 (gated_group_norm_kernel<bf16_t><<<blocks, 128, 0, st>>>((const float*)o, n, (const bf16_t*)gate, ldg,

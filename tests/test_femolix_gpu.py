@@ -152,6 +152,44 @@ def test_kernels_against_unfused_ops(dt, tol):
             assert close(g1, g2, tol)
 
 
+@pytest.mark.parametrize("group,ngroups,ntok,pad", [(128, 1, 1, 0), (128, 3, 7, 4), (256, 1, 5, 8), (256, 3, 33, 4), (128, 5, 3, 1),
+                                                    (384, 2, 9, 4)])
+@pytest.mark.parametrize("act", ["silu", "sigmoid"])
+def test_gated_group_norm_wide_rows(group, ngroups, ntok, pad, act):
+    """bf16 groups of 128 and 256: several groups per warp, the last ones missing, rows whose stride (pad 1) or group keeps them
+    on the element-wise kernel. One bf16 rounding."""
+    from gllm_b200.ops import ref, sm100_seq as S
+    torch.manual_seed(group + ntok)
+    n = group * ngroups
+    o = torch.randn(ntok, n, device=DEV)
+    gate = torch.randn(ntok, n + pad, device=DEV).bfloat16()[:, :n]
+    out = torch.zeros(ntok, n + pad, device=DEV).bfloat16()
+    for w in (torch.randn(group, device=DEV).bfloat16(), torch.randn(n, device=DEV).bfloat16()):
+        got = S.gated_group_norm(o, gate, w, group, 1e-5, act, 0.5, out[:, :n])
+        want = ref.gated_group_norm(o, gate.float(), w.float(), group, 1e-5, act, 0.5, None, torch.float32)
+        assert bool(((got.float() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-6).all())
+        assert out[:, n:].abs().sum().item() == 0
+
+
+@pytest.mark.parametrize("taps", [1, 2, 4])
+@pytest.mark.parametrize("qlens", [[600], [1, 1, 2050, 3, 1, 4, 5], [17, 1, 15, 700]])
+def test_conv_rows_fetched_ahead(qlens, taps):
+    """Blocks of 8 and 16 rows with four fetched ahead: sequence borders at every place of a group of four, a last block cut short."""
+    from gllm_b200.ops import ref, sm100_seq as S
+    torch.manual_seed(taps)
+    ns, C = len(qlens), 36
+    ctx = [5 * (i % 2) for i in range(ns)]
+    qsl = torch.tensor([0] + qlens, device=DEV).cumsum(0).to(torch.int32)
+    sl = torch.tensor([c + q for c, q in zip(ctx, qlens)], dtype=torch.int32, device=DEV)
+    rs = torch.randperm(ns + 1, device=DEV)[:ns].to(torch.int32)
+    xz = torch.randn(sum(qlens), 2 * C, device=DEV).bfloat16()
+    w, b = torch.randn(C, taps, device=DEV), torch.randn(C, device=DEV)
+    st = torch.randn(ns + 1, max(taps - 1, 1), C, device=DEV).bfloat16()[:, :max(taps - 1, 1)]
+    st1, st2 = st.clone(), st.clone()
+    c1, c2 = S.causal_conv_silu(xz, C, w, b, st1, rs, sl, qsl), ref.causal_conv_silu(xz, C, w, b, st2, rs, sl, qsl)
+    assert close(c1, c2, 1e-2) and torch.equal(st1, st2)
+
+
 def test_tensor_core_attention_with_chunk_mask_and_strided_output():
     """bf16, head size 64 / 128 with equal value size: the chunk mask runs on the tensor-core kernels (decode and
     prefill) and must agree with the plain kernel and the PyTorch form, also when it writes a scaled column slice."""
