@@ -534,14 +534,16 @@ static int pick_bn(int M, int N, int epi, int forced) {
   const int num_m = (M + kBlockM - 1) / kBlockM;
   int best = 128;
   double best_cost = 1e30;
-  const int cands[4] = {256, 128, 64, 32};
-  for (int i = 0; i < 4; ++i) {
+  const int cands[5] = {256, 192, 128, 64, 32};
+  for (int i = 0; i < 5; ++i) {
     const int bn = cands[i];
-    if (epi == kEpiSiluMul && bn < 64) continue;
+    if (epi == kEpiSiluMul && (bn < 64 || bn == 192)) continue;         // gated weights are interleaved for 128 and 256
     const int tiles = num_m * ((N + bn - 1) / bn);
     const int waves = (tiles + sms - 1) / sms;
-    // per-tile cost model: MMA time ∝ bn, plus a fixed per-tile overhead (A traffic, epilogue)
-    const double cost = waves * (bn + 48.0);
+    // time of one round of tiles, measured at K = 7168: 43.3 us at 256 wide, 38.4 at 192, 33.4 at 128 (the 128 rows of A cost the
+    // same at every width). 192 fills the last round where 256 does not: 4096 rows, N = 1536: 86.7 us at 256, 100 at 128, 76.7 at
+    // 192; N = 576: 46, 68, 41; N = 6144 stays at 256 (149.5 against 154).
+    const double cost = waves * (bn + 310.0);
     if (cost < best_cost) {
       best_cost = cost;
       best = bn;
@@ -690,6 +692,8 @@ static int gemm_bf16_impl(const void* A, int64_t lda, const void* W, int64_t ldw
                               : launch_gemm<BN_, kEpiStore>(ta, tb, p, st);
   switch (bn) {
     DISPATCH(256)
+    case 192:
+      return launch_gemm<192, kEpiStore>(ta, tb, p, st);
     DISPATCH(128)
     DISPATCH(64)
     case 32:

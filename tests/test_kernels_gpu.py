@@ -820,3 +820,16 @@ def test_linear_few_rows(m, n, k):
         for act, f in (("silu", torch.nn.functional.silu), ("gelu", lambda z: torch.nn.functional.gelu(z, approximate="tanh"))):
             g, u = (x.float() @ gu.float().t()).chunk(2, -1)
             assert _rel_err(sm100.linear_silu_mul(x, inter, act=act), f(g) * u) < 6e-3      # one bf16 rounding and fast exp
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 8, 64), (128, 192, 128), (129, 184, 72), (300, 200, 1000), (2100, 576, 328)])
+def test_gemm_tiles_of_192(m, n, k, monkeypatch):
+    """Tiles 192 wide: columns and rows beyond the last tile, K not a multiple of a 64-deep block, a bias; fp32 sums, one rounding."""
+    from gllm_b200.ops import sm100
+    monkeypatch.setattr(sm100, "_FORCE_BN", 192)
+    torch.manual_seed(n + k)
+    x, w = torch.randn(m, k, device=_dev()).bfloat16(), torch.randn(n, k, device=_dev()).bfloat16()
+    b = torch.randn(n, device=_dev()).bfloat16()
+    want = x.double() @ w.double().t() + b.double()
+    tol = want.abs() * 2.0 ** -8 + (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24
+    assert bool(((sm100.linear(x, w, b).double() - want).abs() <= tol).all())
