@@ -654,6 +654,10 @@ static int gemm_bf16_impl(const void* A, int64_t lda, const void* W, int64_t ldw
     fprintf(stderr, "[gllm_b200] gemm_bf16: K, N and leading dims must be multiples of 8\n");
     return 1;
   }
+  if (((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(bias)) & 15) != 0) {   // 16-byte stores and loads
+    fprintf(stderr, "[gllm_b200] gemm_bf16: output and bias must lie on 16-byte boundaries\n");
+    return 1;
+  }
   int bn = 128, split = 1;
   choose_cfg(M, N, K, epi, force_bn, ws != nullptr && tile_cnt != nullptr ? ws_bytes : 0, max_tiles, &bn, &split);
   CUtensorMap ta, tb;

@@ -35,6 +35,7 @@ struct SmallMParams {
   float* ws;              // [num_n_tiles * S][128][BT] fp32 partials
   uint32_t* counters;     // [num_n_tiles], zero on entry, self-resetting
   int silu;               // gated epilogue (1: silu, 2: the tanh form of gelu): weight rows interleaved per 128: tile 2g = gate, tile 2g+1 = up
+  int wide_c;             // C and its rows on 8-byte boundaries: four columns per store
   int stages;
   uint32_t tmem_cols;
 };
@@ -232,7 +233,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
               const int m = m0 + uu * 4 + mr;
               if (m < p.M) {
                 __nv_bfloat16* dst = p.C + static_cast<size_t>(m) * p.ldc + ncol;
-                if (ncol + 3 < p.N) {
+                if (p.wide_c && ncol + 3 < p.N) {
                   *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(acc[uu].x, acc[uu].y), pack_bf16(acc[uu].z, acc[uu].w));
                 } else {
                   const float a[4] = {acc[uu].x, acc[uu].y, acc[uu].z, acc[uu].w};
@@ -271,8 +272,13 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 const float o1 = act(g[uu].y) * up[uu].y;
                 const float o2 = act(g[uu].z) * up[uu].z;
                 const float o3 = act(g[uu].w) * up[uu].w;
-                *reinterpret_cast<uint2*>(p.C + static_cast<size_t>(m) * p.ldc + f) =
-                    make_uint2(pack_bf16(o0, o1), pack_bf16(o2, o3));
+                __nv_bfloat16* dst = p.C + static_cast<size_t>(m) * p.ldc + f;
+                if (p.wide_c) {
+                  *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(o0, o1), pack_bf16(o2, o3));
+                } else {
+                  dst[0] = __float2bfloat16(o0); dst[1] = __float2bfloat16(o1);
+                  dst[2] = __float2bfloat16(o2); dst[3] = __float2bfloat16(o3);
+                }
               }
             }
           }
@@ -348,6 +354,7 @@ GLLM_EXPORT int gllm_gemm_smallm(const void* A, int64_t lda, const void* W, int6
   }
   p.C = reinterpret_cast<__nv_bfloat16*>(C);
   p.ldc = static_cast<int>(ldc);
+  p.wide_c = (ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 7) == 0) ? 1 : 0;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.ws = reinterpret_cast<float*>(ws);
   p.counters = reinterpret_cast<uint32_t*>(counters);

@@ -428,6 +428,10 @@ GLLM_EXPORT int gllm_gemm_fp8_block(const void* A8, const void* a_s, const void*
     fprintf(stderr, "[gllm_b200] gemm_fp8_block: K %% 128 and N %% 8 required (gated: N %% 256, no bias)\n");
     return 1;
   }
+  if (ldc % 8 != 0 || ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(bias)) & 15) != 0) {
+    fprintf(stderr, "[gllm_b200] gemm_fp8_block: output rows and bias must lie on 16-byte boundaries\n");
+    return 1;
+  }
   Fp8Params p;
   p.M = M; p.N = N; p.K = K;
   p.C = reinterpret_cast<__nv_bfloat16*>(C);

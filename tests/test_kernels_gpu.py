@@ -822,6 +822,46 @@ def test_linear_few_rows(m, n, k):
             assert _rel_err(sm100.linear_silu_mul(x, inter, act=act), f(g) * u) < 6e-3      # one bf16 rounding and fast exp
 
 
+@pytest.mark.parametrize("m", [3, 17, 32])
+@pytest.mark.parametrize("ldc,shift", [(13, 0), (514, 1), (516, 2), (516, 4)])     # the last one: 8-byte boundaries
+def test_gemm_smallm_any_output(m, ldc, shift):
+    """Outputs whose rows lie off the 8-byte boundaries that the split-K sums are stored on: element-wise stores instead."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(ldc + m)
+    n, k = (5, 4096) if ldc == 13 else (512, 4096)
+    x, w = torch.randn(m, k, device=_dev()).bfloat16(), torch.randn(n, k, device=_dev()).bfloat16()
+    buf = torch.full((m * ldc + 8,), 7.0, device=_dev()).bfloat16()
+    want = x.double() @ w.double().t()
+    tol = want.abs() * 2.0 ** -8 + (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24
+    out = torch.as_strided(buf, (m, n), (ldc, 1), shift)
+    sm100.linear(x, w, out=out)
+    assert bool(((out.double() - want).abs() <= tol).all())
+    if ldc != 13:
+        gated = torch.as_strided(buf, (m, n // 2), (ldc, 1), shift)
+        wk = w * k ** -0.5
+        g, u = (x.float() @ wk.float().t()).chunk(2, -1)
+        sm100.linear_silu_mul(x, ref.interleave_gate_up(wk), out=gated)
+        assert _rel_err(gated, torch.nn.functional.silu(g) * u) < 6e-3      # one bf16 rounding and fast exp
+    written = torch.zeros_like(buf, dtype=torch.bool)
+    torch.as_strided(written, (m, n), (ldc, 1), shift).fill_(True)
+    assert bool((buf[~written] == 7.0).all())
+
+
+def test_gemm_refuses_unaligned_output():
+    """The tiled GEMMs store 16 bytes at a time: an output or bias off that boundary is an error, never a launch."""
+    from gllm_b200.ops import sm100
+    x, w = torch.randn(64, 256, device=_dev()).bfloat16(), torch.randn(256, 256, device=_dev()).bfloat16()
+    buf = torch.zeros(64 * 264 + 8, device=_dev()).bfloat16()
+    off = torch.as_strided(buf, (64, 256), (264, 1), 4)
+    w8, ws = w.to(torch.float8_e4m3fn), torch.ones(2, 2, device=_dev())
+    for call in (lambda: sm100.linear(x, w, out=off), lambda: sm100.linear(x, w, buf[4:260]),
+                 lambda: sm100.linear_fp8_block(x, w8, ws, out=off), lambda: sm100.linear_fp8_block(x, w8, ws, buf[4:260]),
+                 lambda: sm100.linear_fp8_block(x, w8, ws, out=torch.as_strided(buf, (64, 256), (260, 1)))):
+        with pytest.raises(RuntimeError):
+            call()
+    assert bool((buf == 0).all())
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 8, 64), (128, 192, 128), (129, 184, 72), (300, 200, 1000), (2100, 576, 328)])
 def test_gemm_tiles_of_192(m, n, k, monkeypatch):
     """Tiles 192 wide: columns and rows beyond the last tile, K not a multiple of a 64-deep block, a bias; fp32 sums, one rounding."""
