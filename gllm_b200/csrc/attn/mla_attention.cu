@@ -50,6 +50,7 @@ struct MlaParams {
   int tokens, max_blocks, H, page_size;
   float scale_log2;
   int window;                 // a token at position i sees keys j with i - j < window (0: the whole past)
+  WaitConfig waits;
   const float* sink;          // [H] one more logit per head in the denominator, without a value (null: none)
 };
 
@@ -80,7 +81,7 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
   griddep_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int hg = (p.H + 15) / 16;
-  const WaitGuard guard{dead};
+  const WaitGuard guard{dead, p.waits};
 
   // ---------------- this CTA's share [t0, t1) of all tiles ----------------
   if (threadIdx.x == 0) {
@@ -139,13 +140,15 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
   };
   auto load_tile = [&] {
     if (ld.cur >= t1) return;
-    const int s = ld.it % kMlaStages;
-    if (!__any_sync(0xffffffffu, guard.gave_up())) {
-      if (lane == 0) mbar_expect_tx(&full_bar[s], kMlaTileBytes);
-      __syncwarp();
-      if (lane < pages_per_tile)
-        tma_load_3d(smem + s * kMlaTileBytes + lane * page_bytes, &tmap, &full_bar[s], 0, 0, ld.page * (kLat / 64));
+    if (__any_sync(0xffffffffu, guard.gave_up())) {    // nothing more is issued: ld.it counts what was
+      ld.cur = t1;
+      return;
     }
+    const int s = ld.it % kMlaStages;
+    if (lane == 0) mbar_expect_tx(&full_bar[s], kMlaTileBytes);
+    __syncwarp();
+    if (lane < pages_per_tile)
+      tma_load_3d(smem + s * kMlaTileBytes + lane * page_bytes, &tmap, &full_bar[s], 0, 0, ld.page * (kLat / 64));
     ++ld.it;
     ++ld.cur;
     if (++ld.at == ld.end) {
@@ -340,7 +343,7 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
   if (threadIdx.x == 0) p.meta[blockIdx.x] = meta;
   if (warp == 0 && guard.gave_up()) {                                  // copies in flight end before the CTA does
     for (uint32_t k = ld.it < kMlaStages ? 0u : ld.it - kMlaStages; k < ld.it; ++k)
-      for (uint32_t n = 0; n < (1u << 20) && !mbar_try_wait(&full_bar[k % kMlaStages], (k / kMlaStages) & 1); ++n) {}
+      guard.land(&full_bar[k % kMlaStages], (k / kMlaStages) & 1);
   }
 }
 
@@ -507,6 +510,7 @@ GLLM_EXPORT int gllm_mla_attention(const void* q, void* out, const void* cache, 
   p.tokens = tokens; p.max_blocks = max_blocks; p.H = H; p.page_size = page_size;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.window = window;
+  p.waits = g_wait_config;
   p.sink = reinterpret_cast<const float*>(sink);
   static PerDeviceOnce configured;
   if (configured.need()) {
@@ -519,8 +523,6 @@ GLLM_EXPORT int gllm_mla_attention(const void* q, void* out, const void* cache, 
                             static_cast<const float*>(p.part_lse), static_cast<const int4*>(p.meta), p.out, H));
   return 0;
 }
-
-GLLM_EXPORT int gllm_waits_given_up_mla() { return read_waits_given_up(); }
 
 // rows [nseq + 1] int32 (written), lat [total, 512], pe [total, 64]; total = the sequences' lengths, each rounded up to 64
 GLLM_EXPORT int gllm_mla_gather(const void* cache, const void* block_table, int max_blocks, const void* seq_lens, int nseq,

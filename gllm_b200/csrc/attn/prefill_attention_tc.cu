@@ -67,6 +67,7 @@ struct TcAttnParams {
   int64_t out_ts;     // output row stride (elements)
   int window;         // sliding window: a query at i sees keys j with i - j < window (0 = the whole past)
   AttnExtras ex;      // distance bias or table (kernel template BIAS), turned values, output gate
+  WaitConfig waits;
   int q_tiles;        // query tiles per CTA (2, or 1 where that gives every SM at most one CTA)
   const int32_t* kv_row;   // DENSE: first row of each sequence of this launch in the expanded keys and values
 };
@@ -167,7 +168,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   uint64_t* q_full = p_full + 2;                       // [2 tiles] Q staged (TMA)
   uint64_t* mma_end = q_full + 2;                      // [1]       every product has finished
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_end + 1);
-  const WaitGuard guard{tmem_slot + 1};
+  const WaitGuard guard{tmem_slot + 1, p.waits};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int seq = blockIdx.y + p.seq_offset;
@@ -271,13 +272,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         page_v = page;
         page = next;
       }
-      if (!ok && n_max > 0) {                              // copies in flight land before the CTA ends
+      if (n_max > 0) {                                     // copies in flight land before the CTA ends, whichever role gave up
         for (int t = 0; t < 2; ++t)
-          for (uint32_t n = 0; (t ? n1 : n0) > 0 && n < (1u << 16) && !mbar_try_wait(&q_full[t], 0); ++n) {}
-        for (int i = max(0, tk - SM::kKStages); i < tk; ++i)
-          for (uint32_t n = 0; n < (1u << 16) && !mbar_try_wait(&k_full[i % SM::kKStages], (i / SM::kKStages) & 1); ++n) {}
-        for (int i = max(0, tv - SM::kVStages); i < tv; ++i)
-          for (uint32_t n = 0; n < (1u << 16) && !mbar_try_wait(&v_full[i % SM::kVStages], (i / SM::kVStages) & 1); ++n) {}
+          if ((t ? n1 : n0) > 0) guard.land(&q_full[t], 0);
+        for (int i = max(0, tk - SM::kKStages); i < tk; ++i) guard.land(&k_full[i % SM::kKStages], (i / SM::kKStages) & 1);
+        for (int i = max(0, tv - SM::kVStages); i < tv; ++i) guard.land(&v_full[i % SM::kVStages], (i / SM::kVStages) & 1);
       }
     } else if (warp == kTcSoftmaxWarps + 1 && lane == 0) {
       // ------------------------------------------------------------------ MMA issuer
@@ -329,7 +328,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         umma_commit(&step[(tile + 1) & 3]);
       }
       umma_commit(mma_end);                              // nothing is in flight when the columns are given back
-      for (uint32_t n = 0; n < (1u << 22) && !mbar_try_wait(mma_end, 0); ++n) {}
+      guard.land(mma_end, 0);
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kTcRegsSoftmax));
@@ -588,6 +587,7 @@ static int launch_prefill_tc(const CUtensorMap& tk, const CUtensorMap& tv, const
     configured.done();
   }
   // One query tile per CTA while that leaves at most one CTA per SM (short prompts): two would only halve the SMs at work
+  p.waits = g_wait_config;
   const int toks = kTcRows / p.GP, z = p.Hkv * (p.G / p.GP);
   const int64_t single = static_cast<int64_t>((max_q_len + toks - 1) / toks) * num_seqs * z;
   p.q_tiles = single <= num_sms() ? 1 : 2;
@@ -668,8 +668,6 @@ static int attn_prefill_tc_impl(const void* q, int64_t q_ts, void* out, const vo
   return GLLM_TC(false, kNoBias);
 #undef GLLM_TC
 }
-
-GLLM_EXPORT int gllm_waits_given_up_attn() { return read_waits_given_up(); }
 
 GLLM_EXPORT int gllm_attn_prefill_tc(const void* q, int64_t q_ts, void* out, const void* k_cache, const void* v_cache,
                                      int64_t num_pages, const void* block_table, const void* seq_lens,

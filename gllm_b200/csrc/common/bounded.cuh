@@ -1,40 +1,75 @@
 // Bounded mbarrier waits. A wait that never ends would hang the GPU for everyone on it, so after a limit the kernel records
 // that it gave up, every later wait of the CTA returns at once, the roles run their loops out without issuing copies or
-// products, wait (again bounded) for what is in flight and return. The count is read by `gllm_waits_given_up_*`.
+// products, what is in flight lands and the kernel returns. Its results are wrong then: the record is one word of pinned host
+// memory, which the engine reads before it uses a step's tokens (ops/lib.py) and fails on.
 #pragma once
 
+#include "host_utils.h"
 #include "ptx.cuh"
 
 namespace b200 {
 
-// each translation unit has its own counter (no relocatable device code)
-static __device__ unsigned int g_waits_given_up;
+struct WaitConfig {              // part of a kernel's parameters
+  uint32_t* word;                // set to 1 when a wait gives up (null: nobody reads it)
+  uint32_t limit_ns;             // at most 2^32 - 1; 0 (tests): a phase that has not completed is given up
+};
+
+// one per process, set when the library is loaded
+inline WaitConfig g_wait_config{nullptr, 2000000000u};
+
+__device__ __forceinline__ uint32_t global_ns() {        // wraps every 4.3 s
+  uint32_t t;
+  asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
+  return t;
+}
 
 struct WaitGuard {
   volatile uint32_t* dead;       // shared memory, zero at the start of the CTA
+  WaitConfig cfg;
 
   __device__ __forceinline__ bool gave_up() const { return *dead != 0; }
 
-  // true: the phase completed. try_wait suspends the thread for a while in hardware, so 2^22 tries are well over a second's
-  // worth of polling only when something is stuck
+  // true: the phase completed. try_wait suspends the thread in hardware, so the clock is read rarely
   __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity) const {
-    if (mbar_try_wait(bar, parity)) return true;
-    for (uint32_t n = 1; n < (1u << 22); ++n) {
-      if (mbar_try_wait(bar, parity)) return true;
-      if ((n & 1023u) == 0u && *dead != 0) return false;
-    }
-    if (*dead == 0) {
-      *dead = 1;
-      atomicAdd(&g_waits_given_up, 1u);
+    if (cfg.limit_ns != 0 ? mbar_try_wait(bar, parity) : mbar_test_wait(bar, parity)) return true;
+    return wait_on(bar, parity);
+  }
+
+  // copies and products in flight: they end by themselves, whatever the limit of the waits
+  __device__ __forceinline__ static void land(uint64_t* bar, uint32_t parity) {
+    if (mbar_try_wait(bar, parity)) return;
+    const uint32_t t0 = global_ns();
+    do {
+#pragma unroll 1
+      for (int n = 0; n < 64; ++n)
+        if (mbar_try_wait(bar, parity)) return;
+    } while (global_ns() - t0 < 2000000000u);
+  }
+
+ private:
+  __device__ __forceinline__ bool wait_on(uint64_t* bar, uint32_t parity) const {
+    const uint32_t t0 = global_ns();
+    while (*dead == 0) {
+      if (global_ns() - t0 >= cfg.limit_ns) {
+        *dead = 1;
+        if (cfg.word != nullptr) {
+          st_relaxed_sys(cfg.word, 1u);
+          __threadfence_system();
+        }
+        return false;
+      }
+#pragma unroll 1
+      for (int n = 0; n < 64; ++n)
+        if (mbar_try_wait(bar, parity)) return true;
     }
     return false;
   }
 };
 
-inline int read_waits_given_up() {
-  unsigned int v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_waits_given_up, sizeof v) != cudaSuccess) return -1;
-  return static_cast<int>(v);
-}
-
 }  // namespace b200
+
+// word: 4 bytes of pinned host memory, kept for the process's life
+extern "C" __attribute__((visibility("default"), weak)) int gllm_set_waits(void* word, unsigned int limit_ns) {
+  b200::g_wait_config = b200::WaitConfig{reinterpret_cast<uint32_t*>(word), limit_ns};
+  return 0;
+}

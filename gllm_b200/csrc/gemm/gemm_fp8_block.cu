@@ -54,6 +54,7 @@ struct Fp8Params {
   int n_per_expert;      // rows of one expert slab
   int64_t ws_stride_e;   // floats per expert in w_s
   int silu;              // 1: out[:, j] = silu(gate[j]) * up[j]; the tile holds [64 gate | 64 up] boxes in turn
+  WaitConfig waits;
   int up_row;            // > 0 (with silu): the weight is [gate rows ; up rows], up rows start here; the boxes are fetched
                          // from the two halves. 0: the rows are interleaved per 64 already
 };
@@ -98,7 +99,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   uint64_t* tmem_empty = tmem_full + 2;
   uint64_t* mma_end = tmem_empty + 2;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(mma_end + 1);
-  const WaitGuard guard{tmem_ptr_smem + 1};
+  const WaitGuard guard{tmem_ptr_smem + 1, p.waits};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool grouped = p.tile_expert != nullptr;
@@ -149,10 +150,9 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                         kEvictNormal);
         }
       }
-      if (!ok) {                                          // copies in flight land before the CTA ends
-        for (uint32_t i = it > T::kStages ? it - T::kStages : 0; i < it; ++i)
-          for (uint32_t n = 0; n < (1u << 16) && !mbar_try_wait(&full_bar[i % T::kStages], (i / T::kStages) & 1); ++n) {}
-      }
+      // copies in flight land before the CTA ends, whichever role gave up
+      for (uint32_t i = it > T::kStages ? it - T::kStages : 0; i < it; ++i)
+        guard.land(&full_bar[i % T::kStages], (i / T::kStages) & 1);
     }
     if (warp == 1 && lane == 0) {
       constexpr uint32_t idesc = make_idesc_e4m3(kFBM, BN);
@@ -177,7 +177,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         }
       }
       umma_commit(mma_end);                               // nothing is in flight when the columns are given back
-      for (uint32_t n = 0; n < (1u << 22) && !mbar_try_wait(mma_end, 0); ++n) {}
+      guard.land(mma_end, 0);
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFRegsFold));
@@ -380,7 +380,7 @@ static int launch_fp8_tile(const CUtensorMap& ta, const CUtensorMap& tb, const F
 // Tile width: the one with the least (waves x time of a tile's K block). A block of 128 rows costs about 560 cycles 256 wide,
 // 330 at 128 and 230 at 64 (there the copies of the activation tile bound it), so narrow tiles only pay when the wide ones
 // leave SMs idle: a decode batch's 7168 columns are 28 tiles of 256. Grouped calls do not know how many row tiles are live.
-static int launch_fp8(const void* A8, const void* W8, uint64_t w_rows, const Fp8Params& p, cudaStream_t st) {
+static int launch_fp8(const void* A8, const void* W8, uint64_t w_rows, Fp8Params p, cudaStream_t st) {
   const int64_t m_tiles = (p.M + kFBM - 1) / kFBM;
   const int width[3] = {256, 128, 64}, cost[3] = {560, 330, 230};
   int bn = 256;
@@ -392,6 +392,7 @@ static int launch_fp8(const void* A8, const void* W8, uint64_t w_rows, const Fp8
       if (best < 0 || t < best) { best = t; bn = width[i]; }
     }
   }
+  p.waits = g_wait_config;
   CUtensorMap ta, tb;
   if (make_tmap_2d(&ta, A8, p.M, p.K, p.K, kFBM, kFBK, CU_TENSOR_MAP_DATA_TYPE_UINT8)) return 1;
   if (make_tmap_2d(&tb, W8, w_rows, p.K, p.K, 64, kFBK, CU_TENSOR_MAP_DATA_TYPE_UINT8)) return 1;
@@ -403,8 +404,6 @@ static int launch_fp8(const void* A8, const void* W8, uint64_t w_rows, const Fp8
 }  // namespace b200
 
 using namespace b200;
-
-GLLM_EXPORT int gllm_waits_given_up_fp8() { return read_waits_given_up(); }
 
 // live_tiles: device count of the 128-row tiles that exist (null: all M rows)
 GLLM_EXPORT int gllm_fp8_quant_group(const void* x, int64_t ldx, void* q, void* scales, int M, int K, const void* live_tiles,

@@ -24,6 +24,7 @@ from gllm_b200.input_data import BatchArrays, InputData
 from gllm_b200.layers import functional as Fn
 from gllm_b200.memory_manager import HybridCache, KVCache
 from gllm_b200.model_loader import ModelLoader
+from gllm_b200.ops.lib import raise_if_waits_gave_up, watch_waits
 from gllm_b200.parallel import state as ps
 from gllm_b200.parallel.tp import make_tp_comm
 from gllm_b200.utils.logging import logger
@@ -43,8 +44,8 @@ class StepResult:
             return []
         if self.event is not None:
             self.event.synchronize()
-            return self.tokens_host[: self.num_emit].tolist()
-        return self.tokens[: self.num_emit].tolist()
+        raise_if_waits_gave_up()
+        return (self.tokens if self.event is None else self.tokens_host)[: self.num_emit].tolist()
 
 
 class ModelRunner:
@@ -88,6 +89,7 @@ class ModelRunner:
         is_cuda = self.device.type == "cuda"
         if is_cuda:
             torch.cuda.set_device(self.device)
+            watch_waits()
         t0 = time.time()
         self.model = self.loader.load_model(self.device, progress)
         self.spec = self.model.spec
@@ -217,6 +219,7 @@ class ModelRunner:
     def step_logits(self, batch: BatchArrays) -> torch.Tensor:
         """One eager step that returns fp32 logits [len(batch.logits_idx), V] instead of sampling (logit tracing,
         numerics checks). `batch.logits_idx` may name any rows of the batch."""
+        raise_if_waits_gave_up()
         self.stats["steps"] += 1
         self.stats["tokens"] += batch.num_tokens
         if batch.logits_idx.shape[0] == 0:
@@ -299,6 +302,7 @@ class ModelRunner:
     # -------------------------------------------------------------------------------------------
     def step(self, batch: BatchArrays, hidden: Optional[torch.Tensor] = None,
              residual: Optional[torch.Tensor] = None, recv_tiles=None) -> StepResult:
+        raise_if_waits_gave_up()          # of earlier steps: a stage without the sampler reads no tokens
         inp = self.input_data
         self.stats["steps"] += 1
         self.stats["tokens"] += batch.num_tokens

@@ -82,6 +82,7 @@ def _declare(lib):
     sig("gllm_moe_combine", [P, P, P, P, I, I, I, P])
     sig("gllm_fp8_quant_group", [P, L, P, P, I, I, P, P])
     sig("gllm_moe_grouped_gemm_fp8", [P, P, P, P, P, L, I, I, I, I, P, P, I, P])
+    sig("gllm_set_waits", [P, c_uint32])
     sig("gllm_gemm_fp8_block", [P, P, P, P, P, L, I, I, I, P, I, P])
 
 
@@ -125,10 +126,44 @@ def load():
         lib = ctypes.CDLL(LIB_PATH)
         _declare(lib)
         _LIB = lib
+        if torch.cuda.is_initialized():
+            watch_waits()
         return lib
     except Exception as e:  # noqa: BLE001
         _LIB_ERR = e
         raise
+
+
+_WAIT_WORD = None     # (pinned tensor that lives as long as the process, the same word as a numpy array)
+WAIT_LIMIT_NS = 2_000_000_000     # below 2^32
+
+
+def watch_waits(limit_ns: int = WAIT_LIMIT_NS):
+    """Gives the kernels with bounded waits (csrc/common/bounded.cuh) the word that they set when a wait ran out, and the
+    limit. The word is pinned host memory: reading it needs no copy and no synchronisation beyond that of the step."""
+    global _WAIT_WORD
+    lib = load()
+    if not hasattr(lib, "gllm_set_waits"):
+        return                       # a library of other kernel families
+    if _WAIT_WORD is None:
+        word = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+        _WAIT_WORD = (word, word.numpy())
+    check(lib.gllm_set_waits(_WAIT_WORD[0].data_ptr(), limit_ns), "set_waits")
+
+
+def waits_gave_up(clear: bool = False) -> bool:
+    """Whether a wait of a kernel that has finished ran out since the last clear."""
+    if _WAIT_WORD is None:
+        return False
+    seen = bool(_WAIT_WORD[1][0])
+    if clear:
+        _WAIT_WORD[1][0] = 0
+    return seen
+
+
+def raise_if_waits_gave_up():
+    if waits_gave_up(clear=True):
+        raise RuntimeError("a kernel's bounded wait ran out: the results since the last check are invalid")
 
 
 def available() -> bool:

@@ -36,12 +36,10 @@ def _count(n=1):
 
 
 def waits_given_up() -> int:
-    """Bounded waits that ran out in this process's kernels (csrc/common/bounded.cuh); 0 in a healthy run."""
-    L = _lib.load()
-    return sum(getattr(L, f"gllm_waits_given_up_{f}")() for f in _WAIT_FAMILIES)
-
-
-_WAIT_FAMILIES = ("fp8", "attn", "mla")
+    """1 if a bounded wait of this process's kernels has run out (csrc/common/bounded.cuh); 0 in a healthy run."""
+    _lib.watch_waits()
+    torch.cuda.synchronize()
+    return int(_lib.waits_gave_up())
 
 
 # ----------------------------------------------------------------------------------------------

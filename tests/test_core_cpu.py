@@ -367,6 +367,28 @@ def test_incremental_decode_batch_equals_full_rebuild():
             s.token_ids.append(int(rng.integers(3, 200)))
 
 
+def test_a_wait_that_gave_up_stops_the_engine(monkeypatch):
+    """The word that a kernel sets when a bounded wait ran out: neither a step's tokens nor the next step get past it."""
+    import torch
+    from gllm_b200 import LLM
+    from gllm_b200.model_runner import StepResult
+    from gllm_b200.models.presets import tiny
+    from gllm_b200.ops import lib
+    word = np.zeros(1, np.int32)
+    monkeypatch.setattr(lib, "_WAIT_WORD", (None, word))
+    res = StepResult(tokens=torch.tensor([7], dtype=torch.int32), num_emit=1)
+    assert res.tokens_list() == [7]
+    word[0] = 1
+    with pytest.raises(RuntimeError, match="bounded wait"):
+        res.tokens_list()
+    assert word[0] == 0 and res.tokens_list() == [7]
+    llm = LLM(tiny(), load_format="dummy", num_cpu_pages=64, model_max_length=64, log_stats=False)
+    word[0] = 1
+    with pytest.raises(RuntimeError, match="bounded wait"):
+        llm.generate(tokens=[[1, 2, 3]], output_lens=[2], ignore_eos=True)
+    llm.shutdown()
+
+
 def test_oversized_requests_do_not_hang_the_scheduler():
     """A prompt that can never be resident is rejected (finished with no output) and an output budget that the
     pool cannot hold is capped — neither may block the queue forever."""

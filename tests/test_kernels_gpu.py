@@ -284,6 +284,45 @@ def test_prefill_attention_tc_edges(hq, hkv, d, page, many, monkeypatch):
     assert sm100.waits_given_up() == 0
 
 
+@pytest.mark.parametrize("family", ["fp8", "attn", "mla"])
+def test_wait_that_gives_up_reaches_the_caller(family):
+    """A wait limit of zero: whatever is not there at the first look is given up. The kernel returns, the engine's check raises,
+    and the next call is right again."""
+    from gllm_b200.model_runner import StepResult
+    from gllm_b200.ops import lib, sm100
+    torch.manual_seed(1)
+    if family == "fp8":
+        x, w = torch.randn(300, 1024, device=_dev()).bfloat16(), torch.randn(512, 1024, device=_dev()).to(torch.float8_e4m3fn)
+        ws = torch.ones(4, 8, device=_dev())
+        call = lambda: sm100.linear_fp8_block(x, w, ws)
+        want = x.float() @ w.float().t()
+    elif family == "attn":
+        lens = [300, 129]
+        a = _make_paged(lens, lens, 8, 2, 128, 16, _dev(), seed=1)
+        call = lambda: sm100.paged_attention(*a, 128 ** -0.5, 8, 128, 0, 2, 300, 300)
+        want = ref.paged_attention(*a, 128 ** -0.5, 8, 128)
+    else:
+        cache = (torch.randn(500, 1, 9, 16, 64, device=_dev()) * 0.5).bfloat16()
+        bt = torch.arange(500, dtype=torch.int32, device=_dev()).view(4, 125)
+        q = (torch.randn(64, 16, 576, device=_dev()) * 0.3).bfloat16()       # shares of 14 tiles: copies are waited for
+        pos, seq = torch.full((64,), 1999, dtype=torch.int32, device=_dev()), torch.arange(64, device=_dev()).int() % 4
+        call = lambda: sm100.mla_attention(q, cache, bt, seq, pos, 192 ** -0.5)
+        want = _mla_ref(q, cache, bt, seq, pos, 192 ** -0.5)
+    assert _rel_err(call(), want) < 5e-2 and sm100.waits_given_up() == 0
+    done = StepResult(tokens=torch.zeros(1, dtype=torch.int32), num_emit=1)
+    try:
+        lib.watch_waits(limit_ns=0)
+        call()
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="bounded wait"):
+            done.tokens_list()
+    finally:
+        lib.watch_waits()
+        lib.waits_gave_up(clear=True)
+    assert _rel_err(call(), want) < 5e-2 and sm100.waits_given_up() == 0
+    assert done.tokens_list() == [0]
+
+
 def test_sampler_greedy_and_filter():
     from gllm_b200.ops import sm100
     torch.manual_seed(6)
