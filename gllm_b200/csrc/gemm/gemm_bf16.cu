@@ -50,7 +50,7 @@ struct GemmParams {
   // grouped (MoE) mode: M tile t multiplies the weight slab of expert tile_expert[t]
   const int32_t* tile_expert;
   const int32_t* num_m_tiles_ptr;  // device scalar: number of live M tiles
-  int moe_experts;                 // > 0: num_m_tiles_ptr points to moe_align's whole block (counts and offsets of that many experts)
+  int moe_experts;                 // MOE: num_m_tiles_ptr points to moe_align's whole block (counts and offsets of that many experts)
   int n_per_expert;
   // per-row destination table (EP combine push): row r of C is stored at row_dest[r] (any rank's memory
   // mapped over NVLink); 0 = padding row, not stored. comm/ep_a2a.cu builds the table.
@@ -89,11 +89,18 @@ struct GemmCfg {
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align*/ + 256 + kEpiBytes;
 };
 
-template <int BN, int EPI>
+// what only expert tiles need (a template flag: in the dense kernel the map alone cost 1 % of a 64-row feed-forward)
+template <bool MOE>
+struct MoeMaps {};
+template <>
+struct MoeMaps<true> {
+  CUtensorMap a16;               // A in boxes of 16 rows
+};
+
+template <int BN, int EPI, bool MOE>
 __global__ void __launch_bounds__(kNumThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                 const __grid_constant__ CUtensorMap tmap_a16,   // A in boxes of 16 rows (grouped mode with moe_experts)
-                 const GemmParams p) {
+                 const __grid_constant__ MoeMaps<MOE> moe, const GemmParams p) {
   using Cfg = GemmCfg<BN>;
   constexpr int S = Cfg::kStages;
 
@@ -120,7 +127,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   // 64) and stored, what the rest of the tile holds is multiplied and dropped. 48 tokens x 8 of 128 experts (2048 -> 2 x 768
   // -> 2048): first product 152 -> 102 us, second 65 -> 55 us.
   auto tile_rows = [&](int mt) {
-    if (p.moe_experts <= 0) return kBlockM;
+    if (!MOE) return kBlockM;
     const int e = p.tile_expert[mt];
     const int end = p.num_m_tiles_ptr[2 + 2 * p.moe_experts + e] + p.num_m_tiles_ptr[2 + e];
     return min(kBlockM, end - mt * kBlockM);
@@ -198,7 +205,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           while (static_cast<int32_t>(ld_acquire_sys(p.a_ready + mt) - want) < 0) guard.poll();
           asm volatile("fence.proxy.async;" ::: "memory");
         }
-        const int boxes = (tile_rows(mt) + 15) / 16;
+        const int boxes = MOE ? (tile_rows(mt) + 15) / 16 : 0;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % S;
           const uint32_t ph = (it / S) & 1;
@@ -209,12 +216,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             continue;
           }
           mbar_wait(&empty_bar[s], ph ^ 1);
-          if (boxes <= 4) {
-            mbar_expect_tx(&full_bar[s], Cfg::kStageBytes - Cfg::kABytes + boxes * (16 * kBlockK * 2));
-            tma_load_2d(sb, &tmap_b, &full_bar[s], kb * kBlockK, n0 + b_row_off, kEvictNormal);
-            for (int i = 0; i < boxes; ++i)
-              tma_load_2d(sa + i * (16 * kBlockK * 2), &tmap_a16, &full_bar[s], kb * kBlockK, m0 + i * 16, kEvictNormal);
-            continue;
+          if constexpr (MOE) {
+            if (boxes <= 4) {
+              mbar_expect_tx(&full_bar[s], Cfg::kStageBytes - Cfg::kABytes + boxes * (16 * kBlockK * 2));
+              tma_load_2d(sb, &tmap_b, &full_bar[s], kb * kBlockK, n0 + b_row_off, kEvictNormal);
+              for (int i = 0; i < boxes; ++i)
+                tma_load_2d(sa + i * (16 * kBlockK * 2), &moe.a16, &full_bar[s], kb * kBlockK, m0 + i * 16, kEvictNormal);
+              continue;
+            }
           }
           mbar_expect_tx(&full_bar[s], Cfg::kStageBytes);
           if (p.batch > 0) tma_load_3d(sa, &tmap_a, &full_bar[s], kb * kBlockK, (mt - bidx * tpb) * kBlockM, bidx);
@@ -279,7 +288,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         row_in = row < p.rows_per_batch;
         c_off = static_cast<int64_t>(bidx) * p.c_batch_stride;
       }
-      if (p.moe_experts > 0) row_in = row_in && q * 32 + lane < tile_rows(m0 / kBlockM);
+      if (MOE) row_in = row_in && q * 32 + lane < tile_rows(m0 / kBlockM);
       const uint32_t t_row = tmem_base + buf * BN + (static_cast<uint32_t>(q * 32) << 16);
 
       // destination row pointer (local C, or the owner rank's staging buffer for RS)
@@ -506,12 +515,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   }
 }
 
-template <int BN, int EPI>
+template <int BN, int EPI, bool MOE = false>
 static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
-                       cudaStream_t stream, const CUtensorMap* ta16 = nullptr) {
+                       cudaStream_t stream, const MoeMaps<MOE>& moe = {}) {
   using Cfg = GemmCfg<BN>;
   static PerDeviceOnce configured;
-  auto kern = gemm_bf16_kernel<BN, EPI>;
+  auto kern = gemm_bf16_kernel<BN, EPI, MOE>;
   if (configured.need()) {
     CUDA_CHECK_RET(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         Cfg::kSmemBytes));
@@ -523,8 +532,7 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
   const int tiles = num_m * num_n * split;
   const int sms = (num_sms() / split) * split;  // split-K slices of a tile must run in the same round
   const int grid = tiles < sms ? tiles : sms;
-  CUDA_CHECK_RET(launch_pdl(kern, dim3(grid), dim3(kNumThreads), Cfg::kSmemBytes, stream, ta, tb,
-                            ta16 != nullptr ? *ta16 : ta, p));
+  CUDA_CHECK_RET(launch_pdl(kern, dim3(grid), dim3(kNumThreads), Cfg::kSmemBytes, stream, ta, tb, moe, p));
   return 0;
 }
 
@@ -786,10 +794,11 @@ static int moe_grouped_gemm_impl(const void* A, int64_t lda, const void* W, void
   if (max_tiles <= 0) return 0;
   if ((K % 8) != 0 || (N % 8) != 0 || (lda % 8) != 0 || (ldc % 8) != 0) return 1;
   const int bn = 128;  // 64|64 gate/up interleave for the SiLU epilogue; good balance for expert tiles
-  CUtensorMap ta, tb, ta16;
+  CUtensorMap ta, tb;
+  MoeMaps<true> moe;
   const int M = max_tiles * kBlockM;
   if (make_tmap_2d(&ta, A, M, K, lda * 2, kBlockM, kBlockK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)) return 1;
-  if (make_tmap_2d(&ta16, A, M, K, lda * 2, 16, kBlockK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)) return 1;
+  if (make_tmap_2d(&moe.a16, A, M, K, lda * 2, 16, kBlockK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)) return 1;
   if (make_tmap_2d(&tb, W, static_cast<uint64_t>(E) * N, K, static_cast<uint64_t>(K) * 2, bn, kBlockK,
                    CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)) return 1;
   GemmParams p;
@@ -806,8 +815,8 @@ static int moe_grouped_gemm_impl(const void* A, int64_t lda, const void* W, void
   p.glu_alpha = glu_alpha;
   p.act = act;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  return epi == kEpiSiluMul ? launch_gemm<128, kEpiSiluMul>(ta, tb, p, st, &ta16)
-                            : launch_gemm<128, kEpiStore>(ta, tb, p, st, &ta16);
+  return epi == kEpiSiluMul ? launch_gemm<128, kEpiSiluMul, true>(ta, tb, p, st, moe)
+                            : launch_gemm<128, kEpiStore, true>(ta, tb, p, st, moe);
 }
 
 GLLM_EXPORT int gllm_moe_grouped_gemm(const void* A, int64_t lda, const void* W, void* C, int64_t ldc,
