@@ -248,8 +248,8 @@ _SCAN_WORK_BYTES = 256 << 20        # its workspace at a time; more channels tak
 
 def selective_scan(xc, dt_raw, proj, xz, a, d_skip, dt_bias, ssm_state, rec_slots, seq_lens, query_start_loc,
                    channels, nstate, dt_rank, max_q_len: Optional[int] = None):
-    """With `max_q_len` (the longest portion of the batch), portions of `_SCAN_MIN_TOKENS` tokens and more run cut in time;
-    the length of a sequence's own portion decides, not what else is in the batch."""
+    """With `max_q_len` (the longest portion of the batch, or a bound on it), portions of `_SCAN_MIN_TOKENS` tokens and more run
+    cut in time; the length of a sequence's own portion decides, not what else is in the batch."""
     assert xc.is_contiguous() and dt_raw.is_contiguous() and proj.stride(1) == 1 and xz.stride(1) == 1
     assert a.dtype == torch.float32 and a.is_contiguous()
     out = torch.empty_like(xc)
@@ -265,7 +265,7 @@ def selective_scan(xc, dt_raw, proj, xz, a, d_skip, dt_bias, ssm_state, rec_slot
         if rc != 2:                          # 2: more states than a thread holds
             check(rc, "scan_chunk")
             sm100._count(3 * -(-channels // width))
-            if seq_lens.shape[0] == 1:
+            if seq_lens.shape[0] == 1 and t >= _SCAN_MIN_TOKENS:      # all rows are the one sequence's
                 return out
             max_len = _SCAN_MIN_TOKENS - 1
     # long chunks of few sequences: 4 threads per channel (more warps in flight); decode-like batches: 1
@@ -358,8 +358,8 @@ def linear_state_scan(q, k, v, beta, a, neg_a, dt_bias, decay, state, rec_slots,
                       qk_heads, dim, v_dim, silu_in, unit_qk, q_scale, delta, zk=None, zk_bias=None, inv_tau=1.0,
                       step=False, d_skip=None, out=None, max_q_len: Optional[int] = None):
     """`step`: the softplus behind the decay is also the write strength; `d_skip` [heads] fp32: o += d_skip v.
-    With `max_q_len` (the longest portion of the batch), the delta rule runs in the chunked form on portions of
-    `_DELTA_MIN_TOKENS` tokens and more; the length of a sequence's own portion decides, not what else is in the batch."""
+    With `max_q_len` (the longest portion of the batch, or a bound on it), the delta rule runs in the chunked form on portions
+    of `_DELTA_MIN_TOKENS` tokens and more; the length of a sequence's own portion decides, not what else is in the batch."""
     t = q.shape[0]
     for x in (q, k, v, beta, a, zk):
         assert x is None or (x.stride(1) == 1 and x.dtype == q.dtype)
@@ -384,7 +384,7 @@ def linear_state_scan(q, k, v, beta, a, neg_a, dt_bias, decay, state, rec_slots,
             not step and d_skip is None and q.dtype == torch.bfloat16 and _delta_chunked(
                 q, k, v, beta, a, neg_a, dt_bias, state, rec_slots, seq_lens, query_start_loc, heads, qk_heads, dim, v_dim,
                 unit_qk, q_scale, out):
-        if nseq == 1:
+        if nseq == 1 and t >= _DELTA_MIN_TOKENS:                      # all rows are the one sequence's
             return out
         max_len = _DELTA_MIN_TOKENS - 1
     blocks = nseq * heads * ((v_dim + 31) // 32)

@@ -383,3 +383,23 @@ def test_chunked_delta_rule(H, G, D, V, lens, ctx, decay):
         err[name] = [float((x.double().cpu() - e).norm() / e.norm()) for x, e in ((o, exact[0]), (st, exact[1]))]
     for c, s in zip(err["chunk"], err["serial"]):
         assert c <= max(1.2 * s, 2e-6), err
+
+
+@pytest.mark.parametrize("lens", [[5], [20], [40], [5, 40]])
+def test_delta_rule_with_a_bound_on_the_lengths(lens):
+    """`max_q_len` may be larger than every portion: each portion is computed, by the kernel that its own length asks for."""
+    from gllm_b200.ops import sm100_seq as S
+    torch.manual_seed(lens[0])
+    dev, t, n, H, D, V = "cuda", sum(lens), len(lens), 2, 128, 64
+    q, k, v = (torch.randn(t, H * w, device=dev).bfloat16() for w in (D, D, V))
+    beta, a = (torch.randn(t, H, device=dev).bfloat16() for _ in range(2))
+    neg_a, dt_bias = -torch.rand(H, device=dev), torch.zeros(H, device=dev)
+    qsl = torch.tensor([0] + lens, device=dev).cumsum(0).to(torch.int32)
+    sl, rs = torch.tensor(lens, device=dev, dtype=torch.int32), torch.arange(n, device=dev, dtype=torch.int32)
+    got = []
+    for bound in (max(lens), 1000):
+        st = torch.zeros(n, H, D, V, device=dev)
+        torch.full((t, H * V), 3.0, device=dev)              # what an unwritten output is likely to hold
+        got.append((S.linear_state_scan(q, k, v, beta, a, neg_a, dt_bias, None, st, rs, sl, qsl, H, H, D, V, False, True, 1.0,
+                                        True, max_q_len=bound), st))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and bool(got[0][1].abs().sum() > 0)

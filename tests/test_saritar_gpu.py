@@ -238,3 +238,22 @@ def test_scan_cut_in_time(N, C, qlens, ctx):
         err.append([float((g.double().cpu() - e).norm() / e.norm()) for g, e in ((y, want), (st, ends))])
     for cut, serial in zip(*err):
         assert cut <= max(1.2 * serial, 1e-6), err
+
+
+@pytest.mark.parametrize("lens", [[5], [100], [130], [100, 130]])
+def test_scan_with_a_bound_on_the_lengths(lens):
+    """`max_q_len` may be larger than every portion: each portion is computed, by the kernel that its own length asks for."""
+    from gllm_b200.ops import sm100_seq as S
+    torch.manual_seed(lens[0])
+    N, C, R, t, n = 8, 70, 4, sum(lens), len(lens)
+    qsl = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    sl, rs = torch.tensor(lens, dtype=torch.int32, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV)
+    x, dtr, xz = (torch.randn(t, w, device=DEV).bfloat16() for w in (C, C, 2 * C))
+    proj = torch.randn(t, R + 2 * N, device=DEV).bfloat16()
+    A, Dk, db = -torch.rand(C, N, device=DEV) * 4, torch.randn(C, device=DEV), torch.full((C,), -3.0, device=DEV)
+    got = []
+    for bound in (max(lens), 1000):
+        st = torch.zeros(n, N, C, device=DEV)
+        torch.full((t, C), 3.0, device=DEV).bfloat16()       # what an unwritten output is likely to hold
+        got.append((S.selective_scan(x, dtr, proj, xz, A, Dk, db, st, rs, sl, qsl, C, N, R, max_q_len=bound), st))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and bool(got[0][1].abs().sum() > 0)
