@@ -12,6 +12,11 @@
 // their products are exact; fp32 operands (S, B, T, U, P) are split into three bf16 parts, which hold all 24 bits: three
 // products against an exact operand, the six that matter between two split ones.
 //
+// Values that are no numbers: a product with a zero above the diagonal would carry a token's NaN or infinity to the tokens before
+// it in its 16-row tile. Rows of B and U enter the products with zeros in such places; the place of the first one in each
+// column is kept, and the column's results from that token on, and its state, are set to NaN. The token-serial kernel has NaN
+// or an infinity there.
+//
 // What bounds it: the chain of chunks of a sequence; per chunk some 3200 mma.sync, the splits and three block barriers.
 // 4 x 1500 tokens, 32 heads of 128 x 128: 437 us, token-serial 3943 us; 1 x 6000 tokens, 8 heads of 128 x 256: 680 / 7352 us
 // (B200). The whole mixer on 6000 ragged tokens at width 4096: 7171 -> 1310 us.
@@ -97,7 +102,9 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(
       const double up = __shfl_up_sync(0xffffffffu, run, o);
       if (lane >= o) run += up;
     }
-    const double l1 = run, l0 = run - (double)a1;
+    // not run - a1: a decay that is no number stays out of the token before it
+    const double up = __shfl_up_sync(0xffffffffu, run, 1);
+    const double l1 = run, l0 = (lane > 0 ? up : 0.0) + (double)a0;
     sLh[2 * lane] = (float)l0;
     sLl[2 * lane] = (float)(l0 - (double)(float)l0);
     sLh[2 * lane + 1] = (float)l1;
@@ -222,9 +229,9 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 8
     for (int s = 0; s < 32; ++s) {
-      const float tv = sT[(32 + xi) * LA + 32 + s];
+      const float tv = sT[(32 + xi) * LA + 32 + s];      // zero for s > xi, and sX[s] may be no number there
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] = fmaf(-tv, sX[s * LX + xj + e], acc[e]);
+      for (int e = 0; e < 8; ++e) acc[e] = s <= xi ? fmaf(-tv, sX[s * LX + xj + e], acc[e]) : acc[e];
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) sT[(32 + xi) * LA + xj + e] = acc[e];
@@ -284,6 +291,7 @@ __global__ void __launch_bounds__(256, 1) delta_chunk_kernel(
   extern __shared__ __align__(16) uint8_t smem_raw[];
   bf16_t* sm = reinterpret_cast<bf16_t*>(smem_raw);
   bf16_t *sS = sm + SM::S, *sB = sm + SM::B, *sU = sm + SM::U, *sW = sm + SM::W;
+  __shared__ int s_bad[VT];                         // first token of the chunk whose B or U is no number, per column
   constexpr int kPS = NP * LV, kPT = kC * LV;       // one part of S, of a token operand
 
   const int h = h0 + blockIdx.x, v0 = blockIdx.y * VT, s = blockIdx.z;
@@ -339,6 +347,7 @@ __global__ void __launch_bounds__(256, 1) delta_chunk_kernel(
     }
     asm volatile("cp.async.commit_group;");
   };
+  if (threadIdx.x < VT) s_bad[threadIdx.x] = kC;    // visible to all after the first barrier of the loop
   put_state();
   fetch(q0, 0);
   const uint32_t* unit = work + ((size_t)chunk_base(qsl, s) * gridDim.x + blockIdx.x) * kUnit;
@@ -381,6 +390,13 @@ __global__ void __launch_bounds__(256, 1) delta_chunk_kernel(
           mma16816(qs_[nv + 1], aq, r[2], r[3]);
         }
     }
+    bool bad = false;
+    auto number = [&](float x, int row, int col) {
+      if (fabsf(x) <= 3.402823466e38f) return x;
+      bad = true;
+      atomicMin(&s_bad[col], row);
+      return 0.f;
+    };
     auto put_rows = [&](bf16_t* dst, int i, int row, float x, float y) {
       uint32_t hi, mid, lo;
       split3(x, y, hi, mid, lo);
@@ -396,7 +412,9 @@ __global__ void __launch_bounds__(256, 1) delta_chunk_kernel(
         const int row = r ? tb : ta;
         const float bk = r ? wb.x : wa.x, be = r ? wb.y : wa.y;
         const float2 vv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sV + row * LV + (cb + i) * 8 + 2 * t4));
-        put_rows(sB, i, row, be * vv.x - bk * ks_[i][2 * r], be * vv.y - bk * ks_[i][2 * r + 1]);
+        const int col = (cb + i) * 8 + 2 * t4;
+        put_rows(sB, i, row, number(be * vv.x - bk * ks_[i][2 * r], row, col),
+                 number(be * vv.y - bk * ks_[i][2 * r + 1], row, col + 1));
       }
     __syncthreads();                                // B is complete
     uint4 P[4][3];
@@ -433,10 +451,12 @@ __global__ void __launch_bounds__(256, 1) delta_chunk_kernel(
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const float w = r ? wb.w : wa.w;
-        put_rows(sU, i, r ? tb : ta, acc[i][2 * r], acc[i][2 * r + 1]);
-        put_rows(sW, i, r ? tb : ta, w * acc[i][2 * r], w * acc[i][2 * r + 1]);
+        const int row = r ? tb : ta, col = (cb + i) * 8 + 2 * t4;
+        const float ux = number(acc[i][2 * r], row, col), uy = number(acc[i][2 * r + 1], row, col + 1);
+        put_rows(sU, i, row, ux, uy);
+        put_rows(sW, i, row, w * ux, w * uy);
       }
-    __syncthreads();                                // U is complete
+    const bool dirty = __syncthreads_or(bad);       // U is complete
     // ---- o = exp(L) Q S + P U
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -444,6 +464,13 @@ __global__ void __launch_bounds__(256, 1) delta_chunk_kernel(
       acc[i][2] = wb.z * qs_[i][2]; acc[i][3] = wb.z * qs_[i][3];
     }
     tri(P, sU);
+    if (dirty) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if ((e < 2 ? ta : tb) >= s_bad[(cb + i) * 8 + 2 * t4 + (e & 1)]) acc[i][e] = __int_as_float(0x7fffffff);
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -471,6 +498,13 @@ __global__ void __launch_bounds__(256, 1) delta_chunk_kernel(
           mma16816(S[ni], ak, r[0], r[1]);
           mma16816(S[ni + 1], ak, r[2], r[3]);
         }
+    }
+    if (dirty) {
+#pragma unroll
+      for (int ni = 0; ni < NI; ++ni)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (s_bad[(wn * NI + ni) * 8 + 2 * t4 + (e & 1)] < kC) S[ni][e] = __int_as_float(0x7fffffff);
     }
     put_state();
   }

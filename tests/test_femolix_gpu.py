@@ -403,3 +403,35 @@ def test_delta_rule_with_a_bound_on_the_lengths(lens):
         got.append((S.linear_state_scan(q, k, v, beta, a, neg_a, dt_bias, None, st, rs, sl, qsl, H, H, D, V, False, True, 1.0,
                                         True, max_q_len=bound), st))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and bool(got[0][1].abs().sum() > 0)
+
+
+@pytest.mark.parametrize("what", ["v", "k", "q", "beta", "a"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("at", [0, 13, 30, 47, 70, 127])
+def test_chunked_delta_rule_keeps_earlier_tokens_clean(what, value, at):
+    """One element that is no number: the chunked form is finite exactly where the token-serial one is (the tokens before it, and
+    for a value the other columns), with the same results there, and the state alike."""
+    from gllm_b200.ops import sm100_seq as S
+    torch.manual_seed(at)
+    dev, H, D, V, lens = "cuda", 2, 128, 72, [40, 150, 35]
+    t, n = sum(lens), len(lens)
+    x = {"q": torch.randn(t, H * D), "k": torch.randn(t, H * D), "v": torch.randn(t, H * V), "beta": torch.randn(t, H),
+         "a": torch.randn(t, H)}
+    row = lens[0] + at                                       # in the middle sequence
+    x[what][row, H - 1 if what in ("beta", "a") else 5] = value
+    x = {name: y.to(dev).bfloat16() for name, y in x.items()}
+    neg_a, dt_bias = -torch.rand(H, device=dev) * 0.2, torch.zeros(H, device=dev)
+    qsl = torch.tensor([0] + lens, device=dev).cumsum(0).to(torch.int32)
+    sl, rs = torch.tensor([45, 150, 35], device=dev, dtype=torch.int32), torch.arange(n, device=dev, dtype=torch.int32)
+    st0, got = torch.randn(n, H, D, V, device=dev), []
+    for mx in (max(lens), None):
+        st = st0.clone()
+        got.append((S.linear_state_scan(x["q"], x["k"], x["v"], x["beta"], x["a"], neg_a, dt_bias, None, st, rs, sl, qsl, H, H,
+                                        D, V, False, True, D ** -0.5, True, max_q_len=mx), st))
+    for c, s in zip(*got):
+        fin = torch.isfinite(s)
+        assert torch.equal(torch.isfinite(c), fin)
+        zero = torch.zeros_like(s)
+        a, b = torch.where(fin, c, zero), torch.where(fin, s, zero)
+        assert float((a - b).norm()) <= 2e-5 * float(b.norm())      # sums of some 150 tokens in fp32, in another order
+    assert bool(torch.isfinite(got[0][0][:row]).all())
