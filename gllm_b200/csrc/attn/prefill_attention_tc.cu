@@ -293,13 +293,22 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
           for (int kk = 0; kk < 4; ++kk) umma_bf16<1>(d_tmem, da + kk * 2, db + kk * 2, idesc_s, (kd | kk) != 0);
         }
       };
+      // Only the 16-key steps that some row of the query tile sees: a masked key has P = 0, but 0 times a value that is no
+      // number is none either, so keys behind the tile's last token (or before its window) stay out of the product.
+      uint32_t in_o = 0;                                   // bit t: O of query tile t has been written
       auto issue_pv = [&](int t, int tile) {
+        const int tok0 = tok_cta + t * toks_per_tile, key0 = (tile0 + tile) * KV;
+        const int end = ctx_len + min(tok0 + toks_per_tile, q_len) - key0;
+        const int low = p.window > 0 ? ctx_len + tok0 - p.window + 1 - key0 : 0;
         const uint32_t v_addr = smem_u32(smem + SM::kVOff + (tile % SM::kVStages) * SM::kVBytes);
         const uint64_t dv = make_sw128_desc(v_addr, (KV * 128) >> 4, 1024 >> 4);
 #pragma unroll
-        for (int kk = 0; kk < KV / 16; ++kk)             // 16 keys per step: 8 columns of P, 16 rows of V
+        for (int kk = 0; kk < KV / 16; ++kk) {           // 16 keys per step: 8 columns of P, 16 rows of V
+          if (kk * 16 >= end || kk * 16 + 15 < low) continue;
           umma_bf16_ts(tmem + SM::kTmemO + t * DV, tmem + t * KV + kk * 8, dv + static_cast<uint64_t>(kk) * (2048 >> 4), idesc_pv,
-                       (tile | kk) != 0);
+                       (in_o >> t) & 1u);
+          in_o |= 1u << t;
+        }
       };
       bool ok = n_max > 0;
       for (int t = 0; t < 2; ++t)

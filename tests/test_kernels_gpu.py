@@ -284,6 +284,25 @@ def test_prefill_attention_tc_edges(hq, hkv, d, page, many, monkeypatch):
     assert sm100.waits_given_up() == 0
 
 
+@pytest.mark.parametrize("window,bad,clean", [(None, 180, (40, 168)), (100, 60, (168, 340))])
+@pytest.mark.parametrize("seqs", [1, 12])                   # one query tile per CTA, or two
+def test_prefill_value_that_is_no_number(window, bad, clean, seqs):
+    """A NaN in one cached value row reaches only query tiles of 128 rows that see a key of its 16-key step: not the tile whose
+    last token (168 - 1) lies before that step, nor one whose window (from 168 - 99 on) starts behind it."""
+    from gllm_b200.ops import sm100_seq as S
+    h, d, page, ctx, n = 4, 128, 16, 40, 300
+    q, kc, vc, bt, sl, qsl = _make_paged([ctx + n] * seqs, [n] * seqs, h, h, d, page, _dev(), seed=2)
+    pos = torch.arange(ctx, ctx + n, dtype=torch.int32, device=_dev()).repeat(seqs)
+    want = ref.window_attention(q, kc, vc, bt, sl, qsl, d ** -0.5, h, d, window, None)
+    for i in range(seqs):
+        vc[bt[i, bad // page].long(), :, :, bad % page] = float("nan")
+    got = S.window_attention(q, kc, vc, bt, sl, qsl, pos, d ** -0.5, h, d, window, None, 0, n)
+    ok = (pos >= clean[0]) & (pos < clean[1])
+    assert _rel_err(got[ok], want[ok]) < 1e-2
+    sees = (pos >= bad) & (pos < (bad + window if window else ctx + n))
+    assert bool(torch.isnan(got[sees]).all())
+
+
 @pytest.mark.parametrize("family", ["fp8", "attn", "mla"])
 def test_wait_that_gives_up_reaches_the_caller(family):
     """A wait limit of zero: whatever is not there at the first look is given up. The kernel returns, the engine's check raises,
