@@ -181,7 +181,9 @@ class ModelRunner:
         else:
             torch.cuda.empty_cache()
             free, _ = torch.cuda.mem_get_info(self.device)
-            num = int((free // max(per_page, 1)) * cfg.gpu_memory_util)
+            # what the layers allocate beside the cache, and the probe, which runs without one, has not seen
+            free -= getattr(self.model, "step_scratch_bytes", lambda max_len: 0)(self.model_max_length)
+            num = int((max(free, 0) // max(per_page, 1)) * cfg.gpu_memory_util)
         if ps.get_world_size() > 1 and torch.distributed.is_initialized():
             all_n = [None] * ps.get_world_size()
             torch.distributed.all_gather_object(all_n, num)

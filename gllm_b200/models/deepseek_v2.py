@@ -11,8 +11,8 @@ On sm_100a the attention runs in the *absorbed* form: q_nope·W_UK per head (bat
 views, written straight into the 576-wide query), fused RoPE + latent-cache write, split-KV multi-query attention
 over the paged latent cache (csrc/attn/mla_attention.cu), then out_lat·W_UV per head (the same batched GEMM,
 written in the [T, heads·v] layout o_proj reads). No cuBLAS and no host synchronisation on that path, so decode
-batches run inside CUDA graphs. Prompt portions of 32 tokens and more (on average) take the
-*expanded* form instead: the cached latents are gathered, one GEMM makes every head's keys and values, and the tcgen05
+batches run inside CUDA graphs. Prompt portions of 32 tokens and more take the
+*expanded* form instead: the cached latents are gathered, a GEMM makes every head's keys and values, and the tcgen05
 prefill attention runs on them. The CPU / odd-shape path below evaluates the expanded form with PyTorch ops per sequence
 (the numerical oracle of the GPU path).
 """
@@ -143,23 +143,46 @@ class MLAAttention(nn.Module):
 
     # Expanded heads cost a GEMM of 2 * 256 * 512 operations per cached row and head, and then 640 per (query, key) pair
     # instead of 2176 on a kernel eight times as fast: they win from some twenty new tokens per sequence on; below that a portion
-    # is a few rows of one 128-row tile. 5 prompts of 4096 tokens together, 16 heads: 2459 -> 479 us. Their keys and values stay
-    # below this many bytes.
+    # is a few rows of one 128-row tile. 5 prompts of 4096 tokens together, 16 heads: 2459 -> 479 us. A sequence's own portion
+    # decides. What a call holds at a time is bounded: the gathered latents (more sequences take another round) and the keys
+    # and values of as many heads as fit.
     _EXPAND_MIN_TOKENS = 32
-    _EXPAND_MAX_BYTES = 1 << 30
+    _EXPAND_KV_BYTES = 1 << 30
+    _EXPAND_LATENT_BYTES = 256 << 20
+    _LATENT_ROW_BYTES = 576 * 2
 
-    def _expanded_rows(self, inp) -> int:
-        """Rows of latents to expand for this batch's prompt portions (each sequence rounded up to 64), or 0: attend in
-        the absorbed form."""
+    def _expands(self) -> bool:
+        return (self.kv_lora, self.rope_dim, self.nope, self.v_dim) == (512, 64, 128, 128)
+
+    def expand_scratch_bytes(self, max_len: int) -> int:
+        """What the expanded form allocates beside the cache at most, for sequences of up to `max_len` tokens."""
+        if not self._expands():
+            return 0
+        return self._EXPAND_KV_BYTES + max(self._EXPAND_LATENT_BYTES, (max_len + 63) // 64 * 64 * self._LATENT_ROW_BYTES)
+
+    def _expanded_plan(self, inp):
+        """(rounds, rest) of this batch. rounds: (first sequence, end, rows of latents) of the prompt portions to expand, each
+        sequence rounded up to 64 rows; empty: all attend in the absorbed form. rest: None if the rows in the absorbed form are
+        the leading ones of the decoding sequences, else (their rows, their sequences)."""
         n0, b = inp.num_decode_seqs, getattr(inp, "batch", None)
-        if b is None or inp.padded_tokens or n0 == inp.num_seqs or (self.nope, self.v_dim) != (128, 128):
-            return 0
-        seq_lens = b.seq_lens[n0:inp.num_seqs].astype(np.int64)
-        new = int(b.query_start_loc[inp.num_seqs]) - int(b.query_start_loc[n0])
-        rows = int(((seq_lens + 63) // 64 * 64).sum())
-        if new < self._EXPAND_MIN_TOKENS * len(seq_lens) or rows * self.num_heads * 512 > self._EXPAND_MAX_BYTES:
-            return 0
-        return rows
+        if b is None or inp.padded_tokens or n0 == inp.num_seqs or not self._expands():
+            return [], None
+        q_lens = np.diff(b.query_start_loc[:inp.num_seqs + 1].astype(np.int64))
+        expand = q_lens >= self._EXPAND_MIN_TOKENS
+        expand[:n0] = False
+        rows = np.where(expand, (b.seq_lens[:inp.num_seqs].astype(np.int64) + 63) // 64 * 64, 0)
+        rounds, first, held = [], n0, 0
+        for s in range(n0, inp.num_seqs):
+            if held and (held + int(rows[s])) * self._LATENT_ROW_BYTES > self._EXPAND_LATENT_BYTES:
+                rounds.append((first, s, held))
+                first, held = s, 0
+            held += int(rows[s])
+        if held:
+            rounds.append((first, inp.num_seqs, held))
+        if not rounds or expand[n0:].all():
+            return rounds, None
+        keep = ~np.repeat(expand, q_lens)
+        return rounds, (np.flatnonzero(keep), np.repeat(np.arange(inp.num_seqs), q_lens)[keep])
 
     def _forward_absorbed(self, inp, q, kv_c, k_pe, cache):
         """sm_100a path: multi-query attention over the latent cache (csrc/attn/mla_attention.cu) for decoding sequences and
@@ -168,23 +191,37 @@ class MLAAttention(nn.Module):
         from gllm_b200.ops import sm100
         t, hl = q.shape[0], self.num_heads
         out = torch.empty(t, hl, self.v_dim, dtype=q.dtype, device=q.device)
-        rows = self._expanded_rows(inp)
-        n = inp.num_decode_seqs if rows else t           # leading rows in the absorbed form
+        rounds, rest = self._expanded_plan(inp)
+        n = inp.num_decode_seqs if rounds else t         # leading rows in the absorbed form
         pos = inp.positions if inp.positions.dim() == 1 else inp.positions[0]
-        if n:
+        if rest is not None:
+            # short portions among long ones: everything is rotated in place, their rows are picked out
+            sm100.mla_rope_cache(q[:, :, self.nope:], None, k_pe, kv_c, self.rope.cos_sin, pos, inp.slot_mapping, cache)
+            rows, seqs = torch.from_numpy(np.stack(rest).astype(np.int32)).to(q.device, non_blocking=True)
+            w_uk, w_uv = self._absorbed_weights()
+            some = q.index_select(0, rows)
+            q_full = torch.empty(len(rest[0]), hl, 576, dtype=q.dtype, device=q.device)
+            sm100.gemm_batched(some[:, :, : self.nope], w_uk, q_full[:, :, :512])
+            q_full[:, :, 512:] = some[:, :, self.nope:]
+            out_lat = sm100.mla_attention(q_full, cache, inp.block_table, seqs, pos.index_select(0, rows), self.scaling)
+            part = torch.empty(len(rest[0]), hl, self.v_dim, dtype=q.dtype, device=q.device)
+            sm100.gemm_batched(out_lat, w_uv, part)
+            out.index_copy_(0, rows.long(), part)
+        elif n:
             w_uk, w_uv = self._absorbed_weights()
             q_full = torch.empty(n, hl, 576, dtype=q.dtype, device=q.device)
             sm100.gemm_batched(q[:n, :, : self.nope], w_uk, q_full[:, :, :512])   # per head: q_nope · W_UK
             sm100.mla_rope_cache(q[:n, :, self.nope:], q_full, k_pe[:n], kv_c[:n], self.rope.cos_sin, pos[:n],
                                  inp.slot_mapping[:n], cache)
-            out_lat = sm100.mla_attention(q_full, cache, inp.block_table, None if rows else inp.tok_seq, pos[:n],
+            out_lat = sm100.mla_attention(q_full, cache, inp.block_table, None if rounds else inp.tok_seq, pos[:n],
                                           self.scaling)
             sm100.gemm_batched(out_lat, w_uv, out[:n])                            # per head: out_lat · W_UV
-        if rows:
+        if rounds and rest is None:
             sm100.mla_rope_cache(q[n:, :, self.nope:], None, k_pe[n:], kv_c[n:], self.rope.cos_sin, pos[n:],
                                  inp.slot_mapping[n:], cache)
-            sm100.mla_expanded_attention(q, cache, inp.block_table, inp.seq_lens, inp.query_start_loc, self.kv_b_w, rows,
-                                         inp.num_decode_seqs, inp.max_q_len, self.scaling, out)
+        for first, end, held in rounds:
+            sm100.mla_expanded_attention(q, cache, inp.block_table, inp.seq_lens, inp.query_start_loc, self.kv_b_w, held, first,
+                                         inp.max_q_len, self.scaling, out, end, self._EXPAND_MIN_TOKENS, self._EXPAND_KV_BYTES)
         return out.view(t, hl * self.v_dim)
 
 
@@ -249,6 +286,10 @@ class DeepseekForCausalLM(CausalLM):
 
     @property
     def head_dim(self): return self.kv_latent_dim
+
+    def step_scratch_bytes(self, max_len: int) -> int:
+        """What a step allocates beside the cache that the memory probe, which runs without one, does not see."""
+        return max((L.attn.expand_scratch_bytes(max_len) for L in self.layers), default=0)
 
     def _load_attention(self, reader, pre, nm, at: MLAAttention):
         tp, tr = self.tp_size, self.tp_rank

@@ -367,6 +367,40 @@ def test_incremental_decode_batch_equals_full_rebuild():
             s.token_ids.append(int(rng.integers(3, 200)))
 
 
+@pytest.mark.parametrize("decodes", [0, 2])
+@pytest.mark.parametrize("q_lens,ctx", [([40, 32, 500], [0, 7, 64]), ([31, 40], [900, 0]), ([40, 5, 32, 31, 64], [0, 1, 2, 3, 4000]),
+                                        ([3, 31], [9, 9])])
+def test_latent_attention_chooses_per_sequence(decodes, q_lens, ctx):
+    """Portions of 32 tokens and more are expanded whatever is beside them, in rounds whose latents stay below the limit (one
+    sequence at least); every other row is attended once in the absorbed form, by its own sequence."""
+    from types import SimpleNamespace
+    from gllm_b200.models.deepseek_v2 import MLAAttention
+    q, c = np.array([1] * decodes + q_lens), np.array([30] * decodes + ctx)
+    n, qsl, lens = len(q), np.concatenate([[0], np.cumsum(q)]).astype(np.int32), (q + c).astype(np.int32)
+    batch = SimpleNamespace(query_start_loc=qsl, seq_lens=lens)
+    inp = SimpleNamespace(num_decode_seqs=decodes, num_seqs=n, padded_tokens=0, batch=batch)
+    att = SimpleNamespace(kv_lora=512, rope_dim=64, nope=128, v_dim=128, _EXPAND_MIN_TOKENS=32, _LATENT_ROW_BYTES=1152,
+                          _expands=lambda: True)
+    long = [s for s in range(decodes, n) if q[s] >= 32]
+    rows = {s: -(-int(lens[s]) // 64) * 64 for s in long}
+    for limit in (1 << 30, 200 * 1152, 1):
+        att._EXPAND_LATENT_BYTES = limit
+        rounds, rest = MLAAttention._expanded_plan(att, inp)
+        seen = []
+        for first, end, held in rounds:
+            mine = [s for s in long if first <= s < end]
+            assert mine and held == sum(rows[s] for s in mine) and (held * 1152 <= limit or len(mine) == 1)
+            seen += mine
+        assert seen == long and [r[0] for r in rounds[1:]] == [r[1] for r in rounds[:-1]]
+        other = [(t, s) for s in range(n) if s not in long for t in range(qsl[s], qsl[s + 1])]
+        if not rounds:
+            assert rest is None                       # all rows, in the absorbed form
+        elif rest is None:
+            assert other == [(t, t) for t in range(decodes)]
+        else:
+            assert other == list(zip(rest[0].tolist(), rest[1].tolist()))
+
+
 def test_a_wait_that_gave_up_stops_the_engine(monkeypatch):
     """The word that a kernel sets when a bounded wait ran out: neither a step's tokens nor the next step get past it."""
     import torch

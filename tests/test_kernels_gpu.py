@@ -2,6 +2,7 @@
 import math
 import os
 
+import numpy as np
 import pytest
 import torch
 
@@ -854,6 +855,58 @@ def test_mla_expanded_attention(heads, page, n_dec):
         s.masked_fill_(torch.arange(n, device=_dev())[None] > torch.arange(n - (b - a), n, device=_dev())[:, None], float("-inf"))
         want[a:b] = torch.einsum("hqk,khd->qhd", s.softmax(-1), kv[..., 128:])
     assert _rel_err(out[n_dec:], want[n_dec:]) < 1.2e-2, _rel_err(out[n_dec:], want[n_dec:])
+
+
+@pytest.mark.parametrize("decodes,q_lens,ctx", [(2, [40, 5, 70, 31], [0, 90, 200, 3]), (0, [31, 33], [65, 1]), (3, [100, 64], [64, 0])])
+@pytest.mark.parametrize("kv_rows,latent_rows", [(1 << 20, 1 << 20), (320 * 3, 1 << 20), (1, 256)])    # heads: all, some, one
+def test_latent_attention_block_mixed_batches(decodes, q_lens, ctx, kv_rows, latent_rows, monkeypatch):
+    """The block on batches of decoding sequences, short and long portions, with limits that make it take rounds of heads and of
+    sequences, against the same block that attends everything in the absorbed form; the cache after it bit for bit. Both round
+    to bf16 at other places; 5 heads, so that a round is cut short."""
+    from types import SimpleNamespace
+    from gllm_b200.layers.rotary import build_rope
+    from gllm_b200.models.decoder import ModelSpec
+    from gllm_b200.models.deepseek_v2 import MLAAttention
+    torch.manual_seed(4)
+    dev, page, heads, width = _dev(), 16, 5, 256
+    spec = ModelSpec(arch="DeepseekV3ForCausalLM", hidden_size=width, num_layers=1, num_heads=heads, num_kv_heads=heads, head_dim=192,
+                     intermediate_size=64, vocab_size=64, rms_eps=1e-6, dtype=torch.bfloat16, use_mla=True,
+                     extra={"qk_nope_head_dim": 128, "qk_rope_head_dim": 64, "v_head_dim": 128, "kv_lora_rank": 512,
+                            "q_lora_rank": 0})
+    att = MLAAttention(spec, 0, build_rope(64, 1024, 1e4, None, 64, False, device=dev), dev)
+    for p in att.parameters():
+        if p.dim() == 2:
+            p.data.copy_(torch.randn(p.shape, device=dev) * p.shape[1] ** -0.5)
+    att.process_weights()
+    q, c = [1] * decodes + q_lens, [50, 1, 129][:decodes] + ctx
+    lens = [a + b for a, b in zip(q, c)]
+    need = [-(-n // page) for n in lens]
+    perm, at = torch.randperm(sum(need)).tolist(), 0
+    bt = torch.zeros(len(lens), max(need), dtype=torch.int32)
+    for i, k in enumerate(need):
+        bt[i, :k] = torch.tensor(perm[at:at + k])
+        at += k
+    qsl = np.concatenate([[0], np.cumsum(q)]).astype(np.int32)
+    pos = torch.cat([torch.arange(a, a + b) for a, b in zip(c, q)]).int()
+    seq = torch.repeat_interleave(torch.arange(len(q)), torch.tensor(q)).int()
+    slots = torch.stack([bt[s, p // page] * page + p % page for s, p in zip(seq.tolist(), pos.tolist())]).int()
+    g = lambda x: torch.as_tensor(x, dtype=torch.int32).to(dev)   # noqa: E731
+    inp = SimpleNamespace(num_decode_seqs=decodes, num_seqs=len(q), padded_tokens=0, max_q_len=max(q),
+                          batch=SimpleNamespace(query_start_loc=qsl, seq_lens=np.array(lens, np.int32)), positions=g(pos),
+                          slot_mapping=g(slots), block_table=g(bt), tok_seq=g(seq), seq_lens=g(lens), query_start_loc=g(qsl))
+    tpc = SimpleNamespace(materialize=lambda h: h)
+    cache0 = torch.randn(sum(need), 1, 9, page, 64, device=dev).bfloat16()
+    h = torch.randn(sum(q), width, device=dev).bfloat16()
+    got = []
+    for least in (32, 10 ** 6):
+        monkeypatch.setattr(MLAAttention, "_EXPAND_MIN_TOKENS", least)
+        monkeypatch.setattr(MLAAttention, "_EXPAND_KV_BYTES", kv_rows * 512)
+        monkeypatch.setattr(MLAAttention, "_EXPAND_LATENT_BYTES", latent_rows * 1152)
+        cache = cache0.clone()
+        got.append((att(inp, h, SimpleNamespace(k_cache=[cache]), tpc), cache))
+    assert torch.equal(got[0][1], got[1][1])
+    for a, b in zip(q, qsl):
+        assert _rel_err(got[0][0][b:b + a], got[1][0][b:b + a]) < 1.2e-2
 
 
 @pytest.mark.parametrize("m", [1, 2])
