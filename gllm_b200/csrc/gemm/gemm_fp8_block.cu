@@ -320,13 +320,14 @@ fp8_quant_group_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_fp
   griddep_launch();
   griddep_wait();
   const int rows = live_tiles != nullptr ? min(M, *live_tiles * kFBM) : M;
-  const int row0 = blockIdx.y * 8;
-  if (row0 >= rows) return;
   const int groups = K / 128, lane = threadIdx.x & 15;
+  // one grid axis: the second one ends at 65,535 blocks, 524,280 rows
+  const int across = (groups + 7) / 8, row0 = static_cast<int>(blockIdx.x / across) * 8, g0 = static_cast<int>(blockIdx.x % across) * 8;
+  if (row0 >= rows) return;
   uint4 raw[4];
 #pragma unroll
   for (int n = 0; n < 4; ++n) {
-    const int pair = n * 16 + (threadIdx.x >> 4), row = row0 + (pair & 7), g = blockIdx.x * 8 + (pair >> 3);
+    const int pair = n * 16 + (threadIdx.x >> 4), row = row0 + (pair & 7), g = g0 + (pair >> 3);
     raw[n] = make_uint4(0u, 0u, 0u, 0u);
     if (row < rows && g < groups) {
       const __nv_bfloat16* src = x + static_cast<size_t>(row) * ldx + g * 128 + lane * 8;
@@ -340,7 +341,7 @@ fp8_quant_group_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_fp
   }
 #pragma unroll
   for (int n = 0; n < 4; ++n) {
-    const int pair = n * 16 + (threadIdx.x >> 4), row = row0 + (pair & 7), g = blockIdx.x * 8 + (pair >> 3);
+    const int pair = n * 16 + (threadIdx.x >> 4), row = row0 + (pair & 7), g = g0 + (pair >> 3);
     const uint32_t w[4] = {raw[n].x, raw[n].y, raw[n].z, raw[n].w};
     float f[8], amax = 0.f;
 #pragma unroll
@@ -410,7 +411,7 @@ GLLM_EXPORT int gllm_fp8_quant_group(const void* x, int64_t ldx, void* q, void* 
                                      void* stream) {
   if (M <= 0) return 0;
   if (K % 128 != 0) return 1;
-  CUDA_CHECK_RET(launch_pdl(fp8_quant_group_kernel, dim3((K / 128 + 7) / 8, (M + 7) / 8), dim3(256), 0,
+  CUDA_CHECK_RET(launch_pdl(fp8_quant_group_kernel, dim3(static_cast<unsigned>((K / 128 + 7) / 8) * ((M + 7) / 8)), dim3(256), 0,
                             reinterpret_cast<cudaStream_t>(stream), reinterpret_cast<const __nv_bfloat16*>(x), ldx,
                             reinterpret_cast<__nv_fp8_e4m3*>(q), reinterpret_cast<float*>(scales), M, K,
                             reinterpret_cast<const int32_t*>(live_tiles),

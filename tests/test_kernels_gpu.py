@@ -595,6 +595,21 @@ def test_moe_expert_tiles_partly_filled(counts):
     assert _rel_err(y, want) < 6e-3, _rel_err(y, want)
 
 
+@pytest.mark.parametrize("m,k", [(7, 1152), (8 * 65535 + 9, 128)])       # the second: more row groups than a grid's y axis has
+def test_fp8_quantiser_rows(m, k):
+    """Scales amax / 448 (an approximate division, 2 ulp) and e4m3 values of rows before and past 524,280."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(k)
+    x = torch.randn(m, k, device=_dev()).bfloat16()
+    q, s = sm100.fp8_quant_group(x)
+    amax = x.float().view(m, k // 128, 128).abs().amax(-1)
+    assert torch.allclose(s.t(), amax / 448, rtol=2.0 ** -21, atol=0)
+    back = q.float().view(m, k // 128, 128) * s.t()[..., None]
+    # e4m3 keeps 3 bits behind the leading one (2^-4), and steps of 2^-9 below 2^-6
+    err = (back - x.float().view(m, k // 128, 128)).abs()
+    assert bool((err <= x.float().view(m, k // 128, 128).abs() * 2.0 ** -4 * 1.001 + s.t()[..., None] * 2.0 ** -10 * 1.001).all())
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 256, 128), (77, 1536, 512), (300, 4096, 7168), (1024, 2048, 2048),
                                    (64, 576, 7168),       # 576 = kv_a_proj_with_mqa (MLA): N not a multiple of 128
                                    (129, 8200, 640), (3000, 1032, 384), (2500, 4352, 1152)])   # tiles of 64, 128, 256
