@@ -666,6 +666,10 @@ static int gemm_bf16_impl(const void* A, int64_t lda, const void* W, int64_t ldw
     fprintf(stderr, "[gllm_b200] gemm_bf16: output and bias must lie on 16-byte boundaries\n");
     return 1;
   }
+  if (epi == kEpiSiluMul && (force_bn == 192 || force_bn == 32)) {   // no gated form: plain stores would not fit the output
+    fprintf(stderr, "[gllm_b200] gemm_bf16: no gated tiles %d wide\n", force_bn);
+    return 1;
+  }
   int bn = 128, split = 1;
   choose_cfg(M, N, K, epi, force_bn, ws != nullptr && tile_cnt != nullptr ? ws_bytes : 0, max_tiles, &bn, &split);
   CUtensorMap ta, tb;

@@ -948,6 +948,16 @@ def test_linear_few_rows(m, n, k):
             assert _rel_err(sm100.linear_silu_mul(x, inter, act=act), f(g) * u) < 6e-3      # one bf16 rounding and fast exp
 
 
+@pytest.mark.parametrize("bn", [32, 192])
+def test_gemm_gated_refuses_tile_widths_without_a_gated_form(bn, monkeypatch):
+    """The plain epilogue would store twice the output's columns."""
+    from gllm_b200.ops import sm100
+    monkeypatch.setattr(sm100, "_FORCE_BN", bn)
+    x, w = torch.randn(64, 128, device=_dev()).bfloat16(), torch.randn(256, 128, device=_dev()).bfloat16()
+    with pytest.raises(RuntimeError):
+        sm100.linear(x, w, epi=1)
+
+
 @pytest.mark.parametrize("m", [3, 17, 32])
 @pytest.mark.parametrize("ldc,shift", [(13, 0), (514, 1), (516, 2), (516, 4)])     # the last one: 8-byte boundaries
 def test_gemm_smallm_any_output(m, ldc, shift):
