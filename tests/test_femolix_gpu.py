@@ -435,3 +435,32 @@ def test_chunked_delta_rule_keeps_earlier_tokens_clean(what, value, at):
         a, b = torch.where(fin, c, zero), torch.where(fin, s, zero)
         assert float((a - b).norm()) <= 2e-5 * float(b.norm())      # sums of some 150 tokens in fp32, in another order
     assert bool(torch.isfinite(got[0][0][:row]).all())
+
+
+@pytest.mark.parametrize("state", [True, False])
+@pytest.mark.parametrize("unit", [True, False])
+def test_chunked_delta_rule_in_rounds_of_heads(state, unit, monkeypatch):
+    """A workspace for two of three heads: rounds of two and one, each with its own strides, the same bits as all at once. Without
+    a carried state, and without unit lengths; against the token-serial kernel (fp32 sums over some 100 tokens in another order)."""
+    from gllm_b200.ops import sm100_seq as S
+    torch.manual_seed(3)
+    dev, H, D, V, lens, ctx = "cuda", 3, 64, 40, [70, 5, 33, 128], [4, 0, 9, 0]
+    t, n = sum(lens), len(lens)
+    q, k, v = (torch.randn(t, H * w, device=dev) for w in (D, D, V))
+    q, k, v = q.bfloat16(), (k if unit else k * D ** -0.5).bfloat16(), v.bfloat16()
+    beta, a = (torch.randn(t, H, device=dev).bfloat16() for _ in range(2))
+    neg_a, dt_bias = -torch.rand(H, device=dev), torch.zeros(H, device=dev)
+    qsl = torch.tensor([0] + lens, device=dev).cumsum(0).to(torch.int32)
+    sl = torch.tensor([x + c for x, c in zip(lens, ctx)], device=dev, dtype=torch.int32)
+    rs = torch.randperm(n, device=dev).to(torch.int32)
+    st0, got = torch.randn(n, H, D, V, device=dev), []
+    slots, unit_bytes = t // 64 + n, S._L().gllm_delta_unit_bytes()
+    for work, mx in ((1 << 28, max(lens)), (2 * slots * unit_bytes, max(lens)), (1 << 28, None)):
+        monkeypatch.setattr(S, "_DELTA_WORK_BYTES", work)
+        st = st0.clone()
+        o = S.linear_state_scan(q, k, v, beta, a, neg_a, dt_bias, None, st if state else None, rs if state else None, sl, qsl, H, H,
+                                D, V, False, unit, 0.3, True, max_q_len=mx)
+        got.append((o, st))
+    for whole, rounds, serial in zip(*got):
+        assert torch.equal(whole, rounds)
+        assert float((whole - serial).norm()) <= 1e-5 * float(serial.norm())

@@ -257,3 +257,30 @@ def test_scan_with_a_bound_on_the_lengths(lens):
         torch.full((t, C), 3.0, device=DEV).bfloat16()       # what an unwritten output is likely to hold
         got.append((S.selective_scan(x, dtr, proj, xz, A, Dk, db, st, rs, sl, qsl, C, N, R, max_q_len=bound), st))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and bool(got[0][1].abs().sum() > 0)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("state", [True, False])
+def test_scan_in_rounds_of_channels(dt, state, monkeypatch):
+    """A workspace for 128 channels: rounds of 128, 128 and 1, the same bits as all at once; with and without a carried state, in
+    fp32 and bf16. Against the token-serial kernel: fp32 sums in another order, and for bf16 outputs one rounding (2^-8)."""
+    from gllm_b200.ops import sm100_seq as S
+    torch.manual_seed(5)
+    N, C, R, qlens, ctx = 12, 257, 6, [150, 7, 129, 256], [4, 0, 0, 66]
+    t, n = sum(qlens), len(qlens)
+    qsl = torch.tensor([0] + qlens, device=DEV).cumsum(0).to(torch.int32)
+    sl = torch.tensor([c + q for c, q in zip(ctx, qlens)], dtype=torch.int32, device=DEV)
+    rs = torch.randperm(n, device=DEV).to(torch.int32)
+    x, dtr, xz = (torch.randn(t, w, device=DEV).to(dt) for w in (C, C, 2 * C))
+    proj = torch.randn(t, R + 2 * N, device=DEV).to(dt)
+    A, Dk, db = -torch.rand(C, N, device=DEV) * 4, torch.randn(C, device=DEV), torch.full((C,), -3.0, device=DEV)
+    st0, got = torch.randn(n, N, C, device=DEV), []
+    for work, mx in ((1 << 28, max(qlens)), (0, max(qlens)), (1 << 28, None)):
+        monkeypatch.setattr(S, "_SCAN_WORK_BYTES", work)
+        st = st0.clone()
+        o = S.selective_scan(x, dtr, proj, xz, A, Dk, db, st if state else None, rs if state else None, sl, qsl, C, N, R,
+                             max_q_len=mx)
+        got.append((o, st))
+    for (whole, rounds, serial), tol in zip(zip(*got), (1e-5 if dt == torch.float32 else 2.0 ** -8, 1e-5)):
+        assert torch.equal(whole, rounds)
+        assert float((whole.float() - serial.float()).norm()) <= tol * float(serial.float().norm())
