@@ -380,18 +380,17 @@ static int launch_fp8_tile(const CUtensorMap& ta, const CUtensorMap& tb, const F
 
 // Tile width: the one with the least (waves x time of a tile's K block). A block of 128 rows costs about 560 cycles 256 wide,
 // 330 at 128 and 230 at 64 (there the copies of the activation tile bound it), so narrow tiles only pay when the wide ones
-// leave SMs idle: a decode batch's 7168 columns are 28 tiles of 256. Grouped calls do not know how many row tiles are live.
-static int launch_fp8(const void* A8, const void* W8, uint64_t w_rows, Fp8Params p, cudaStream_t st) {
+// leave SMs idle: a decode batch's 7168 columns are 28 tiles of 256. `live`: the most row tiles that can hold rows; grouped calls
+// (256 or 128 wide) do not know more on the host.
+static int launch_fp8(const void* A8, const void* W8, uint64_t w_rows, Fp8Params p, int64_t live, cudaStream_t st) {
   const int64_t m_tiles = (p.M + kFBM - 1) / kFBM;
   const int width[3] = {256, 128, 64}, cost[3] = {560, 330, 230};
   int bn = 256;
-  if (p.tile_expert == nullptr) {
-    int64_t best = -1;
-    for (int i = 0; i < (p.silu ? 2 : 3); ++i) {
-      const int64_t tiles = m_tiles * ((p.N + width[i] - 1) / width[i]);
-      const int64_t t = (tiles + num_sms() - 1) / num_sms() * cost[i];
-      if (best < 0 || t < best) { best = t; bn = width[i]; }
-    }
+  int64_t best = -1;
+  for (int i = 0; i < (p.silu || p.tile_expert != nullptr ? 2 : 3); ++i) {
+    const int64_t tiles = live * ((p.N + width[i] - 1) / width[i]);
+    const int64_t t = (tiles + num_sms() - 1) / num_sms() * cost[i];
+    if (best < 0 || t < best) { best = t; bn = width[i]; }
   }
   p.waits = g_wait_config;
   CUtensorMap ta, tb;
@@ -443,15 +442,15 @@ GLLM_EXPORT int gllm_gemm_fp8_block(const void* A8, const void* a_s, const void*
   p.tile_expert = nullptr; p.num_m_tiles_ptr = nullptr; p.n_per_expert = 0; p.ws_stride_e = 0;
   p.silu = silu ? 1 : 0;
   p.up_row = silu ? N / 2 : 0;
-  return launch_fp8(A8, W8, N, p, reinterpret_cast<cudaStream_t>(stream));
+  return launch_fp8(A8, W8, N, p, (M + kFBM - 1) / kFBM, reinterpret_cast<cudaStream_t>(stream));
 }
 
 // Grouped (MoE) block-scaled fp8 GEMM: A8 [max_tiles*128, K] e4m3 (expert-sorted, 128-row tiles), a_s
 // [K/128, max_tiles*128]; W8 [E, N, K] e4m3, w_s [E, N/64, K/128] (one scale row per 64 weight rows);
-// epi 1 = SiLU gate on [64 gate | 64 up] interleaved tiles -> C [rows, N/2].
+// epi 1 = SiLU gate on [64 gate | 64 up] interleaved tiles -> C [rows, N/2]. At most max_live of the max_tiles tiles hold rows.
 GLLM_EXPORT int gllm_moe_grouped_gemm_fp8(const void* A8, const void* a_s, const void* W8, const void* w_s, void* C,
-                                          int64_t ldc, int max_tiles, int N, int K, int E, const void* tile_expert,
-                                          const void* num_tiles_ptr, int epi, void* stream) {
+                                          int64_t ldc, int max_tiles, int max_live, int N, int K, int E,
+                                          const void* tile_expert, const void* num_tiles_ptr, int epi, void* stream) {
   if (max_tiles <= 0) return 0;
   if (K % 128 != 0 || N % 128 != 0) {
     fprintf(stderr, "[gllm_b200] moe_grouped_gemm_fp8: K %% 128 and N %% 128 required\n");
@@ -471,5 +470,6 @@ GLLM_EXPORT int gllm_moe_grouped_gemm_fp8(const void* A8, const void* a_s, const
   p.ws_stride_e = static_cast<int64_t>(N / 64) * (K / 128);
   p.silu = epi == 1 ? 1 : 0;
   p.up_row = 0;
-  return launch_fp8(A8, W8, static_cast<uint64_t>(E) * N, p, reinterpret_cast<cudaStream_t>(stream));
+  return launch_fp8(A8, W8, static_cast<uint64_t>(E) * N, p, max_live < max_tiles ? max_live : max_tiles,
+                    reinterpret_cast<cudaStream_t>(stream));
 }

@@ -143,6 +143,7 @@ def fused_experts_fp8(x: torch.Tensor, w13: torch.Tensor, w13_s: torch.Tensor, w
     if t == 0:
         return out
     max_tiles = (t * k + 127) // 128 + e_local
+    max_live = t * k // 128 + min(e_local, t * k)      # full tiles, and one partly filled tile per expert that has a row
     rows = max_tiles * 128
     meta = _buf("meta", (2 + 3 * e_local + 1,), torch.int32, dev)
     tile_expert = _buf("tile_expert", (max_tiles,), torch.int32, dev)
@@ -159,10 +160,10 @@ def fused_experts_fp8(x: torch.Tensor, w13: torch.Tensor, w13_s: torch.Tensor, w
     check(L.gllm_moe_align_gather(_p(topk_ids), _p(expert_map), t, k, e_local, _p(meta), _p(tile_expert), max_tiles,
                                   _p(slot_pos), _p(x), x.stride(0), _p(xs), h, None, st), "moe_align_gather")
     check(L.gllm_fp8_quant_group(_p(xs), h, _p(xs8), _p(xs_s), rows, h, _p(meta), st), "fp8_quant(xs)")   # meta[0]: live tiles
-    check(L.gllm_moe_grouped_gemm_fp8(_p(xs8), _p(xs_s), _p(w13), _p(w13_s), _p(hbuf), inter, max_tiles, two_i, h,
+    check(L.gllm_moe_grouped_gemm_fp8(_p(xs8), _p(xs_s), _p(w13), _p(w13_s), _p(hbuf), inter, max_tiles, max_live, two_i, h,
                                       e_local, _p(tile_expert), _p(meta), 1, st), "moe_grouped_gemm_fp8(1)")
     check(L.gllm_fp8_quant_group(_p(hbuf), inter, _p(h8), _p(h_s), rows, inter, _p(meta), st), "fp8_quant(h)")
-    check(L.gllm_moe_grouped_gemm_fp8(_p(h8), _p(h_s), _p(w2), _p(w2_s), _p(ybuf), h, max_tiles, h, inter, e_local,
+    check(L.gllm_moe_grouped_gemm_fp8(_p(h8), _p(h_s), _p(w2), _p(w2_s), _p(ybuf), h, max_tiles, max_live, h, inter, e_local,
                                       _p(tile_expert), _p(meta), 0, st), "moe_grouped_gemm_fp8(2)")
     check(L.gllm_moe_combine(_p(ybuf), _p(slot_pos), _p(topk_w), _p(out), t, k, h, st), "moe_combine")
     _count(9)
