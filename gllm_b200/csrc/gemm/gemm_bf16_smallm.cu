@@ -296,7 +296,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   }
 }
 
-// defined in gemv_bf16.cu
+// defined in gemv_bf16.cu: one or two rows on small matrices; -1: not taken
 int gemv_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int M, int N, int K, const void* bias,
               int act, cudaStream_t st);
 

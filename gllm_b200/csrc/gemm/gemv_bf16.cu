@@ -6,10 +6,19 @@
 // or two weight rows with the whole of K: no tensor core, no split of K, no second pass over partial sums. Its first 4 KB of
 // weights are in flight before the previous kernel ends, the next 4 KB while one is multiplied; the rows of A wait in shared
 // memory. Products and sums are fp32 (a lane's in order, then a tree over the lanes).
-// Cold weights, against the tensor-core kernel that splits K (us per GEMM): layers of 1024 -> 4096, 2048 -> 1024, 1024 -> 2 x 3072,
-// 3072 -> 1024: one row 5.5 -> 3.3, two 5.5 -> 4.1; layers of a width of 4096 (12288 inside): 19.9 -> 16.7 and 20.0 -> 19.4;
-// 1024 -> 151,936: 52.6 -> 45.8 and 53.3 -> 49.7. Three rows lose where the matrix is large (74 against 53): the arithmetic of
-// the plain cores then outlasts the weights.
+// Taken where the busiest SM streams at most 560 KB (one row) or 140 KB (two), whole rounds of its 16 warps counted, and the rows
+// of A fit 48 KB. The tensor-core kernel has 192 KB per SM in flight before the previous kernel ends where this one has 64, and its
+// last round is not partly empty, so it wins on large matrices; two rows unpack A again for every weight row. Timed on whole
+// captured decode steps, all layers (ms, one row / two; 0: none, then up to 560 / 140 KB, then up to 800 / 400 KB):
+//     0.6B shape          0.979 / 0.995    0.712 / 0.833    0.712 / 0.830
+//     1.7B, 16 layers     0.872 / 0.895    0.741 / 0.852    0.737 / 0.836
+//     4B, 16 layers       1.255 / 1.247    1.189 / 1.248    1.142 / 1.261
+//     8B, 20 layers       2.065 / 2.062    2.009 / 2.060    2.081 / 2.116    (everything: +10 % / +15 %)
+//     half of it          1.386 / 1.375    1.307 / 1.346    1.346 / 1.400
+//     an eighth           0.775 / 0.782    0.640 / 0.739    0.638 / 0.747
+//     70B, an eighth, 10  0.698 / 0.703    0.688 / 0.692    0.690 / 0.723
+// One GEMM at a time says otherwise (4096 -> 2 x 12288, 12288 -> 4096 cold: 19.9 -> 16.7 us on average for a layer of the 8B shape).
+// Three rows lose where the matrix is large (74 against 53 us): the arithmetic of the plain cores then outlasts the weights.
 #include "../common/host_utils.h"
 #include "../common/ptx.cuh"
 
@@ -39,6 +48,9 @@ __device__ __forceinline__ uint64_t pair_f32(uint32_t v) {
 __device__ __forceinline__ void fma_pair(uint64_t& acc, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
+
+// most bytes of weights that the busiest SM streams
+static constexpr int64_t kMostOneRow = 560 * 1024, kMostTwoRows = 140 * 1024;
 
 // MT: rows of A; R weight rows per warp, U 16-byte loads per lane and row at a time.
 // ACT 0: plain (+ bias); 1: silu(gate) * up; 2: tanh gelu. Gated weights are interleaved per 128 rows (128 gate, 128 up), R = 2.
@@ -137,8 +149,11 @@ __global__ void __launch_bounds__(128) gemv_kernel(const GemvParams p) {
 template <int MT, int R, int U, int ACT>
 static int launch_gemv(GemvParams p, cudaStream_t st) {
   p.units = ACT != 0 ? p.N / 2 : (p.N + R - 1) / R;
-  const int want = (p.units + 3) / 4, most = num_sms() * 4;
-  CUDA_CHECK_RET(launch_pdl(gemv_kernel<MT, R, U, ACT>, dim3(want < most ? want : most), dim3(128), MT * p.K * 2, st, p));
+  const int want = (p.units + 3) / 4, sms = num_sms(), grid = want < 4 * sms ? want : 4 * sms;
+  // what the busiest SM streams: whole rounds of its warps, the last one included
+  const int64_t rounds = (p.units + 4 * grid - 1) / (4 * grid), warps = (grid + sms - 1) / sms * 4;
+  if (rounds * warps * R * p.K * 2 > (MT == 1 ? kMostOneRow : kMostTwoRows)) return -1;
+  CUDA_CHECK_RET(launch_pdl(gemv_kernel<MT, R, U, ACT>, dim3(grid), dim3(128), MT * p.K * 2, st, p));
   return 0;
 }
 

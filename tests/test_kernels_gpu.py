@@ -948,6 +948,25 @@ def test_linear_few_rows(m, n, k):
             assert _rel_err(sm100.linear_silu_mul(x, inter, act=act), f(g) * u) < 6e-3      # one bf16 rounding and fast exp
 
 
+@pytest.mark.parametrize("m,n", [(1, 9472), (1, 9473), (2, 2368), (2, 2369)])       # 148 SMs x 16 warps: four full rounds, one
+@pytest.mark.parametrize("gated", [False, True])
+def test_linear_few_rows_at_the_rules_border(m, n, gated):
+    """The last matrix that the plain-core kernel takes and the first that goes to the tensor-core one, K = 4096 (131 KB a round
+    and SM; gated, two rows per warp: half as many rounds)."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(n)
+    x = torch.randn(m, 4096, device=_dev()).bfloat16()
+    if not gated:
+        w = torch.randn(n, 4096, device=_dev()).bfloat16()
+        want = x.double() @ w.double().t()
+        tol = want.abs() * 2.0 ** -8 + (x.double().abs() @ w.double().abs().t()) * 4096 * 2.0 ** -24
+        assert bool(((sm100.linear(x, w).double() - want).abs() <= tol).all())
+        return
+    w = torch.randn(n // 256 * 256 + 256 * (n & 1), 4096, device=_dev()).bfloat16() * 4096 ** -0.5
+    g, u = (x.float() @ w.float().t()).chunk(2, -1)
+    assert _rel_err(sm100.linear_silu_mul(x, ref.interleave_gate_up(w)), torch.nn.functional.silu(g) * u) < 6e-3
+
+
 @pytest.mark.parametrize("bn", [32, 192])
 def test_gemm_gated_refuses_tile_widths_without_a_gated_form(bn, monkeypatch):
     """The plain epilogue would store twice the output's columns."""
