@@ -15,6 +15,8 @@
 //   warp 9 (1 thread)  MMA issuer   : S  = Q K^T  (tcgen05.mma, A = Q smem K-major, B = K tile K-major, D in TMEM)
 //                                     O += P V    (A = P in TMEM, B = V tile **MN-major**, D in TMEM)
 //
+// The schedule is the published one of FlashAttention on this generation (Dao and others, "FlashAttention-4"): two query tiles
+// in turn, P over S in TMEM, and a reference of the exponentials that follows the row's maximum in steps.
 // The tensor core runs one query tile's PV_j and S_j+1 while the other tile's softmax works on S_j. Products of one thread
 // execute in order, so S_j+1 may take P_j's columns without a wait between the two, and the barrier that announces S_j+1 also
 // says that PV_j is in O.

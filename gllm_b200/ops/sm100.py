@@ -244,8 +244,9 @@ _attn_ws = {}
 _FUSED_MERGE = os.environ.get("GLLM_ATTN_FUSED_MERGE", "0") == "1"
 # tcgen05 / TMEM prefill attention (csrc/attn/prefill_attention_tc.cu) is the default prefill kernel (validated on
 # B200: profiles/attn_prefill_tc.md; 1.3-2.1x the mma.sync kernel); GLLM_ATTN_TC=0 selects the mma.sync kernel, which
-# also serves the shapes outside the tcgen05 kernel's envelope. ATTN_TC_KV bounds its page size (64 or 128;
-# 64 measured faster at every shape). Module attributes so tests / benches can flip them.
+# also serves the shapes outside the tcgen05 kernel's envelope. ATTN_TC_KV (64 or 128) bounds the page size that it takes, and
+# nothing else: it walks 128 keys at a time whatever the pages. The other paged kernels end at pages of 64, hence the default.
+# Module attributes so tests / benches can flip them.
 ATTN_TC = os.environ.get("GLLM_ATTN_TC", "1") == "1"
 ATTN_TC_KV = int(os.environ.get("GLLM_ATTN_TC_KV", "64"))
 

@@ -258,6 +258,21 @@ def test_prefill_attention_tc(hq, hkv, d, kv_tile, monkeypatch):
     assert _rel_err(o, o_ref) < 1e-2, _rel_err(o, o_ref)
 
 
+@pytest.mark.parametrize("page", [32, 64, 128])
+@pytest.mark.parametrize("hq,hkv,d", [(8, 2, 128), (4, 4, 64)])
+def test_prefill_attention_tc_page_sizes(hq, hkv, d, page, monkeypatch):
+    """Pages below, at and above half of the 128 keys that the kernel walks at a time: two boxes of 64 rows for a page of 128,
+    which ATTN_TC_KV = 128 admits."""
+    from gllm_b200.ops import sm100
+    monkeypatch.setattr(sm100, "ATTN_TC", True)
+    monkeypatch.setattr(sm100, "ATTN_TC_KV", max(64, page))
+    q_lens, ctx = [1, 40, 127, 128, 300, 64], [127, 0, 129, 128, 1, 700]
+    seq_lens = [a + b for a, b in zip(q_lens, ctx)]
+    q, kc, vc, bt, sl, qsl = _make_paged(seq_lens, q_lens, hq, hkv, d, page, _dev(), seed=5)
+    o = sm100.paged_attention(q, kc, vc, bt, sl, qsl, d ** -0.5, hq, d, 0, len(q_lens), max(q_lens), max(seq_lens))
+    assert _rel_err(o, ref.paged_attention(q, kc, vc, bt, sl, qsl, d ** -0.5, hq, d)) < 1e-2
+
+
 @pytest.mark.parametrize("hq,hkv,d", [(8, 1, 128), (4, 4, 128), (6, 2, 64)])
 @pytest.mark.parametrize("page", [8, 16, 64])
 @pytest.mark.parametrize("many", [False, True])       # few CTAs: one query tile each; many: two
