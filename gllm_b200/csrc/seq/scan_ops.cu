@@ -21,47 +21,54 @@ using namespace seqk;
 
 constexpr int kL = 64;                              // tokens of a chunk
 constexpr int kNM = 16;                             // states a thread holds
+constexpr int kRows = 2 * kL;                       // tokens of the longest sequence that is walked whole
 
 // Chunk slots: sequence s owns slots from qsl[s] / 64 + s on (at least one per started 64 tokens); some stay empty.
 __device__ __forceinline__ int chunk_base(const int* qsl, int s) { return qsl[s] / kL + s; }
 
 // Channels [c0, c0 + CW) of the batch; ends [slot][n][CW]: end states (FINAL 0: written) or entering states (FINAL 1: read);
-// steps [slot][CW]: sums of dt. Sequences of fewer than min_len tokens are the serial kernel's.
+// steps [slot][CW]: sums of dt. Sequences of fewer than min_len tokens are not cut: FINAL walks them whole, from the carried
+// state (a kernel of their own behind the three took as long again: 8 portions of 100 tokens and one of 150).
 template <typename T, bool FINAL>
-__global__ void __launch_bounds__(128) scan_chunk_kernel(
+__global__ void __launch_bounds__(128, FINAL ? 6 : 7) scan_chunk_kernel(
     const T* __restrict__ xc, const T* __restrict__ dt_raw, const T* __restrict__ proj, long ldp, const T* __restrict__ xz,
     long ldxz, const float* __restrict__ A, const float* __restrict__ Dskip, const float* __restrict__ dt_bias,
-    float* __restrict__ state, const int* __restrict__ rec_slots, const int* __restrict__ qsl, int nseq, int C, int N, int R,
-    int c0, int CW, int min_len, float* __restrict__ ends, float* __restrict__ steps, T* __restrict__ out) {
+    float* __restrict__ state, const int* __restrict__ rec_slots, const int* __restrict__ seq_lens, const int* __restrict__ qsl,
+    int nseq, int C, int N, int R, int c0, int CW, int min_len, float* __restrict__ ends, float* __restrict__ steps, T* __restrict__ out) {
   constexpr int TCH = 8;
-  __shared__ __align__(16) float sBC[kL][2 * kNM];
+  __shared__ __align__(16) float sBC[FINAL ? kRows : kL][2 * kNM];
   const int u = blockIdx.y;
   int lo = 0, hi = nseq - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (chunk_base(qsl, mid) <= u) lo = mid; else hi = mid - 1;
   }
-  const int q0 = qsl[lo], q1 = qsl[lo + 1], base = q0 + (u - chunk_base(qsl, lo)) * kL;
-  if (base < q0 || q1 - q0 < min_len || base >= q1) return;         // uniform over the block
-  const bool last = base + kL >= q1;
+  const int q0 = qsl[lo], q1 = qsl[lo + 1];
+  const int base = q0 + (u - chunk_base(qsl, lo)) * kL;
+  const bool whole = q1 - q0 < min_len;
+  if (base < q0 || base >= q1 || (whole && base != q0)) return;     // uniform over the block
+  const bool last = whole || base + kL >= q1;
   if (!FINAL && last) return;                       // nobody continues from its end
-  const int len = min(kL, q1 - base);
-  for (int i = threadIdx.x; i < len * 2 * kNM; i += 128) {
-    const int k = i / (2 * kNM), n = i % kNM, half = (i / kNM) & 1;
-    sBC[k][half * kNM + n] = n < N ? to_f(proj[(size_t)(base + k) * ldp + R + half * N + n]) : 0.f;
-  }
+  const int len = (FINAL && whole ? q1 : min(base + kL, q1)) - base;      // whole: fewer than min_len tokens, at most kRows
   const int w = blockIdx.x * 128 + threadIdx.x;     // channel inside this round's range
   const bool active = w < CW;
   const int c = c0 + (active ? w : CW - 1);         // idle threads mirror the last channel (loads only)
   float S[kNM], a[kNM];
   float* e0 = ends + ((size_t)u * N) * CW + (active ? w : CW - 1);
+  const bool carried = whole && state != nullptr && seq_lens[lo] > q1 - q0;
+  const float* from = carried ? state + (size_t)rec_slots[lo] * N * C + c : e0;
+  const size_t step = carried ? C : CW;
 #pragma unroll
   for (int n = 0; n < kNM; ++n) {
     a[n] = n < N ? A[(size_t)c * N + n] : 0.f;
-    S[n] = FINAL && n < N ? e0[(size_t)n * CW] : 0.f;
+    S[n] = FINAL && n < N && (carried || !whole) ? from[n * step] : 0.f;
   }
   const float dsk = Dskip[c], bias = dt_bias[c];
   float sum = 0.f;
+  for (int i = threadIdx.x; i < len * 2 * kNM; i += 128) {
+    const int k = i / (2 * kNM), n = i % kNM, half = (i / kNM) & 1;
+    sBC[k][half * kNM + n] = n < N ? to_f(proj[(size_t)(base + k) * ldp + R + half * N + n]) : 0.f;
+  }
   __syncthreads();
   for (int k0 = 0; k0 < len; k0 += TCH) {
     float dtv[TCH], xv[TCH], zv[TCH];
@@ -162,13 +169,13 @@ int launch_scan(const void* xc, const void* dt_raw, const void* proj, long ldp, 
     float* steps = work + (size_t)slots * N * cw;
     const dim3 grid((cw + 127) / 128, slots);
     scan_chunk_kernel<T, false><<<grid, 128, 0, st>>>((const T*)xc, (const T*)dt_raw, (const T*)proj, ldp, (const T*)xz, ldxz,
-                                                      A, Dskip, dt_bias, state, rec_slots, qsl, nseq, C, N, R, c0, cw, min_len,
-                                                      work, steps, (T*)out);
+                                                      A, Dskip, dt_bias, state, rec_slots, seq_lens, qsl, nseq, C, N, R, c0, cw,
+                                                      min_len, work, steps, (T*)out);
     scan_carry_kernel<<<dim3((cw + 127) / 128, N, nseq), 128, 0, st>>>(A, state, rec_slots, seq_lens, qsl, C, N, c0, cw,
                                                                        min_len, work, steps);
     scan_chunk_kernel<T, true><<<grid, 128, 0, st>>>((const T*)xc, (const T*)dt_raw, (const T*)proj, ldp, (const T*)xz, ldxz,
-                                                     A, Dskip, dt_bias, state, rec_slots, qsl, nseq, C, N, R, c0, cw, min_len,
-                                                     work, steps, (T*)out);
+                                                     A, Dskip, dt_bias, state, rec_slots, seq_lens, qsl, nseq, C, N, R, c0, cw,
+                                                     min_len, work, steps, (T*)out);
   }
   CUDA_CHECK_RET(cudaGetLastError());
   return 0;
@@ -176,14 +183,14 @@ int launch_scan(const void* xc, const void* dt_raw, const void* proj, long ldp, 
 
 }  // namespace
 
-// The sequences with at least min_len new tokens, `width` channels at a time; returns 2 outside its envelope (the caller then
-// uses the token-serial kernel): N <= 16. `work`: (ntok / 64 + nseq) * (N + 1) * min(width, C) floats.
+// Sequences with at least min_len new tokens are cut, the others walked whole, `width` channels at a time; returns 2 outside its
+// envelope (the caller then uses the token-serial kernel): N <= 16. `work`: (ntok / 64 + nseq) * (N + 1) * min(width, C) floats.
 GLLM_EXPORT int gllm_scan_chunk(const void* xc, const void* dt_raw, const void* proj, long ldp, const void* xz, long ldxz,
                                 const void* A, const void* Dskip, const void* dt_bias, void* state, const void* rec_slots,
                                 const void* seq_lens, const void* qsl, int ntok, int nseq, int C, int N, int R, int min_len,
                                 int width, void* work, void* out, int is_f32, void* stream) {
   if (nseq <= 0 || ntok <= 0) return 0;
-  if (N < 1 || N > kNM || width < 1 || nseq > 65535 || ntok / kL + nseq > 65535) return 2;
+  if (N < 1 || N > kNM || width < 1 || min_len > kRows + 1 || nseq > 65535 || ntok / kL + nseq > 65535) return 2;
   auto go = is_f32 ? launch_scan<float> : launch_scan<__nv_bfloat16>;
   return go(xc, dt_raw, proj, ldp, xz, ldxz, (const float*)A, (const float*)Dskip, (const float*)dt_bias, (float*)state,
             (const int*)rec_slots, (const int*)seq_lens, (const int*)qsl, ntok, nseq, C, N, R, min_len, width, (float*)work,

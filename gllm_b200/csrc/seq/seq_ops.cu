@@ -480,14 +480,13 @@ __global__ void conv_state_update_kernel(const T* __restrict__ xz, long ldxz, in
 
 // Mamba-1 recurrence: one thread per channel holds its N states in registers and walks the sequence's tokens in
 // chunks of TCH: the chunk's B and C rows (shared by all channels) are staged in shared memory by the whole block and
-// the thread's own dt / x / z values are fetched up front, so the serial loop runs out of registers and smem. max_len > 0:
-// longer sequences are another kernel's (scan_ops.cu).
+// the thread's own dt / x / z values are fetched up front, so the serial loop runs out of registers and smem.
 template <typename T, int NMAX, int PARTS>
 __global__ void __launch_bounds__(64) selective_scan_kernel(
     const T* __restrict__ xc, const T* __restrict__ dt_raw, const T* __restrict__ proj, long ldp,
     const T* __restrict__ xz, long ldxz, const float* __restrict__ A, const float* __restrict__ Dskip,
     const float* __restrict__ dt_bias, float* __restrict__ state, const int* __restrict__ rec_slots,
-    const int* __restrict__ seq_lens, const int* __restrict__ qsl, int C, int N, int R, T* __restrict__ out, int max_len) {
+    const int* __restrict__ seq_lens, const int* __restrict__ qsl, int C, int N, int R, T* __restrict__ out) {
   constexpr int TCH = 8;
   __shared__ float sBC[TCH][2 * NMAX];
   const int s = blockIdx.x;
@@ -495,7 +494,7 @@ __global__ void __launch_bounds__(64) selective_scan_kernel(
   constexpr int NS = NMAX / PARTS;
   const int c0 = (blockIdx.y * 64 + threadIdx.x) / PARTS, part = threadIdx.x % PARTS;
   const int q0 = qsl[s], q1 = qsl[s + 1];
-  if (q1 <= q0 || (max_len > 0 && q1 - q0 > max_len)) return;      // uniform over the block
+  if (q1 <= q0) return;                       // uniform over the block
   const bool active = c0 < C;
   const int c = active ? c0 : C - 1;          // idle threads mirror the last channel (loads only)
   const bool carried = state != nullptr && (seq_lens[s] - (q1 - q0)) > 0;
@@ -606,11 +605,11 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const T* __restrict__ A,
 template <typename T, int PARTS>
 int scan_dispatch(int nmax, dim3 grid, cudaStream_t st, const void* xc, const void* dt_raw, const void* proj, long ldp,
                   const void* xz, long ldxz, const float* A, const float* Dskip, const float* dt_bias, float* state,
-                  const int* rec_slots, const int* seq_lens, const int* qsl, int C, int N, int R, void* out, int max_len) {
+                  const int* rec_slots, const int* seq_lens, const int* qsl, int C, int N, int R, void* out) {
 #define GLLM_SCAN(NM)                                                                                             \
   selective_scan_kernel<T, NM, PARTS><<<grid, 64, 0, st>>>((const T*)xc, (const T*)dt_raw, (const T*)proj, ldp,          \
                                                     (const T*)xz, ldxz, A, Dskip, dt_bias, state, rec_slots,      \
-                                                    seq_lens, qsl, C, N, R, (T*)out, max_len)
+                                                    seq_lens, qsl, C, N, R, (T*)out)
   if (nmax <= 8) GLLM_SCAN(8);
   else if (nmax <= 16) GLLM_SCAN(16);
   else if (nmax <= 32) GLLM_SCAN(32);
@@ -789,7 +788,7 @@ GLLM_EXPORT int gllm_seq_conv_silu(const void* xz, long ldxz, int ntok, int nseq
 GLLM_EXPORT int gllm_seq_selective_scan(const void* xc, const void* dt_raw, const void* proj, long ldp, const void* xz,
                                         long ldxz, const void* A, const void* Dskip, const void* dt_bias, void* state,
                                         const void* rec_slots, const void* seq_lens, const void* qsl, int nseq, int C,
-                                        int N, int R, void* out, int is_f32, int parts, int max_len, void* stream) {
+                                        int N, int R, void* out, int is_f32, int parts, void* stream) {
   if (nseq <= 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
   int rc;
@@ -798,11 +797,11 @@ GLLM_EXPORT int gllm_seq_selective_scan(const void* xc, const void* dt_raw, cons
     if (is_f32)
       rc = scan_dispatch<float, 4>(N, grid4, st, xc, dt_raw, proj, ldp, xz, ldxz, (const float*)A,
                                    (const float*)Dskip, (const float*)dt_bias, (float*)state, (const int*)rec_slots,
-                                   (const int*)seq_lens, (const int*)qsl, C, N, R, out, max_len);
+                                   (const int*)seq_lens, (const int*)qsl, C, N, R, out);
     else
       rc = scan_dispatch<__nv_bfloat16, 4>(N, grid4, st, xc, dt_raw, proj, ldp, xz, ldxz, (const float*)A,
                                            (const float*)Dskip, (const float*)dt_bias, (float*)state,
-                                           (const int*)rec_slots, (const int*)seq_lens, (const int*)qsl, C, N, R, out, max_len);
+                                           (const int*)rec_slots, (const int*)seq_lens, (const int*)qsl, C, N, R, out);
     if (rc) return rc;
     CUDA_CHECK_RET(cudaGetLastError());
     return 0;
@@ -811,11 +810,11 @@ GLLM_EXPORT int gllm_seq_selective_scan(const void* xc, const void* dt_raw, cons
   if (is_f32)
     rc = scan_dispatch<float, 1>(N, grid, st, xc, dt_raw, proj, ldp, xz, ldxz, (const float*)A, (const float*)Dskip,
                               (const float*)dt_bias, (float*)state, (const int*)rec_slots, (const int*)seq_lens,
-                              (const int*)qsl, C, N, R, out, max_len);
+                              (const int*)qsl, C, N, R, out);
   else
     rc = scan_dispatch<__nv_bfloat16, 1>(N, grid, st, xc, dt_raw, proj, ldp, xz, ldxz, (const float*)A,
                                       (const float*)Dskip, (const float*)dt_bias, (float*)state,
-                                      (const int*)rec_slots, (const int*)seq_lens, (const int*)qsl, C, N, R, out, max_len);
+                                      (const int*)rec_slots, (const int*)seq_lens, (const int*)qsl, C, N, R, out);
   if (rc) return rc;
   CUDA_CHECK_RET(cudaGetLastError());
   return 0;

@@ -48,7 +48,7 @@ def _L():
             "gllm_seq_routed_experts": [P, G, P, P, P, P, I, I, I, I, P, P, I, I, F, F, I, P],
             "gllm_seq_softcap": [P, G, I, I, F, I, P],
             "gllm_seq_conv_silu": [P, G, I, I, I, P, P, I, P, P, P, P, P, I, I, P, I, P],
-            "gllm_seq_selective_scan": [P, P, P, G, P, G, P, P, P, P, P, P, P, I, I, I, I, P, I, I, I, P],
+            "gllm_seq_selective_scan": [P, P, P, G, P, G, P, P, P, P, P, P, P, I, I, I, I, P, I, I, P],
             "gllm_scan_chunk": [P, P, P, G, P, G] + [P] * 7 + [I] * 7 + [P, P, I, P],
             "gllm_seq_relu2": [P, P, G, I, P],
             "gllm_seq_gemm_simt": [P, G, P, G, P, G, I, I, I, I, P, P],
@@ -249,11 +249,12 @@ _SCAN_WORK_BYTES = 256 << 20        # its workspace at a time; more channels tak
 def selective_scan(xc, dt_raw, proj, xz, a, d_skip, dt_bias, ssm_state, rec_slots, seq_lens, query_start_loc,
                    channels, nstate, dt_rank, max_q_len: Optional[int] = None):
     """With `max_q_len` (the longest portion of the batch, or a bound on it), portions of `_SCAN_MIN_TOKENS` tokens and more run
-    cut in time; the length of a sequence's own portion decides, not what else is in the batch."""
+    cut in time, whatever else is in the batch, and the shorter ones beside them are walked whole in the same launches. Without
+    any of that length, the token-serial kernel takes the batch (the same state, bit for bit; outputs sum their states in
+    another order)."""
     assert xc.is_contiguous() and dt_raw.is_contiguous() and proj.stride(1) == 1 and xz.stride(1) == 1
     assert a.dtype == torch.float32 and a.is_contiguous()
     out = torch.empty_like(xc)
-    max_len = 0
     if max_q_len is not None and max_q_len >= _SCAN_MIN_TOKENS:
         t, slots = xc.shape[0], xc.shape[0] // 64 + seq_lens.shape[0]
         width = max(128, min(channels, _SCAN_WORK_BYTES // (4 * slots * (nstate + 1)) // 128 * 128))
@@ -265,16 +266,14 @@ def selective_scan(xc, dt_raw, proj, xz, a, d_skip, dt_bias, ssm_state, rec_slot
         if rc != 2:                          # 2: more states than a thread holds
             check(rc, "scan_chunk")
             sm100._count(3 * -(-channels // width))
-            if seq_lens.shape[0] == 1 and t >= _SCAN_MIN_TOKENS:      # all rows are the one sequence's
-                return out
-            max_len = _SCAN_MIN_TOKENS - 1
+            return out
     # long chunks of few sequences: 4 threads per channel (more warps in flight); decode-like batches: 1
     nseq = seq_lens.shape[0]
     parts = 4 if (nstate % 4 == 0 and nstate >= 8 and xc.shape[0] >= 16 * nseq and nseq * channels < (1 << 20)) else 1
     check(_L().gllm_seq_selective_scan(_p(xc), _p(dt_raw), _p(proj), proj.stride(0), _p(xz), xz.stride(0), _p(a),
                                        _p(d_skip), _p(dt_bias), _p(ssm_state), _p(rec_slots), _p(seq_lens),
                                        _p(query_start_loc), seq_lens.shape[0], channels, nstate, dt_rank, _p(out),
-                                       _f32(xc), parts, max_len, stream_ptr()), "seq_selective_scan")
+                                       _f32(xc), parts, stream_ptr()), "seq_selective_scan")
     sm100._count()
     return out
 

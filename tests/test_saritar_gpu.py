@@ -242,7 +242,8 @@ def test_scan_cut_in_time(N, C, qlens, ctx):
 
 @pytest.mark.parametrize("lens", [[5], [100], [130], [100, 130]])
 def test_scan_with_a_bound_on_the_lengths(lens):
-    """`max_q_len` may be larger than every portion: each portion is computed, by the kernel that its own length asks for."""
+    """`max_q_len` may be larger than every portion: each portion is computed. A short one is then walked by the cut form's last
+    pass: the same state bit for bit, outputs within one bf16 rounding (their states are summed in another order)."""
     from gllm_b200.ops import sm100_seq as S
     torch.manual_seed(lens[0])
     N, C, R, t, n = 8, 70, 4, sum(lens), len(lens)
@@ -256,7 +257,9 @@ def test_scan_with_a_bound_on_the_lengths(lens):
         st = torch.zeros(n, N, C, device=DEV)
         torch.full((t, C), 3.0, device=DEV).bfloat16()       # what an unwritten output is likely to hold
         got.append((S.selective_scan(x, dtr, proj, xz, A, Dk, db, st, rs, sl, qsl, C, N, R, max_q_len=bound), st))
-    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and bool(got[0][1].abs().sum() > 0)
+    (a, sa), (b, sb) = got
+    assert torch.equal(sa, sb) and bool(sa.abs().sum() > 0)
+    assert bool(((a.float() - b.float()).abs() <= a.float().abs() * 2.0 ** -7 + 1e-6).all())
 
 
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
