@@ -35,11 +35,12 @@ struct SmallMParams {
   float* ws;              // [num_n_tiles * S][128][BT] fp32 partials
   uint32_t* counters;     // [num_n_tiles], zero on entry, self-resetting
   int silu;               // gated epilogue (1: silu, 2: the tanh form of gelu): weight rows interleaved per 128: tile 2g = gate, tile 2g+1 = up
-  int wide_c;             // C and its rows on 8-byte boundaries: four columns per store
   int stages;
   uint32_t tmem_cols;
 };
 
+// WIDE: C and its rows lie on 8-byte boundaries, four columns per store
+template <bool WIDE>
 __global__ void __launch_bounds__(kSmThreads, 1)
 gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                    const SmallMParams p) {
@@ -233,7 +234,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
               const int m = m0 + uu * 4 + mr;
               if (m < p.M) {
                 __nv_bfloat16* dst = p.C + static_cast<size_t>(m) * p.ldc + ncol;
-                if (p.wide_c && ncol + 3 < p.N) {
+                if (WIDE && ncol + 3 < p.N) {
                   *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(acc[uu].x, acc[uu].y), pack_bf16(acc[uu].z, acc[uu].w));
                 } else {
                   const float a[4] = {acc[uu].x, acc[uu].y, acc[uu].z, acc[uu].w};
@@ -273,7 +274,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 const float o2 = act(g[uu].z) * up[uu].z;
                 const float o3 = act(g[uu].w) * up[uu].w;
                 __nv_bfloat16* dst = p.C + static_cast<size_t>(m) * p.ldc + f;
-                if (p.wide_c) {
+                if (WIDE) {
                   *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(o0, o1), pack_bf16(o2, o3));
                 } else {
                   dst[0] = __float2bfloat16(o0); dst[1] = __float2bfloat16(o1);
@@ -354,7 +355,6 @@ GLLM_EXPORT int gllm_gemm_smallm(const void* A, int64_t lda, const void* W, int6
   }
   p.C = reinterpret_cast<__nv_bfloat16*>(C);
   p.ldc = static_cast<int>(ldc);
-  p.wide_c = (ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 7) == 0) ? 1 : 0;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.ws = reinterpret_cast<float*>(ws);
   p.counters = reinterpret_cast<uint32_t*>(counters);
@@ -372,12 +372,14 @@ GLLM_EXPORT int gllm_gemm_smallm(const void* A, int64_t lda, const void* W, int6
   if (make_tmap_2d(&tx, A, M, K, lda * 2, p.BT, kBK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)) return 1;
   static PerDeviceOnce configured;
   if (configured.need()) {
-    CUDA_CHECK_RET(cudaFuncSetAttribute(gemm_smallm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    CUDA_CHECK_RET(cudaFuncSetAttribute(gemm_smallm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    CUDA_CHECK_RET(cudaFuncSetAttribute(gemm_smallm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     configured.done();
   }
   const int units = num_n * p.S;
   const int grid = units < sms ? units : sms;
-  CUDA_CHECK_RET(launch_pdl(gemm_smallm_kernel, dim3(grid), dim3(kSmThreads), smem_bytes,
+  const bool wide = ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 7) == 0;
+  CUDA_CHECK_RET(launch_pdl(wide ? gemm_smallm_kernel<true> : gemm_smallm_kernel<false>, dim3(grid), dim3(kSmThreads), smem_bytes,
                             reinterpret_cast<cudaStream_t>(stream), tw, tx, p));
   return 0;
 }
