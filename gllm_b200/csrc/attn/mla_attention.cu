@@ -160,6 +160,7 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
   if (warp == 0) {
     fetch_page();
     for (int i = 0; i < kMlaStages - 1; ++i) load_tile();
+    guard.first(&full_bar[1]);
   }
 
   const int g = lane >> 2, t = lane & 3;

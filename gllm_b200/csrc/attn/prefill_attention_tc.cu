@@ -314,7 +314,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
           in_o |= 1u << t;
         }
       };
-      bool ok = n_max > 0;
+      bool ok = n_max > 0 && guard.first(&k_full[0]);
       for (int t = 0; t < 2; ++t)
         if (t ? n1 : n0) ok = ok && guard.wait(&q_full[t], 0);
       ok = ok && guard.wait(&k_full[0], 0);

@@ -11,7 +11,7 @@ namespace b200 {
 
 struct WaitConfig {              // part of a kernel's parameters
   uint32_t* word;                // set to 1 when a wait gives up (null: nobody reads it)
-  uint32_t limit_ns;             // at most 2^32 - 1; 0 (tests): a phase that has not completed is given up
+  uint32_t limit_ns;             // at most 2^32 - 1; 0 (tests): a role's first wait is given up
 };
 
 // one per process, set when the library is loaded
@@ -31,8 +31,15 @@ struct WaitGuard {
 
   // true: the phase completed. try_wait suspends the thread in hardware, so the clock is read rarely
   __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity) const {
-    if (cfg.limit_ns != 0 ? mbar_try_wait(bar, parity) : mbar_test_wait(bar, parity)) return true;
+    if (mbar_try_wait(bar, parity)) return true;
     return wait_on(bar, parity);
+  }
+
+  // a role's first wait, looked at once: with a limit of 0 (tests) it is given up unless the phase has completed already
+  __device__ __forceinline__ bool first(uint64_t* bar) const {
+    if (cfg.limit_ns != 0 || mbar_test_wait(bar, 0)) return true;
+    give_up();
+    return false;
   }
 
   // copies and products in flight: they end by themselves, whatever the limit of the waits
@@ -47,15 +54,18 @@ struct WaitGuard {
   }
 
  private:
+  __device__ __forceinline__ void give_up() const {
+    *dead = 1;
+    if (cfg.word != nullptr) {
+      st_relaxed_sys(cfg.word, 1u);
+      __threadfence_system();
+    }
+  }
   __device__ __forceinline__ bool wait_on(uint64_t* bar, uint32_t parity) const {
     const uint32_t t0 = global_ns();
     while (*dead == 0) {
       if (global_ns() - t0 >= cfg.limit_ns) {
-        *dead = 1;
-        if (cfg.word != nullptr) {
-          st_relaxed_sys(cfg.word, 1u);
-          __threadfence_system();
-        }
+        give_up();
         return false;
       }
 #pragma unroll 1

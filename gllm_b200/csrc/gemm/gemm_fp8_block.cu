@@ -157,7 +157,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     if (warp == 1 && lane == 0) {
       constexpr uint32_t idesc = make_idesc_e4m3(kFBM, BN);
       uint32_t it = 0;  // global k-block counter == TMEM hand-off counter
-      bool ok = true;
+      bool ok = guard.first(&full_bar[0]);
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % T::kStages;
