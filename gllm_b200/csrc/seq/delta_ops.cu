@@ -230,11 +230,18 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(
   __syncthreads();
   {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-    for (int s = 0; s < 32; ++s) {
-      const float tv = sT[(32 + xi) * LA + 32 + s];      // zero for s > xi, and sX[s] may be no number there
+    // zero for s > xi, where sX[s] may be no number: a warp's eight rows end with its own eight columns
+    for (int s0 = 0; s0 <= 8 * warp; s0 += 8) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] = s <= xi ? fmaf(-tv, sX[s * LX + xj + e], acc[e]) : acc[e];
+      for (int i = 0; i < 8; ++i) {
+        const int s = s0 + i;
+        const float tv = sT[(32 + xi) * LA + 32 + s];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float x = sX[s * LX + xj + e];
+          acc[e] = fmaf(-tv, s <= xi ? x : 0.f, acc[e]);
+        }
+      }
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) sT[(32 + xi) * LA + xj + e] = acc[e];
@@ -393,12 +400,17 @@ __global__ void __launch_bounds__(256, 1) delta_chunk_kernel(
           mma16816(qs_[nv + 1], aq, r[2], r[3]);
         }
     }
-    bool bad = false;
-    auto number = [&](float x, int row, int col) {
-      if (fabsf(x) <= 3.402823466e38f) return x;
-      bad = true;
-      atomicMin(&s_bad[col], row);
-      return 0.f;
+    uint32_t odd = 0;                               // places of this thread's 16 values that are no numbers
+    auto number = [&](float x, int i, int e) {
+      const bool ok = fabsf(x) <= 3.402823466e38f;
+      odd |= ok ? 0u : 1u << (4 * i + e);
+      return ok ? x : 0.f;
+    };
+    auto note = [&]() {
+      for (uint32_t m = odd; m != 0; m &= m - 1) {
+        const int at = __ffs(m) - 1;
+        atomicMin(&s_bad[(cb + (at >> 2)) * 8 + 2 * t4 + (at & 1)], (at & 2) ? tb : ta);
+      }
     };
     auto put_rows = [&](bf16_t* dst, int i, int row, float x, float y) {
       uint32_t hi, mid, lo;
@@ -415,11 +427,11 @@ __global__ void __launch_bounds__(256, 1) delta_chunk_kernel(
         const int row = r ? tb : ta;
         const float bk = r ? wb.x : wa.x, be = r ? wb.y : wa.y;
         const float2 vv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sV + row * LV + (cb + i) * 8 + 2 * t4));
-        const int col = (cb + i) * 8 + 2 * t4;
-        put_rows(sB, i, row, number(be * vv.x - bk * ks_[i][2 * r], row, col),
-                 number(be * vv.y - bk * ks_[i][2 * r + 1], row, col + 1));
+        put_rows(sB, i, row, number(be * vv.x - bk * ks_[i][2 * r], i, 2 * r),
+                 number(be * vv.y - bk * ks_[i][2 * r + 1], i, 2 * r + 1));
       }
-    __syncthreads();                                // B is complete
+    if (odd != 0) note();
+    const bool dirty = __syncthreads_or(odd != 0);  // B is complete
     uint4 P[4][3];
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk)
@@ -449,17 +461,22 @@ __global__ void __launch_bounds__(256, 1) delta_chunk_kernel(
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
     tri(T, sB);
+    if (dirty) {                                    // a decay or key that is no number is in T's rows, too
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][e] = number(acc[i][e], i, e);
+      if (odd != 0) note();
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const float w = r ? wb.w : wa.w;
-        const int row = r ? tb : ta, col = (cb + i) * 8 + 2 * t4;
-        const float ux = number(acc[i][2 * r], row, col), uy = number(acc[i][2 * r + 1], row, col + 1);
-        put_rows(sU, i, row, ux, uy);
-        put_rows(sW, i, row, w * ux, w * uy);
+        put_rows(sU, i, r ? tb : ta, acc[i][2 * r], acc[i][2 * r + 1]);
+        put_rows(sW, i, r ? tb : ta, w * acc[i][2 * r], w * acc[i][2 * r + 1]);
       }
-    const bool dirty = __syncthreads_or(bad);       // U is complete
+    __syncthreads();                                // U is complete
     // ---- o = exp(L) Q S + P U
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
