@@ -306,12 +306,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         const int low = p.window > 0 ? ctx_len + tok0 - p.window + 1 - key0 : 0;
         const uint32_t v_addr = smem_u32(smem + SM::kVOff + (tile % SM::kVStages) * SM::kVBytes);
         const uint64_t dv = make_sw128_desc(v_addr, (KV * 128) >> 4, 1024 >> 4);
+        const uint32_t o_tmem = tmem + SM::kTmemO + t * DV, p_tmem = tmem + t * KV;
+        const uint32_t acc = (in_o >> t) & 1u;
+        if (end >= KV && low <= 0) {                     // all but the first and the last tiles
 #pragma unroll
-        for (int kk = 0; kk < KV / 16; ++kk) {           // 16 keys per step: 8 columns of P, 16 rows of V
-          if (kk * 16 >= end || kk * 16 + 15 < low) continue;
-          umma_bf16_ts(tmem + SM::kTmemO + t * DV, tmem + t * KV + kk * 8, dv + static_cast<uint64_t>(kk) * (2048 >> 4), idesc_pv,
-                       (in_o >> t) & 1u);
+          for (int kk = 0; kk < KV / 16; ++kk)           // 16 keys per step: 8 columns of P, 16 rows of V
+            umma_bf16_ts(o_tmem, p_tmem + kk * 8, dv + static_cast<uint64_t>(kk) * (2048 >> 4), idesc_pv, kk != 0 ? 1u : acc);
           in_o |= 1u << t;
+        } else {
+          const int k0 = max(low, 0) / 16, k1 = min((end + 15) / 16, KV / 16);
+#pragma unroll 1
+          for (int kk = k0; kk < k1; ++kk)
+            umma_bf16_ts(o_tmem, p_tmem + kk * 8, dv + static_cast<uint64_t>(kk) * (2048 >> 4), idesc_pv, kk != k0 ? 1u : acc);
+          if (k0 < k1) in_o |= 1u << t;
         }
       };
       bool ok = n_max > 0 && guard.first(&k_full[0]);
