@@ -363,11 +363,13 @@ __global__ void conv_silu_kernel(const T* __restrict__ xz, long ldxz, int C, con
 
 // The same convolution for bf16 rows whose channels come in aligned groups of 4: a thread owns 4 channels (8-byte loads
 // and stores, weights in registers: 8 channels would halve the occupancy) and walks `rows` consecutive batch rows with
-// the last TAPS - 1 inputs in registers, so every input row is read once per block instead of TAPS times. The next four
-// rows' loads are in flight while four are computed (6000 rows of 8192 channels: 105 -> 86 us against one row ahead).
+// the last TAPS - 1 inputs in registers, so every input row is read once per block instead of TAPS times. The next kAhead
+// rows' loads are in flight while as many are computed: four in long batches (6000 rows of 8192 channels: 105 -> 86 us against one
+// row ahead), one in short ones, whose blocks have a row or eight (200 single tokens: 18.6 us with four, 16.3 with one; 900 rows
+// 17.3 / 16.3).
 // Sequences of one token also update their carried inputs here (longer ones: the kernel
 // below, after every block has read them).
-template <int TAPS>
+template <int TAPS, int kAhead>
 __global__ void __launch_bounds__(128) conv_silu_vec_kernel(
     const __nv_bfloat16* __restrict__ xz, long ldxz, int C, const float* __restrict__ w, const float* __restrict__ b,
     __nv_bfloat16* __restrict__ state, const int* __restrict__ rec_slots, const int* __restrict__ seq_lens,
@@ -394,7 +396,6 @@ __global__ void __launch_bounds__(128) conv_silu_vec_kernel(
   };
   float win[TAPS][4];                            // win[0 .. TAPS-2]: inputs before the row; win[TAPS-1]: the row's own
   int s = find_seq(qsl, nseq, t0), q0 = 0, q1 = -1;
-  constexpr int kAhead = 4;
   uint2 q[kAhead], q2[kAhead];
   auto fetch = [&](int tb, uint2 (&v)[kAhead]) {
 #pragma unroll
@@ -762,7 +763,7 @@ GLLM_EXPORT int gllm_seq_conv_silu(const void* xz, long ldxz, int ntok, int nseq
     const int rows = ntok >= 2048 ? 16 : (ntok >= 512 ? 8 : 1);
     dim3 vgrid((ntok + rows - 1) / rows, (C / 4 + 127) / 128);
 #define GLLM_CONV_VEC(TAPS)                                                                                        \
-  conv_silu_vec_kernel<TAPS><<<vgrid, 128, 0, st>>>(                                                               \
+  (rows == 16 ? conv_silu_vec_kernel<TAPS, 4> : conv_silu_vec_kernel<TAPS, 1>)<<<vgrid, 128, 0, st>>>(              \
       (const __nv_bfloat16*)xz, ldxz, C, (const float*)w, (const float*)b, (__nv_bfloat16*)state,                  \
       (const int*)rec_slots, (const int*)seq_lens, (const int*)qsl, nseq, ntok, rows, (__nv_bfloat16*)out, act,    \
       (const float*)in_bias)
