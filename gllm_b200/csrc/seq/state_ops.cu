@@ -439,12 +439,13 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ o, int n, cons
 
 // The same for bf16 rows whose groups are 128 or 256 wide and lie on 8-byte boundaries (o: 16): 16- and 8-byte accesses, and a
 // warp has the loads of 4 x 128 columns in flight, where 4-byte loads of one group at a time were bound by their latency.
-// 6000 tokens x 32 groups of 128: 97 -> 58 us.
-template <int NCH>
+// 6000 tokens x 32 groups of 128: 97 -> 58 us. Where the groups do not fill the machine, four in a row only make a warp slower
+// (one token, 32 groups of 128: 3.2 us element-wise, 4.1 with four): one group per warp there.
+template <int NCH, int kRows>
 __global__ void __launch_bounds__(128) gated_group_norm_vec_kernel(
     const float* __restrict__ o, int n, const __nv_bfloat16* __restrict__ gate, long ldg, const __nv_bfloat16* __restrict__ w,
     int wlen, float eps, int act, float out_scale, __nv_bfloat16* __restrict__ out, long ldo, int ntok) {
-  constexpr int kGroup = 128 * NCH, kRows = 4 / NCH;
+  constexpr int kGroup = 128 * NCH;
   const int lane = threadIdx.x & 31, ngroups = n / kGroup;
   const long g0 = ((long)blockIdx.x * 4 + (threadIdx.x >> 5)) * kRows, total = (long)ntok * ngroups;
   if (g0 >= total) return;
@@ -916,8 +917,9 @@ GLLM_EXPORT int gllm_seq_gated_group_norm(const void* o, int n, const void* gate
   const long warps = (long)ntok * (n / group);
   if (!is_f32 && (group == 128 || group == 256) && ((uintptr_t)o & 15) == 0 && wlen % 4 == 0 && ldg % 4 == 0 && ldo % 4 == 0 &&
       (((uintptr_t)gate | (uintptr_t)w | (uintptr_t)out) & 7) == 0) {
-    const unsigned vblocks = (unsigned)((warps * (group / 128) + 15) / 16);
-    auto run = group == 128 ? gated_group_norm_vec_kernel<1> : gated_group_norm_vec_kernel<2>;
+    const bool few = group == 128 && warps < 64 * b200::num_sms();
+    const unsigned vblocks = (unsigned)(few ? (warps + 3) / 4 : (warps * (group / 128) + 15) / 16);
+    auto run = few ? gated_group_norm_vec_kernel<1, 1> : group == 128 ? gated_group_norm_vec_kernel<1, 4> : gated_group_norm_vec_kernel<2, 2>;
     run<<<vblocks, 128, 0, st>>>((const float*)o, n, (const __nv_bfloat16*)gate, ldg, (const __nv_bfloat16*)w, wlen, eps, act,
                                  out_scale, (__nv_bfloat16*)out, ldo, ntok);
     CUDA_CHECK_RET(cudaGetLastError());
