@@ -89,42 +89,86 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
     *dead = 0;
     fence_mbar_init();
   }
-  const int per = (p.tokens + kMlaThreads - 1) / kMlaThreads;          // tokens scanned by one thread
-  const int s0 = min(static_cast<int>(threadIdx.x) * per, p.tokens), s1 = min(s0 + per, p.tokens);
-  int own = 0;
-  for (int i = s0; i < s1; ++i) own += MlaSpan(p, i).n;
-  int upto = own;
+  int tok, grp, off, t0, t1, share, last_cta = -1;
+  const int grid = static_cast<int>(gridDim.x), cta = static_cast<int>(blockIdx.x);
+  if (p.tokens <= 32) {
+    // A lane per token, every warp for itself. Where each (token, heads) can have whole shares, none begins inside another's: a CTA
+    // that goes on into the next one waits for its queries once more (4 tokens of 300 keys, 16 heads: 14.6 us against 11.4).
+    const int own = lane < p.tokens ? MlaSpan(p, lane).n : 0;
+    auto upto = [&](int v) {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, upto, o);
-    if (lane >= o) upto += v;
-  }
-  if (lane == 31) warp_sum[warp] = upto;
-  __syncthreads();
-  int total = 0, before = upto - own;
-#pragma unroll
-  for (int w = 0; w < kMlaWarps; ++w) {
-    if (w < warp) before += warp_sum[w];
-    total += warp_sum[w];
-  }
-  total *= hg;
-  const int share = max((total + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x), kMlaMinTiles);
-  const int t0 = min(static_cast<int>(blockIdx.x) * share, total), t1 = min(t0 + share, total);
-  if (t0 >= t1) {
-    if (threadIdx.x == 0) p.meta[blockIdx.x] = make_int4(-1, 0, 0, 0);
-    return;
-  }
-  if (t0 >= before * hg && t0 < (before + own) * hg) {                 // one thread: the token that the share starts in
-    int tok = s0, acc = before, n = MlaSpan(p, s0).n;
-    while (t0 >= (acc + n) * hg) {
-      acc += n;
-      n = MlaSpan(p, ++tok).n;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+      }
+      return v;
+    };
+    const int to = upto(own), total = __shfl_sync(0xffffffffu, to, 31) * hg;
+    share = max((total + grid - 1) / grid, kMlaMinTiles);
+    const int parts = (own + share - 1) / share, pto = upto(parts);
+    const bool aligned = __shfl_sync(0xffffffffu, pto, 31) * hg <= grid;
+    const int at = aligned ? cta : cta * share, from = (aligned ? pto - parts : to - own) * hg, width = aligned ? parts : own;
+    const uint32_t mine = __ballot_sync(0xffffffffu, at >= from && at < from + width * hg);
+    if (mine == 0) {                                                   // idle, and so all of the block
+      if (threadIdx.x == 0) p.meta[cta] = make_int4(-1, 0, 0, 0);
+      return;
     }
-    const int in = t0 - acc * hg;
-    first[0] = tok; first[1] = in / n; first[2] = in % n;
+    tok = __ffs(mine) - 1;
+    const int in = at - __shfl_sync(0xffffffffu, from, tok), w = __shfl_sync(0xffffffffu, width, tok),
+              n = __shfl_sync(0xffffffffu, own, tok);
+    grp = in / w;
+    if (aligned) {
+      off = in % w * share;
+      t0 = 0;
+      t1 = min(share, n - off);
+      last_cta = cta + w - 1 - in % w;
+    } else {
+      off = in % w;
+      t0 = at;
+      t1 = min(t0 + share, total);
+    }
+    __syncthreads();                                                   // the barriers are initialised
+  } else {
+    const int per = (p.tokens + kMlaThreads - 1) / kMlaThreads;        // tokens scanned by one thread
+    const int s0 = min(static_cast<int>(threadIdx.x) * per, p.tokens), s1 = min(s0 + per, p.tokens);
+    int own = 0;
+    for (int i = s0; i < s1; ++i) own += MlaSpan(p, i).n;
+    int upto = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    if (lane == 31) warp_sum[warp] = upto;
+    __syncthreads();
+    int total = 0, before = upto - own;
+#pragma unroll
+    for (int w = 0; w < kMlaWarps; ++w) {
+      if (w < warp) before += warp_sum[w];
+      total += warp_sum[w];
+    }
+    total *= hg;
+    share = max((total + grid - 1) / grid, kMlaMinTiles);
+    t0 = min(cta * share, total);
+    t1 = min(t0 + share, total);
+    if (t0 >= t1) {
+      if (threadIdx.x == 0) p.meta[cta] = make_int4(-1, 0, 0, 0);
+      return;
+    }
+    if (t0 >= before * hg && t0 < (before + own) * hg) {               // one thread: the token that the share starts in
+      int at = s0, acc = before, n = MlaSpan(p, s0).n;
+      while (t0 >= (acc + n) * hg) {
+        acc += n;
+        n = MlaSpan(p, ++at).n;
+      }
+      const int in = t0 - acc * hg;
+      first[0] = at; first[1] = in / n; first[2] = in % n;
+    }
+    __syncthreads();
+    tok = first[0];
+    grp = first[1];
+    off = first[2];
   }
-  __syncthreads();
-  int tok = first[0], grp = first[1], off = first[2];
 
   // ---------------- copies, issued by warp 0: one TMA box per page, K == V, two tiles ahead of the products ----------------
   const int page_bytes = p.page_size * kLat * 2, slab = p.page_size * 128;
@@ -187,7 +231,7 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
     const int len = min(span.n - off, t1 - cur);
     const bool whole = off == 0 && len == span.n;
     const int slot = 2 * blockIdx.x + (cur == t0 ? 0 : 1);
-    if (off == 0 && !whole) meta = make_int4(tok, grp, (cur + span.n - 1) / share, slot);
+    if (off == 0 && !whole) meta = make_int4(tok, grp, last_cta >= 0 ? last_cta : (cur + span.n - 1) / share, slot);
     const int hbase = grp * 16, n_rows = min(16, p.H - hbase);
     uint32_t qa[kLat / 32][4];                        // Q fragments of this warp's columns; rows beyond the head count are zero
     {
