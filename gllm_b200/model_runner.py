@@ -11,6 +11,7 @@ copy issued asynchronously), or the (hidden, residual) views to ship to the next
 """
 from __future__ import annotations
 
+import gc
 import os
 import time
 from dataclasses import dataclass
@@ -249,7 +250,18 @@ class ModelRunner:
         return h, r
 
     def capture_graphs(self):
-        """Decode-only batches replay a CUDA graph per power-of-two bucket (forward -> logits)."""
+        """Decode-only batches replay a CUDA graph per power-of-two bucket (forward -> logits). The collector stays out of it:
+        a graph of an engine that is gone, destroyed by a collection during a capture, invalidates that capture."""
+        gc.collect()
+        was = gc.isenabled()
+        gc.disable()
+        try:
+            self._capture_graphs()
+        finally:
+            if was:
+                gc.enable()
+
+    def _capture_graphs(self):
         inp = self.input_data
         self.graph_pool = None
         self.graph_logits: Dict[int, torch.Tensor] = {}

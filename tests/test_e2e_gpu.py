@@ -91,6 +91,38 @@ def test_qwen3_vl_gpu_matches_cpu_engine():
     assert [x[0] for x in outs["cpu"]] == [x[0] for x in outs["cuda"]], outs
 
 
+def test_collected_graphs_do_not_disturb_a_capture():
+    """A graph held by a reference cycle, and a collector that would run at every allocation: the engine's captures stand."""
+    import gc
+    from gllm_b200 import LLM
+    from gllm_b200.models.presets import tiny
+
+    class Cycle:
+        pass
+
+    def leave_a_graph():
+        x, g, c = torch.zeros(4, device="cuda"), torch.cuda.CUDAGraph(), Cycle()
+        with torch.cuda.graph(g):
+            x += 1
+        c.me, c.graph = c, g
+
+    old = gc.get_threshold()
+    gc.disable()
+    try:
+        for _ in range(4):
+            leave_a_graph()
+        gc.enable()
+        gc.set_threshold(1, 1, 1)
+        llm = LLM(tiny("Qwen3ForCausalLM", hidden_size=256, head_dim=64, torch_dtype="bfloat16"), load_format="dummy",
+                  num_gpu_pages=64, model_max_length=128, max_cuda_graph_bs=2, log_stats=False)
+        out = llm.generate(tokens=[[1, 2, 3]], output_lens=[4], ignore_eos=True)
+        assert len(out[0].token_ids) == 7 and gc.isenabled()
+        llm.shutdown()
+    finally:
+        gc.set_threshold(*old)
+        gc.enable()
+
+
 def test_deepseek_mla_gpu_matches_cpu_engine():
     """DeepSeek-V3 style model (MLA latent cache 512+64, grouped top-k MoE with a shared expert): the sm_100a
     absorbed-MLA kernel path with CUDA graphs vs the PyTorch expanded-form oracle on the CPU."""
