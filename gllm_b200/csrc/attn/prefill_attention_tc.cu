@@ -172,6 +172,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   uint64_t* mma_end = q_full + 2;                      // [1]       every product has finished
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_end + 1);
   const WaitGuard guard{tmem_slot + 1, p.waits};
+  volatile int* sees = reinterpret_cast<int*>(tmem_slot + 2);   // [2 tiles][low, end): keys that a query tile sees, from tile0 on
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int seq = blockIdx.y + p.seq_offset;
@@ -197,15 +198,69 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   };
   const int n0 = tiles_of(0), n1 = tiles_of(1), n_max = max(n0, n1);
 
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < SM::kKStages; ++i) mbar_init(&k_full[i], 1);
-    for (int i = 0; i < SM::kVStages; ++i) mbar_init(&v_full[i], 1);
-    mbar_init(s_full, 1);
-    for (int i = 0; i < 4; ++i) mbar_init(&step[i], 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&p_full[i], 4); mbar_init(&q_full[i], 1); }
-    mbar_init(mma_end, 1);
-    *guard.dead = 0;
-    fence_mbar_init();
+  // One lane per box (DENSE: per slab). The block-table entries are fetched one tile ahead: read where it is used, each
+  // cost the copies of a tile some 470 cycles, and with 16-token pages that chain alone took as long as four softmax tiles.
+  const int box = min(p.page_size, 64);                // rows of a box
+  const int boxes = DENSE ? 1 : KV / box;
+  const int j = lane % boxes, sl = lane / boxes;       // this lane's box and 64-wide slab
+  const int32_t* bt = p.block_table + static_cast<size_t>(seq) * p.max_blocks;
+  const int last_page = (seq_len - 1) / p.page_size;
+  const int row0 = DENSE ? p.kv_row[blockIdx.y] : 0;
+  auto page_of = [&](int tile) {                       // masked columns read the last page: keep the data finite
+    return DENSE ? 0 : bt[min(((tile0 + tile) * KV + j * box) / p.page_size, last_page)];
+  };
+  // Boxes of the last K / V tile that hold a key some query of this CTA sees, in steps of 16 keys (a step of the product with V); the
+  // others stay out. (Worked out per tile, the division held the copies up by 6 to 9 % in long prompts.)
+  const int rows_last = min((ctx_len + min(tok_cta + toks_per_cta, q_len) - (tile0 + n_max - 1) * KV + 15) & ~15, KV);
+  const int boxes_last = DENSE ? 1 : min((rows_last + box - 1) / box, boxes);
+  auto load = [&](int tile, int page, uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int width, bool is_v) {
+    const int n = tile + 1 < n_max ? boxes : boxes_last;
+    if (lane == 0) mbar_expect_tx(bar, (DENSE ? KV : n * box) * width * 2);
+    __syncwarp();
+    if (sl >= width / 64 || j >= n) return;
+    if constexpr (DENSE) {
+      const int row = row0 + (tile0 + tile) * KV;
+      if (sl < 2) tma_load_2d(dst + sl * (KV * 128), map, bar, kvh * 256 + (is_v ? 128 : 0) + sl * 64, row, kEvictNormal);
+      else tma_load_2d(dst + sl * (KV * 128), &tmap_pe, bar, 0, row, kEvictNormal);
+    } else {
+      tma_load_3d(dst + sl * (KV * 128) + j * box * 128, map, bar, 0, ((tile0 + tile) * KV + j * box) % p.page_size,
+                  (page * p.Hkv + kvh) * (width / 64) + sl);
+    }
+  };
+  auto load_q = [&](int t) {                           // rows tok * GP + head of a query tile, 64 columns per box
+    if ((t ? n1 : n0) == 0) return;
+    if (lane == 0) mbar_expect_tx(&q_full[t], SM::kQBytes);
+    __syncwarp();
+    if (lane < DK / 64)
+      tma_load_3d(smem + t * SM::kQBytes + lane * (kTcRows * 128), &tmap_q, &q_full[t], lane * 64, hbase,
+                  q_begin + tok_cta + t * toks_per_tile);
+  };
+  int page = 0;                                        // of the K tile to come
+  if (warp == kTcSoftmaxWarps) {
+    // The first copies are on their way while the others wait for tensor memory.
+    if (lane < 3) tma_prefetch_desc(lane == 0 ? &tmap_q : lane == 1 ? &tmap_k : DENSE ? &tmap_pe : &tmap_v);
+    if (n_max > 0) page = page_of(0);
+    if (lane == 0) {
+      for (int i = 0; i < SM::kKStages; ++i) mbar_init(&k_full[i], 1);
+      for (int i = 0; i < SM::kVStages; ++i) mbar_init(&v_full[i], 1);
+      mbar_init(s_full, 1);
+      for (int i = 0; i < 4; ++i) mbar_init(&step[i], 1);
+      for (int i = 0; i < 2; ++i) { mbar_init(&p_full[i], 4); mbar_init(&q_full[i], 1); }
+      mbar_init(mma_end, 1);
+      *guard.dead = 0;
+      for (int t = 0; t < 2; ++t) {
+        const int tok0 = tok_cta + t * toks_per_tile;
+        sees[2 * t] = p.window > 0 ? max(ctx_len + tok0 - p.window + 1 - tile0 * KV, 0) : 0;
+        sees[2 * t + 1] = ctx_len + min(tok0 + toks_per_tile, q_len) - tile0 * KV;
+      }
+      fence_mbar_init();
+    }
+    __syncwarp();
+    if (n_max > 0) {
+      load_q(0);
+      load(0, page, smem + SM::kKOff, &tmap_k, &k_full[0], DK, false);
+      load_q(1);
+    }
   }
   if (warp == kTcSoftmaxWarps + 1) tmem_alloc<1>(tmem_slot, SM::kTmemCols);
   tc_fence_before();
@@ -217,62 +272,25 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTcRegsIssue));
     if (warp == kTcSoftmaxWarps) {
       // ------------------------------------------------------------------ TMA producer
-      // One lane per box (DENSE: per slab). The block-table entries are fetched one tile ahead: read where it is used, each
-      // cost the copies of a tile some 470 cycles, and with 16-token pages that chain alone took as long as four softmax tiles.
-      const int box = min(p.page_size, 64);                // rows of a box
-      const int boxes = DENSE ? 1 : KV / box;
-      const int j = lane % boxes, sl = lane / boxes;       // this lane's box and 64-wide slab
-      const bool has_k = sl < DK / 64, has_v = sl < DV / 64;
-      const int32_t* bt = p.block_table + static_cast<size_t>(seq) * p.max_blocks;
-      const int last_page = (seq_len - 1) / p.page_size;
-      const int row0 = DENSE ? p.kv_row[blockIdx.y] : 0;
-      auto page_of = [&](int tile) {                       // masked columns read the last page: keep the data finite
-        return DENSE ? 0 : bt[min(((tile0 + tile) * KV + j * box) / p.page_size, last_page)];
-      };
-      auto load = [&](int tile, int page, uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int width, bool is_v) {
-        if constexpr (DENSE) {
-          const int row = row0 + (tile0 + tile) * KV;
-          if (sl < 2) tma_load_2d(dst + sl * (KV * 128), map, bar, kvh * 256 + (is_v ? 128 : 0) + sl * 64, row, kEvictNormal);
-          else tma_load_2d(dst + sl * (KV * 128), &tmap_pe, bar, 0, row, kEvictNormal);
-        } else {
-          tma_load_3d(dst + sl * (KV * 128) + j * box * 128, map, bar, 0, ((tile0 + tile) * KV + j * box) % p.page_size,
-                      (page * p.Hkv + kvh) * (width / 64) + sl);
-        }
-      };
-      auto load_q = [&](int t) {                           // rows tok * GP + head of a query tile, 64 columns per box
-        if ((t ? n1 : n0) == 0) return;
-        if (lane == 0) mbar_expect_tx(&q_full[t], SM::kQBytes);
-        __syncwarp();
-        if (lane < DK / 64)
-          tma_load_3d(smem + t * SM::kQBytes + lane * (kTcRows * 128), &tmap_q, &q_full[t], lane * 64, hbase,
-                      q_begin + tok_cta + t * toks_per_tile);
-      };
-      load_q(0);
       auto after_step = [&](int j) { return j < 0 || guard.wait(&step[j & 3], (j >> 2) & 1); };
-      int tk = 0, tv = 0, page_v = 0;                      // tiles issued
+      int tk = n_max > 0 ? 1 : 0, tv = 0;                  // tiles issued
       bool ok = true;
-      int page = n_max > 0 ? page_of(0) : 0;               // of the K tile to come, and of the V tile behind it
-      for (int tile = 0; tile <= n_max && n_max > 0; ++tile) {
+      int page_v = page;
+      page = n_max > 1 ? page_of(1) : 0;
+      for (int tile = 1; tile <= n_max; ++tile) {
         const int next = tile + 1 < n_max ? page_of(tile + 1) : 0;
         if (tile < n_max) {                                // K_tile
           const int ks = tile % SM::kKStages;
           ok = __all_sync(0xffffffffu, after_step(tile - SM::kKStages));
           if (!ok) break;
-          if (lane == 0) mbar_expect_tx(&k_full[ks], SM::kKBytes);
-          __syncwarp();
-          if (has_k) load(tile, page, smem + SM::kKOff + ks * SM::kKBytes, &tmap_k, &k_full[ks], DK, false);
+          load(tile, page, smem + SM::kKOff + ks * SM::kKBytes, &tmap_k, &k_full[ks], DK, false);
           ++tk;
-          if (tile == 0) load_q(1);
         }
-        if (tile > 0) {                                    // V_tile-1
-          const int v = tile - 1, vs = v % SM::kVStages;
-          ok = __all_sync(0xffffffffu, after_step(v - SM::kVStages + 1));
-          if (!ok) break;
-          if (lane == 0) mbar_expect_tx(&v_full[vs], SM::kVBytes);
-          __syncwarp();
-          if (has_v) load(v, page_v, smem + SM::kVOff + vs * SM::kVBytes, &tmap_v, &v_full[vs], DV, true);
-          ++tv;
-        }
+        const int v = tile - 1, vs = v % SM::kVStages;     // V_tile-1
+        ok = __all_sync(0xffffffffu, after_step(v - SM::kVStages + 1));
+        if (!ok) break;
+        load(v, page_v, smem + SM::kVOff + vs * SM::kVBytes, &tmap_v, &v_full[vs], DV, true);
+        ++tv;
         page_v = page;
         page = next;
       }
@@ -299,26 +317,21 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       };
       // Only the 16-key steps that some row of the query tile sees: a masked key has P = 0, but 0 times a value that is no
       // number is none either, so keys behind the tile's last token (or before its window) stay out of the product.
-      uint32_t in_o = 0;                                   // bit t: O of query tile t has been written
-      auto issue_pv = [&](int t, int tile) {
-        const int tok0 = tok_cta + t * toks_per_tile, key0 = (tile0 + tile) * KV;
-        const int end = ctx_len + min(tok0 + toks_per_tile, q_len) - key0;
-        const int low = p.window > 0 ? ctx_len + tok0 - p.window + 1 - key0 : 0;
+      // (The range is kept in shared memory: in registers it made this role spill.)
+      auto issue_pv = [&](int t, int tile, int low, int end) {
         const uint32_t v_addr = smem_u32(smem + SM::kVOff + (tile % SM::kVStages) * SM::kVBytes);
         const uint64_t dv = make_sw128_desc(v_addr, (KV * 128) >> 4, 1024 >> 4);
         const uint32_t o_tmem = tmem + SM::kTmemO + t * DV, p_tmem = tmem + t * KV;
-        const uint32_t acc = (in_o >> t) & 1u;
+        const uint32_t acc = low < 0 ? 1u : 0u;          // an earlier tile wrote O
         if (end >= KV && low <= 0) {                     // all but the first and the last tiles
 #pragma unroll
           for (int kk = 0; kk < KV / 16; ++kk)           // 16 keys per step: 8 columns of P, 16 rows of V
             umma_bf16_ts(o_tmem, p_tmem + kk * 8, dv + static_cast<uint64_t>(kk) * (2048 >> 4), idesc_pv, kk != 0 ? 1u : acc);
-          in_o |= 1u << t;
         } else {
           const int k0 = max(low, 0) / 16, k1 = min((end + 15) / 16, KV / 16);
 #pragma unroll 1
           for (int kk = k0; kk < k1; ++kk)
             umma_bf16_ts(o_tmem, p_tmem + kk * 8, dv + static_cast<uint64_t>(kk) * (2048 >> 4), idesc_pv, kk != k0 ? 1u : acc);
-          if (k0 < k1) in_o |= 1u << t;
         }
       };
       bool ok = n_max > 0 && guard.first(&k_full[0]);
@@ -337,10 +350,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         for (int t = 0; t < 2 && ok; ++t) {
           const int n = t ? n1 : n0;
           if (tile < n) {
+            const int low = sees[2 * t] - tile * KV, end = sees[2 * t + 1] - tile * KV;
             ok = guard.wait(&p_full[t], tile & 1);
             if (!ok) break;
             tc_fence_after();
-            issue_pv(t, tile);
+            issue_pv(t, tile, low, end);
             if (tile + 1 < n) issue_s(t, tile + 1);
             if (t == 0) umma_commit(s_full);
           }
@@ -393,6 +407,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       };
       const uint32_t t_s = tmem + lane_base + qt * KV, t_o = tmem_o + lane_base;
       constexpr bool kRaw = BIAS == kNoBias && !CAP;
+      const int left_last = ctx_len + last_tok + 1 - (tile0 + n_tiles - 1) * KV;      // keys that the query tile sees of its last tile
+      const bool short_last = !DENSE && left_last <= KV / 2;   // tiles of 64 keys gain nothing by it
       for (int tile = 0; tile < n_tiles; ++tile) {
         // smallest distance of the tile (uniform over the query tile); at the table's end every score gets the same entry
         const int d0 = ctx_len + tok_base - ((tile0 + tile) * KV + KV - 1);
@@ -403,6 +419,70 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         const bool need_mask = key0 + KV - 1 > ctx_len + tok_base ||
                                (p.window > 0 && key0 < ctx_len + last_tok - p.window + 1);
         await(tile);
+        // the reference of the exponents follows the row's maximum only in steps of 2^8: P, l and O are all relative to it
+        auto follow = [&](float m_new) {
+          float alpha = 1.f;
+          if (m_new > m_run + kTcLazy) {
+            alpha = exp2f(m_run - m_new);
+            m_run = m_new;
+          }
+          if (tile > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+#pragma unroll 1
+            for (int c = 0; c < DV; c += 16) {
+              uint32_t v[16];
+              tmem_ld_32x16(t_o + c, v);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * alpha);
+              tmem_st_32x16(t_o + c, v);
+            }
+          }
+          return alpha;
+        };
+        if (short_last && tile + 1 == n_tiles) {
+          // A last tile that is half empty or more (all there is of a short prompt): 32 keys at a time, S read twice, nothing
+          // done for the rest, which the product leaves out too.
+          const int groups = (left_last + 31) / 32;
+          auto score = [&](uint32_t raw, int c) {
+            float x = __uint_as_float(raw);
+            if (BIAS == kTableBias) x = fmaf(x, p.scale_log2, far_tile ? b1 : trow[(KV - 1 - c) * p.GP]);
+            else if (BIAS == kLogBias) x = fmaf(x, p.scale_log2, -dist_bias_log2(b1, b2, lim - (key0 + c)));
+            else if (CAP) x = p.cap_log2 * tanh_exp(x * p.scale_over_cap);
+            return key0 + c > lim || key0 + c < low ? -INFINITY : x;
+          };
+          float mx = -INFINITY;
+#pragma unroll 1
+          for (int g = 0; g < groups; ++g) {
+            uint32_t v[32];
+            tmem_ld_32x32(t_s + g * 32, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) mx = fmaxf(mx, score(v[e], g * 32 + e));
+          }
+          const float alpha = follow(fmaxf(m_run, kRaw ? mx * p.scale_log2 : mx));
+          const float m_use = m_run == -INFINITY ? 0.f : m_run;
+          float sum = 0.f;
+#pragma unroll 1
+          for (int g = 0; g < groups; ++g) {
+            uint32_t v[32], pk[16];
+            tmem_ld_32x32(t_s + g * 32, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              const float y0 = exp2f(fmaf(score(v[2 * e], g * 32 + 2 * e), kRaw ? p.scale_log2 : 1.f, -m_use)),
+                          y1 = exp2f(fmaf(score(v[2 * e + 1], g * 32 + 2 * e + 1), kRaw ? p.scale_log2 : 1.f, -m_use));
+              sum += y0 + y1;
+              pk[e] = pack_bf16(y0, y1);
+            }
+            tmem_st_32x16(t_s + g * 16, pk);               // into columns whose scores have been read
+          }
+          l_run = l_run * alpha + sum;
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&p_full[qt]);
+          continue;
+        }
         // the whole row of the tile stays in registers: S leaves TMEM once
         float f[KV];
         {
@@ -438,24 +518,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
           for (int i = 0; i < 4; ++i) m4[i] = fmaxf(m4[i], e + 4 < KV ? fmaxf(f[e + i], f[e + 4 + i]) : f[e + i]);
         }
         const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-        // the reference of the exponents follows the row's maximum only in steps of 2^8: P, l and O are all relative to it
-        const float m_new = fmaxf(m_run, kRaw ? mx * p.scale_log2 : mx);
-        float alpha = 1.f;
-        if (m_new > m_run + kTcLazy) {
-          alpha = exp2f(m_run - m_new);
-          m_run = m_new;
-        }
-        if (tile > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-#pragma unroll 1
-          for (int c = 0; c < DV; c += 16) {
-            uint32_t v[16];
-            tmem_ld_32x16(t_o + c, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int e = 0; e < 16; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) * alpha);
-            tmem_st_32x16(t_o + c, v);
-          }
-        }
+        const float alpha = follow(fmaxf(m_run, kRaw ? mx * p.scale_log2 : mx));
         const float m_use = m_run == -INFINITY ? 0.f : m_run;
         const uint64_t sc2 = pack2(kRaw ? p.scale_log2 : 1.f, kRaw ? p.scale_log2 : 1.f), nm2 = pack2(-m_use, -m_use);
         uint64_t sum2[2] = {0, 0};
