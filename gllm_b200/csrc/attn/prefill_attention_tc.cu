@@ -317,13 +317,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       };
       // Only the 16-key steps that some row of the query tile sees: a masked key has P = 0, but 0 times a value that is no
       // number is none either, so keys behind the tile's last token (or before its window) stay out of the product.
-      // (The range is kept in shared memory: in registers it made this role spill.)
+      // (The range is kept in shared memory: in registers it made this role spill.) DENSE takes its tiles of 64 keys whole, as the
+      // absorbed form does: with a range the prompts of 4096 tokens, 16 heads, take 427 us instead of 419.
       auto issue_pv = [&](int t, int tile, int low, int end) {
         const uint32_t v_addr = smem_u32(smem + SM::kVOff + (tile % SM::kVStages) * SM::kVBytes);
         const uint64_t dv = make_sw128_desc(v_addr, (KV * 128) >> 4, 1024 >> 4);
         const uint32_t o_tmem = tmem + SM::kTmemO + t * DV, p_tmem = tmem + t * KV;
         const uint32_t acc = low < 0 ? 1u : 0u;          // an earlier tile wrote O
-        if (end >= KV && low <= 0) {                     // all but the first and the last tiles
+        if (DENSE || (end >= KV && low <= 0)) {          // all but the first and the last tiles
 #pragma unroll
           for (int kk = 0; kk < KV / 16; ++kk)           // 16 keys per step: 8 columns of P, 16 rows of V
             umma_bf16_ts(o_tmem, p_tmem + kk * 8, dv + static_cast<uint64_t>(kk) * (2048 >> 4), idesc_pv, kk != 0 ? 1u : acc);
@@ -350,7 +351,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         for (int t = 0; t < 2 && ok; ++t) {
           const int n = t ? n1 : n0;
           if (tile < n) {
-            const int low = sees[2 * t] - tile * KV, end = sees[2 * t + 1] - tile * KV;
+            const int low = DENSE ? -tile : sees[2 * t] - tile * KV, end = DENSE ? KV : sees[2 * t + 1] - tile * KV;
             ok = guard.wait(&p_full[t], tile & 1);
             if (!ok) break;
             tc_fence_after();
