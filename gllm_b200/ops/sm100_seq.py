@@ -327,9 +327,11 @@ def qk_norm_rope_kv_write(qkv, num_heads, num_kv_heads, dim, v_dim, q_norm_w, k_
     return q
 
 
-# Where the chunked delta rule starts to pay (32 heads of 128 x 128, chunked against serial): 4 portions of 8 tokens 57 / 26 us,
-# of 16 tokens 60 / 42 us, one of 64 tokens 29 / 76 us.
-_DELTA_MIN_TOKENS = 32
+# Where the chunked delta rule starts to pay, calls chained on the device, chunked against serial in us, 32 and 8 heads of 128 x 128:
+# 4 portions of 16 tokens 33 / 40 and 22 / 21, 32 of them 174 / 273 and 55 / 75, one of 24 tokens 21 / 30, 8 of 31 55 / 141 and
+# 23 / 42. From 32 tokens on, as it was, 8 portions of 31 tokens beside one of 33 (8 heads) took 62 us in the two forms one after
+# the other where the serial one alone takes 45; now 23.
+_DELTA_MIN_TOKENS = 16
 _DELTA_WORK_BYTES = 256 << 20       # its workspace (31 KB per chunk and head) at a time; more heads take another round
 
 
