@@ -312,6 +312,7 @@ class InputData:
         self.num_tokens = self.num_seqs = self.num_decode_seqs = self.num_emit = 0
         self.max_q_len = self.max_seq_len = 0
         self.padded_tokens = 0  # > 0 when padded to a CUDA-graph bucket
+        self.latent_plan = None  # how latent attention splits the loaded batch (models/deepseek_v2.py), made by its first layer
         self.decode_splits = None  # None: pick per batch (eager); int: fixed (CUDA graphs)
 
     def _put(self, pair, arr: np.ndarray):
@@ -339,6 +340,7 @@ class InputData:
         self.num_emit = int(batch.logits_idx.shape[0])
         self.max_q_len, self.max_seq_len = batch.max_q_len, batch.max_seq_len
         self.padded_tokens = 0
+        self.latent_plan = None
         self._put(self._tokens, batch.tokens)
         if self.mrope:
             pos = batch.positions if batch.positions.ndim == 2 else np.broadcast_to(batch.positions, (3, batch.num_tokens))
@@ -378,6 +380,7 @@ class InputData:
         and write their K/V into the reserved dummy page (reference: input_data.py:319-367)."""
         b = self.num_seqs
         assert self.num_decode_seqs == b and bucket >= b
+        self.latent_plan = None
         if bucket == b:
             self.padded_tokens = b
             return

@@ -163,26 +163,45 @@ class MLAAttention(nn.Module):
     def _expanded_plan(self, inp):
         """(rounds, rest) of this batch. rounds: (first sequence, end, rows of latents) of the prompt portions to expand, each
         sequence rounded up to 64 rows; empty: all attend in the absorbed form. rest: None if the rows in the absorbed form are
-        the leading ones of the decoding sequences, else (their rows, their sequences)."""
+        the leading ones of the decoding sequences, else [their rows ; their sequences]."""
         n0, b = inp.num_decode_seqs, getattr(inp, "batch", None)
-        if b is None or inp.padded_tokens or n0 == inp.num_seqs or not self._expands():
+        if b is None or inp.padded_tokens or n0 == inp.num_seqs or inp.max_q_len < self._EXPAND_MIN_TOKENS or \
+                not self._expands():
             return [], None
         q_lens = np.diff(b.query_start_loc[:inp.num_seqs + 1].astype(np.int64))
         expand = q_lens >= self._EXPAND_MIN_TOKENS
         expand[:n0] = False
         rows = np.where(expand, (b.seq_lens[:inp.num_seqs].astype(np.int64) + 63) // 64 * 64, 0)
-        rounds, first, held = [], n0, 0
-        for s in range(n0, inp.num_seqs):
-            if held and (held + int(rows[s])) * self._LATENT_ROW_BYTES > self._EXPAND_LATENT_BYTES:
-                rounds.append((first, s, held))
-                first, held = s, 0
-            held += int(rows[s])
-        if held:
-            rounds.append((first, inp.num_seqs, held))
+        total = int(rows.sum())
+        if total * self._LATENT_ROW_BYTES <= self._EXPAND_LATENT_BYTES:
+            rounds = [(n0, inp.num_seqs, total)] if total else []
+        else:
+            rounds, first, held = [], n0, 0
+            for s in range(n0, inp.num_seqs):
+                if held and (held + int(rows[s])) * self._LATENT_ROW_BYTES > self._EXPAND_LATENT_BYTES:
+                    rounds.append((first, s, held))
+                    first, held = s, 0
+                held += int(rows[s])
+            if held:
+                rounds.append((first, inp.num_seqs, held))
         if not rounds or expand[n0:].all():
             return rounds, None
         keep = ~np.repeat(expand, q_lens)
-        return rounds, (np.flatnonzero(keep), np.repeat(np.arange(inp.num_seqs), q_lens)[keep])
+        return rounds, np.stack([np.flatnonzero(keep), np.repeat(np.arange(inp.num_seqs), q_lens)[keep]]).astype(np.int32)
+
+    def _plan_on_device(self, inp, device):
+        """`_expanded_plan` with `rest` as tensors (rows, sequences), kept on the step's input for the layers behind the first:
+        `InputData.load` drops it."""
+        plan = getattr(inp, "latent_plan", None)
+        if plan is None:
+            rounds, rest = self._expanded_plan(inp)
+            if rest is not None:
+                rows, seqs = torch.from_numpy(rest).to(device, non_blocking=True)
+                rest = (rows.long(), seqs)
+            plan = (rounds, rest)
+            if hasattr(inp, "latent_plan"):
+                inp.latent_plan = plan
+        return plan
 
     def _forward_absorbed(self, inp, q, kv_c, k_pe, cache):
         """sm_100a path: multi-query attention over the latent cache (csrc/attn/mla_attention.cu) for decoding sequences and
@@ -191,22 +210,22 @@ class MLAAttention(nn.Module):
         from gllm_b200.ops import sm100
         t, hl = q.shape[0], self.num_heads
         out = torch.empty(t, hl, self.v_dim, dtype=q.dtype, device=q.device)
-        rounds, rest = self._expanded_plan(inp)
-        n = inp.num_decode_seqs if rounds else t         # leading rows in the absorbed form
         pos = inp.positions if inp.positions.dim() == 1 else inp.positions[0]
+        rounds, rest = self._plan_on_device(inp, q.device)
+        n = inp.num_decode_seqs if rounds else t         # leading rows in the absorbed form
         if rest is not None:
             # short portions among long ones: everything is rotated in place, their rows are picked out
             sm100.mla_rope_cache(q[:, :, self.nope:], None, k_pe, kv_c, self.rope.cos_sin, pos, inp.slot_mapping, cache)
-            rows, seqs = torch.from_numpy(np.stack(rest).astype(np.int32)).to(q.device, non_blocking=True)
+            rows, seqs = rest
             w_uk, w_uv = self._absorbed_weights()
             some = q.index_select(0, rows)
-            q_full = torch.empty(len(rest[0]), hl, 576, dtype=q.dtype, device=q.device)
+            q_full = torch.empty(rows.shape[0], hl, 576, dtype=q.dtype, device=q.device)
             sm100.gemm_batched(some[:, :, : self.nope], w_uk, q_full[:, :, :512])
             q_full[:, :, 512:] = some[:, :, self.nope:]
             out_lat = sm100.mla_attention(q_full, cache, inp.block_table, seqs, pos.index_select(0, rows), self.scaling)
-            part = torch.empty(len(rest[0]), hl, self.v_dim, dtype=q.dtype, device=q.device)
+            part = torch.empty(rows.shape[0], hl, self.v_dim, dtype=q.dtype, device=q.device)
             sm100.gemm_batched(out_lat, w_uv, part)
-            out.index_copy_(0, rows.long(), part)
+            out.index_copy_(0, rows, part)
         elif n:
             w_uk, w_uv = self._absorbed_weights()
             q_full = torch.empty(n, hl, 576, dtype=q.dtype, device=q.device)

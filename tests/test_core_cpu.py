@@ -378,7 +378,7 @@ def test_latent_attention_chooses_per_sequence(decodes, q_lens, ctx):
     q, c = np.array([1] * decodes + q_lens), np.array([30] * decodes + ctx)
     n, qsl, lens = len(q), np.concatenate([[0], np.cumsum(q)]).astype(np.int32), (q + c).astype(np.int32)
     batch = SimpleNamespace(query_start_loc=qsl, seq_lens=lens)
-    inp = SimpleNamespace(num_decode_seqs=decodes, num_seqs=n, padded_tokens=0, batch=batch)
+    inp = SimpleNamespace(num_decode_seqs=decodes, num_seqs=n, padded_tokens=0, batch=batch, max_q_len=int(q.max()))
     att = SimpleNamespace(kv_lora=512, rope_dim=64, nope=128, v_dim=128, _EXPAND_MIN_TOKENS=32, _LATENT_ROW_BYTES=1152,
                           _expands=lambda: True)
     long = [s for s in range(decodes, n) if q[s] >= 32]
