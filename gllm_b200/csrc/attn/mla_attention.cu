@@ -467,15 +467,17 @@ __global__ void mla_rope_cache_kernel(const __nv_bfloat16* q_pe, int64_t q_ts, i
 }
 
 // First row of every sequence in the gathered latents (each takes whole 64-row tiles): rows[s] = sum of the lengths before it,
-// rounded up to 64. Sequences of fewer than min_len new tokens take none.
-__global__ void mla_rows_kernel(const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ q_start, int min_len, int nseq,
-                                int32_t* __restrict__ rows) {
+// rounded up to 64. Sequences of fewer than min_len new tokens, or of fewer than min_work / 2 (query, key) pairs, take none.
+__global__ void mla_rows_kernel(const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ q_start, int min_len, int min_work,
+                                int nseq, int32_t* __restrict__ rows) {
   __shared__ int32_t part[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int base = 0;
   for (int s0 = 0; s0 <= nseq; s0 += blockDim.x) {
     const int s = s0 + threadIdx.x;
-    const int n = s < nseq && q_start[s + 1] - q_start[s] >= min_len ? (seq_lens[s] + 63) / 64 * 64 : 0;
+    const int len = s < nseq ? seq_lens[s] : 0, q = s < nseq ? q_start[s + 1] - q_start[s] : 0;
+    const bool expand = s < nseq && q >= min_len && static_cast<int64_t>(q) * (2 * static_cast<int64_t>(len) - q) >= min_work;
+    const int n = expand ? (len + 63) / 64 * 64 : 0;
     int sum = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -571,14 +573,14 @@ GLLM_EXPORT int gllm_mla_attention(const void* q, void* out, const void* cache, 
 }
 
 // rows [nseq + 1] int32 (written), lat [total, 512], pe [total, 64]; total = the lengths of the sequences with at least min_len
-// new tokens, each rounded up to 64
+// new tokens and min_work / 2 pairs, each rounded up to 64
 GLLM_EXPORT int gllm_mla_gather(const void* cache, const void* block_table, int max_blocks, const void* seq_lens,
-                                const void* q_start, int min_len, int nseq, int total, int page_size, void* rows, void* lat,
-                                void* pe, void* stream) {
+                                const void* q_start, int min_len, int min_work, int nseq, int total, int page_size, void* rows,
+                                void* lat, void* pe, void* stream) {
   if (nseq <= 0 || total <= 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   mla_rows_kernel<<<1, 256, 0, st>>>(reinterpret_cast<const int32_t*>(seq_lens), reinterpret_cast<const int32_t*>(q_start),
-                                     min_len, nseq, reinterpret_cast<int32_t*>(rows));
+                                     min_len, min_work, nseq, reinterpret_cast<int32_t*>(rows));
   mla_gather_kernel<<<(total + 7) / 8, 256, 0, st>>>(
       reinterpret_cast<const __nv_bfloat16*>(cache), reinterpret_cast<const int32_t*>(block_table), max_blocks,
       reinterpret_cast<const int32_t*>(seq_lens), reinterpret_cast<const int32_t*>(rows), nseq, total, page_size,

@@ -71,7 +71,6 @@ struct TcAttnParams {
   AttnExtras ex;      // distance bias or table (kernel template BIAS), turned values, output gate
   WaitConfig waits;
   int q_tiles;        // query tiles per CTA (2, or 1 where that gives every SM at most one CTA)
-  int min_len;             // DENSE: sequences of fewer new tokens are left alone
   const int32_t* kv_row;   // DENSE: first row of each sequence of this launch in the expanded keys and values
 };
 
@@ -180,7 +179,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   const int kvh = blockIdx.z / groups_per_kv;
   const int hbase = kvh * p.G + (blockIdx.z % groups_per_kv) * p.GP;
   const int q_begin = p.q_start[seq], q_len = p.q_start[seq + 1] - q_begin;
-  if (DENSE && q_len < p.min_len) return;
+  if (DENSE && p.kv_row[blockIdx.y + 1] == p.kv_row[blockIdx.y]) return;      // no rows: not expanded
   const int toks_per_tile = kTcRows / p.GP;
   const int toks_per_cta = toks_per_tile * p.q_tiles;
   const int n_blocks = (q_len + toks_per_cta - 1) / toks_per_cta;
@@ -742,7 +741,6 @@ static int attn_prefill_tc_impl(const void* q, int64_t q_ts, void* out, const vo
   p.window = window;
   p.ex = ex;
   p.kv_row = nullptr;
-  p.min_len = 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 #define GLLM_TC(CAP, BIAS)                                                                                    \
   (D == 128 ? launch_prefill_tc<128, 128, false, CAP, BIAS>(tk, tv, tk, p, num_seqs, num_tokens, max_q_len, st) \
@@ -782,11 +780,10 @@ GLLM_EXPORT int gllm_attn_prefill_tc_cap(const void* q, int64_t q_ts, void* out,
 // Causal attention of expanded latent heads: q [tokens, H, 192] (token stride q_ts), kv [rows, H, 256] = [128 key | 128 value
 // columns], pe [rows, 64] = the key columns shared by all heads, both from kv_row[s] on for sequence s of this launch (64-row
 // tiles); out [tokens, H, 128] with rows out_ts elements apart. Sequences seq_offset .. + num_seqs of seq_lens / q_start, those with
-// at least min_len new tokens. A slice of heads is passed by q, out and kv that start at it. Returns 2 for unaligned queries.
+// rows (kv_row has one entry more than sequences). A slice of heads is passed by q, out and kv that start at it. Returns 2 for unaligned queries.
 GLLM_EXPORT int gllm_attn_prefill_expanded(const void* q, int64_t q_ts, void* out, int64_t out_ts, const void* kv, const void* pe, int64_t rows,
                                            const void* kv_row, const void* seq_lens, const void* q_start, int num_tokens,
-                                           int num_seqs, int seq_offset, int max_q_len, int min_len, int H, float scale,
-                                           void* stream) {
+                                           int num_seqs, int seq_offset, int max_q_len, int H, float scale, void* stream) {
   if (num_seqs <= 0 || max_q_len <= 0) return 0;
   if (q_ts % 8 != 0 || (reinterpret_cast<uintptr_t>(q) & 15) != 0) return 2;
   CUtensorMap tkv, tpe;
@@ -803,7 +800,6 @@ GLLM_EXPORT int gllm_attn_prefill_expanded(const void* q, int64_t q_ts, void* ou
   p.page_size = 64; p.seq_offset = seq_offset;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.out_ts = out_ts;
-  p.min_len = min_len;
   p.kv_row = reinterpret_cast<const int32_t*>(kv_row);
   return launch_prefill_tc<192, 128, true>(tkv, tkv, tpe, p, num_seqs, num_tokens, max_q_len,
                                            reinterpret_cast<cudaStream_t>(stream));

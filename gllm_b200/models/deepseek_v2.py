@@ -144,15 +144,22 @@ class MLAAttention(nn.Module):
     # Expanded heads cost a GEMM of 2 * 256 * 512 operations per cached row and head, and then 640 per (query, key) pair
     # instead of 2176 on a kernel eight times as fast: they win from some twenty new tokens per sequence on; below that a portion
     # is a few rows of one 128-row tile. 5 prompts of 4096 tokens together, 16 heads: 2459 -> 479 us. A sequence's own portion
-    # decides. What a call holds at a time is bounded: the gathered latents (more sequences take another round) and the keys
+    # decides: its length, and its (query, key) pairs over all heads. Below 2^18 of them the absorbed form takes at most 4 us
+    # (16 per 2^20), less than the host needs for the launches that the expanded form and the picking of rows add: 12 portions of 6
+    # to 50 tokens over some hundred cached ones, 16 heads, took 250 us for the block where all absorbed they take 166.
+    # What a call holds at a time is bounded: the gathered latents (more sequences take another round) and the keys
     # and values of as many heads as fit.
     _EXPAND_MIN_TOKENS = 32
+    _EXPAND_MIN_PAIRS = 1 << 18
     _EXPAND_KV_BYTES = 1 << 30
     _EXPAND_LATENT_BYTES = 256 << 20
     _LATENT_ROW_BYTES = 576 * 2
 
     def _expands(self) -> bool:
         return (self.kv_lora, self.rope_dim, self.nope, self.v_dim) == (512, 64, 128, 128)
+
+    def _expand_min_work(self) -> int:
+        return -(-2 * self._EXPAND_MIN_PAIRS // self.num_heads)
 
     def expand_scratch_bytes(self, max_len: int) -> int:
         """What the expanded form allocates beside the cache at most, for sequences of up to `max_len` tokens."""
@@ -169,9 +176,10 @@ class MLAAttention(nn.Module):
                 not self._expands():
             return [], None
         q_lens = np.diff(b.query_start_loc[:inp.num_seqs + 1].astype(np.int64))
-        expand = q_lens >= self._EXPAND_MIN_TOKENS
+        lens = b.seq_lens[:inp.num_seqs].astype(np.int64)
+        expand = (q_lens >= self._EXPAND_MIN_TOKENS) & (q_lens * (2 * lens - q_lens) >= self._expand_min_work())
         expand[:n0] = False
-        rows = np.where(expand, (b.seq_lens[:inp.num_seqs].astype(np.int64) + 63) // 64 * 64, 0)
+        rows = np.where(expand, (lens + 63) // 64 * 64, 0)
         total = int(rows.sum())
         if total * self._LATENT_ROW_BYTES <= self._EXPAND_LATENT_BYTES:
             rounds = [(n0, inp.num_seqs, total)] if total else []
@@ -240,7 +248,8 @@ class MLAAttention(nn.Module):
                                  inp.slot_mapping[n:], cache)
         for first, end, held in rounds:
             sm100.mla_expanded_attention(q, cache, inp.block_table, inp.seq_lens, inp.query_start_loc, self.kv_b_w, held, first,
-                                         inp.max_q_len, self.scaling, out, end, self._EXPAND_MIN_TOKENS, self._EXPAND_KV_BYTES)
+                                         inp.max_q_len, self.scaling, out, end, self._EXPAND_MIN_TOKENS, self._EXPAND_KV_BYTES,
+                                         self._expand_min_work())
         return out.view(t, hl * self.v_dim)
 
 

@@ -495,8 +495,9 @@ def mla_rope_cache(q_pe: torch.Tensor, q_full: Optional[torch.Tensor], k_pe: tor
 def mla_expanded_attention(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, seq_lens: torch.Tensor,
                            query_start_loc: torch.Tensor, kv_b_w: torch.Tensor, rows: int, first_seq: int, max_q_len: int,
                            scale: float, out: torch.Tensor, end_seq: Optional[int] = None, min_len: int = 0,
-                           kv_bytes: Optional[int] = None) -> torch.Tensor:
-    """Causal attention of the sequences [first_seq, end_seq) that have at least `min_len` new tokens, in the expanded form: their
+                           kv_bytes: Optional[int] = None, min_work: int = 0) -> torch.Tensor:
+    """Causal attention of the sequences [first_seq, end_seq) that have at least `min_len` new tokens and at least `min_work` by
+    new tokens x (2 x length - new tokens), twice their (query, key) pairs, in the expanded form: their
     cached latents are gathered (`rows` of them, every sequence rounded up to 64), kv_b_w [H * 256, 512] makes each head's 128
     key and 128 value columns from them, and the tcgen05 prefill kernel runs on keys [128 | 64 shared] and values 128 wide.
     q [T, H, 192] rotated; out [T, H, 128]: the rows of those sequences are written. With `kv_bytes`, so many heads at a time
@@ -510,8 +511,8 @@ def mla_expanded_attention(q: torch.Tensor, cache: torch.Tensor, block_table: to
     lat = torch.empty(rows, 512, dtype=_BF16, device=dev)
     pe = torch.empty(rows, 64, dtype=_BF16, device=dev)
     check(L.gllm_mla_gather(_p(cache), _p(block_table[first_seq:]), block_table.stride(0), _p(seq_lens[first_seq:]),
-                            _p(query_start_loc[first_seq:]), min_len, n, rows, cache.shape[3], _p(start), _p(lat), _p(pe), st),
-          "mla_gather")
+                            _p(query_start_loc[first_seq:]), min_len, min_work, n, rows, cache.shape[3], _p(start), _p(lat), _p(pe),
+                            st), "mla_gather")
     _count(2)
     rounds = -(-h // max(1, min(h, kv_bytes // (rows * 512)))) if kv_bytes else 1
     step = -(-h // rounds)
@@ -519,7 +520,7 @@ def mla_expanded_attention(q: torch.Tensor, cache: torch.Tensor, block_table: to
         nh = min(step, h - h0)
         kv = linear(lat, kv_b_w[h0 * 256:(h0 + nh) * 256])
         check(L.gllm_attn_prefill_expanded(_p(q[:, h0:]), q.stride(0), _p(out[:, h0:]), out.stride(0), _p(kv), _p(pe), rows,
-                                           _p(start), _p(seq_lens), _p(query_start_loc), t, n, first_seq, max_q_len, min_len, nh,
+                                           _p(start), _p(seq_lens), _p(query_start_loc), t, n, first_seq, max_q_len, nh,
                                            float(scale), st), "attn_prefill_expanded")
         _count()
     return out

@@ -368,10 +368,11 @@ def test_incremental_decode_batch_equals_full_rebuild():
 
 
 @pytest.mark.parametrize("decodes", [0, 2])
+@pytest.mark.parametrize("work", [0, 40 * 40 + 1])
 @pytest.mark.parametrize("q_lens,ctx", [([40, 32, 500], [0, 7, 64]), ([31, 40], [900, 0]), ([40, 5, 32, 31, 64], [0, 1, 2, 3, 4000]),
                                         ([3, 31], [9, 9])])
-def test_latent_attention_chooses_per_sequence(decodes, q_lens, ctx):
-    """Portions of 32 tokens and more are expanded whatever is beside them, in rounds whose latents stay below the limit (one
+def test_latent_attention_chooses_per_sequence(decodes, work, q_lens, ctx):
+    """Portions of 32 tokens and more, with enough (query, key) pairs, are expanded whatever is beside them, in rounds whose latents stay below the limit (one
     sequence at least); every other row is attended once in the absorbed form, by its own sequence."""
     from types import SimpleNamespace
     from gllm_b200.models.deepseek_v2 import MLAAttention
@@ -380,8 +381,8 @@ def test_latent_attention_chooses_per_sequence(decodes, q_lens, ctx):
     batch = SimpleNamespace(query_start_loc=qsl, seq_lens=lens)
     inp = SimpleNamespace(num_decode_seqs=decodes, num_seqs=n, padded_tokens=0, batch=batch, max_q_len=int(q.max()))
     att = SimpleNamespace(kv_lora=512, rope_dim=64, nope=128, v_dim=128, _EXPAND_MIN_TOKENS=32, _LATENT_ROW_BYTES=1152,
-                          _expands=lambda: True)
-    long = [s for s in range(decodes, n) if q[s] >= 32]
+                          _expands=lambda: True, _expand_min_work=lambda: work)
+    long = [s for s in range(decodes, n) if q[s] >= 32 and q[s] * (2 * int(lens[s]) - q[s]) >= work]
     rows = {s: -(-int(lens[s]) // 64) * 64 for s in long}
     for limit in (1 << 30, 200 * 1152, 1):
         att._EXPAND_LATENT_BYTES = limit

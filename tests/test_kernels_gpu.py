@@ -928,15 +928,17 @@ def test_latent_attention_block_mixed_batches(decodes, q_lens, ctx, kv_rows, lat
     cache0 = torch.randn(sum(need), 1, 9, page, 64, device=dev).bfloat16()
     h = torch.randn(sum(q), width, device=dev).bfloat16()
     got = []
-    for least in (32, 10 ** 6):
+    for least, pairs in ((32, 0), (32, heads * 2400), (10 ** 6, 0)):
         monkeypatch.setattr(MLAAttention, "_EXPAND_MIN_TOKENS", least)
+        monkeypatch.setattr(MLAAttention, "_EXPAND_MIN_PAIRS", pairs)
         monkeypatch.setattr(MLAAttention, "_EXPAND_KV_BYTES", kv_rows * 512)
         monkeypatch.setattr(MLAAttention, "_EXPAND_LATENT_BYTES", latent_rows * 1152)
         cache = cache0.clone()
         got.append((att(inp, h, SimpleNamespace(k_cache=[cache]), tpc), cache))
-    assert torch.equal(got[0][1], got[1][1])
-    for a, b in zip(q, qsl):
-        assert _rel_err(got[0][0][b:b + a], got[1][0][b:b + a]) < 1.2e-2
+    for x in got[:2]:
+        assert torch.equal(x[1], got[2][1])
+        for a, b in zip(q, qsl):
+            assert _rel_err(x[0][b:b + a], got[2][0][b:b + a]) < 1.2e-2
 
 
 @pytest.mark.parametrize("m", [1, 2])
