@@ -381,8 +381,8 @@ static int launch_fp8_tile(const CUtensorMap& ta, const CUtensorMap& tb, const F
 // Tile width: the one with the least (waves x time of a tile's K block). A block of 128 rows takes 0.60 us 256 wide, 0.48 at 128
 // and 0.43 at 64 (there the chain of copies, products and folds bounds it), so narrow tiles only pay when the wide ones leave SMs
 // idle: a decode batch's 7168 columns are 28 tiles of 256. Over 80 shapes (1 to 1000 rows, 1536 to 36,864 columns, K 1536 to
-// 18,432) timed at all three widths the choice is 0.3 % slower than the best on average. A few rows are the exception: 112 CTAs that
-// all read the same one to four rows of A wait for them, 56 do not (7168 x 18432, one row: 70 us 64 wide, 66.5 at 128; eight: 59.7). `live`: the most row tiles that can hold rows; grouped calls
+// 18,432) timed at all three widths the choice is 0.3 % slower than the best on average. One to four rows of 7168 columns alone
+// take 70 us 64 wide and 66.5 at 128 (K = 18432), but the whole MLP of one row 124.2 against 125.2. `live`: the most row tiles that can hold rows; grouped calls
 // (256 or 128 wide) do not know more on the host.
 static int launch_fp8(const void* A8, const void* W8, uint64_t w_rows, Fp8Params p, int64_t live, cudaStream_t st) {
   const int64_t m_tiles = (p.M + kFBM - 1) / kFBM;
@@ -392,7 +392,6 @@ static int launch_fp8(const void* A8, const void* W8, uint64_t w_rows, Fp8Params
   for (int i = 0; i < (p.silu || p.tile_expert != nullptr ? 2 : 3); ++i) {
     const int64_t tiles = live * ((p.N + width[i] - 1) / width[i]);
     const int64_t t = (tiles + num_sms() - 1) / num_sms() * cost[i];
-    if (width[i] == 64 && p.M < 8 && tiles > 96) continue;
     if (best < 0 || t < best) { best = t; bn = width[i]; }
   }
   p.waits = g_wait_config;
