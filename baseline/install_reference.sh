@@ -1,5 +1,5 @@
 #!/usr/bin/env bash
-# Offline install of the UNMODIFIED reference into baseline/_ref (git-ignored; travels with gpurun snapshots).
+# Offline install of the UNMODIFIED reference into baseline/_ref (git-ignored).
 #
 # The reference's setup.py extracts its native kernels from a vLLM wheel (setup.py:186-215); with no network we
 # hand it, through its own GLLM_PRECOMPILED_WHEEL_LOCATION switch, a local wheel-shaped zip whose members are

@@ -2,7 +2,7 @@
 `ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum ...` (per-kernel device time without launch gaps).
 
     ncu --clock-control none --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum \
-        --csv --log-file gpurun_out/layer.csv python benchmarks/ncu_decode_layer.py --batch 64 --ctx 512
+        --csv --log-file layer.csv python benchmarks/ncu_decode_layer.py --batch 64 --ctx 512
 """
 import argparse
 import os

@@ -1,7 +1,7 @@
 """Prefill-shaped hot kernels, launched a few times each — target of `ncu --set full` (Qwen3-8B shapes, 4096 tokens).
 
     ncu --set full --clock-control none -k regex:'gemm_bf16_kernel|attn_prefill' -s 3 -c 3 \
-        -o gpurun_out/prefill python benchmarks/ncu_prefill_ops.py
+        -o prefill python benchmarks/ncu_prefill_ops.py
 """
 import os
 import sys
