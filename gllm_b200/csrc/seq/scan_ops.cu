@@ -1,16 +1,24 @@
-// Mamba-1 recurrence cut in time (selective_scan; csrc/seq/seq_ops.cu holds the token-serial form):
+// Mamba-1 recurrence of prompt portions (selective_scan; csrc/seq/seq_ops.cu holds the token-serial form for decoding):
 //     S_n <- exp(dt a_n) S_n + dt x B_n;  y = sum_n S_n C_n + D x;  out = y silu(z)          N states per channel, fp32
-// The decays are diagonal, so a chunk of 64 tokens takes an entering state S_0 to exp(a_n sum dt) S_0 + (its own end state).
-// Three kernels: every chunk's end state from zero and its sum of steps; the chain over a sequence's chunks (one thread per
-// channel and state); every chunk again from its entering state, with the outputs. One thread per channel, all its states in
-// registers, no shuffles. Same formulas, order and functions per token as the serial kernel.
+// Two or four lanes share a channel and hold an equal part of its states in registers; a block of 128 threads walks its channels
+// through one piece of a sequence, 16 tokens at a time. For each 16 tokens the block first forms the steps dt = softplus(.), dt x
+// and B, C in shared memory (two channels of a row per thread), then walks them (no arithmetic but the recurrence's own), then
+// forms the gated outputs; the next tokens' inputs are on their way during the walk.
 //
-// What bounds it: issue slots, about 11 per (token, channel, state) and pass, most of them the accurate expf. The serial kernel
-// does the exponentials once, but its longest sequence is one chain of tokens on a part of the machine, and the four threads of
-// a channel each form the same steps and gates.
-// 8192 ragged tokens in 4 sequences, 8192 channels, 16 states: 527 + 29 + 740 us, token-serial 2999 us (B200); one sequence of
-// 8192 tokens: 1.28 ms / 8.5 ms. The hardware's 2^x on an exponent in two parts would take 250 us off, but its error is up to
-// 1.8 times that of expf (state of 2048 tokens against float64: 3.1e-7 / 1.8e-7).
+// Usually a piece is a whole sequence: one launch, every exponential once. Where the sequences are too few to fill the machine
+// (scan_piece in ops/sm100_seq.py), they are cut in pieces and three kernels run: every piece's end state from zero and its sum
+// of steps (the decays are diagonal, so a piece takes an entering state S_0 to exp(a_n sum dt) S_0 + its own end state); the
+// chain over a sequence's pieces; every piece again from its entering state, with the outputs.
+//
+// What bounds it: the 2^x unit (8 cycles per warp and exponential: 64 of about 100 cycles per token of a warp with 16 channels)
+// and issue slots. So the arithmetic is on pairs (f32x2), log2(e) is multiplied into A, softplus and silu are formed once per
+// token and channel in forms of their own instead of expf, log1pf and a division (790 -> 730 us), and the exponential is the bare
+// instruction with its bias taken out (a quarter of them as polynomials on the fma units: 730 instead of 614 us). 128 registers,
+// for the scheduler to overlap four tokens: 572 us, at 96 628.
+// 8192 ragged tokens in 4 sequences, 8192 channels, 16 states: 1342 -> 572 us (B200); one sequence of 16384 tokens, 2048 channels,
+// cut in pieces: 710 -> 480. Before, every batch ran as chunks of 64 tokens in two passes, a thread per channel, with expf.
+// Error against float64 after 2048 tokens, steps around 0.01 (fp32 outputs / states): 8.3e-8 / 1.8e-7; chunks with expf 8.0e-8 /
+// 1.8e-7; token-serial with expf 9.3e-8 / 1.8e-7.
 #include <cuda_bf16.h>
 
 #include "common/host_utils.h"
@@ -19,138 +27,316 @@
 namespace {
 using namespace seqk;
 
-constexpr int kL = 64;                              // tokens of a chunk
-constexpr int kNM = 16;                             // states a thread holds
-constexpr int kRows = 2 * kL;                       // tokens of the longest sequence that is walked whole
+constexpr int kNM = 16;                             // most states of a channel
+constexpr int kThreads = 128;
+constexpr int kTile = 16;                           // tokens between two barriers
 
-// Chunk slots: sequence s owns slots from qsl[s] / 64 + s on (at least one per started 64 tokens); some stay empty.
-__device__ __forceinline__ int chunk_base(const int* qsl, int s) { return qsl[s] / kL + s; }
+// ---- pairs of fp32 ----
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk(float a, float b) { f2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
+__device__ __forceinline__ void un(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ float rcp(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
-// Channels [c0, c0 + CW) of the batch; ends [slot][n][CW]: end states (FINAL 0: written) or entering states (FINAL 1: read);
-// steps [slot][CW]: sums of dt. Sequences of fewer than min_len tokens are not cut: FINAL walks them whole, from the carried
-// state (a kernel of their own behind the three took as long again: 8 portions of 100 tokens and one of 150).
-template <typename T, bool FINAL>
-__global__ void __launch_bounds__(128, FINAL ? 6 : 7) scan_chunk_kernel(
-    const T* __restrict__ xc, const T* __restrict__ dt_raw, const T* __restrict__ proj, long ldp, const T* __restrict__ xz,
-    long ldxz, const float* __restrict__ A, const float* __restrict__ Dskip, const float* __restrict__ dt_bias,
-    float* __restrict__ state, const int* __restrict__ rec_slots, const int* __restrict__ seq_lens, const int* __restrict__ qsl,
-    int nseq, int C, int N, int R, int c0, int CW, int min_len, float* __restrict__ ends, float* __restrict__ steps, T* __restrict__ out) {
-  constexpr int TCH = 8;
-  __shared__ __align__(16) float sBC[FINAL ? kRows : kL][2 * kNM];
+// 2^t of both halves on the 2^x unit. Its results lie 1.5e-8 to 2e-8 below 2^t on average for t in (-1, 0), which adds up over the
+// tokens that a state remembers. The caller adds kBias = 1.9e-8 / ln 2 to t in the fma that forms it (states after 2048 tokens
+// against float64, steps of 0.001 to 0.1: 1.46e-7 with 2.2e-8, 1.41e-7 with 2.6e-8, 1.53e-7 with 3.4e-8; expf 1.43e-7).
+constexpr float kBias = 2.7e-8f;
+__device__ __forceinline__ f2 exp2_unit(f2 t) {
+  float t0, t1;
+  un(t, t0, t1);
+  return pk(ex2(t0), ex2(t1));
+}
+__device__ __forceinline__ f2 rcp2(f2 v) {
+  float a, b;
+  un(v, a, b);
+  return pk(rcp(a), rcp(b));
+}
+// log(1 + e^v) of both halves = max(v, 0) + log1p(e), e = e^-|v|; log1p(e) = 2 atanh(s), s = e / (2 + e) <= 1/3, by the polynomial of
+// least relative error (4.5e-9) in s^2. Relative error below 1.5e-7 at any v, where expf and log1pf one after the other have as much.
+__device__ __forceinline__ f2 softplus2(f2 v) {
+  float v0, v1;
+  un(v, v0, v1);
+  const f2 e = exp2_unit(fma2(pk(fabsf(v0), fabsf(v1)), pk(-1.4426950408889634f, -1.4426950408889634f), pk(kBias, kBias)));
+  const f2 r = rcp2(add2(e, pk(2.f, 2.f)));
+  f2 s = mul2(e, r);
+  const f2 ns = mul2(s, pk(-1.f, -1.f));
+  s = fma2(r, fma2(ns, e, fma2(ns, pk(2.f, 2.f), e)), s);
+  const f2 q = mul2(s, s), twice = add2(s, s);
+  f2 w = fma2(q, pk(0.14005993f, 0.14005993f), pk(0.14000903f, 0.14000903f));
+  w = fma2(q, w, pk(0.20010763f, 0.20010763f));
+  w = fma2(q, w, pk(0.3333321f, 0.3333321f));
+  return add2(pk(fmaxf(v0, 0.f), fmaxf(v1, 0.f)), fma2(twice, mul2(q, w), twice));
+}
+// z / (1 + e^-z)
+__device__ __forceinline__ f2 silu2(f2 z) {
+  const f2 e = exp2_unit(fma2(z, pk(-1.4426950408889634f, -1.4426950408889634f), pk(kBias, kBias)));
+  const f2 d = add2(e, pk(1.f, 1.f)), r = rcp2(d);
+  const f2 better = fma2(r, fma2(mul2(r, pk(-1.f, -1.f)), d, pk(1.f, 1.f)), r);        // NaN where d is infinite
+  float d0, d1, r0, r1, b0, b1;
+  un(d, d0, d1);
+  un(r, r0, r1);
+  un(better, b0, b1);
+  return mul2(z, pk(d0 < 1e37f ? b0 : r0, d1 < 1e37f ? b1 : r1));
+}
+
+// Piece slots: sequence s owns slots from qsl[s] / piece + s on (at least one per started piece); some stay empty.
+__device__ __forceinline__ int piece_base(const int* qsl, int s, int piece) { return qsl[s] / piece + s; }
+
+struct ScanArgs {
+  const float *A, *Dskip, *dt_bias;
+  float* state;
+  const int *rec_slots, *seq_lens, *qsl;
+  int nseq, C, N, R, c0, CW, piece;
+  long ldp, ldxz;
+  int wide;                                          // channels 2 i, 2 i + 1 of x, dt, z and out can be moved together
+  float *ends, *steps;
+};
+
+template <typename T> struct Pair;
+template <> struct Pair<__nv_bfloat16> { using V = uint32_t; };
+template <> struct Pair<float> { using V = float2; };
+__device__ __forceinline__ f2 pair_f(uint32_t v) { return pk(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
+__device__ __forceinline__ f2 pair_f(float2 v) { return pk(v.x, v.y); }
+__device__ __forceinline__ void pair_make(uint32_t& v, __nv_bfloat16 a, __nv_bfloat16 b) {
+  v = (uint32_t)__bfloat16_as_ushort(a) | ((uint32_t)__bfloat16_as_ushort(b) << 16);
+}
+__device__ __forceinline__ void pair_make(float2& v, float a, float b) { v = make_float2(a, b); }
+
+// Channels [c0, c0 + CW) of the batch; ends [slot][n][CW]: end states (FINAL 0: written) or entering states (FINAL 1: read, but a
+// sequence of one piece starts from the carried state itself); steps [slot][CW]: sums of dt. LPC lanes per channel, NS states at most.
+template <typename T, bool FINAL, int LPC, int NS>
+__global__ void __launch_bounds__(kThreads, LPC == 2 ? 4 : 6)
+scan_walk_kernel(const T* __restrict__ xc, const T* __restrict__ dt_raw, const T* __restrict__ proj, const T* __restrict__ xz,
+                 T* __restrict__ out, const ScanArgs p) {
+  using V = typename Pair<T>::V;
+  constexpr int NL = NS / LPC, NP = NL / 2;                                // states and pairs of a lane
+  constexpr int CH = kThreads / LPC;                                       // channels of the block
+  constexpr int RP = 2 * kThreads / CH, RT = kTile / RP;                   // rows of the block at a time; rows of a thread
+  __shared__ __align__(16) float4 sD[kTile][CH];                           // dt, dt, dt x, dt x
+  __shared__ __align__(16) float sBC[kTile][2 * NS];
+  __shared__ __align__(16) float sY[FINAL ? kTile : 1][CH];
   const int u = blockIdx.y;
-  int lo = 0, hi = nseq - 1;
+  int lo = 0, hi = p.nseq - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (chunk_base(qsl, mid) <= u) lo = mid; else hi = mid - 1;
+    if (piece_base(p.qsl, mid, p.piece) <= u) lo = mid; else hi = mid - 1;
   }
-  const int q0 = qsl[lo], q1 = qsl[lo + 1];
-  const int base = q0 + (u - chunk_base(qsl, lo)) * kL;
-  const bool whole = q1 - q0 < min_len;
-  if (base < q0 || base >= q1 || (whole && base != q0)) return;     // uniform over the block
-  const bool last = whole || base + kL >= q1;
-  if (!FINAL && last) return;                       // nobody continues from its end
-  const int len = (FINAL && whole ? q1 : min(base + kL, q1)) - base;      // whole: fewer than min_len tokens, at most kRows
-  const int w = blockIdx.x * 128 + threadIdx.x;     // channel inside this round's range
-  const bool active = w < CW;
-  const int c = c0 + (active ? w : CW - 1);         // idle threads mirror the last channel (loads only)
-  float S[kNM], a[kNM];
-  float* e0 = ends + ((size_t)u * N) * CW + (active ? w : CW - 1);
-  const bool carried = whole && state != nullptr && seq_lens[lo] > q1 - q0;
-  const float* from = carried ? state + (size_t)rec_slots[lo] * N * C + c : e0;
-  const size_t step = carried ? C : CW;
+  const int q0 = p.qsl[lo], q1 = p.qsl[lo + 1];
+  const long off = (long)(u - piece_base(p.qsl, lo, p.piece)) * p.piece;
+  if (off >= q1 - q0) return;                        // uniform over the block
+  const int base = q0 + (int)off, len = min(q1 - base, p.piece);
+  const bool whole = q1 - q0 <= p.piece, last = base + len >= q1;
+  if (!FINAL && last) return;                        // nobody continues from its end
+  const int tid = threadIdx.x, j = tid % LPC, ch = tid / LPC, C = p.C, N = p.N;
+  const int w0 = blockIdx.x * CH, w = w0 + ch;       // channel inside this round's range
+  const bool active = w < p.CW;
+  const int wc = active ? w : p.CW - 1, c = p.c0 + wc;                     // idle threads mirror the last channel (loads only)
+
+  f2 S[NP], a[NP];                                   // states; A log2(e)
+  {
+    const bool carried = whole && p.state != nullptr && p.seq_lens[lo] > q1 - q0;
+    const float* from = carried ? p.state + (size_t)p.rec_slots[lo] * N * C + c : p.ends + (size_t)u * N * p.CW + wc;
+    const size_t step = carried ? C : p.CW;
+    float sv[NL], av[NL];
 #pragma unroll
-  for (int n = 0; n < kNM; ++n) {
-    a[n] = n < N ? A[(size_t)c * N + n] : 0.f;
-    S[n] = FINAL && n < N && (carried || !whole) ? from[n * step] : 0.f;
-  }
-  const float dsk = Dskip[c], bias = dt_bias[c];
-  float sum = 0.f;
-  for (int i = threadIdx.x; i < len * 2 * kNM; i += 128) {
-    const int k = i / (2 * kNM), n = i % kNM, half = (i / kNM) & 1;
-    sBC[k][half * kNM + n] = n < N ? to_f(proj[(size_t)(base + k) * ldp + R + half * N + n]) : 0.f;
-  }
-  __syncthreads();
-  for (int k0 = 0; k0 < len; k0 += TCH) {
-    float dtv[TCH], xv[TCH], zv[TCH];
-#pragma unroll
-    for (int k = 0; k < TCH; ++k) {
-      const size_t t = base + min(k0 + k, len - 1);
-      dtv[k] = to_f(dt_raw[t * C + c]);
-      xv[k] = to_f(xc[t * C + c]);
-      if (FINAL) zv[k] = to_f(xz[t * ldxz + C + c]);
+    for (int e = 0; e < NL; ++e) {
+      const int n = j * NL + e;
+      av[e] = n < N ? p.A[(size_t)c * N + n] * 1.4426950408889634f : 0.f;
+      sv[e] = FINAL && n < N && (carried || !whole) ? from[n * step] : 0.f;
     }
 #pragma unroll
-    for (int k = 0; k < TCH; ++k) {
-      if (k0 + k < len) {
-        const float v = dtv[k] + bias;
-        const float dt = v > 20.0f ? v : log1pf(expf(v));
-        const float x = xv[k], dx = dt * x;
-        const float4* bc = reinterpret_cast<const float4*>(sBC[k0 + k]);
-        float y4[4] = {0.f, 0.f, 0.f, 0.f};
-        sum += dt;
+    for (int e = 0; e < NP; ++e) { S[e] = pk(sv[2 * e], sv[2 * e + 1]); a[e] = pk(av[2 * e], av[2 * e + 1]); }
+  }
+
+  // the two channels and the rows (r0, r0 + RP, ...) of each tile whose steps and outputs this thread forms
+  const int cp = 2 * (tid % (CH / 2)), r0 = tid / (CH / 2), cc = p.c0 + w0 + cp;
+  const bool on0 = w0 + cp < p.CW, on1 = w0 + cp + 1 < p.CW;
+  const f2 bias = pk(on0 ? p.dt_bias[cc] : 0.f, on1 ? p.dt_bias[cc + 1] : 0.f);
+  const f2 dsk = pk(on0 ? p.Dskip[cc] : 0.f, on1 ? p.Dskip[cc + 1] : 0.f);
+  f2 sum = 0;
+  auto load = [&](const T* src) {                    // channels cc, cc + 1 of a row
+    V v;
+    if (p.wide) {
+      v = *reinterpret_cast<const V*>(src);
+    } else {
+      pair_make(v, src[0], on1 ? src[1] : src[0]);
+    }
+    return v;
+  };
+  constexpr int kBC = kTile * 2 * NS / kThreads;     // B and C values of a thread
+  V dv[RT], xv[RT], zv[RT];
+  T bc[kBC];
+  auto fetch = [&](int t0) {
 #pragma unroll
-        for (int g = 0; g < kNM / 4; ++g) {
-          const float4 bv = bc[g], cv = bc[kNM / 4 + g];
-          const float b[4] = {bv.x, bv.y, bv.z, bv.w}, cc[4] = {cv.x, cv.y, cv.z, cv.w};
+    for (int i = 0; i < RT; ++i) {
+      const size_t t = base + min(t0 + r0 + i * RP, len - 1);
+      if (on0) {
+        dv[i] = load(dt_raw + t * C + cc);
+        xv[i] = load(xc + t * C + cc);
+        if (FINAL) zv[i] = load(xz + t * p.ldxz + C + cc);
+      }
+    }
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int n = 4 * g + e;
-            S[n] = expf(dt * a[n]) * S[n] + dx * b[e];
-            if (FINAL) y4[e] = fmaf(S[n], cc[e], y4[e]);
+    for (int i = 0; i < kBC; ++i) {
+      const int k = i * kThreads + tid, r = k / (2 * NS), v = k % (2 * NS), half = v / NS, n = min(v % NS, N - 1);
+      bc[i] = proj[(size_t)(base + min(t0 + r, len - 1)) * p.ldp + p.R + half * N + n];
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < RT; ++i) dv[i] = xv[i] = zv[i] = V{};
+  fetch(0);
+  for (int t0 = 0; t0 < len; t0 += kTile) {
+    // steps and scaled inputs; tokens past the end leave the states alone (dt = dt x = B = 0)
+    f2 xf[RT], zf[RT];
+#pragma unroll
+    for (int i = 0; i < RT; ++i) {
+      const int r = r0 + i * RP;
+      xf[i] = pair_f(xv[i]);
+      zf[i] = pair_f(zv[i]);
+      f2 step = softplus2(add2(pair_f(dv[i]), bias)), in = mul2(step, xf[i]);
+      if (t0 + r >= len) step = in = 0;
+      sum = add2(sum, step);
+      float s0, s1, m0, m1;
+      un(step, s0, s1);
+      un(in, m0, m1);
+      sD[r][cp] = make_float4(s0, s0, m0, m0);
+      sD[r][cp + 1] = make_float4(s1, s1, m1, m1);
+    }
+#pragma unroll
+    for (int i = 0; i < kBC; ++i) {
+      const int k = i * kThreads + tid, r = k / (2 * NS), n = k % NS;
+      (&sBC[0][0])[k] = t0 + r < len && n < N ? to_f(bc[i]) : 0.f;
+    }
+    __syncthreads();
+    if (t0 + kTile < len) fetch(t0 + kTile);         // on their way during the walk
+    const int rows = min(kTile, len - t0);
+#pragma unroll 1
+    for (int g = 0; g < rows; g += 4) {
+      float y[4];
+      const f2 bias2 = pk(kBias, kBias);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const ulonglong2 d = *reinterpret_cast<const ulonglong2*>(&sD[g + k][ch]);
+        const f2 dt2 = d.x, dx2 = d.y;
+        f2 b[NP], cv[NP];
+#pragma unroll
+        for (int e = 0; e < NP; e += 2) {
+          const ulonglong2 bb = *reinterpret_cast<const ulonglong2*>(&sBC[g + k][j * NL + 2 * e]);
+          b[e] = bb.x;
+          b[e + 1] = bb.y;
+          if (FINAL) {
+            const ulonglong2 c2 = *reinterpret_cast<const ulonglong2*>(&sBC[g + k][NS + j * NL + 2 * e]);
+            cv[e] = c2.x;
+            cv[e + 1] = c2.y;
           }
         }
+        f2 y2 = 0;
+#pragma unroll
+        for (int e = 0; e < NP; ++e) {
+          const f2 dec = exp2_unit(fma2(dt2, a[e], bias2));
+          S[e] = fma2(dec, S[e], mul2(dx2, b[e]));
+          if (FINAL) y2 = e == 0 ? mul2(S[e], cv[e]) : fma2(S[e], cv[e], y2);
+        }
         if (FINAL) {
-          const float z = zv[k], y = fmaf(dsk, x, (y4[0] + y4[1]) + (y4[2] + y4[3]));
-          if (active) out[(size_t)(base + k0 + k) * C + c] = from_f<T>(y * (z / (1.0f + expf(-z))));
+          float h0, h1;
+          un(y2, h0, h1);
+          y[k] = h0 + h1;
+        }
+      }
+      if (FINAL) {
+        // the lanes' partial sums of the four tokens, transposed
+        const bool odd = j & 1;
+        const float q_0 = __shfl_xor_sync(0xffffffffu, odd ? y[0] : y[1], 1), q_1 = __shfl_xor_sync(0xffffffffu, odd ? y[2] : y[3], 1);
+        const float k0 = (odd ? y[1] : y[0]) + q_0, k1 = (odd ? y[3] : y[2]) + q_1;
+        if (LPC == 2) {
+          sY[g + j][ch] = k0;
+          sY[g + 2 + j][ch] = k1;
+        } else {
+          const bool up = j & 2;
+          sY[g + j][ch] = (up ? k1 : k0) + __shfl_xor_sync(0xffffffffu, up ? k0 : k1, 2);
+        }
+      }
+    }
+    __syncthreads();
+    if (FINAL && on0) {
+#pragma unroll
+      for (int i = 0; i < RT; ++i) {
+        const int r = r0 + i * RP;
+        if (r < rows) {
+          const f2 y = *reinterpret_cast<const f2*>(&sY[r][cp]);
+          float y0, y1;
+          un(mul2(fma2(dsk, xf[i], y), silu2(zf[i])), y0, y1);
+          const T o0 = from_f<T>(y0), o1 = from_f<T>(y1);
+          T* dst = out + (size_t)(base + t0 + r) * C + cc;
+          if (p.wide) {
+            V v;
+            pair_make(v, o0, o1);
+            *reinterpret_cast<V*>(dst) = v;
+          } else {
+            dst[0] = o0;
+            if (on1) dst[1] = o1;
+          }
         }
       }
     }
   }
+  if (!FINAL) {                                      // sums of the rows that other threads formed
+    float* part = &sD[0][0].x;
+    un(sum, part[r0 * CH + cp], part[r0 * CH + cp + 1]);
+    __syncthreads();
+    if (tid < CH && w0 + tid < p.CW) {
+      float all = 0.f;
+      for (int r = 0; r < RP; ++r) all += part[r * CH + tid];
+      p.steps[(size_t)u * p.CW + w0 + tid] = all;
+    }
+  }
   if (!active) return;
+  float sv[NL];
+#pragma unroll
+  for (int e = 0; e < NP; ++e) un(S[e], sv[2 * e], sv[2 * e + 1]);
   if (!FINAL) {
 #pragma unroll
-    for (int n = 0; n < kNM; ++n)
-      if (n < N) e0[(size_t)n * CW] = S[n];
-    steps[(size_t)u * CW + w] = sum;
-  } else if (last && state != nullptr) {
-    float* st = state + (size_t)rec_slots[lo] * N * C;
+    for (int e = 0; e < NL; ++e)
+      if (j * NL + e < N) p.ends[((size_t)u * N + j * NL + e) * p.CW + w] = sv[e];
+  } else if (last && p.state != nullptr) {
+    float* st = p.state + (size_t)p.rec_slots[lo] * N * C + c;
 #pragma unroll
-    for (int n = 0; n < kNM; ++n)
-      if (n < N) st[(size_t)n * C + c] = S[n];
+    for (int e = 0; e < NL; ++e)
+      if (j * NL + e < N) st[(size_t)(j * NL + e) * C] = sv[e];
   }
 }
 
-// end states from zero -> entering states, along the chunks of each sequence
-__global__ void __launch_bounds__(128) scan_carry_kernel(const float* __restrict__ A, const float* __restrict__ state,
-                                                         const int* __restrict__ rec_slots, const int* __restrict__ seq_lens,
-                                                         const int* __restrict__ qsl, int C, int N, int c0, int CW,
-                                                         int min_len, float* __restrict__ ends,
-                                                         const float* __restrict__ steps) {
-  constexpr int U = 8;                              // chunks fetched at a time: the chain itself is two operations
+// end states from zero -> entering states, along the pieces of each sequence
+__global__ void __launch_bounds__(128) scan_carry_kernel(const ScanArgs p) {
+  constexpr int U = 8;                              // pieces fetched at a time: the chain itself is two operations
   const int w = blockIdx.x * 128 + threadIdx.x, n = blockIdx.y, s = blockIdx.z;
-  const int q0 = qsl[s], q1 = qsl[s + 1];
-  if (w >= CW || q1 <= q0 || q1 - q0 < min_len) return;
-  const int c = c0 + w, chunks = (q1 - q0 + kL - 1) / kL;
-  const float a = A[(size_t)c * N + n];
-  const bool carried = state != nullptr && seq_lens[s] > q1 - q0;
-  float S = carried ? state[((size_t)rec_slots[s] * N + n) * C + c] : 0.f;
-  const size_t u0 = chunk_base(qsl, s);
-  float* e = ends + (u0 * N + n) * CW + w;
-  const float* d = steps + u0 * CW + w;
-  const size_t stride = (size_t)N * CW;
-  for (int i0 = 0; i0 < chunks; i0 += U) {
+  const int q0 = p.qsl[s], q1 = p.qsl[s + 1];
+  if (w >= p.CW || q1 - q0 <= p.piece) return;      // one piece: it starts from the carried state itself
+  const int c = p.c0 + w, pieces = (q1 - q0 + p.piece - 1) / p.piece;
+  const float a = p.A[(size_t)c * p.N + n];
+  const bool carried = p.state != nullptr && p.seq_lens[s] > q1 - q0;
+  float S = carried ? p.state[((size_t)p.rec_slots[s] * p.N + n) * p.C + c] : 0.f;
+  const size_t u0 = piece_base(p.qsl, s, p.piece);
+  float* e = p.ends + (u0 * p.N + n) * p.CW + w;
+  const float* d = p.steps + u0 * p.CW + w;
+  const size_t stride = (size_t)p.N * p.CW;
+  for (int i0 = 0; i0 < pieces; i0 += U) {
     float g[U], end[U];
 #pragma unroll
     for (int i = 0; i < U; ++i) {
       const int k = i0 + i;
-      const bool ok = k < chunks - 1;               // the last chunk hands nothing on
-      g[i] = ok ? d[(size_t)k * CW] : 0.f;
+      const bool ok = k < pieces - 1;               // the last piece hands nothing on
+      g[i] = ok ? d[(size_t)k * p.CW] : 0.f;
       end[i] = ok ? e[k * stride] : 0.f;
     }
 #pragma unroll
     for (int i = 0; i < U; ++i) {
       const int k = i0 + i;
-      if (k < chunks) {
+      if (k < pieces) {
         e[k * stride] = S;
         S = expf(g[i] * a) * S + end[i];
       }
@@ -158,41 +344,57 @@ __global__ void __launch_bounds__(128) scan_carry_kernel(const float* __restrict
   }
 }
 
-template <typename T>
-int launch_scan(const void* xc, const void* dt_raw, const void* proj, long ldp, const void* xz, long ldxz, const float* A,
-                const float* Dskip, const float* dt_bias, float* state, const int* rec_slots, const int* seq_lens,
-                const int* qsl, int ntok, int nseq, int C, int N, int R, int min_len, int width, float* work, void* out,
-                cudaStream_t st) {
-  const int slots = ntok / kL + nseq;
-  for (int c0 = 0; c0 < C; c0 += width) {
-    const int cw = width < C - c0 ? width : C - c0;
-    float* steps = work + (size_t)slots * N * cw;
-    const dim3 grid((cw + 127) / 128, slots);
-    scan_chunk_kernel<T, false><<<grid, 128, 0, st>>>((const T*)xc, (const T*)dt_raw, (const T*)proj, ldp, (const T*)xz, ldxz,
-                                                      A, Dskip, dt_bias, state, rec_slots, seq_lens, qsl, nseq, C, N, R, c0, cw,
-                                                      min_len, work, steps, (T*)out);
-    scan_carry_kernel<<<dim3((cw + 127) / 128, N, nseq), 128, 0, st>>>(A, state, rec_slots, seq_lens, qsl, C, N, c0, cw,
-                                                                       min_len, work, steps);
-    scan_chunk_kernel<T, true><<<grid, 128, 0, st>>>((const T*)xc, (const T*)dt_raw, (const T*)proj, ldp, (const T*)xz, ldxz,
-                                                     A, Dskip, dt_bias, state, rec_slots, seq_lens, qsl, nseq, C, N, R, c0, cw,
-                                                     min_len, work, steps, (T*)out);
+template <typename T, int LPC, int NS>
+int launch_scan(const void* xc, const void* dt_raw, const void* proj, const void* xz, ScanArgs p, int ntok, int width, float* work,
+                void* out, cudaStream_t st) {
+  constexpr int CH = kThreads / LPC;
+  const int C = p.C, slots = ntok / p.piece + p.nseq;
+  const bool cut = ntok > p.piece;
+  if (!cut) width = C;
+  p.wide = C % 2 == 0 && width % 2 == 0 && p.ldxz % 2 == 0 &&
+           (((uintptr_t)xc | (uintptr_t)dt_raw | (uintptr_t)xz | (uintptr_t)out) & (2 * sizeof(T) - 1)) == 0;
+  for (p.c0 = 0; p.c0 < C; p.c0 += width) {
+    p.CW = width < C - p.c0 ? width : C - p.c0;
+    p.ends = work;
+    p.steps = work + (size_t)slots * p.N * p.CW;
+    const dim3 grid((p.CW + CH - 1) / CH, slots);
+    if (cut) {
+      scan_walk_kernel<T, false, LPC, NS><<<grid, kThreads, 0, st>>>((const T*)xc, (const T*)dt_raw, (const T*)proj, (const T*)xz, (T*)out, p);
+      scan_carry_kernel<<<dim3((p.CW + 127) / 128, p.N, p.nseq), 128, 0, st>>>(p);
+    }
+    scan_walk_kernel<T, true, LPC, NS><<<grid, kThreads, 0, st>>>((const T*)xc, (const T*)dt_raw, (const T*)proj, (const T*)xz, (T*)out, p);
   }
   CUDA_CHECK_RET(cudaGetLastError());
   return 0;
 }
 
+template <typename T>
+int pick_scan(int lanes, const void* xc, const void* dt_raw, const void* proj, const void* xz, const ScanArgs& p, int ntok,
+              int width, float* work, void* out, cudaStream_t st) {
+  auto go = p.N <= 8 ? launch_scan<T, 2, 8> : lanes == 2 ? launch_scan<T, 2, 16> : launch_scan<T, 4, 16>;
+  return go(xc, dt_raw, proj, xz, p, ntok, width, work, out, st);
+}
+
 }  // namespace
 
-// Sequences with at least min_len new tokens are cut, the others walked whole, `width` channels at a time; returns 2 outside its
-// envelope (the caller then uses the token-serial kernel): N <= 16. `work`: (ntok / 64 + nseq) * (N + 1) * min(width, C) floats.
-GLLM_EXPORT int gllm_scan_chunk(const void* xc, const void* dt_raw, const void* proj, long ldp, const void* xz, long ldxz,
-                                const void* A, const void* Dskip, const void* dt_bias, void* state, const void* rec_slots,
-                                const void* seq_lens, const void* qsl, int ntok, int nseq, int C, int N, int R, int min_len,
-                                int width, void* work, void* out, int is_f32, void* stream) {
+// Sequences longer than `piece` tokens are cut, `width` channels at a time; none is if piece >= ntok, and `work` is not used then.
+// Returns 2 outside its envelope (the caller then uses the token-serial kernel): N <= 16. `work`: (ntok / piece + nseq) * (N + 1) *
+// min(width, C) floats.
+GLLM_EXPORT int gllm_scan_walk(const void* xc, const void* dt_raw, const void* proj, long ldp, const void* xz, long ldxz,
+                               const void* A, const void* Dskip, const void* dt_bias, void* state, const void* rec_slots,
+                               const void* seq_lens, const void* qsl, int ntok, int nseq, int C, int N, int R, int piece,
+                               int width, void* work, void* out, int is_f32, void* stream) {
   if (nseq <= 0 || ntok <= 0) return 0;
-  if (N < 1 || N > kNM || width < 1 || min_len > kRows + 1 || nseq > 65535 || ntok / kL + nseq > 65535) return 2;
-  auto go = is_f32 ? launch_scan<float> : launch_scan<__nv_bfloat16>;
-  return go(xc, dt_raw, proj, ldp, xz, ldxz, (const float*)A, (const float*)Dskip, (const float*)dt_bias, (float*)state,
-            (const int*)rec_slots, (const int*)seq_lens, (const int*)qsl, ntok, nseq, C, N, R, min_len, width, (float*)work,
-            out, (cudaStream_t)stream);
+  if (N < 1 || N > kNM || width < 1 || piece < 1 || nseq > 65535 || ntok / piece + nseq > 65535) return 2;
+  ScanArgs p{};
+  p.A = (const float*)A; p.Dskip = (const float*)Dskip; p.dt_bias = (const float*)dt_bias;
+  p.state = (float*)state;
+  p.rec_slots = (const int*)rec_slots; p.seq_lens = (const int*)seq_lens; p.qsl = (const int*)qsl;
+  p.nseq = nseq; p.C = C; p.N = N; p.R = R; p.piece = piece; p.ldp = ldp; p.ldxz = ldxz;
+  // Two lanes per channel spend fewer instructions, four have twice the warps: from three warps per scheduler on, two are faster
+  // (8192 channels, 4 portions of 2048: 572 / 609 us; one of 8192: 1000 / 1090; 4096 channels, 700 tokens: 91 / 63).
+  const int pieces = piece < ntok ? ntok / piece : nseq;
+  const int lanes = static_cast<int64_t>(C) / 16 * pieces >= 3 * 4 * b200::num_sms() ? 2 : 4;
+  return (is_f32 ? pick_scan<float> : pick_scan<__nv_bfloat16>)(lanes, xc, dt_raw, proj, xz, p, ntok, width, (float*)work, out,
+                                                                (cudaStream_t)stream);
 }

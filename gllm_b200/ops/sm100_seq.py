@@ -49,7 +49,7 @@ def _L():
             "gllm_seq_softcap": [P, G, I, I, F, I, P],
             "gllm_seq_conv_silu": [P, G, I, I, I, P, P, I, P, P, P, P, P, I, I, P, I, P],
             "gllm_seq_selective_scan": [P, P, P, G, P, G, P, P, P, P, P, P, P, I, I, I, I, P, I, I, P],
-            "gllm_scan_chunk": [P, P, P, G, P, G] + [P] * 7 + [I] * 7 + [P, P, I, P],
+            "gllm_scan_walk": [P, P, P, G, P, G] + [P] * 7 + [I] * 7 + [P, P, I, P],
             "gllm_seq_relu2": [P, P, G, I, P],
             "gllm_seq_gemm_simt": [P, G, P, G, P, G, I, I, I, I, P, P],
             "gllm_attn_decode_win": [P, G, P, P, P, G, P, P, I, I, I, I, I, I, I, F, I, P, P],
@@ -242,30 +242,42 @@ def causal_conv_silu(xz, channels, w, b, conv_state, rec_slots, seq_lens, query_
     return out
 
 
-_SCAN_MIN_TOKENS = 128              # two chunks: below that the cut form is one chunk in three launches
-_SCAN_WORK_BYTES = 256 << 20        # its workspace at a time; more channels take another round
+_SCAN_WORK_BYTES = 256 << 20        # workspace of a scan cut in time, at a time; more channels take another round
+
+
+def scan_piece(tokens: int, longest: int, channels: int) -> int:
+    """Tokens of a piece of the scan (csrc/seq/scan_ops.cu), for `tokens` tokens in all and at most `longest` in one portion: all of
+    them (nothing is cut), or a multiple of 64. Walking whole portions takes 572 us per 2^26 tokens x channels and no less than
+    0.105 us per token of the longest one; cut, everything is done twice: 940 us, and two launches more (measured, B200). Portions
+    of up to 512 tokens are never cut: there is little to gain, and their bits do not depend on what else is known of the batch."""
+    work = tokens * channels / 2.0 ** 26
+    if longest <= 512 or max(572.0 * work, 0.105 * longest) <= 940.0 * work + 13.0:
+        return tokens
+    return max(64, int(tokens * channels / 8 / (592 * 12)) // 64 * 64)      # twelve pieces for every scheduler
 
 
 def selective_scan(xc, dt_raw, proj, xz, a, d_skip, dt_bias, ssm_state, rec_slots, seq_lens, query_start_loc,
                    channels, nstate, dt_rank, max_q_len: Optional[int] = None):
-    """With `max_q_len` (the longest portion of the batch, or a bound on it), portions of `_SCAN_MIN_TOKENS` tokens and more run
-    cut in time, whatever else is in the batch, and the shorter ones beside them are walked whole in the same launches. Without
-    any of that length, the token-serial kernel takes the batch (the same state, bit for bit; outputs sum their states in
-    another order)."""
+    """With `max_q_len` (the longest portion of the batch, or a bound on it) above one token, four lanes walk a channel
+    (csrc/seq/scan_ops.cu); batches of single tokens, or without a bound, take the token-serial kernel."""
     assert xc.is_contiguous() and dt_raw.is_contiguous() and proj.stride(1) == 1 and xz.stride(1) == 1
     assert a.dtype == torch.float32 and a.is_contiguous()
     out = torch.empty_like(xc)
-    if max_q_len is not None and max_q_len >= _SCAN_MIN_TOKENS:
-        t, slots = xc.shape[0], xc.shape[0] // 64 + seq_lens.shape[0]
-        width = max(128, min(channels, _SCAN_WORK_BYTES // (4 * slots * (nstate + 1)) // 128 * 128))
-        work = torch.empty(slots * (nstate + 1) * min(width, channels), dtype=torch.float32, device=xc.device)
-        rc = _L().gllm_scan_chunk(_p(xc), _p(dt_raw), _p(proj), proj.stride(0), _p(xz), xz.stride(0), _p(a), _p(d_skip),
-                                  _p(dt_bias), _p(ssm_state), _p(rec_slots), _p(seq_lens), _p(query_start_loc), t,
-                                  seq_lens.shape[0], channels, nstate, dt_rank, _SCAN_MIN_TOKENS, width, _p(work), _p(out),
-                                  _f32(xc), stream_ptr())
-        if rc != 2:                          # 2: more states than a thread holds
-            check(rc, "scan_chunk")
-            sm100._count(3 * -(-channels // width))
+    if max_q_len is not None and max_q_len > 1 and xc.shape[0] > 0:
+        t, nseq = xc.shape[0], seq_lens.shape[0]
+        piece = scan_piece(t, min(max_q_len, t), channels)
+        width, work, rounds = channels, None, 1
+        if piece < t:
+            slots = t // piece + nseq
+            width = max(128, min(channels, _SCAN_WORK_BYTES // (4 * slots * (nstate + 1)) // 128 * 128))
+            work = torch.empty(slots * (nstate + 1) * min(width, channels), dtype=torch.float32, device=xc.device)
+            rounds = 3 * -(-channels // width)
+        rc = _L().gllm_scan_walk(_p(xc), _p(dt_raw), _p(proj), proj.stride(0), _p(xz), xz.stride(0), _p(a), _p(d_skip),
+                                 _p(dt_bias), _p(ssm_state), _p(rec_slots), _p(seq_lens), _p(query_start_loc), t, nseq,
+                                 channels, nstate, dt_rank, piece, width, _p(work), _p(out), _f32(xc), stream_ptr())
+        if rc != 2:                          # 2: more states than four lanes hold
+            check(rc, "scan_walk")
+            sm100._count(rounds)
             return out
     # long chunks of few sequences: 4 threads per channel (more warps in flight); decode-like batches: 1
     nseq = seq_lens.shape[0]

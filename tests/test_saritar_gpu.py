@@ -287,3 +287,42 @@ def test_scan_in_rounds_of_channels(dt, state, monkeypatch):
     for (whole, rounds, serial), tol in zip(zip(*got), (1e-5 if dt == torch.float32 else 2.0 ** -8, 1e-5)):
         assert torch.equal(whole, rounds)
         assert float((whole.float() - serial.float()).norm()) <= tol * float(serial.float().norm())
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,C", [(16, 128), (16, 2176), (9, 65), (8, 64), (3, 34), (1, 7)])
+@pytest.mark.parametrize("piece", [None, 16, 40])
+def test_scan_walk_against_float64(dt, N, C, piece, monkeypatch):
+    """Portions around the 16 tokens between two barriers, whole and cut in pieces, with two and four lanes per channel (2176
+    channels fill the machine), steps from 0 (inputs of -60) to 60. fp32: a state keeps at most max(len) rounded sums of relative
+    error 2^-23 each; bf16 outputs are rounded once (2^-8), their inputs are exact in float64."""
+    from gllm_b200.ops import sm100_seq as S
+    torch.manual_seed(N)
+    lens, ctx, R = [1, 15, 16, 17, 0, 33, 100, 2] + [20] * (16 if C > 2000 else 0), [4, 0, 3, 0, 0, 66, 1, 0] + [0] * 16, 5
+    lens, ctx = [n for n in lens if n], [c for n, c in zip(lens, ctx) if n]
+    t, n = sum(lens), len(lens)
+    qsl = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    sl = torch.tensor([a + b for a, b in zip(lens, ctx)], dtype=torch.int32, device=DEV)
+    rs = torch.randperm(n, device=DEV).to(torch.int32)
+    x, dtr, xz = (torch.randn(t, w, device=DEV).to(dt) for w in (C, C, 2 * C))
+    dtr[0, 0], dtr[1, C - 1], dtr[-1, 0] = 60.0, -60.0, 20.5
+    proj = torch.randn(t, R + 2 * N, device=DEV).to(dt)
+    A, Dk, db = -torch.rand(C, N, device=DEV) * 4, torch.randn(C, device=DEV), torch.full((C,), -3.0, device=DEV)
+    st0 = torch.randn(n, N, C, device=DEV)
+    if piece:
+        monkeypatch.setattr(S, "scan_piece", lambda *a: piece)
+    st = st0.clone()
+    got = S.selective_scan(x, dtr, proj, xz, A, Dk, db, st, rs, sl, qsl, C, N, R, max_q_len=max(lens))
+    want, ends, at = torch.empty(t, C, dtype=torch.float64, device=DEV), st0.double(), 0
+    for i, q in enumerate(lens):
+        h = st0[rs[i]].double() if ctx[i] else torch.zeros(N, C, dtype=torch.float64, device=DEV)
+        for k in range(at, at + q):
+            s = torch.nn.functional.softplus(dtr[k].double() + db.double(), threshold=50)
+            h = torch.exp(s * A.double().t()) * h + (s * x[k].double()) * proj[k, R:R + N].double()[:, None]
+            y = (h * proj[k, R + N:].double()[:, None]).sum(0) + Dk.double() * x[k].double()
+            want[k] = y * torch.nn.functional.silu(xz[k, C:].double())
+        ends[rs[i]] = h
+        at += q
+    bound = max(lens) * 2.0 ** -23
+    assert float((st.double() - ends).norm() / ends.norm()) < bound
+    assert float((got.double() - want).norm() / want.norm()) < bound + (2.0 ** -8 if dt == torch.bfloat16 else 0)
