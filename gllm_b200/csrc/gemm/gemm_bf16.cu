@@ -18,6 +18,7 @@
 // and its GEMM -> NCCL all_reduce sequence (gllm/layers/linear.py:247-250).
 #include "../common/host_utils.h"
 #include "../common/ptx.cuh"
+#include "gemm_pair.h"
 #include <string.h>
 
 namespace b200 {
@@ -562,6 +563,17 @@ static int pick_bn(int M, int N, int epi, int forced) {
   return best;
 }
 
+// A round of 256 x 256 tiles on pairs of SMs (gemm_bf16_pair.cu) takes as long as 128 rows of a 190-wide tile on one (500 in
+// the units of pick_bn): 4096 rows, K = 7168: N = 1536 78.5 us on pairs, 78.3 here (two rounds each), N = 576 44.9 / 43.4 (one
+// round each); where pairs need fewer rounds or equal ones of 256 columns they win: 8192 x 16384 x 4096 716 / 808 us, 4096 x
+// 6144 x 4096 141 / 151, 600 x 6144 x 4096 29 / 33, 8192 x 8192 x 256 50 / 82.
+static bool pairs_are_faster(int M, int N, int bn) {
+  const int sms = num_sms(), rows = (M + kBlockM - 1) / kBlockM;
+  const int here = (rows * ((N + bn - 1) / bn) + sms - 1) / sms;
+  const int pairs = ((M + 255) / 256 * ((N + 255) / 256) + sms / 2 - 1) / (sms / 2);
+  return pairs * 500 < here * (bn + 310);
+}
+
 // Decode-sized M: few output tiles, so tile shape and a K split are chosen together. Cost model in SM clocks,
 // calibrated on B200 (profiles/gemm_splitk.md): a 64-deep k-block costs ~650 clk for BN=256 and ~420 clk for
 // BN<=128 (SMEM fill bound: 16 KB of A per k-block regardless of BN), a split-K round adds ~2000 + 24*BN.
@@ -674,6 +686,12 @@ static int gemm_bf16_impl(const void* A, int64_t lda, const void* W, int64_t ldw
   }
   int bn = 128, split = 1;
   choose_cfg(M, N, K, epi, force_bn, ws != nullptr && tile_cnt != nullptr ? ws_bytes : 0, max_tiles, &bn, &split);
+  const bool decode = ws != nullptr && tile_cnt != nullptr && ws_bytes > 0 && M <= g_max_split_m;   // pick_split's sizes
+  if (comm == nullptr && !decode && split == 1 && (epi == kEpiSiluMul || force_bn == 0) && pairs_are_faster(M, N, bn)) {
+    const PairGemm g{A, W, lda, ldw, reinterpret_cast<__nv_bfloat16*>(C), ldc, M, N, K,
+                     reinterpret_cast<const __nv_bfloat16*>(bias), epi == kEpiSiluMul, glu_limit, glu_alpha, gelu};
+    return gemm_bf16_pair(g, reinterpret_cast<cudaStream_t>(stream));
+  }
   CUtensorMap ta, tb;
   if (make_tmap_2d(&ta, A, M, K, lda * 2, kBlockM, kBlockK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)) return 1;
   if (make_tmap_2d(&tb, W, N, K, ldw * 2, bn, kBlockK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)) return 1;

@@ -319,7 +319,7 @@ def test_prefill_value_that_is_no_number(window, bad, clean, seqs):
     assert bool(torch.isnan(got[sees]).all())
 
 
-@pytest.mark.parametrize("family", ["fp8", "attn", "mla"])
+@pytest.mark.parametrize("family", ["fp8", "attn", "mla", "gemm"])
 def test_wait_that_gives_up_reaches_the_caller(family):
     """A wait limit of zero: whatever is not there at the first look is given up. The kernel returns, the engine's check raises,
     and the next call is right again."""
@@ -330,6 +330,10 @@ def test_wait_that_gives_up_reaches_the_caller(family):
         x, w = torch.randn(300, 1024, device=_dev()).bfloat16(), torch.randn(512, 1024, device=_dev()).to(torch.float8_e4m3fn)
         ws = torch.ones(4, 8, device=_dev())
         call = lambda: sm100.linear_fp8_block(x, w, ws)
+        want = x.float() @ w.float().t()
+    elif family == "gemm":
+        x, w = torch.randn(600, 1024, device=_dev()).bfloat16(), torch.randn(6144, 1024, device=_dev()).bfloat16()
+        call = lambda: sm100.linear(x, w)
         want = x.float() @ w.float().t()
     elif family == "attn":
         lens = [300, 129]
@@ -1045,3 +1049,39 @@ def test_gemm_tiles_of_192(m, n, k, monkeypatch):
     want = x.double() @ w.double().t() + b.double()
     tol = want.abs() * 2.0 ** -8 + (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24
     assert bool(((sm100.linear(x, w, b).double() - want).abs() <= tol).all())
+
+
+@pytest.mark.parametrize("m,n,k", [(513, 5000, 8), (600, 6136, 264), (769, 5128, 1000), (4200, 4104, 136), (2305, 19208, 64)])
+def test_gemm_on_pairs_of_sms(m, n, k):
+    """Sizes that run on pairs: rows and columns beyond the last tile of 256 (one row, one CTA's half, eight columns), one to four
+    rounds, K not a multiple of a 64-deep block; rows of the output on a wider stride, the row behind the last untouched. fp32
+    sums, one rounding."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(n + k)
+    x, w = torch.randn(m, k, device=_dev()).bfloat16(), torch.randn(n, k, device=_dev()).bfloat16()
+    b = torch.randn(n, device=_dev()).bfloat16()
+    buf = torch.full((m + 1, n + 8), 7.0, device=_dev(), dtype=torch.bfloat16)
+    sm100.linear(x, w, b, out=buf[:m, :n])
+    want = x.double() @ w.double().t() + b.double()
+    tol = want.abs() * 2.0 ** -8 + (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24
+    assert bool(((buf[:m, :n].double() - want).abs() <= tol).all())
+    assert bool((buf[m] == 7).all()) and bool((buf[:, n:] == 7).all())
+
+
+@pytest.mark.parametrize("act", ["silu", "gelu", "glu"])
+@pytest.mark.parametrize("m,f,k", [(600, 2944, 264), (2305, 4992, 72)])
+def test_gemm_on_pairs_of_sms_gated(m, f, k, act):
+    """Both halves of a gated tile lie in each CTA. One rounding of the output; the gate functions are fp32 on fp32 sums."""
+    from gllm_b200.ops import ref, sm100, sm100_latent
+    torch.manual_seed(f)
+    x, w = torch.randn(m, k, device=_dev()).bfloat16(), (torch.randn(2 * f, k, device=_dev()) * k ** -0.5).bfloat16()
+    wi = ref.interleave_gate_up(w, 128)
+    g, u = (x.double() @ w.double().t()).chunk(2, -1)
+    if act == "glu":
+        got = sm100_latent.linear_glu_clamp(x, wi, 1.5, 1.7)
+        g, u = g.clamp(max=1.5), u.clamp(-1.5, 1.5)
+        want = g * torch.sigmoid(1.7 * g) * (u + 1)
+    else:
+        got = sm100.linear_silu_mul(x, wi, act=act)
+        want = (torch.nn.functional.silu(g) if act == "silu" else torch.nn.functional.gelu(g, approximate="tanh")) * u
+    assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -16 * (1 + want.abs())).all())
