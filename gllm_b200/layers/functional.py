@@ -42,6 +42,14 @@ def linear_silu_mul(x, w_interleaved, out=None, act="silu"):
     return y if out is None else out.copy_(y)
 
 
+def rmsnorm_two(x1, w1, x2, w2, eps):
+    """(rmsnorm(x1) * w1, rmsnorm(x2) * w2) of two column ranges of the same rows."""
+    if x1.is_cuda and all(x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and x.shape[1] % 8 == 0 and x.shape[1] <= 8192
+                          for x in (x1, x2)):
+        return _sm().rmsnorm_two(x1, w1, x2, w2, eps)
+    return rmsnorm(x1.contiguous(), w1, eps)[0], rmsnorm(x2.contiguous(), w2, eps)[0]
+
+
 def rmsnorm(x, w, eps, residual=None, out=None):
     """-> (normed, residual_out). With `residual`, computes residual += x first (in place on GPU)."""
     if x.is_cuda:

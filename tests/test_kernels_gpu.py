@@ -1085,3 +1085,16 @@ def test_gemm_on_pairs_of_sms_gated(m, f, k, act):
         got = sm100.linear_silu_mul(x, wi, act=act)
         want = (torch.nn.functional.silu(g) if act == "silu" else torch.nn.functional.gelu(g, approximate="tanh")) * u
     assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -16 * (1 + want.abs())).all())
+
+
+@pytest.mark.parametrize("t,widths", [(1, (1536, 512)), (5, (8, 8192)), (130, (72, 1000))])
+def test_rmsnorm_two(t, widths):
+    """Two norms over column ranges of the same rows: each as the single one has it (fp32 sums in another order, one rounding)."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(t)
+    x = torch.randn(t, sum(widths) + 64, device=_dev()).bfloat16()
+    x1, x2 = x[:, :widths[0]], x[:, widths[0]:sum(widths)]
+    w1, w2 = (torch.randn(n, device=_dev()).bfloat16() for n in widths)
+    for got, v, w in zip(sm100.rmsnorm_two(x1, w1, x2, w2, 1e-6), (x1, x2), (w1, w2)):
+        want = v.double() * torch.rsqrt(v.double().square().mean(-1, keepdim=True) + 1e-6) * w.double()
+        assert got.is_contiguous() and bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-6).all())
