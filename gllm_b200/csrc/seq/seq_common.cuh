@@ -34,6 +34,13 @@ template <int NT> __device__ __forceinline__ float block_sum(float v, float* scr
   for (int i = 0; i < NT / 32; ++i) t += scratch[i];
   return t;
 }
+// 1 / (1 + e^-v) from the 2^x and 1/x units, within 2^-21 of it: for results that are rounded to bf16 (2^-9)
+__device__ __forceinline__ float sigmoid_unit(float v) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * v));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+  return r;
+}
 // sequence that owns batch row t: largest s with qsl[s] <= t
 __device__ __forceinline__ int find_seq(const int* __restrict__ qsl, int nseq, int t) {
   if (t < nseq && qsl[t] <= t && t < qsl[t + 1]) return t;   // single-token sequences lead the batch: row t is theirs

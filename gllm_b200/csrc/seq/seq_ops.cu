@@ -363,13 +363,14 @@ __global__ void conv_silu_kernel(const T* __restrict__ xz, long ldxz, int C, con
 
 // The same convolution for bf16 rows whose channels come in aligned groups of 4: a thread owns 4 channels (8-byte loads
 // and stores, weights in registers: 8 channels would halve the occupancy) and walks `rows` consecutive batch rows with
-// the last TAPS - 1 inputs in registers, so every input row is read once per block instead of TAPS times. The next kAhead
-// rows' loads are in flight while as many are computed: four in long batches (6000 rows of 8192 channels: 105 -> 86 us against one
-// row ahead), one in short ones, whose blocks have a row or eight (200 single tokens: 18.6 us with four, 16.3 with one; 900 rows
-// 17.3 / 16.3).
+// the last TAPS - 1 inputs in registers, so every input row is read once per block instead of TAPS times. What bounds it is the
+// bytes on their way: in long batches (LONG) the next 16 rows' are, through a ring in shared memory of which each thread fills and
+// reads its own 8 bytes of a row (no barrier); one row ahead in registers in short ones, whose blocks have a row or eight. Then the
+// issue slots, hence the sigmoid from the units. 6000 rows of 8192 channels: 86 us (16 rows per block, four ahead in registers, the
+// sigmoid by __expf and __fdividef), 81 with the ring and 64 rows, 69 with the units; 8192 rows: 119, 104, 87.
 // Sequences of one token also update their carried inputs here (longer ones: the kernel
 // below, after every block has read them).
-template <int TAPS, int kAhead>
+template <int TAPS, bool LONG>
 __global__ void __launch_bounds__(128) conv_silu_vec_kernel(
     const __nv_bfloat16* __restrict__ xz, long ldxz, int C, const float* __restrict__ w, const float* __restrict__ b,
     __nv_bfloat16* __restrict__ state, const int* __restrict__ rec_slots, const int* __restrict__ seq_lens,
@@ -396,15 +397,35 @@ __global__ void __launch_bounds__(128) conv_silu_vec_kernel(
   };
   float win[TAPS][4];                            // win[0 .. TAPS-2]: inputs before the row; win[TAPS-1]: the row's own
   int s = find_seq(qsl, nseq, t0), q0 = 0, q1 = -1;
+  constexpr int kAhead = LONG ? 4 : 1, kGroups = 4;      // rows of a copy group; groups on their way
+  __shared__ uint2 ring[LONG ? kGroups * kAhead : 1][128];
   uint2 q[kAhead], q2[kAhead];
   auto fetch = [&](int tb, uint2 (&v)[kAhead]) {
 #pragma unroll
-    for (int i = 0; i < kAhead; ++i)
-      if (tb + i < t1) v[i] = *reinterpret_cast<const uint2*>(xz + (size_t)(tb + i) * ldxz + c);
+    for (int i = 0; i < kAhead; ++i) {
+      const __nv_bfloat16* src = xz + (size_t)(tb + i) * ldxz + c;
+      if constexpr (LONG) {
+        if (tb + i < t1)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                           (uint32_t)__cvta_generic_to_shared(&ring[(tb - t0 + i) % (kGroups * kAhead)][threadIdx.x])),
+                       "l"(src) : "memory");
+      } else if (tb + i < t1) {
+        v[i] = *reinterpret_cast<const uint2*>(src);
+      }
+    }
+    if constexpr (LONG) asm volatile("cp.async.commit_group;" ::: "memory");
   };
   fetch(t0, q);
+  if constexpr (LONG)
+    for (int g = 1; g < kGroups; ++g) fetch(t0 + g * kAhead, q);
   for (int tb = t0; tb < t1; tb += kAhead) {
-    fetch(tb + kAhead, q2);
+    if constexpr (LONG) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kGroups - 1) : "memory");
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) q[i] = ring[(tb - t0 + i) % (kGroups * kAhead)][threadIdx.x];
+    } else {
+      fetch(tb + kAhead, q2);
+    }
 #pragma unroll
     for (int i = 0; i < kAhead; ++i) {
       const int t = tb + i;
@@ -436,7 +457,7 @@ __global__ void __launch_bounds__(128) conv_silu_vec_kernel(
         float acc = br[e];
 #pragma unroll
         for (int j = 0; j < TAPS; ++j) acc = fmaf(wr[e * TAPS + j], win[j][e], acc);
-        o[e] = __float2bfloat16_rn(act == 0 ? acc * __fdividef(1.0f, 1.0f + __expf(-acc)) : acc);
+        o[e] = __float2bfloat16_rn(act == 0 ? acc * sigmoid_unit(acc) : acc);
 #pragma unroll
         for (int j = 0; j + 1 < TAPS; ++j) win[j][e] = win[j + 1][e];
       }
@@ -452,8 +473,12 @@ __global__ void __launch_bounds__(128) conv_silu_vec_kernel(
         *reinterpret_cast<uint2*>(st + (size_t)(TAPS - 2) * C) = cur;
       }
     }
+    if constexpr (LONG) {
+      fetch(tb + kGroups * kAhead, q);                   // into the places that have been read
+    } else {
 #pragma unroll
-    for (int i = 0; i < kAhead; ++i) q[i] = q2[i];
+      for (int i = 0; i < kAhead; ++i) q[i] = q2[i];
+    }
   }
 }
 
@@ -760,10 +785,14 @@ GLLM_EXPORT int gllm_seq_conv_silu(const void* xz, long ldxz, int ntok, int nseq
     const bool vec = C % 4 == 0 && ldxz % 4 == 0 && ((uintptr_t)xz & 7) == 0 && taps >= 1 && taps <= 4 &&
                      ((uintptr_t)state & 7) == 0 && ((uintptr_t)out & 7) == 0 && ((uintptr_t)w & 15) == 0 &&
                      ((uintptr_t)b & 15) == 0;
-    const int rows = ntok >= 2048 ? 16 : (ntok >= 512 ? 8 : 1);
-    dim3 vgrid((ntok + rows - 1) / rows, (C / 4 + 127) / 128);
+    // Rows of a block: as many as leave eight blocks for every SM, for a block starts with a chain of loads (its sequence, the rows
+    // before its first).
+    const int across = (C / 4 + 127) / 128;
+    int rows = ntok >= 2048 ? 64 : (ntok >= 512 ? 8 : 1);
+    while (rows > 16 && (int64_t)((ntok + rows - 1) / rows) * across < 8 * b200::num_sms()) rows /= 2;
+    dim3 vgrid((ntok + rows - 1) / rows, across);
 #define GLLM_CONV_VEC(TAPS)                                                                                        \
-  (rows == 16 ? conv_silu_vec_kernel<TAPS, 4> : conv_silu_vec_kernel<TAPS, 1>)<<<vgrid, 128, 0, st>>>(              \
+  (rows >= 16 ? conv_silu_vec_kernel<TAPS, true> : conv_silu_vec_kernel<TAPS, false>)<<<vgrid, 128, 0, st>>>(              \
       (const __nv_bfloat16*)xz, ldxz, C, (const float*)w, (const float*)b, (__nv_bfloat16*)state,                  \
       (const int*)rec_slots, (const int*)seq_lens, (const int*)qsl, nseq, ntok, rows, (__nv_bfloat16*)out, act,    \
       (const float*)in_bias)

@@ -19,13 +19,6 @@ using namespace seqk;
 
 __device__ __forceinline__ float sigmoid_f(float v) { return 1.0f / (1.0f + expf(-v)); }
 __device__ __forceinline__ float silu_f(float v) { return v / (1.0f + expf(-v)); }
-// the same sigmoid from the 2^x and 1/x units, within 2^-21 of it: for results that are rounded to bf16 (2^-9)
-__device__ __forceinline__ float sigmoid_unit(float v) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * v));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-  return r;
-}
 
 // x <- rms(alpha * x + y) * w (fp32 stream, in place); out = the same row in the compute dtype (optional)
 template <typename T>
