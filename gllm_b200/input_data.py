@@ -290,6 +290,15 @@ class InputData:
             return ([(h, h.numpy()) for h in hosts], torch.zeros(shape, dtype=dtype, device=self.device))
 
         self._flip = 0
+        # Small arrays of a step go to the device as one block and are put into their buffers by one kernel
+        # (csrc/elemwise/batch_load.cu): staging block (two, like the arrays' own), its place on the device, one row per array.
+        self._blocks = None
+        if pin:
+            hosts = [torch.zeros(self._BLOCK_WORDS, dtype=i32, pin_memory=True) for _ in range(2)]
+            self._blocks = [(h, {np.dtype(np.int32): h.numpy(), np.dtype(np.float32): h.numpy().view(np.float32)}) for h in hosts]
+            self._block_dev = torch.zeros(self._BLOCK_WORDS, dtype=i32, device=self.device)
+            self._parts = np.zeros((16, 5), np.int64)
+        self._num_parts = self._block_at = self._most_words = 0
 
         self._tokens = buf((max_tokens,), i32)
         self._positions = buf((3, max_tokens) if mrope else (max_tokens,), i32)
@@ -315,11 +324,28 @@ class InputData:
         self.latent_plan = None  # how latent attention splits the loaded batch (models/deepseek_v2.py), made by its first layer
         self.decode_splits = None  # None: pick per batch (eager); int: fixed (CUDA graphs)
 
+    # A decode step of 64 sequences has some 2000 words beside its block table. Above the limit an array is copied by itself: there
+    # the bytes count, and the block would only be moved twice. One sequence: 8 copies 20 us, the block and its kernel 5.
+    _BLOCK_WORDS, _PART_WORDS = 16384, 4096
+
     def _put(self, pair, arr: np.ndarray):
-        """numpy array -> this step's pinned staging buffer (plain numpy store through a shared-memory view: no
-        tensor wrapping per array) -> one non-blocking H2D copy."""
+        """numpy array -> this step's pinned staging block, to be sent with the others by `_send_block`, or, if it is large, its
+        own pinned staging buffer and one non-blocking H2D copy (plain numpy stores through shared-memory views: no tensor
+        wrapping per array)."""
         stages, dev = pair
         host, host_np = stages[self._flip]
+        n = arr.size
+        if self._blocks is not None and 0 < n <= self._PART_WORDS and self._block_at + n <= self._BLOCK_WORDS and \
+                self._num_parts < 16:
+            at = self._block_at
+            self._blocks[self._flip][1][host_np.dtype][at:at + n].reshape(arr.shape)[...] = arr
+            rows, cols, pitch = (1, n, n) if arr.ndim == 1 else (*arr.shape, dev.stride(0))
+            assert rows <= dev.shape[0] and cols <= dev.shape[-1]
+            self._parts[self._num_parts] = dev.data_ptr(), pitch, at, rows, cols
+            self._num_parts += 1
+            self._block_at = at + n
+            self._most_words = max(self._most_words, n)
+            return
         if arr.ndim == 1:
             n = arr.shape[0]
             host_np[:n] = arr
@@ -328,6 +354,14 @@ class InputData:
             r, c = arr.shape
             host_np[:r, :c] = arr
             dev[:r, :c].copy_(host[:r, :c], non_blocking=True)
+
+    def _send_block(self):
+        if self._num_parts:
+            from gllm_b200.ops import sm100
+            n = self._block_at
+            self._block_dev[:n].copy_(self._blocks[self._flip][0][:n], non_blocking=True)
+            sm100.batch_load(self._block_dev, self._parts, self._num_parts, self._most_words)
+        self._num_parts = self._block_at = self._most_words = 0
 
     def load(self, batch: BatchArrays):
         assert batch.num_tokens <= self.max_tokens, (batch.num_tokens, self.max_tokens)
@@ -367,6 +401,7 @@ class InputData:
                 self._put(self._top_p, batch.top_p)
                 self._put(self._rep_penalty, batch.rep_penalty)
                 self._put(self._state_slot, batch.state_slot)
+        self._send_block()
 
     def apply_feed(self, prev_tokens_out: torch.Tensor):
         """Lookahead step: the input tokens are the previous step's sampled tokens, still on the device."""

@@ -172,6 +172,13 @@ def rmsnorm_two(x1: torch.Tensor, w1: torch.Tensor, x2: torch.Tensor, w2: torch.
     return o1, o2
 
 
+def batch_load(block: torch.Tensor, parts, n: int, most: int):
+    """Arrays of a step out of `block` (32-bit words) into their buffers. parts: int64 rows (device pointer, row pitch, first word
+    in the block, rows, columns), the first `n` of them; most: words of the largest."""
+    check(_lib.load().gllm_batch_load(_p(block), parts.ctypes.data, n, most, stream_ptr()), "batch_load")
+    _count()
+
+
 def silu_and_mul(x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     assert x.dtype == _BF16 and x.dim() == 2 and x.stride(1) == 1
     t, two_i = x.shape

@@ -1069,9 +1069,10 @@ def test_gemm_on_pairs_of_sms(m, n, k):
 
 
 @pytest.mark.parametrize("act", ["silu", "gelu", "glu"])
-@pytest.mark.parametrize("m,f,k", [(600, 2944, 264), (2305, 4992, 72)])
-def test_gemm_on_pairs_of_sms_gated(m, f, k, act):
-    """Both halves of a gated tile lie in each CTA. One rounding of the output; the gate functions are fp32 on fp32 sums."""
+@pytest.mark.parametrize("m,f,k", [(600, 2944, 264), (2305, 4992, 72), (33, 128, 72), (64, 12288, 136), (128, 4736, 200)])
+def test_gemm_gated_tiles(m, f, k, act):
+    """On pairs of SMs, where both halves of a gated tile lie in each CTA; up to 128 rows in tiles of 96 features, whose rows
+    straddle the blocks that gate and up rows alternate in. One rounding of the output; the gate functions are fp32 on fp32 sums."""
     from gllm_b200.ops import ref, sm100, sm100_latent
     torch.manual_seed(f)
     x, w = torch.randn(m, k, device=_dev()).bfloat16(), (torch.randn(2 * f, k, device=_dev()) * k ** -0.5).bfloat16()
@@ -1098,3 +1099,30 @@ def test_rmsnorm_two(t, widths):
     for got, v, w in zip(sm100.rmsnorm_two(x1, w1, x2, w2, 1e-6), (x1, x2), (w1, w2)):
         want = v.double() * torch.rsqrt(v.double().square().mean(-1, keepdim=True) + 1e-6) * w.double()
         assert got.is_contiguous() and bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-6).all())
+
+
+@pytest.mark.parametrize("seqs,blocks,tokens", [(1, 1, 1), (3, 7, 3), (64, 60, 64), (64, 70, 4100), (200, 100, 5000)])
+def test_batch_arrays_reach_their_buffers(seqs, blocks, tokens):
+    """A step's arrays on the device are the host's, whether they go in the staging block or are copied by themselves (more than
+    4096 words each, or beyond the block's 16,384), over several steps that alternate the staging buffers; rows beyond them stay."""
+    import numpy as np
+    from gllm_b200.input_data import BatchArrays, InputData
+    inp, rng = InputData(6000, 256, 128, "cuda:0"), np.random.RandomState(seqs)
+    i32, f32 = np.int32, np.float32
+    for step in range(3):
+        ints = lambda n: rng.randint(0, 1 << 30, n).astype(i32)
+        b = BatchArrays(tokens=ints(tokens), positions=ints(tokens), slot_mapping=ints(tokens),
+                        block_table=rng.randint(0, 1 << 30, (seqs, blocks)).astype(i32), seq_lens=ints(seqs),
+                        query_start_loc=ints(seqs + 1), logits_idx=ints(seqs), emit_seq=np.arange(seqs, dtype=i32),
+                        temperature=rng.rand(seqs).astype(f32), top_k=ints(seqs), top_p=rng.rand(seqs).astype(f32),
+                        rep_penalty=rng.rand(seqs).astype(f32), state_slot=ints(seqs), num_decode_seqs=0, num_seqs=seqs,
+                        num_tokens=tokens, max_q_len=2, max_seq_len=9, rec_slots=ints(seqs), all_greedy=False)
+        inp.load(b)
+        for pair, want in ((inp._tokens, b.tokens), (inp._positions, b.positions), (inp._slots, b.slot_mapping),
+                           (inp._seq_lens, b.seq_lens), (inp._qsl, b.query_start_loc), (inp._logits_idx, b.logits_idx),
+                           (inp._temperature, b.temperature), (inp._top_k, b.top_k), (inp._top_p, b.top_p),
+                           (inp._rep_penalty, b.rep_penalty), (inp._state_slot, b.state_slot), (inp._rec_slots, b.rec_slots)):
+            got = pair[1].cpu().numpy()
+            assert np.array_equal(got[:len(want)], want) and not got[len(want):].any()
+        table = inp._block_table[1].cpu().numpy()
+        assert np.array_equal(table[:seqs, :blocks], b.block_table) and not table[seqs:].any() and not table[:, blocks:].any()
