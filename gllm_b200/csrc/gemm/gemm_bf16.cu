@@ -169,6 +169,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     // ===================== TMA producer =====================
     if (lane == 0) {
       uint32_t it = 0;
+      auto load_b = [&](uint8_t* dst, uint64_t* bar, int k0, int row) {
+        if constexpr (EPI == kEpiSiluMul && BN == 192) {     // 96 features: three boxes of 32 gate rows, three of their up rows
+#pragma unroll
+          for (int i = 0; i < 6; ++i) {
+            const int f = row / 2 + (i % 3) * 32;            // rows are interleaved per 128
+            tma_load_2d(dst + i * 32 * kBlockK * 2, &tmap_b, bar, k0, f / 128 * 256 + f % 128 + (i / 3) * 128, kEvictNormal);
+          }
+        } else {
+          tma_load_2d(dst, &tmap_b, bar, k0, row, kEvictNormal);
+        }
+      };
       // weights (B) do not depend on the previous kernel: put the first stages' B tiles in flight, then wait
       uint32_t pre = 0;
       if (!grouped) {
@@ -181,7 +192,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           for (uint32_t i = 0; i < pre; ++i) {
             uint8_t* sb = smem + i * Cfg::kStageBytes + Cfg::kABytes;
             mbar_expect_tx(&full_bar[i], Cfg::kStageBytes);
-            tma_load_2d(sb, &tmap_b, &full_bar[i], (kb0 + static_cast<int>(i)) * kBlockK, n0, kEvictNormal);
+            load_b(sb, &full_bar[i], (kb0 + static_cast<int>(i)) * kBlockK, n0);
           }
         }
         griddep_wait();
@@ -229,7 +240,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           mbar_expect_tx(&full_bar[s], Cfg::kStageBytes);
           if (p.batch > 0) tma_load_3d(sa, &tmap_a, &full_bar[s], kb * kBlockK, (mt - bidx * tpb) * kBlockM, bidx);
           else tma_load_2d(sa, &tmap_a, &full_bar[s], kb * kBlockK, m0, kEvictNormal);
-          tma_load_2d(sb, &tmap_b, &full_bar[s], kb * kBlockK, n0 + b_row_off, kEvictNormal);
+          load_b(sb, &full_bar[s], kb * kBlockK, n0 + b_row_off);
         }
       }
     }
@@ -373,7 +384,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       // Output tiles go through a per-warp swizzled smem transpose so that every global (or peer / NVLink)
       // store instruction writes full 128-byte row segments instead of 32 scattered 16-byte pieces.
       constexpr int OUT_W = (EPI == kEpiSiluMul) ? BN / 2 : BN;   // output columns of this tile
-      constexpr int W = OUT_W < 64 ? OUT_W : 64;                  // columns per staged chunk
+      constexpr int W = OUT_W % 64 != 0 ? 32 : 64;                // columns per staged chunk
       constexpr int LPR = W / 8;                                  // lanes (16 B each) per staged row
       constexpr int RPI = 32 / LPR;                               // rows per store instruction
       uint8_t* stg = epi_smem + (warp - 2) * 4096;
@@ -446,13 +457,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll 1
         for (int c = c_lo; c < c_hi; c += W) {
 #pragma unroll
-          for (int h = 0; h < W; h += 16) {
+          for (int h = 0; h < W; h += 32) {
             if (c + h >= c_hi) break;
-            uint32_t g[16], u[16];
+            uint32_t g[32], u[32];
             load_acc(c + h, g);
             load_acc(H + c + h, u);
 #pragma unroll
-            for (int j = 0; j < 16; j += 8) {
+            for (int j = 0; j < 32; j += 8) {
               float f[8];
 #pragma unroll
               for (int e = 0; e < 8; ++e) {
@@ -694,7 +705,12 @@ static int gemm_bf16_impl(const void* A, int64_t lda, const void* W, int64_t ldw
   }
   CUtensorMap ta, tb;
   if (make_tmap_2d(&ta, A, M, K, lda * 2, kBlockM, kBlockK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)) return 1;
-  if (make_tmap_2d(&tb, W, N, K, ldw * 2, bn, kBlockK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)) return 1;
+  // One row of gated tiles: the weights are the traffic, and 128 SMs that read 192 rows each draw more than 96 that read 256
+  // (64 rows, 24,576 x 4096 and the 4096 x 12,288 behind it: 76.9 -> 70.4 us).
+  const int sms = num_sms();
+  if (epi == kEpiSiluMul && comm == nullptr && split == 1 && M <= kBlockM && (N + 255) / 256 < sms && (N + 191) / 192 <= sms) bn = 192;
+  if (make_tmap_2d(&tb, W, N, K, ldw * 2, epi == kEpiSiluMul && bn == 192 ? 32 : bn, kBlockK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16))
+    return 1;
   GemmParams p;
   memset(&p, 0, sizeof(p));
   p.split_k = split;
@@ -728,8 +744,7 @@ static int gemm_bf16_impl(const void* A, int64_t lda, const void* W, int64_t ldw
                               : launch_gemm<BN_, kEpiStore>(ta, tb, p, st);
   switch (bn) {
     DISPATCH(256)
-    case 192:
-      return launch_gemm<192, kEpiStore>(ta, tb, p, st);
+    DISPATCH(192)
     DISPATCH(128)
     DISPATCH(64)
     case 32:
