@@ -12,13 +12,13 @@
 //
 // What bounds it: the 2^x unit (8 cycles per warp and exponential: 64 of about 100 cycles per token of a warp with 16 channels)
 // and issue slots. So the arithmetic is on pairs (f32x2), log2(e) is multiplied into A, softplus and silu are formed once per
-// token and channel in forms of their own instead of expf, log1pf and a division (790 -> 730 us), and the exponential is the bare
-// instruction with its bias taken out (a quarter of them as polynomials on the fma units: 730 instead of 614 us). 128 registers,
-// for the scheduler to overlap four tokens: 572 us, at 96 628.
-// 8192 ragged tokens in 4 sequences, 8192 channels, 16 states: 1342 -> 572 us (B200); one sequence of 16384 tokens, 2048 channels,
-// cut in pieces: 710 -> 480. Before, every batch ran as chunks of 64 tokens in two passes, a thread per channel, with expf.
-// Error against float64 after 2048 tokens, steps around 0.01 (fp32 outputs / states): 8.3e-8 / 1.8e-7; chunks with expf 8.0e-8 /
-// 1.8e-7; token-serial with expf 9.3e-8 / 1.8e-7.
+// token and channel in forms of their own instead of expf, log1pf and a division, and the exponential is the bare instruction with
+// its bias taken out (a quarter of them as polynomials on the fma units: 730 instead of 614 us). 128 registers, for the scheduler to
+// overlap four tokens (at 96: 10 % more).
+// 2048 tokens in each of 4 sequences, 8192 channels, 16 states, bf16: 1329 us as chunks of 64 tokens in two passes, a thread per channel,
+// with expf; 610 so (556 with the exponents of softplus and silu rounded to one fp32, which cost up to ten times the error).
+// Relative error of the steps / gates against float64, rms over inputs in (-20, 20): at most 5.1e-8 / 5.1e-8, with expf, log1pf and a
+// division 4.8e-8 / 4.9e-8; largest 1.8e-7 / 1.7e-7 and 1.9e-7 / 2.3e-7.
 #include <cuda_bf16.h>
 
 #include "common/host_utils.h"
@@ -55,32 +55,59 @@ __device__ __forceinline__ f2 rcp2(f2 v) {
   un(v, a, b);
   return pk(rcp(a), rcp(b));
 }
-// log(1 + e^v) of both halves = max(v, 0) + log1p(e), e = e^-|v|; log1p(e) = 2 atanh(s), s = e / (2 + e) <= 1/3, by the polynomial of
-// least relative error (4.5e-9) in s^2. Relative error below 1.5e-7 at any v, where expf and log1pf one after the other have as much.
-__device__ __forceinline__ f2 softplus2(f2 v) {
-  float v0, v1;
+// e^-|v| = e (1 + c) of both halves. The exponent |v| log2 e is formed in two parts: rounded to one it would cost |v| 2^-24, 9e-7
+// at v = -20. Here 2^x keeps denormals: it is formed once per token and channel.
+__device__ __forceinline__ void exp_neg2(f2 v, f2& e, f2& c) {
+  float v0, v1, t0, t1;
   un(v, v0, v1);
-  const f2 e = exp2_unit(fma2(pk(fabsf(v0), fabsf(v1)), pk(-1.4426950408889634f, -1.4426950408889634f), pk(kBias, kBias)));
-  const f2 r = rcp2(add2(e, pk(2.f, 2.f)));
+  v0 = fabsf(v0);
+  v1 = fabsf(v1);
+  const f2 m = pk(v0 > 200.f ? 200.f : v0, v1 > 200.f ? 200.f : v1);       // finite, or NaN
+  const f2 t = mul2(m, pk(1.4426950216293335f, 1.4426950216293335f));
+  const f2 rest = fma2(m, pk(-1.925963033500011e-8f, -1.925963033500011e-8f), fma2(m, pk(-1.4426950216293335f, -1.4426950216293335f), t));
+  c = fma2(rest, pk(0.6931472f, 0.6931472f), pk(1.9e-8f, 1.9e-8f));
+  un(t, t0, t1);
+  asm("ex2.approx.f32 %0, %1;" : "=f"(v0) : "f"(-t0));
+  asm("ex2.approx.f32 %0, %1;" : "=f"(v1) : "f"(-t1));
+  e = pk(v0, v1);
+}
+__device__ __forceinline__ f2 neg2(f2 v) { return v ^ 0x8000000080000000ull; }
+// log(1 + e^v) of both halves = max(v, 0) + log1p(e), e = e^-|v|; log1p(e) = 2 atanh(s), s = e / (2 + e) <= 1/3, by the polynomial of
+// least relative error (4.5e-9) in s^2. Two roundings (2^x, the last sum): what the division leaves over and the second part of e
+// are added at the end, their factors need no accuracy.
+__device__ __forceinline__ f2 softplus2(f2 v) {
+  f2 e, c;
+  exp_neg2(v, e, c);
+  const f2 two = pk(2.f, 2.f), r = rcp2(add2(e, two));
   f2 s = mul2(e, r);
-  const f2 ns = mul2(s, pk(-1.f, -1.f));
-  s = fma2(r, fma2(ns, e, fma2(ns, pk(2.f, 2.f), e)), s);
+  s = fma2(r, fma2(neg2(s), e, fma2(neg2(s), two, e)), s);
+  const f2 left = fma2(neg2(s), e, fma2(neg2(s), two, e));
   const f2 q = mul2(s, s), twice = add2(s, s);
   f2 w = fma2(q, pk(0.14005993f, 0.14005993f), pk(0.14000903f, 0.14000903f));
   w = fma2(q, w, pk(0.20010763f, 0.20010763f));
   w = fma2(q, w, pk(0.3333321f, 0.3333321f));
-  return add2(pk(fmaxf(v0, 0.f), fmaxf(v1, 0.f)), fma2(twice, mul2(q, w), twice));
+  const f2 l = add2(twice, fma2(twice, fma2(q, w, c), mul2(add2(r, r), left)));
+  float v0, v1;
+  un(v, v0, v1);
+  return add2(pk(fmaxf(v0, 0.f), fmaxf(v1, 0.f)), l);
 }
-// z / (1 + e^-z)
+// z / (1 + e^-z) of both halves, as z / (1 + e) or z e / (1 + e) with e = e^-|z|: nothing overflows. What z e and the division leave
+// over and the second part of e are added at the end.
 __device__ __forceinline__ f2 silu2(f2 z) {
-  const f2 e = exp2_unit(fma2(z, pk(-1.4426950408889634f, -1.4426950408889634f), pk(kBias, kBias)));
-  const f2 d = add2(e, pk(1.f, 1.f)), r = rcp2(d);
-  const f2 better = fma2(r, fma2(mul2(r, pk(-1.f, -1.f)), d, pk(1.f, 1.f)), r);        // NaN where d is infinite
-  float d0, d1, r0, r1, b0, b1;
-  un(d, d0, d1);
-  un(r, r0, r1);
+  f2 e, c;
+  exp_neg2(z, e, c);
+  float z0, z1, e0, e1, c0, c1;
+  un(z, z0, z1);
+  un(e, e0, e1);
+  un(c, c0, c1);
+  const f2 m = pk(z0 < 0.f ? e0 : 1.f, z1 < 0.f ? e1 : 1.f), g = pk(z0 < 0.f ? c0 : -c0 * e0, z1 < 0.f ? c1 : -c1 * e1);
+  const f2 num = mul2(z, m), r = rcp2(add2(e, pk(1.f, 1.f))), q = mul2(num, r);
+  const f2 left = add2(fma2(neg2(q), e, add2(num, neg2(q))), fma2(z, m, neg2(num)));
+  const f2 better = fma2(r, fma2(q, g, left), q);                          // NaN where z is infinite
+  float q0, q1, b0, b1;
+  un(q, q0, q1);
   un(better, b0, b1);
-  return mul2(z, pk(d0 < 1e37f ? b0 : r0, d1 < 1e37f ? b1 : r1));
+  return pk(fabsf(z0) <= 3.4028235e38f ? b0 : q0, fabsf(z1) <= 3.4028235e38f ? b1 : q1);
 }
 
 // Piece slots: sequence s owns slots from qsl[s] / piece + s on (at least one per started piece); some stay empty.

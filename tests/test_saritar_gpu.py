@@ -326,3 +326,28 @@ def test_scan_walk_against_float64(dt, N, C, piece, monkeypatch):
     bound = max(lens) * 2.0 ** -23
     assert float((st.double() - ends).norm() / ends.norm()) < bound
     assert float((got.double() - want).norm() / want.norm()) < bound + (2.0 ** -8 if dt == torch.bfloat16 else 0)
+
+
+@pytest.mark.parametrize("lo,hi", [(-20, -10), (-7, -3), (-3, 3), (3, 25), (-100, -80)])
+def test_scan_steps_and_gates_one_by_one(lo, hi):
+    """Portions of one token from empty states with x = B = 1, C = 0, D = 1: the states are softplus(dt), the outputs silu(z). The 2^x
+    unit is within 2^-22 (2 ulp; twice that where it squares a result to reach denormals, below -87), two to three further roundings of
+    2^-24 each; in the denormals their spacing. Infinities and NaN as the token-serial kernel has them."""
+    from gllm_b200.ops import sm100_seq as S
+    n, C, N = 40, 1030, 3
+    torch.manual_seed(hi)
+    v = torch.rand(n, C, device=DEV) * (hi - lo) + lo
+    v[3, :5] = torch.tensor([float("inf"), -float("inf"), float("nan"), 0.0, -0.0], device=DEV)
+    proj = torch.cat([torch.ones(n, N, device=DEV), torch.zeros(n, N, device=DEV)], 1)
+    qsl, ones = torch.arange(n + 1, device=DEV, dtype=torch.int32), torch.ones(n, C, device=DEV)
+    got = []
+    for mx in (2, None):
+        st = torch.empty(n, N, C, device=DEV)
+        y = S.selective_scan(ones, v, proj, torch.cat([ones, v], 1), -torch.rand(C, N, device=DEV), ones[0], torch.zeros(C, device=DEV), st,
+                             qsl[:n], qsl[:n] * 0 + 1, qsl, C, N, 0, max_q_len=mx)
+        got.append((st[:, N - 1], y))
+    d = v.double()
+    for one, serial, want in zip(*got, (torch.logaddexp(d, torch.zeros_like(d)), d * torch.sigmoid(d))):
+        fine = torch.isfinite(d)
+        assert bool(((one.double() - want).abs() <= want.abs() * 2.0 ** (-21.4 if lo > -80 else -20.4) + 2.0 ** -148 * (1 + d.abs()))[fine].all())
+        assert torch.equal(torch.nan_to_num(one[3, :3], 7.0, 8.0, 9.0), torch.nan_to_num(serial[3, :3], 7.0, 8.0, 9.0))
