@@ -16,7 +16,8 @@
 // its bias taken out (a quarter of them as polynomials on the fma units: 730 instead of 614 us). 128 registers, for the scheduler to
 // overlap four tokens (at 96: 10 % more).
 // 2048 tokens in each of 4 sequences, 8192 channels, 16 states, bf16: 1329 us as chunks of 64 tokens in two passes, a thread per channel,
-// with expf; 610 so (556 with the exponents of softplus and silu rounded to one fp32, which cost up to ten times the error).
+// with expf; 661 so (556 with the exponents of softplus and silu rounded to one fp32, which cost up to ten times their error, and
+// without `anchored`).
 // Relative error of the steps / gates against float64, rms over inputs in (-20, 20): at most 5.1e-8 / 5.1e-8, with expf, log1pf and a
 // division 4.8e-8 / 4.9e-8; largest 1.8e-7 / 1.7e-7 and 1.9e-7 / 2.3e-7.
 #include <cuda_bf16.h>
@@ -30,6 +31,7 @@ using namespace seqk;
 constexpr int kNM = 16;                             // most states of a channel
 constexpr int kThreads = 128;
 constexpr int kTile = 16;                           // tokens between two barriers
+constexpr int kAnchor = 4;                          // tiles between two corrections of the states' decay
 
 // ---- pairs of fp32 ----
 typedef unsigned long long f2;
@@ -44,6 +46,9 @@ __device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32
 // 2^t of both halves on the 2^x unit. Its results lie 1.5e-8 to 2e-8 below 2^t on average for t in (-1, 0), which adds up over the
 // tokens that a state remembers. The caller adds kBias = 1.9e-8 / ln 2 to t in the fma that forms it (states after 2048 tokens
 // against float64, steps of 0.001 to 0.1: 1.46e-7 with 2.2e-8, 1.41e-7 with 2.6e-8, 1.53e-7 with 3.4e-8; expf 1.43e-7).
+// A single decay: A log2(e) is rounded before the product, so that decays of e^-5 and less have 1.4 times the rms error of expf(dt A),
+// of a value that is added to 150 times its size, and below 2^-126 they are 0. The states show nothing of it: steps of 0.1 to 2, A to
+// -24, 5.3e-8 against 5.4e-8 with expf.
 constexpr float kBias = 2.7e-8f;
 __device__ __forceinline__ f2 exp2_unit(f2 t) {
   float t0, t1;
@@ -110,6 +115,16 @@ __device__ __forceinline__ f2 silu2(f2 z) {
   return pk(fabsf(z0) <= 3.4028235e38f ? b0 : q0, fabsf(z1) <= 3.4028235e38f ? b1 : q1);
 }
 
+constexpr float kMostF = 3.4028235e38f;
+// What a state lacks after steps of `Dt` in all from S0 on, decays whose product was P: the unit's errors have one sign for decays of
+// about the same size, and a state that keeps thousands of tokens adds them up. exp(A Dt), formed once in 64 tokens, does not. States
+// of 2048 tokens whose decays lie around 0.9999 / 0.999 / 0.99, against float64: 1.4e-6 / 8.4e-7 / 3.4e-7, without it 2.3e-5 / 1.0e-5 /
+// 5.5e-7, chunks of 64 tokens with expf 9e-7 / 1.5e-6 / 4.0e-7. It costs 8 % of the kernel.
+__device__ __forceinline__ float anchored(float a, float Dt, float P, float S0) {
+  const float lack = (exp2f(a * Dt) - P) * S0;
+  return fabsf(lack) <= kMostF ? lack : 0.f;         // infinite states and growing ones stay as they are
+}
+
 // Piece slots: sequence s owns slots from qsl[s] / piece + s on (at least one per started piece); some stay empty.
 __device__ __forceinline__ int piece_base(const int* qsl, int s, int piece) { return qsl[s] / piece + s; }
 
@@ -164,6 +179,8 @@ scan_walk_kernel(const T* __restrict__ xc, const T* __restrict__ dt_raw, const T
   const int wc = active ? w : p.CW - 1, c = p.c0 + wc;                     // idle threads mirror the last channel (loads only)
 
   f2 S[NP], a[NP];                                   // states; A log2(e)
+  f2 S0[NP], P[NP];                                  // states and product of the decays since the last anchor
+  float Dt = 0.f;                                    // sum of the steps since then
   {
     const bool carried = whole && p.state != nullptr && p.seq_lens[lo] > q1 - q0;
     const float* from = carried ? p.state + (size_t)p.rec_slots[lo] * N * C + c : p.ends + (size_t)u * N * p.CW + wc;
@@ -176,7 +193,11 @@ scan_walk_kernel(const T* __restrict__ xc, const T* __restrict__ dt_raw, const T
       sv[e] = FINAL && n < N && (carried || !whole) ? from[n * step] : 0.f;
     }
 #pragma unroll
-    for (int e = 0; e < NP; ++e) { S[e] = pk(sv[2 * e], sv[2 * e + 1]); a[e] = pk(av[2 * e], av[2 * e + 1]); }
+    for (int e = 0; e < NP; ++e) {
+      S0[e] = S[e] = pk(sv[2 * e], sv[2 * e + 1]);
+      a[e] = pk(av[2 * e], av[2 * e + 1]);
+      P[e] = pk(1.f, 1.f);
+    }
   }
 
   // the two channels and the rows (r0, r0 + RP, ...) of each tile whose steps and outputs this thread forms
@@ -249,6 +270,7 @@ scan_walk_kernel(const T* __restrict__ xc, const T* __restrict__ dt_raw, const T
       for (int k = 0; k < 4; ++k) {
         const ulonglong2 d = *reinterpret_cast<const ulonglong2*>(&sD[g + k][ch]);
         const f2 dt2 = d.x, dx2 = d.y;
+        Dt += __uint_as_float((uint32_t)dt2);
         f2 b[NP], cv[NP];
 #pragma unroll
         for (int e = 0; e < NP; e += 2) {
@@ -266,6 +288,7 @@ scan_walk_kernel(const T* __restrict__ xc, const T* __restrict__ dt_raw, const T
         for (int e = 0; e < NP; ++e) {
           const f2 dec = exp2_unit(fma2(dt2, a[e], bias2));
           S[e] = fma2(dec, S[e], mul2(dx2, b[e]));
+          P[e] = mul2(P[e], dec);
           if (FINAL) y2 = e == 0 ? mul2(S[e], cv[e]) : fma2(S[e], cv[e], y2);
         }
         if (FINAL) {
@@ -287,6 +310,19 @@ scan_walk_kernel(const T* __restrict__ xc, const T* __restrict__ dt_raw, const T
           sY[g + j][ch] = (up ? k1 : k0) + __shfl_xor_sync(0xffffffffu, up ? k0 : k1, 2);
         }
       }
+    }
+    if ((t0 / kTile + 1) % kAnchor == 0) {
+#pragma unroll
+      for (int e = 0; e < NP; ++e) {
+        float a0, a1, s0, s1, p0, p1, o0, o1;
+        un(a[e], a0, a1);
+        un(S[e], s0, s1);
+        un(P[e], p0, p1);
+        un(S0[e], o0, o1);
+        S[e] = S0[e] = pk(s0 + anchored(a0, Dt, p0, o0), s1 + anchored(a1, Dt, p1, o1));
+        P[e] = pk(1.f, 1.f);
+      }
+      Dt = 0.f;
     }
     __syncthreads();
     if (FINAL && on0) {

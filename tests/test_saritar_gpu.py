@@ -351,3 +351,27 @@ def test_scan_steps_and_gates_one_by_one(lo, hi):
         fine = torch.isfinite(d)
         assert bool(((one.double() - want).abs() <= want.abs() * 2.0 ** (-21.4 if lo > -80 else -20.4) + 2.0 ** -148 * (1 + d.abs()))[fine].all())
         assert torch.equal(torch.nan_to_num(one[3, :3], 7.0, 8.0, 9.0), torch.nan_to_num(serial[3, :3], 7.0, 8.0, 9.0))
+
+
+@pytest.mark.parametrize("lens,C", [([2048] * 4, 1024), ([600, 130], 96)])
+def test_scan_states_that_decay_slowly(lens, C):
+    """Decays around 0.9999 to 0.99 over whole portions. Against float64: the 2^x unit's errors (at most 2^-23 in a token, of one
+    sign) add up over 64 tokens and not over the portion."""
+    from gllm_b200.ops import sm100_seq as S
+    torch.manual_seed(C)
+    N, t, n = 16, sum(lens), len(lens)
+    qsl = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    sl, rs = torch.tensor(lens, dtype=torch.int32, device=DEV) + 1, torch.arange(n, dtype=torch.int32, device=DEV)
+    steps = 10.0 ** -torch.linspace(2, 4, C, device=DEV, dtype=torch.float64)
+    raw = torch.log(torch.expm1(steps * (0.8 + 0.4 * torch.rand(t, C, device=DEV)))).float()
+    x, xz = torch.randn(t, C, device=DEV), torch.randn(t, 2 * C, device=DEV)
+    proj, st0 = torch.randn(t, 2 * N, device=DEV), torch.randn(n, N, C, device=DEV)
+    A, st = -(0.5 + torch.rand(C, N, device=DEV)), st0.clone()
+    S.selective_scan(x, raw, proj, xz, A, torch.zeros(C, device=DEV), torch.zeros(C, device=DEV), st, rs, sl, qsl, C, N, 0, max_q_len=max(lens))
+    for s in range(n):
+        h = st0[s].double()
+        for k in range(int(qsl[s]), int(qsl[s + 1])):
+            dt = torch.nn.functional.softplus(raw[k].double())
+            h = torch.exp(dt * A.double().t()) * h + (dt * x[k].double()) * proj[k, :N].double()[:, None]
+        err = (st[s].double() - h).norm(dim=0) / h.norm(dim=0)              # per channel
+        assert float(err.max()) <= 64 * 2.0 ** -23, float(err.max())
