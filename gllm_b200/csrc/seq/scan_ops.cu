@@ -178,7 +178,7 @@ scan_walk_kernel(const T* __restrict__ xc, const T* __restrict__ dt_raw, const T
   const bool active = w < p.CW;
   const int wc = active ? w : p.CW - 1, c = p.c0 + wc;                     // idle threads mirror the last channel (loads only)
 
-  f2 S[NP], a[NP];                                   // states; A log2(e)
+  f2 S[NP], a[NP];                                   // states; A log2(e), finite (a step of 0 leaves a state alone at any rate)
   f2 S0[NP], P[NP];                                  // states and product of the decays since the last anchor
   float Dt = 0.f;                                    // sum of the steps since then
   {
@@ -190,6 +190,7 @@ scan_walk_kernel(const T* __restrict__ xc, const T* __restrict__ dt_raw, const T
     for (int e = 0; e < NL; ++e) {
       const int n = j * NL + e;
       av[e] = n < N ? p.A[(size_t)c * N + n] * 1.4426950408889634f : 0.f;
+      if (fabsf(av[e]) > kMostF) av[e] = copysignf(kMostF, av[e]);
       sv[e] = FINAL && n < N && (carried || !whole) ? from[n * step] : 0.f;
     }
 #pragma unroll

@@ -375,3 +375,23 @@ def test_scan_states_that_decay_slowly(lens, C):
             h = torch.exp(dt * A.double().t()) * h + (dt * x[k].double()) * proj[k, :N].double()[:, None]
         err = (st[s].double() - h).norm(dim=0) / h.norm(dim=0)              # per channel
         assert float(err.max()) <= 64 * 2.0 ** -23, float(err.max())
+
+
+@pytest.mark.parametrize("L", [1, 5, 64, 70])
+def test_scan_with_infinite_rates(L):
+    """A = -inf forgets everything at every step, also in portions that end inside a group of four tokens."""
+    from gllm_b200.ops import sm100_seq as S
+    torch.manual_seed(L)
+    N, C, i32 = 3, 40, torch.int32
+    A = -torch.rand(C, N, device=DEV)
+    A[::3] = -float("inf")
+    x, raw, xz, proj = (torch.randn(L, w, device=DEV) for w in (C, C, 2 * C, 2 * N))
+    z, st = torch.zeros(C, device=DEV), torch.randn(1, N, C, device=DEV)
+    y = S.selective_scan(x, raw, proj, xz, A, z, z, st, torch.zeros(1, dtype=i32, device=DEV), torch.tensor([L + 1], dtype=i32, device=DEV),
+                         torch.tensor([0, L], dtype=i32, device=DEV), C, N, 0, max_q_len=max(L, 2))
+    dx = torch.nn.functional.softplus(raw.double()) * x.double()
+    want = dx[:, None, ::3] * proj[:, :N, None].double()                    # [token, state, channel]
+    assert bool(((st[0, :, ::3].double() - want[-1]).abs() <= want[-1].abs() * 2.0 ** -20).all())
+    out = (want * proj[:, N:, None].double()).sum(1) * torch.nn.functional.silu(xz[:, C::3].double())
+    assert bool(((y[:, ::3].double() - out).abs() <= 2.0 ** -20 * (want.abs() * proj[:, N:, None].abs()).sum(1) * 20).all())
+    assert bool(torch.isfinite(y).all()) and bool(torch.isfinite(st).all())
