@@ -34,7 +34,8 @@ template <int NT> __device__ __forceinline__ float block_sum(float v, float* scr
   for (int i = 0; i < NT / 32; ++i) t += scratch[i];
   return t;
 }
-// 1 / (1 + e^-v) from the 2^x and 1/x units, within 2^-21 of it: for results that are rounded to bf16 (2^-9)
+// 1 / (1 + e^-v) from the 2^x and 1/x units: __fdividef(1, 1 + __expf(-v)) without the handling of denormals. Within 2^-21 of it, and
+// within |v| 2^-24 + 2^-21 of it relative to the value, for the exponent is rounded to one fp32.
 __device__ __forceinline__ float sigmoid_unit(float v) {
   float e, r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * v));

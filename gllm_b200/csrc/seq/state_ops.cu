@@ -19,6 +19,17 @@ using namespace seqk;
 
 __device__ __forceinline__ float sigmoid_f(float v) { return 1.0f / (1.0f + expf(-v)); }
 __device__ __forceinline__ float silu_f(float v) { return v / (1.0f + expf(-v)); }
+// sigmoid_f from the 2^x and 1/x units, within 2^-21 of it relative to the value: e = 2^(-|v| log2 e) with the exponent in two parts
+// (rounded to one it would cost |v| 2^-24), then 1 / (1 + e) or e / (1 + e). Denormals of e are kept.
+__device__ __forceinline__ float sigmoid_parts(float v) {
+  const float m = fabsf(v) > 200.f ? 200.f : fabsf(v);                     // finite, or NaN
+  const float t = m * 1.4426950216293335f, rest = fmaf(m, -1.925963033500011e-8f, fmaf(m, -1.4426950216293335f, t));
+  float e, r;
+  asm("ex2.approx.f32 %0, %1;" : "=f"(e) : "f"(-t));
+  e = fmaf(e, 0.6931472f * rest, e);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+  return v < 0.f ? e * r : r;
+}
 
 // x <- rms(alpha * x + y) * w (fp32 stream, in place); out = the same row in the compute dtype (optional)
 template <typename T>
@@ -439,8 +450,9 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ o, int n, cons
 
 // The same for bf16 rows whose groups are 128 or 256 wide and lie on 8-byte boundaries (o: 16): 16- and 8-byte accesses, and a
 // warp has the loads of 4 x 128 columns in flight, where 4-byte loads of one group at a time were bound by their latency.
-// 6000 tokens x 32 groups of 128: 97 -> 58 us, with the gate from the 2^x and 1/x units instead of expf and a division 41. Where the groups do not fill the machine, four in a row only make a warp slower
-// (one token, 32 groups of 128: 3.2 us element-wise, 4.1 with four): one group per warp there.
+// 6000 tokens x 32 groups of 128: 97 -> 61 us, with the gate from the 2^x and 1/x units instead of expf and a division 51. Where the
+// groups do not fill the machine, four in a row only make a warp slower (one token, 32 groups of 128: 3.2 us element-wise, 4.1 with
+// four): one group per warp there.
 template <int NCH, int kRows>
 __global__ void __launch_bounds__(128) gated_group_norm_vec_kernel(
     const float* __restrict__ o, int n, const __nv_bfloat16* __restrict__ gate, long ldg, const __nv_bfloat16* __restrict__ w,
@@ -482,7 +494,7 @@ __global__ void __launch_bounds__(128) gated_group_norm_vec_kernel(
       const uint2 wr = *reinterpret_cast<const uint2*>(w + (col[i] + c * 128) % wlen);
       const float2 w01 = b200::unpack_bf16(wr.x), w23 = b200::unpack_bf16(wr.y);
       auto one = [&](float x, float wt, float g) {
-        const float sg = sigmoid_unit(g);
+        const float sg = sigmoid_parts(g);
         return x * r * wt * (act ? sg : g * sg) * out_scale;
       };
       *reinterpret_cast<uint2*>(out + (size_t)tok[i] * ldo + col[i] + c * 128) =

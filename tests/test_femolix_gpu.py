@@ -171,6 +171,28 @@ def test_gated_group_norm_wide_rows(group, ngroups, ntok, pad, act):
         assert out[:, n:].abs().sum().item() == 0
 
 
+@pytest.mark.parametrize("act", ["silu", "sigmoid"])
+def test_gated_group_norm_gates_one_by_one(act):
+    """Unit rows (norm exactly 1) and gates from -100 to 100: the product before the bf16 rounding is within 2^-20 of float64 at any
+    gate, so a result is at most half a bf16 step and that away."""
+    from gllm_b200.ops import sm100_seq as S
+    torch.manual_seed(3)
+    n, T = 4096, 64
+    o = torch.ones(T, n, device=DEV)
+    gate = (torch.rand(T, n, device=DEV) * 200 - 100).bfloat16()
+    gate[0, :3] = torch.tensor([float("inf"), float("nan"), -float("inf")], device=DEV)
+    w = (1 + torch.rand(n, device=DEV)).bfloat16()
+    scale = 1 + torch.rand(1).item()
+    got = S.gated_group_norm(o, gate, w, 128, 0.0, act, scale).double()
+    sg = torch.sigmoid(gate.double())
+    want = w.double() * float(torch.tensor(scale, dtype=torch.float32)) * (sg if act == "sigmoid" else gate.double() * sg)
+    step = torch.exp2(torch.floor(torch.log2(want.abs().clamp(min=2.0 ** -126))) - 7)
+    ok = (got - want).abs() <= step / 2 + want.abs() * 2.0 ** -20
+    assert bool(ok[1:].all()) and bool(ok[0, 3:].all())
+    assert bool(torch.isnan(got[0, 1])) and float(got[0, 0]) == float(want[0, 0].float().bfloat16())
+    assert bool(torch.isnan(got[0, 2])) if act == "silu" else float(got[0, 2]) == 0.0
+
+
 @pytest.mark.parametrize("taps", [1, 2, 4])
 @pytest.mark.parametrize("qlens", [[600], [1, 1, 2050, 3, 1, 4, 5], [17, 1, 15, 700]])
 def test_conv_rows_fetched_ahead(qlens, taps):
