@@ -37,6 +37,16 @@ from gllm_b200.parallel import state as ps
 from gllm_b200.parallel.tp import TPComm
 
 
+def _joined(a: torch.Tensor, b: torch.Tensor):
+    """[a ; b] without a copy if b's rows follow a's in the same storage, else None."""
+    if b.data_ptr() != a.data_ptr() + a.nbytes or b.dtype != a.dtype or not (a.is_contiguous() and b.is_contiguous()):
+        return None
+    (n, k), (m, l) = a.shape, b.shape
+    if l != k or a.untyped_storage().nbytes() < (a.storage_offset() + (n + m) * k) * a.itemsize:
+        return None
+    return a.as_strided((n + m, k), (k, 1))
+
+
 class MLAAttention(nn.Module):
     def __init__(self, spec: ModelSpec, layer_id: int, rope, device):
         super().__init__()
@@ -56,26 +66,26 @@ class MLAAttention(nn.Module):
         # The projections follow the checkpoint's quantisation (fp8 block-scaled for V3 / R1: (weight, scale_inv)
         # pairs on the UTCQMMA GEMM — reference plumbs quant_config into them, gllm/models/deepseek_v2.py:280-440).
         # kv_b_proj stays bf16: it is only ever used absorbed, as the per-head W_UK / W_UV operands.
-        # The two projections of the hidden state are one weight, [q_a rows ; kv_a rows], and the parameters views of it: one GEMM of
-        # 2112 columns instead of two of 1536 and 576, neither of which fills the machine (K = 7168, 4096 rows: 87 us instead of
-        # 78 + 43, 128 rows: 17 instead of 16.5 + 16.4). Block scales must not straddle the border.
-        self._qkv_a = None
-        if self.q_lora and self.q_lora % 128 == 0:
+        # The two projections of the hidden state lie in one tensor, [q_a rows ; kv_a rows], of which the parameters are views: one GEMM
+        # of 2112 columns instead of two of 1536 and 576, neither of which fills the machine (K = 7168, 4096 rows: 87 us instead of
+        # 78 + 43, 128 rows: 17 instead of 16.5 + 16.4). Block scales must not straddle the border. Only the parameters hold them:
+        # `_qkv_a` looks in each call whether they still lie so (one that was replaced, moved or converted does not).
+        self.joined = bool(self.q_lora) and self.q_lora % 128 == 0
+        if self.joined:
             w, s = _linear_params(self.q_lora + self.kv_lora + self.rope_dim, h, spec, device)
-            self._qkv_a = _qw(w.data, None if s is None else s.data)
 
             def cut(x, n):
                 return (None, None) if x is None else [nn.Parameter(v, requires_grad=False) for v in (x.data[:n], x.data[n:])]
             self.q_a_w, self.kv_a_w = cut(w, self.q_lora)
             self.q_a_ws, self.kv_a_ws = cut(s, self.q_lora // 128)
         if self.q_lora:
-            if self._qkv_a is None:
+            if not self.joined:
                 self.q_a_w, self.q_a_ws = _linear_params(self.q_lora, h, spec, device)
             self.q_a_norm_w = _param(self.q_lora, dtype=dt, device=device, fill=1.0)
             self.q_b_w, self.q_b_ws = _linear_params(self.num_heads * self.qk_dim, self.q_lora, spec, device)
         else:
             self.q_w, self.q_ws = _linear_params(self.num_heads * self.qk_dim, h, spec, device)
-        if self._qkv_a is None:
+        if not self.joined:
             self.kv_a_w, self.kv_a_ws = _linear_params(self.kv_lora + self.rope_dim, h, spec, device)
         self.kv_a_norm_w = _param(self.kv_lora, dtype=dt, device=device, fill=1.0)
         self.kv_b_w = _param(self.num_heads * (self.nope + self.v_dim), self.kv_lora, dtype=dt, device=device)
@@ -85,12 +95,23 @@ class MLAAttention(nn.Module):
         self.num_kv_heads = 1
         self.head_dim = self.kv_lora + self.rope_dim
 
+    def _qkv_a(self):
+        """q_a and kv_a as the weight of one product, or None if their tensors do not follow each other in memory."""
+        if not self.joined:
+            return None
+        w = _joined(self.q_a_w, self.kv_a_w)
+        if w is None or self.q_a_ws is None:
+            return w
+        s = _joined(self.q_a_ws, self.kv_a_ws)
+        return None if s is None else (w, s)
+
     def forward(self, inp, h: torch.Tensor, kv_cache, tpc: TPComm) -> torch.Tensor:
         t = h.shape[0]
         hl = self.num_heads
         h = tpc.materialize(h)
-        if self._qkv_a is not None:
-            both = Fn.linear(h, self._qkv_a)
+        qkv_a = self._qkv_a()
+        if qkv_a is not None:
+            both = Fn.linear(h, qkv_a)
             kv_a = both[:, self.q_lora:]
             qa, kv_c = Fn.rmsnorm_two(both[:, : self.q_lora], self.q_a_norm_w, kv_a[:, : self.kv_lora], self.kv_a_norm_w, self.eps)
             q = Fn.linear(qa, _qw(self.q_b_w, self.q_b_ws))

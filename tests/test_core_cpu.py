@@ -733,3 +733,53 @@ def test_generate_takes_per_request_sampling_parameters():
     assert (outs[0].top_k, outs[1].top_k, outs[1].repetition_penalty, outs[1].top_p) == (1, 5, 1.3, 0.8)
     assert not llm.worker._seq_slots                       # the penalised request gave its state row back
     llm.shutdown()
+
+
+@pytest.mark.parametrize("how,quant", [("assign", None), ("data", None), ("copy", None), ("deepcopy", None), ("float", None),
+                                       ("data", "fp8"), ("copy", "fp8"), ("scale", "fp8")])
+def test_latent_attention_uses_the_parameters_it_has(how, quant, monkeypatch):
+    """The projections of the hidden state are two parameters in one tensor. Whatever becomes of them, the block computes with what
+    they hold now: replaced, written to, copied with the module, converted. (The products are looked at where they are normed: one
+    rounding to bf16.)"""
+    import copy
+    import torch
+    from gllm_b200.layers import functional as Fn
+    from gllm_b200.layers.rotary import build_rope
+    from gllm_b200.models.decoder import ModelSpec, _qw
+    from gllm_b200.models.deepseek_v2 import MLAAttention
+    from gllm_b200.parallel.tp import TPComm
+    torch.manual_seed(0)
+    spec = ModelSpec(arch="DeepseekV3ForCausalLM", hidden_size=128, num_layers=1, num_heads=2, num_kv_heads=2, head_dim=24,
+                     intermediate_size=8, vocab_size=8, dtype=torch.bfloat16, quant=quant, use_mla=True,
+                     extra=dict(qk_nope_head_dim=16, qk_rope_head_dim=8, v_head_dim=16, kv_lora_rank=128, q_lora_rank=256))
+    att = MLAAttention(spec, 0, build_rope(8, 64, 1e4, None, 8, False, device="cpu"), "cpu")
+    draw = lambda p: torch.randn(p.shape).to(p.dtype)  # noqa: E731
+    for p in att.parameters():
+        p.data.copy_(draw(p))
+    seen, norm, norm2 = [], Fn.rmsnorm, Fn.rmsnorm_two
+    monkeypatch.setattr(Fn, "rmsnorm", lambda x, *a, **k: (seen.append(x), norm(x, *a, **k))[1])
+    monkeypatch.setattr(Fn, "rmsnorm_two", lambda x1, w1, x2, w2, eps: (seen.extend((x1, x2)), norm2(x1, w1, x2, w2, eps))[1])
+
+    def check(att, joined):
+        seen.clear()
+        h = torch.randn(5, 128).bfloat16().to(att.q_a_norm_w.dtype)
+        att(None, h, None, TPComm())
+        assert (att._qkv_a() is not None) == joined
+        want = Fn.linear(h, _qw(att.q_a_w, att.q_a_ws)), Fn.linear(h, _qw(att.kv_a_w, att.kv_a_ws))[:, :128]
+        assert all(torch.allclose(g.float(), w.float(), rtol=2.0 ** -7, atol=1e-4) for g, w in zip(seen, want))
+
+    check(att, True)
+    if how == "assign":
+        att.load_state_dict({k: draw(v) for k, v in att.state_dict().items()}, assign=True)
+    elif how == "data":
+        att.q_a_w.data = draw(att.q_a_w)
+    elif how == "copy":
+        att.kv_a_w.data.copy_(draw(att.kv_a_w))
+    elif how == "deepcopy":
+        att = copy.deepcopy(att)
+        att.q_a_w.data.copy_(draw(att.q_a_w))
+    elif how == "scale":
+        att.kv_a_ws.data = torch.rand_like(att.kv_a_ws)
+    else:
+        att.to(torch.float32)
+    check(att, how == "copy")
