@@ -698,7 +698,9 @@ static int gemm_bf16_impl(const void* A, int64_t lda, const void* W, int64_t ldw
   int bn = 128, split = 1;
   choose_cfg(M, N, K, epi, force_bn, ws != nullptr && tile_cnt != nullptr ? ws_bytes : 0, max_tiles, &bn, &split);
   const bool decode = ws != nullptr && tile_cnt != nullptr && ws_bytes > 0 && M <= g_max_split_m;   // pick_split's sizes
-  if (comm == nullptr && !decode && split == 1 && (epi == kEpiSiluMul || force_bn == 0) && pairs_are_faster(M, N, bn)) {
+  // pairs, and gated tiles of 192 below, read gate and up rows that alternate in blocks of 128, as tiles of 256 do
+  const bool free_bn = force_bn == (epi == kEpiSiluMul ? 256 : 0);
+  if (comm == nullptr && !decode && split == 1 && free_bn && pairs_are_faster(M, N, bn)) {
     const PairGemm g{A, W, lda, ldw, reinterpret_cast<__nv_bfloat16*>(C), ldc, M, N, K,
                      reinterpret_cast<const __nv_bfloat16*>(bias), epi == kEpiSiluMul, glu_limit, glu_alpha, gelu};
     return gemm_bf16_pair(g, reinterpret_cast<cudaStream_t>(stream));
@@ -708,7 +710,7 @@ static int gemm_bf16_impl(const void* A, int64_t lda, const void* W, int64_t ldw
   // One row of gated tiles: the weights are the traffic, and 128 SMs that read 192 rows each draw more than 96 that read 256
   // (64 rows, 24,576 x 4096 and the 4096 x 12,288 behind it: 76.9 -> 70.4 us).
   const int sms = num_sms();
-  if (epi == kEpiSiluMul && comm == nullptr && split == 1 && M <= kBlockM && (N + 255) / 256 < sms && (N + 191) / 192 <= sms) bn = 192;
+  if (epi == kEpiSiluMul && free_bn && comm == nullptr && split == 1 && M <= kBlockM && (N + 255) / 256 < sms && (N + 191) / 192 <= sms) bn = 192;
   if (make_tmap_2d(&tb, W, N, K, ldw * 2, epi == kEpiSiluMul && bn == 192 ? 32 : bn, kBlockK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16))
     return 1;
   GemmParams p;

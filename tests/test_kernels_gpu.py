@@ -1023,6 +1023,22 @@ def test_gemm_smallm_any_output(m, ldc, shift):
     assert bool((buf[~written] == 7.0).all())
 
 
+@pytest.mark.parametrize("bn", [64, 128, 256])
+@pytest.mark.parametrize("m", [64, 600, 2305])
+def test_gemm_gated_at_a_forced_tile_width(bn, m, monkeypatch):
+    """A forced width of a gated product says how gate and up rows alternate (blocks of half of it): no other tiles may be taken.
+    One rounding of the output; the gate is fp32 on fp32 sums."""
+    from gllm_b200.ops import ref, sm100
+    torch.manual_seed(bn)
+    monkeypatch.setattr(sm100, "_FORCE_BN", bn)
+    f, k = 4992, 136
+    x, w = torch.randn(m, k, device=_dev()).bfloat16(), (torch.randn(2 * f, k, device=_dev()) * k ** -0.5).bfloat16()
+    g, u = (x.double() @ w.double().t()).chunk(2, -1)
+    want = torch.nn.functional.silu(g) * u
+    got = sm100.linear(x, ref.interleave_gate_up(w, bn // 2), epi=1)
+    assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -16 * (1 + want.abs())).all())
+
+
 def test_gemm_refuses_unaligned_output():
     """The tiled GEMMs store 16 bytes at a time: an output or bias off that boundary is an error, never a launch."""
     from gllm_b200.ops import sm100
