@@ -454,32 +454,40 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         // SiLU-gate: tile columns [0, BN/2) hold gate, [BN/2, BN) hold up for the same
         // BN/2 output features (weights are interleaved per tile at load time).
         constexpr int H = BN / 2;
+        auto gate = [&](int c, int h, auto& g, auto& u) {            // columns [c + h, ...) of gate and up, as many as g holds
+          load_acc(c + h, g);
+          load_acc(H + c + h, u);
+#pragma unroll
+          for (int j = 0; j < static_cast<int>(sizeof(g) / sizeof(uint32_t)); j += 8) {
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float gv = __uint_as_float(g[j + e]);
+              const float uv = __uint_as_float(u[j + e]);
+              if (p.glu_limit > 0.f) {
+                const float gc = fminf(gv, p.glu_limit);
+                const float uc = fminf(fmaxf(uv, -p.glu_limit), p.glu_limit);
+                f[e] = gc / (1.0f + __expf(-p.glu_alpha * gc)) * (uc + 1.0f);
+              } else if (p.gelu) {
+                f[e] = gelu_tanh_fast(gv) * uv;
+              } else {
+                f[e] = gv / (1.0f + __expf(-gv)) * uv;
+              }
+            }
+            stage_put((h + j) / 8, f);
+          }
+        };
 #pragma unroll 1
         for (int c = c_lo; c < c_hi; c += W) {
+          if (share == 16) {                                         // 32 would reach into the sums of the next share or tile
+            uint32_t g[16], u[16];
+            gate(c, 0, g, u);
+          } else {
 #pragma unroll
-          for (int h = 0; h < W; h += 32) {
-            if (c + h >= c_hi) break;
-            uint32_t g[32], u[32];
-            load_acc(c + h, g);
-            load_acc(H + c + h, u);
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              float f[8];
-#pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                const float gv = __uint_as_float(g[j + e]);
-                const float uv = __uint_as_float(u[j + e]);
-                if (p.glu_limit > 0.f) {
-                  const float gc = fminf(gv, p.glu_limit);
-                  const float uc = fminf(fmaxf(uv, -p.glu_limit), p.glu_limit);
-                  f[e] = gc / (1.0f + __expf(-p.glu_alpha * gc)) * (uc + 1.0f);
-                } else if (p.gelu) {
-                  f[e] = gelu_tanh_fast(gv) * uv;
-                } else {
-                  f[e] = gv / (1.0f + __expf(-gv)) * uv;
-                }
-              }
-              stage_put((h + j) / 8, f);
+            for (int h = 0; h < W; h += 32) {
+              if (c + h >= c_hi) break;
+              uint32_t g[32], u[32];
+              gate(c, h, g, u);
             }
           }
           stage_flush(out_n0 + c, out_n0 + c_hi);

@@ -1023,6 +1023,28 @@ def test_gemm_smallm_any_output(m, ldc, shift):
     assert bool((buf[~written] == 7.0).all())
 
 
+@pytest.mark.parametrize("act", ["silu", "gelu", "glu"])
+@pytest.mark.parametrize("m,f,k", [(64, 1536, 4096), (100, 2048, 7168), (128, 1792, 4096)])
+def test_gemm_gated_split_in_eight(m, f, k, act):
+    """K in eight parts, each of whose CTAs gates 16 columns of a tile. fp32 sums in the order of the parts, one rounding."""
+    from gllm_b200.ops import lib, ref, sm100, sm100_latent
+    torch.manual_seed(f)
+    x, w = torch.randn(m, k, device=_dev()).bfloat16(), (torch.randn(2 * f, k, device=_dev()) * k ** -0.5).bfloat16()
+    units = lib.load().gllm_gemm_bf16_tiles_covering(m, 2 * f, k, 1, 256, 0, m, sm100._SMALLM_WS_FLOATS * 4, sm100._SPLITK_MAX_TILES)
+    assert units == f // 128 * 8
+    wi = ref.interleave_gate_up(w, 128)
+    g, u = (x.double() @ w.double().t()).chunk(2, -1)
+    if act == "glu":
+        g, u = g.clamp(max=1.5), u.clamp(-1.5, 1.5)
+        want, call = g * torch.sigmoid(1.7 * g) * (u + 1), lambda: sm100_latent.linear_glu_clamp(x, wi, 1.5, 1.7)
+    else:
+        want = (torch.nn.functional.silu(g) if act == "silu" else torch.nn.functional.gelu(g, approximate="tanh")) * u
+        call = lambda: sm100.linear_silu_mul(x, wi, act=act)  # noqa: E731
+    for _ in range(3):                                       # the counters of a tile are set back behind each product
+        got = call()
+        assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -16 * (1 + want.abs())).all())
+
+
 @pytest.mark.parametrize("bn", [64, 128, 256])
 @pytest.mark.parametrize("m", [64, 600, 2305])
 def test_gemm_gated_at_a_forced_tile_width(bn, m, monkeypatch):
