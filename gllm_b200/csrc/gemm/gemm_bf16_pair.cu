@@ -119,6 +119,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           tma_load_2d_pair(sa, &tmap_a, bar, kb * kPBK, m0, kEvictNormal);
         }
       }
+      // The commits that hand the last stages back arrive in both CTAs, and the cluster's barrier does not order them: the other
+      // CTA sees its own before it ends (the leader's issuer waits for `mma_end`).
+      if (rank == 1)
+        for (uint32_t i = it > S ? it - S : 0; i < it && ok; ++i) ok = guard.wait(&empty_bar[i % S], (i / S) & 1);
       // copies in flight land before the CTAs end, whichever role gave up; the leader's barriers count the other CTA's as well
       if (rank == 0)
         for (uint32_t i = it > S ? it - S : 0; i < it; ++i) guard.land(&full_bar[i % S], (i / S) & 1);
@@ -249,6 +253,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         __syncwarp();
       }
     }
+    // the very last commit as well
+    if (rank == 1 && warp == 2 && lane == 0) WaitGuard::land(mma_end, 0);
   }
   tc_fence_before();
   __syncthreads();
