@@ -130,6 +130,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         WaitGuard::settle();
     }
   } else if (warp == 1) {
+    griddep_wait();                                      // A is copied behind it: the limit of the waits does not count the kernel before
     if (rank == 0 && lane == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(256, BN);
       uint32_t it = 0, n = 0;

@@ -362,6 +362,29 @@ def test_wait_that_gives_up_reaches_the_caller(family):
     assert done.tokens_list() == [0]
 
 
+def test_wait_limit_does_not_count_the_kernel_before():
+    """A GEMM on pairs of SMs starts while ten CTAs of the kernel before it still have a long product to sum up: what it waits for
+    there is not a wait of its own."""
+    from gllm_b200.ops import lib, sm100
+    torch.manual_seed(1)
+    x0, w0 = torch.randn(600, 1 << 17, device=_dev()).bfloat16(), torch.randn(256, 1 << 17, device=_dev()).bfloat16()
+    x, w = torch.randn(600, 1024, device=_dev()).bfloat16(), torch.randn(6144, 1024, device=_dev()).bfloat16()
+    want = x.float() @ w.float().t()
+    sm100.linear(x0, w0), sm100.linear(x, w)
+    assert sm100.waits_given_up() == 0
+    try:
+        lib.watch_waits(limit_ns=100_000)
+        for _ in range(3):
+            sm100.linear(x0, w0)
+            got = sm100.linear(x, w)
+        torch.cuda.synchronize()
+        assert not lib.waits_gave_up()
+    finally:
+        lib.watch_waits()
+        lib.waits_gave_up(clear=True)
+    assert _rel_err(got, want) < 5e-2
+
+
 def test_sampler_greedy_and_filter():
     from gllm_b200.ops import sm100
     torch.manual_seed(6)
