@@ -53,13 +53,6 @@ struct WaitGuard {
     } while (global_ns() - t0 < 2000000000u);
   }
 
-  // a millisecond, for copies in flight that this CTA has no barrier for
-  __device__ __forceinline__ static void settle() {
-    const uint32_t t0 = global_ns();
-    while (global_ns() - t0 < 1000000u) {
-    }
-  }
-
  private:
   __device__ __forceinline__ void give_up() const {
     *dead = 1;

@@ -61,7 +61,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   uint64_t* tmem_full = empty_bar + S;
   uint64_t* tmem_empty = tmem_full + 2;
   uint64_t* mma_end = tmem_empty + 2;
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(mma_end + 1);
+  uint64_t* peer_end = mma_end + 1;                      // leader: the other CTA issues no more copies; how many stages it filled
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(peer_end + 1);
+  uint32_t* peer_stages = tmem_ptr_smem + 2;
   const WaitGuard guard{tmem_ptr_smem + 1, p.waits};
   uint8_t* epi_smem = smem + S * kPStage + 256;
 
@@ -78,6 +80,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     for (int i = 0; i < S; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&tmem_full[i], 1); mbar_init(&tmem_empty[i], 2 * kPEpi); }
     mbar_init(mma_end, 1);
+    mbar_init(peer_end, 1);
+    *peer_stages = 0;
     *guard.dead = 0;
     fence_mbar_init();
   }
@@ -123,11 +127,30 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       // CTA sees its own before it ends (the leader's issuer waits for `mma_end`).
       if (rank == 1)
         for (uint32_t i = it > S ? it - S : 0; i < it && ok; ++i) ok = guard.wait(&empty_bar[i % S], (i / S) & 1);
-      // copies in flight land before the CTAs end, whichever role gave up; the leader's barriers count the other CTA's as well
-      if (rank == 0)
-        for (uint32_t i = it > S ? it - S : 0; i < it; ++i) guard.land(&full_bar[i % S], (i / S) & 1);
-      else if (guard.gave_up())
-        WaitGuard::settle();
+      // Copies in flight land before the CTAs end, whichever role gave up (then the other CTA's waits end too). The leader's barriers
+      // count both CTAs' copies, so it has to know how many stages the other one filled: a stage that only the leader filled is not
+      // waited for in full, one that only the other CTA filled is counted after all.
+      auto warn = [&] {
+        if (guard.gave_up()) st_cluster(cluster_addr(const_cast<uint32_t*>(guard.dead), rank ^ 1), 1);
+      };
+      warn();
+      if (rank == 1) {
+        st_cluster(cluster_addr(peer_stages, 0), it);
+        mbar_arrive_cluster(cluster_addr(peer_end, 0));
+      } else {
+        const uint32_t t0 = global_ns();
+        bool told = mbar_try_wait_cluster(peer_end, 0);
+        while (!told && global_ns() - t0 < 4000000000u) {
+          warn();
+          told = mbar_try_wait_cluster(peer_end, 0);
+        }
+        const uint32_t other = told ? *reinterpret_cast<volatile uint32_t*>(peer_stages) : it, most = other > it ? other : it;
+        for (uint32_t i = other < it ? other : it; i < most; ++i) {
+          if (i < it) mbar_complete_tx(&full_bar[i % S], kPStage);
+          else mbar_expect_tx(&full_bar[i % S], kPStage);
+        }
+        for (uint32_t i = most > S ? most - S : 0; i < most; ++i) guard.land(&full_bar[i % S], (i / S) & 1);
+      }
     }
   } else if (warp == 1) {
     griddep_wait();                                      // A is copied behind it: the limit of the waits does not count the kernel before

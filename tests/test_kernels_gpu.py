@@ -362,6 +362,31 @@ def test_wait_that_gives_up_reaches_the_caller(family):
     assert done.tokens_list() == [0]
 
 
+@pytest.mark.parametrize("m,n,k", [(600, 6144, 64), (600, 6144, 1024), (4200, 4104, 4096)])
+def test_gemm_on_pairs_that_gives_up_ends_soon(m, n, k):
+    """Limits of nothing and of 2 us: the two CTAs of a pair give up at different stages, and still no copy is waited for that was
+    never issued (two seconds each)."""
+    import time
+    from gllm_b200.ops import lib, sm100
+    torch.manual_seed(k)
+    x, w = torch.randn(m, k, device=_dev()).bfloat16(), torch.randn(n, k, device=_dev()).bfloat16()
+    want = sm100.linear(x, w)
+    torch.cuda.synchronize()
+    try:
+        for limit in (0, 2000):
+            lib.watch_waits(limit_ns=limit)
+            for _ in range(5):
+                t0 = time.monotonic()
+                sm100.linear(x, w)
+                torch.cuda.synchronize()
+                assert time.monotonic() - t0 < 0.5, limit
+            assert limit or lib.waits_gave_up()
+    finally:
+        lib.watch_waits()
+        lib.waits_gave_up(clear=True)
+    assert torch.equal(sm100.linear(x, w), want)
+
+
 def test_wait_limit_does_not_count_the_kernel_before():
     """A GEMM on pairs of SMs starts while ten CTAs of the kernel before it still have a long product to sum up: what it waits for
     there is not a wait of its own."""
