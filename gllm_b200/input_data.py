@@ -273,7 +273,7 @@ class InputData:
     """Persistent device-side batch state (stable addresses => CUDA-graph friendly).
 
     One instance per worker. `load(batch)` copies a `BatchArrays` into pinned staging and then
-    into the device buffers with a single non-blocking H2D per array.
+    into the device buffers: the small ones together in one non-blocking H2D, each large one in its own.
     """
 
     def __init__(self, max_tokens: int, max_seqs: int, max_blocks: int, device, mrope: bool = False):
@@ -338,9 +338,10 @@ class InputData:
         if self._blocks is not None and 0 < n <= self._PART_WORDS and self._block_at + n <= self._BLOCK_WORDS and \
                 self._num_parts < 16:
             at = self._block_at
-            self._blocks[self._flip][1][host_np.dtype][at:at + n].reshape(arr.shape)[...] = arr
             rows, cols, pitch = (1, n, n) if arr.ndim == 1 else (*arr.shape, dev.stride(0))
-            assert rows <= dev.shape[0] and cols <= dev.shape[-1]
+            if dev.dim() != arr.ndim or cols > dev.shape[-1] or rows > dev.shape[0]:
+                raise ValueError(f"an array of shape {arr.shape} for a buffer of {tuple(dev.shape)}")
+            self._blocks[self._flip][1][host_np.dtype][at:at + n].reshape(arr.shape)[...] = arr
             self._parts[self._num_parts] = dev.data_ptr(), pitch, at, rows, cols
             self._num_parts += 1
             self._block_at = at + n
@@ -361,7 +362,6 @@ class InputData:
             n = self._block_at
             self._block_dev[:n].copy_(self._blocks[self._flip][0][:n], non_blocking=True)
             sm100.batch_load(self._block_dev, self._parts, self._num_parts, self._most_words)
-        self._num_parts = self._block_at = self._most_words = 0
 
     def load(self, batch: BatchArrays):
         assert batch.num_tokens <= self.max_tokens, (batch.num_tokens, self.max_tokens)
@@ -369,6 +369,7 @@ class InputData:
         assert batch.block_table.shape[1] <= self.max_blocks
         self.batch = batch
         self._flip ^= 1
+        self._num_parts = self._block_at = self._most_words = 0     # also what a load that raised had put in the block
         self.num_tokens, self.num_seqs = batch.num_tokens, batch.num_seqs
         self.num_decode_seqs = batch.num_decode_seqs
         self.num_emit = int(batch.logits_idx.shape[0])

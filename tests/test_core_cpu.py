@@ -783,3 +783,35 @@ def test_latent_attention_uses_the_parameters_it_has(how, quant, monkeypatch):
     else:
         att.to(torch.float32)
     check(att, how == "copy")
+
+
+def test_a_load_that_raises_leaves_nothing_for_the_next(monkeypatch):
+    """A step's small arrays wait in one block until all are there. If one of them does not fit its buffer, as before with the copy of
+    each, that load raises ValueError; the next one sends its own arrays, each buffer once, and nothing else."""
+    import torch
+    from gllm_b200.input_data import InputData
+    from gllm_b200.ops import sm100
+    inp, i32, f32 = InputData(64, 4, 8, "cpu"), np.int32, np.float32
+    hosts = [torch.zeros(inp._BLOCK_WORDS, dtype=torch.int32) for _ in range(2)]         # what a CUDA device has
+    inp._blocks = [(h, {np.dtype(i32): h.numpy(), np.dtype(f32): h.numpy().view(f32)}) for h in hosts]
+    inp._block_dev, inp._parts = torch.zeros(inp._BLOCK_WORDS, dtype=torch.int32), np.zeros((16, 5), np.int64)
+    sent = []
+    monkeypatch.setattr(sm100, "batch_load", lambda block, parts, n, most: sent.append((block.clone(), parts[:n].copy())))
+
+    def batch(n, base, lens):
+        a = lambda k: base + np.arange(k, dtype=i32)  # noqa: E731
+        return BatchArrays(tokens=a(n), positions=a(n), slot_mapping=a(n), block_table=a(6).reshape(2, 3), seq_lens=a(lens),
+                           query_start_loc=a(3), logits_idx=a(2), emit_seq=a(2), temperature=np.ones(2, f32), top_k=a(2),
+                           top_p=np.ones(2, f32), rep_penalty=np.ones(2, f32), state_slot=a(2), num_decode_seqs=0, num_seqs=2,
+                           num_tokens=n, max_q_len=2, max_seq_len=9, rec_slots=a(2), all_greedy=False)
+
+    with pytest.raises(ValueError):
+        inp.load(batch(7, 100, 5))                             # five lengths for four sequences
+    assert not sent
+    inp.load(batch(9, 500, 2))
+    (block, parts), = sent
+    assert len(set(parts[:, 0])) == len(parts) and inp._tokens[1].data_ptr() in parts[:, 0]
+    at = {int(p[0]): p for p in parts}
+    for pair, want in ((inp._tokens, 500 + np.arange(9)), (inp._seq_lens, 500 + np.arange(2)), (inp._block_table, 500 + np.arange(6))):
+        p = at[pair[1].data_ptr()]
+        assert np.array_equal(block.numpy()[p[2]:p[2] + p[3] * p[4]], want)
