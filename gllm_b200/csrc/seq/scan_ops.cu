@@ -8,7 +8,8 @@
 // Usually a piece is a whole sequence: one launch, every exponential once. Where the sequences are too few to fill the machine
 // (scan_piece in ops/sm100_seq.py), they are cut in pieces and three kernels run: every piece's end state from zero and its sum
 // of steps (the decays are diagonal, so a piece takes an entering state S_0 to exp(a_n sum dt) S_0 + its own end state); the
-// chain over a sequence's pieces; every piece again from its entering state, with the outputs.
+// chain over a sequence's pieces; every piece again from its entering state, with the outputs. Short sequences beside those are walked
+// whole in the last one, so that their states do not depend on the batch.
 //
 // What bounds it: the 2^x unit (8 cycles per warp and exponential: 64 of about 100 cycles per token of a warp with 16 channels)
 // and issue slots. So the arithmetic is on pairs (f32x2), log2(e) is multiplied into A, softplus and silu are formed once per
@@ -132,7 +133,7 @@ struct ScanArgs {
   const float *A, *Dskip, *dt_bias;
   float* state;
   const int *rec_slots, *seq_lens, *qsl;
-  int nseq, C, N, R, c0, CW, piece;
+  int nseq, C, N, R, c0, CW, piece, uncut;
   long ldp, ldxz;
   int wide;                                          // channels 2 i, 2 i + 1 of x, dt, z and out can be moved together
   float *ends, *steps;
@@ -170,9 +171,10 @@ scan_walk_kernel(const T* __restrict__ xc, const T* __restrict__ dt_raw, const T
   const int q0 = p.qsl[lo], q1 = p.qsl[lo + 1];
   const long off = (long)(u - piece_base(p.qsl, lo, p.piece)) * p.piece;
   if (off >= q1 - q0) return;                        // uniform over the block
-  const int base = q0 + (int)off, len = min(q1 - base, p.piece);
-  const bool whole = q1 - q0 <= p.piece, last = base + len >= q1;
-  if (!FINAL && last) return;                        // nobody continues from its end
+  const bool whole = q1 - q0 <= max(p.piece, p.uncut);
+  const int base = q0 + (int)off, len = whole ? q1 - q0 : min(q1 - base, p.piece);
+  const bool last = base + len >= q1;
+  if (whole ? off > 0 || !FINAL : !FINAL && last) return;                  // nobody continues from the end of a sequence
   const int tid = threadIdx.x, j = tid % LPC, ch = tid / LPC, C = p.C, N = p.N;
   const int w0 = blockIdx.x * CH, w = w0 + ch;       // channel inside this round's range
   const bool active = w < p.CW;
@@ -379,7 +381,7 @@ __global__ void __launch_bounds__(128) scan_carry_kernel(const ScanArgs p) {
   constexpr int U = 8;                              // pieces fetched at a time: the chain itself is two operations
   const int w = blockIdx.x * 128 + threadIdx.x, n = blockIdx.y, s = blockIdx.z;
   const int q0 = p.qsl[s], q1 = p.qsl[s + 1];
-  if (w >= p.CW || q1 - q0 <= p.piece) return;      // one piece: it starts from the carried state itself
+  if (w >= p.CW || q1 - q0 <= max(p.piece, p.uncut)) return;               // walked whole: from the carried state itself
   const int c = p.c0 + w, pieces = (q1 - q0 + p.piece - 1) / p.piece;
   const float a = p.A[(size_t)c * p.N + n];
   const bool carried = p.state != nullptr && p.seq_lens[s] > q1 - q0;
@@ -441,22 +443,25 @@ int pick_scan(int lanes, const void* xc, const void* dt_raw, const void* proj, c
 
 }  // namespace
 
-// Sequences longer than `piece` tokens are cut, `width` channels at a time; none is if piece >= ntok, and `work` is not used then.
+// Sequences longer than both `piece` and `uncut` tokens are cut, `width` channels at a time; none is if piece >= ntok, and `work` is
+// not used then.
 // Returns 2 outside its envelope (the caller then uses the token-serial kernel): N <= 16. `work`: (ntok / piece + nseq) * (N + 1) *
 // min(width, C) floats.
 GLLM_EXPORT int gllm_scan_walk(const void* xc, const void* dt_raw, const void* proj, long ldp, const void* xz, long ldxz,
                                const void* A, const void* Dskip, const void* dt_bias, void* state, const void* rec_slots,
                                const void* seq_lens, const void* qsl, int ntok, int nseq, int C, int N, int R, int piece,
-                               int width, void* work, void* out, int is_f32, void* stream) {
+                               int uncut, int width, void* work, void* out, int is_f32, void* stream) {
   if (nseq <= 0 || ntok <= 0) return 0;
   if (N < 1 || N > kNM || width < 1 || piece < 1 || nseq > 65535 || ntok / piece + nseq > 65535) return 2;
   ScanArgs p{};
   p.A = (const float*)A; p.Dskip = (const float*)Dskip; p.dt_bias = (const float*)dt_bias;
   p.state = (float*)state;
   p.rec_slots = (const int*)rec_slots; p.seq_lens = (const int*)seq_lens; p.qsl = (const int*)qsl;
-  p.nseq = nseq; p.C = C; p.N = N; p.R = R; p.piece = piece; p.ldp = ldp; p.ldxz = ldxz;
-  // Two lanes per channel spend fewer instructions, four have twice the warps: from three warps per scheduler on, two are faster
-  // (8192 channels, 4 portions of 2048: 572 / 609 us; one of 8192: 1000 / 1090; 4096 channels, 700 tokens: 91 / 63).
+  p.nseq = nseq; p.C = C; p.N = N; p.R = R; p.piece = piece; p.uncut = uncut; p.ldp = ldp; p.ldxz = ldxz;
+  // Two lanes per channel spend fewer instructions, four have twice the warps. With warps for every scheduler two are faster (8192
+  // channels, 4 portions of 2048, 3.5 warps: 661 / 701 us; 2 of 2048, 1.7: 407 / 483; 4096 channels, 4 of 2048, 1.7: 407 / 405), with
+  // few four (4096 channels, 700 tokens, 0.4 warps: 112 / 81; 2000, 300, 100 and 50 tokens, of which one is walked for long: 318 /
+  // 272). Portions are counted as if they were equal, hence the line at three.
   const int pieces = piece < ntok ? ntok / piece : nseq;
   const int lanes = static_cast<int64_t>(C) / 16 * pieces >= 3 * 4 * b200::num_sms() ? 2 : 4;
   return (is_f32 ? pick_scan<float> : pick_scan<__nv_bfloat16>)(lanes, xc, dt_raw, proj, xz, p, ntok, width, (float*)work, out,

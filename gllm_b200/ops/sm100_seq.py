@@ -49,7 +49,7 @@ def _L():
             "gllm_seq_softcap": [P, G, I, I, F, I, P],
             "gllm_seq_conv_silu": [P, G, I, I, I, P, P, I, P, P, P, P, P, I, I, P, I, P],
             "gllm_seq_selective_scan": [P, P, P, G, P, G, P, P, P, P, P, P, P, I, I, I, I, P, I, I, P],
-            "gllm_scan_walk": [P, P, P, G, P, G] + [P] * 7 + [I] * 7 + [P, P, I, P],
+            "gllm_scan_walk": [P, P, P, G, P, G] + [P] * 7 + [I] * 8 + [P, P, I, P],
             "gllm_seq_relu2": [P, P, G, I, P],
             "gllm_seq_gemm_simt": [P, G, P, G, P, G, I, I, I, I, P, P],
             "gllm_attn_decode_win": [P, G, P, P, P, G, P, P, I, I, I, I, I, I, I, F, I, P, P],
@@ -243,23 +243,30 @@ def causal_conv_silu(xz, channels, w, b, conv_state, rec_slots, seq_lens, query_
 
 
 _SCAN_WORK_BYTES = 256 << 20        # workspace of a scan cut in time, at a time; more channels take another round
+_SCAN_UNCUT = 128                   # portions of at most so many tokens are walked whole, whatever is beside them
 
 
 def scan_piece(tokens: int, longest: int, channels: int) -> int:
     """Tokens of a piece of the scan (csrc/seq/scan_ops.cu), for `tokens` tokens in all and at most `longest` in one portion: all of
-    them (nothing is cut), or a multiple of 64. Walking whole portions takes 572 us per 2^26 tokens x channels and no less than
-    0.105 us per token of the longest one; cut, everything is done twice: 940 us, and two launches more (measured, B200). Portions
-    of up to 512 tokens are never cut: there is little to gain, and their bits do not depend on what else is known of the batch."""
+    them (nothing is cut), or a multiple of 64. Walked whole, a batch takes some 480 us per 2^26 tokens x channels and 0.1 us per token
+    of its longest portion; cut, where everything is done twice, some 900 us per 2^26 and 20 us. Measured (B200, 16 states, bf16; whole /
+    cut): 8192 channels, 4 x 2048 tokens 661 / 875 us, 1 x 8192 1314 / 921; 4096 channels, 4 x 2048 405 / 473, 2 x 4096 530 / 473; 2048
+    channels, 8 x 1024 206 / 249, 4 x 2048 269 / 247, 1 x 2048 226 / 78. Pieces give every scheduler twelve, up to 256 tokens: 4096
+    channels, 8192 tokens in pieces of 64, 128, 256, 512, 1024: 498, 485, 485, 495, 571 us."""
     work = tokens * channels / 2.0 ** 26
-    if longest <= 512 or max(572.0 * work, 0.105 * longest) <= 940.0 * work + 13.0:
+    if longest <= 512 or 480.0 * work + 0.1 * longest <= 900.0 * work + 20.0:
         return tokens
-    return max(64, int(tokens * channels / 8 / (592 * 12)) // 64 * 64)      # twelve pieces for every scheduler
+    return max(64, min(256, int(tokens * channels / 8 / (4 * sm100.NUM_SMS * 12)) // 64 * 64))
 
 
 def selective_scan(xc, dt_raw, proj, xz, a, d_skip, dt_bias, ssm_state, rec_slots, seq_lens, query_start_loc,
                    channels, nstate, dt_rank, max_q_len: Optional[int] = None):
-    """With `max_q_len` (the longest portion of the batch, or a bound on it) above one token, four lanes walk a channel
-    (csrc/seq/scan_ops.cu); batches of single tokens, or without a bound, take the token-serial kernel."""
+    """With `max_q_len` (the longest portion of the batch, or a bound on it) above one token, two or four lanes walk a channel
+    (csrc/seq/scan_ops.cu); batches of single tokens, or without a bound, take the token-serial kernel.
+
+    The same batch gives the same bits. A portion's may depend on what is beside it: the states of those of up to `_SCAN_UNCUT` tokens
+    do not, in batches that are walked; their outputs (sums over the states, in the order of the lanes) and portions that are cut do, by
+    roundings of fp32."""
     assert xc.is_contiguous() and dt_raw.is_contiguous() and proj.stride(1) == 1 and xz.stride(1) == 1
     assert a.dtype == torch.float32 and a.is_contiguous()
     out = torch.empty_like(xc)
@@ -274,7 +281,8 @@ def selective_scan(xc, dt_raw, proj, xz, a, d_skip, dt_bias, ssm_state, rec_slot
             rounds = 3 * -(-channels // width)
         rc = _L().gllm_scan_walk(_p(xc), _p(dt_raw), _p(proj), proj.stride(0), _p(xz), xz.stride(0), _p(a), _p(d_skip),
                                  _p(dt_bias), _p(ssm_state), _p(rec_slots), _p(seq_lens), _p(query_start_loc), t, nseq,
-                                 channels, nstate, dt_rank, piece, width, _p(work), _p(out), _f32(xc), stream_ptr())
+                                 channels, nstate, dt_rank, piece, _SCAN_UNCUT, width, _p(work), _p(out), _f32(xc),
+                                 stream_ptr())
         if rc != 2:                          # 2: more states than four lanes hold
             check(rc, "scan_walk")
             sm100._count(rounds)

@@ -311,6 +311,7 @@ def test_scan_walk_against_float64(dt, N, C, piece, monkeypatch):
     st0 = torch.randn(n, N, C, device=DEV)
     if piece:
         monkeypatch.setattr(S, "scan_piece", lambda *a: piece)
+        monkeypatch.setattr(S, "_SCAN_UNCUT", 0)
     st = st0.clone()
     got = S.selective_scan(x, dtr, proj, xz, A, Dk, db, st, rs, sl, qsl, C, N, R, max_q_len=max(lens))
     want, ends, at = torch.empty(t, C, dtype=torch.float64, device=DEV), st0.double(), 0
@@ -395,3 +396,26 @@ def test_scan_with_infinite_rates(L):
     out = (want * proj[:, N:, None].double()).sum(1) * torch.nn.functional.silu(xz[:, C::3].double())
     assert bool(((y[:, ::3].double() - out).abs() <= 2.0 ** -20 * (want.abs() * proj[:, N:, None].abs()).sum(1) * 20).all())
     assert bool(torch.isfinite(y).all()) and bool(torch.isfinite(st).all())
+
+
+@pytest.mark.parametrize("N,C", [(16, 96), (5, 2048)])
+def test_scan_of_a_short_portion_beside_a_long_one(N, C):
+    """Portions of up to 128 tokens alone, and beside one that is cut in pieces: the same states bit for bit, outputs of the same terms
+    (at most 16, 2^-23 each for the order of the sum)."""
+    from gllm_b200.ops import sm100_seq as S
+    torch.manual_seed(C)
+    lens, R = [100, 1500, 128, 1, 7], 3
+    t, n = sum(lens), len(lens)
+    assert S.scan_piece(t, 1500, C) < 128 and S.scan_piece(128, 128, C) == 128
+    qsl = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
+    rs, sl = torch.arange(n, dtype=torch.int32, device=DEV), torch.tensor(lens, dtype=torch.int32, device=DEV) + 1
+    x, raw, xz, proj = (torch.randn(t, w, device=DEV) for w in (C, C, 2 * C, R + 2 * N))
+    A, z, st0 = -torch.rand(C, N, device=DEV), torch.zeros(C, device=DEV), torch.randn(n, N, C, device=DEV)
+    st = st0.clone()
+    y = S.selective_scan(x, raw, proj, xz, A, z, z, st, rs, sl, qsl, C, N, R, max_q_len=1500)
+    for s in (0, 2, 3, 4):
+        a, b, one = int(qsl[s]), int(qsl[s + 1]), st0[s:s + 1].clone()
+        ys = S.selective_scan(x[a:b], raw[a:b], proj[a:b], xz[a:b], A, z, z, one, rs[:1], sl[s:s + 1], qsl[s:s + 2] - a, C, N, R, max_q_len=128)
+        assert torch.equal(one[0], st[s])
+        most = torch.nn.functional.silu(xz[a:b, C:]).abs() * (y[a:b].abs() + 16 * 30)         # |state| |C| below 30
+        assert bool(((ys - y[a:b]).abs() <= 2.0 ** -20 * most).all())
