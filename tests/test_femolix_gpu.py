@@ -196,7 +196,8 @@ def test_gated_group_norm_gates_one_by_one(act):
 @pytest.mark.parametrize("taps", [1, 2, 4])
 @pytest.mark.parametrize("qlens", [[600], [1, 1, 2050, 3, 1, 4, 5], [17, 1, 15, 700]])
 def test_conv_rows_fetched_ahead(qlens, taps):
-    """Blocks of 8 and 16 rows with four fetched ahead: sequence borders at every place of a group of four, a last block cut short."""
+    """Blocks of 8 rows, one fetched ahead, and of 16, all fetched ahead in groups of four: sequence borders at every place of a group,
+    a last block cut short."""
     from gllm_b200.ops import ref, sm100_seq as S
     torch.manual_seed(taps)
     ns, C = len(qlens), 36
@@ -210,6 +211,35 @@ def test_conv_rows_fetched_ahead(qlens, taps):
     st1, st2 = st.clone(), st.clone()
     c1, c2 = S.causal_conv_silu(xz, C, w, b, st1, rs, sl, qsl), ref.causal_conv_silu(xz, C, w, b, st2, rs, sl, qsl)
     assert close(c1, c2, 1e-2) and torch.equal(st1, st2)
+
+
+@pytest.mark.parametrize("C", [5120, 10240])
+@pytest.mark.parametrize("qlens", [[4100], [1, 1, 700, 13, 1500, 18, 1, 1866]])
+def test_conv_rows_beyond_the_ring(C, qlens):
+    """Blocks of 32 (5120 channels) and 64 rows, which fill each of the 16 places of the ring twice and four times: borders inside a
+    block, a last block cut short. Element by element: the sum and the sigmoid are fp32 (2^-18 at any input here), one rounding."""
+    from gllm_b200.ops import ref, sm100_seq as S
+    torch.manual_seed(C)
+    ns, t, taps = len(qlens), sum(qlens), 4
+    ctx = [5 * (i % 2) for i in range(ns)]
+    qsl = torch.tensor([0] + qlens, device=DEV).cumsum(0).to(torch.int32)
+    sl = torch.tensor([c + q for c, q in zip(ctx, qlens)], dtype=torch.int32, device=DEV)
+    rs = torch.randperm(ns + 1, device=DEV)[:ns].to(torch.int32)
+    xz = (torch.randn(t, C, device=DEV) * 4).bfloat16()
+    w, b = torch.randn(C, taps, device=DEV), torch.randn(C, device=DEV)
+    st1 = torch.randn(ns + 1, taps - 1, C, device=DEV).bfloat16()
+    st2, st0 = st1.clone(), st1.clone()
+    got = S.causal_conv_silu(xz, C, w, b, st1, rs, sl, qsl)
+    assert close(got, ref.causal_conv_silu(xz, C, w, b, st2, rs, sl, qsl), 1e-2) and torch.equal(st1, st2)
+    for s in range(ns):
+        a, e = int(qsl[s]), int(qsl[s + 1])
+        before = st0[rs[s]].double() if ctx[s] else torch.zeros(taps - 1, C, dtype=torch.float64, device=DEV)
+        x = torch.cat([before, xz[a:e].double()])
+        terms = [w[:, j].double() * x[j:j + e - a] for j in range(taps)]
+        acc, size = sum(terms) + b.double(), sum(v.abs() for v in terms) + b.double().abs()
+        want = acc * torch.sigmoid(acc)
+        tol = want.abs() * (2.0 ** -8 + 2.0 ** -17) + size * 2.0 ** -22 * (1 + acc.abs()) * torch.sigmoid(acc)   # sum of 5, times silu'
+        assert bool(((got[a:e].double() - want).abs() <= tol).all())
 
 
 def test_tensor_core_attention_with_chunk_mask_and_strided_output():

@@ -208,10 +208,12 @@ def test_greedy_generation_on_the_gpu(models, graphs):
 
 @pytest.mark.parametrize("N,C", [(16, 130), (5, 64), (12, 257)])
 @pytest.mark.parametrize("qlens,ctx", [([1, 128, 127, 129, 300], [4, 0, 2, 66, 0]), ([193], [0])])
-def test_scan_cut_in_time(N, C, qlens, ctx):
-    """Portions of 128 tokens and more run in chunks; both forms against float64 from the same fp32 inputs. The cut form adds
-    one product of a summed decay per chunk and no other rounding: as accurate as the serial form."""
-    from gllm_b200.ops import sm100_seq as S
+def test_scan_cut_in_time(N, C, qlens, ctx, monkeypatch):
+    """Portions of 128 tokens and more in pieces of 64; both forms against float64 from the same fp32 inputs. The cut form adds
+    one product of a summed decay per piece and no other rounding: as accurate as the serial form."""
+    from gllm_b200.ops import sm100, sm100_seq as S
+    monkeypatch.setattr(S, "scan_piece", lambda *a: 64)
+    monkeypatch.setattr(S, "_SCAN_UNCUT", 127)
     torch.manual_seed(N + len(qlens))
     R, t, n = 6, sum(qlens), len(qlens)
     qsl = torch.tensor([0] + qlens, device=DEV).cumsum(0).to(torch.int32)
@@ -232,19 +234,21 @@ def test_scan_cut_in_time(N, C, qlens, ctx):
             want[i] = (h @ pd[i, R + N:] + Dd * xd[i]) * torch.nn.functional.silu(zd[i])
         ends[slot] = h.t()
     err = []
-    for mx in (max(qlens), None):
-        st = st0.clone()
+    for mx, launches in ((max(qlens), 3), (None, 1)):
+        st, before = st0.clone(), sm100.launches()
         y = S.selective_scan(x, dtr, proj, xz, A, Dk, db, st, rs, sl, qsl, C, N, R, max_q_len=mx)
+        assert sm100.launches() - before == launches
         err.append([float((g.double().cpu() - e).norm() / e.norm()) for g, e in ((y, want), (st, ends))])
     for cut, serial in zip(*err):
         assert cut <= max(1.2 * serial, 1e-6), err
 
 
-@pytest.mark.parametrize("lens", [[5], [100], [130], [100, 130]])
-def test_scan_with_a_bound_on_the_lengths(lens):
-    """`max_q_len` may be larger than every portion: each portion is computed. A short one is then walked by the cut form's last
-    pass: the same state bit for bit, outputs within one bf16 rounding (their states are summed in another order)."""
-    from gllm_b200.ops import sm100_seq as S
+@pytest.mark.parametrize("lens,cut", [([5], False), ([100], False), ([100, 130], False), ([400, 400], True), ([300, 7, 128, 400], True)])
+def test_scan_with_a_bound_on_the_lengths(lens, cut):
+    """`max_q_len` may be larger than every portion: each portion is computed, also where the bound makes the batch one that is cut.
+    Portions of up to 128 tokens are walked whole in both: the same state bit for bit; longer ones within fp32 roundings (2^-23 a
+    token); outputs within one bf16 rounding."""
+    from gllm_b200.ops import sm100, sm100_seq as S
     torch.manual_seed(lens[0])
     N, C, R, t, n = 8, 70, 4, sum(lens), len(lens)
     qsl = torch.tensor([0] + lens, device=DEV).cumsum(0).to(torch.int32)
@@ -253,21 +257,27 @@ def test_scan_with_a_bound_on_the_lengths(lens):
     proj = torch.randn(t, R + 2 * N, device=DEV).bfloat16()
     A, Dk, db = -torch.rand(C, N, device=DEV) * 4, torch.randn(C, device=DEV), torch.full((C,), -3.0, device=DEV)
     got = []
-    for bound in (max(lens), 1000):
-        st = torch.zeros(n, N, C, device=DEV)
+    for bound, launches in ((max(lens), 1), (1000, 3 if cut else 1)):
+        st, before = torch.zeros(n, N, C, device=DEV), sm100.launches()
         torch.full((t, C), 3.0, device=DEV).bfloat16()       # what an unwritten output is likely to hold
         got.append((S.selective_scan(x, dtr, proj, xz, A, Dk, db, st, rs, sl, qsl, C, N, R, max_q_len=bound), st))
+        assert sm100.launches() - before == launches
     (a, sa), (b, sb) = got
-    assert torch.equal(sa, sb) and bool(sa.abs().sum() > 0)
-    assert bool(((a.float() - b.float()).abs() <= a.float().abs() * 2.0 ** -7 + 1e-6).all())
+    for s, m in enumerate(lens):
+        assert bool(sa[s].abs().sum() > 0)
+        assert torch.equal(sa[s], sb[s]) if m <= 128 or not cut else float((sa[s] - sb[s]).norm() / sa[s].norm()) <= m * 2.0 ** -23
+    # sums of eight terms in fp32, of either form's states, and a rounding of 2^-8 each
+    assert bool(((a.float() - b.float()).abs() <= a.float().abs() * 2.0 ** -7 + 1e-5).all())
 
 
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("state", [True, False])
 def test_scan_in_rounds_of_channels(dt, state, monkeypatch):
-    """A workspace for 128 channels: rounds of 128, 128 and 1, the same bits as all at once; with and without a carried state, in
-    fp32 and bf16. Against the token-serial kernel: fp32 sums in another order, and for bf16 outputs one rounding (2^-8)."""
-    from gllm_b200.ops import sm100_seq as S
+    """Portions cut in pieces of 64 with a workspace for 128 channels: rounds of 128, 128 and 1, the same bits as all at once; with and
+    without a carried state, in fp32 and bf16. Against the token-serial kernel: fp32 sums in another order, and for bf16 outputs one
+    rounding (2^-8)."""
+    from gllm_b200.ops import sm100, sm100_seq as S
+    monkeypatch.setattr(S, "scan_piece", lambda *a: 64)
     torch.manual_seed(5)
     N, C, R, qlens, ctx = 12, 257, 6, [150, 7, 129, 256], [4, 0, 0, 66]
     t, n = sum(qlens), len(qlens)
@@ -278,11 +288,12 @@ def test_scan_in_rounds_of_channels(dt, state, monkeypatch):
     proj = torch.randn(t, R + 2 * N, device=DEV).to(dt)
     A, Dk, db = -torch.rand(C, N, device=DEV) * 4, torch.randn(C, device=DEV), torch.full((C,), -3.0, device=DEV)
     st0, got = torch.randn(n, N, C, device=DEV), []
-    for work, mx in ((1 << 28, max(qlens)), (0, max(qlens)), (1 << 28, None)):
+    for work, mx, launches in ((1 << 28, max(qlens), 3), (0, max(qlens), 9), (1 << 28, None, 1)):
         monkeypatch.setattr(S, "_SCAN_WORK_BYTES", work)
-        st = st0.clone()
+        st, before = st0.clone(), sm100.launches()
         o = S.selective_scan(x, dtr, proj, xz, A, Dk, db, st if state else None, rs if state else None, sl, qsl, C, N, R,
                              max_q_len=mx)
+        assert sm100.launches() - before == launches
         got.append((o, st))
     for (whole, rounds, serial), tol in zip(zip(*got), (1e-5 if dt == torch.float32 else 2.0 ** -8, 1e-5)):
         assert torch.equal(whole, rounds)
