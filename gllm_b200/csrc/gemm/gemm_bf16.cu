@@ -565,7 +565,7 @@ static int pick_bn(int M, int N, int epi, int forced) {
   const int cands[5] = {256, 192, 128, 64, 32};
   for (int i = 0; i < 5; ++i) {
     const int bn = cands[i];
-    if (epi == kEpiSiluMul && (bn < 64 || bn == 192)) continue;         // gated weights are interleaved for 128 and 256
+    if (epi == kEpiSiluMul && (bn < 64 || bn == 192)) continue;         // gated rows alternate in blocks of half a tile: 256, 128, 64
     const int tiles = num_m * ((N + bn - 1) / bn);
     const int waves = (tiles + sms - 1) / sms;
     // time of one round of tiles, measured at K = 7168: 43.3 us at 256 wide, 38.4 at 192, 33.4 at 128 (the 128 rows of A cost the

@@ -13,13 +13,14 @@
 // TMEM buffers ping-pong per K block so the tensor core runs block kb+1 while the CUDA cores fold
 // block kb. Same TMA (SWIZZLE_128B, 128 fp8 = one 128-byte row) / mbarrier ring as gemm_bf16.cu.
 //
-// What bounds it: a 128 x 256 x 128 block takes the tensor core 512 cycles; folding it takes 256 cycles of TMEM reads and 128
-// issue slots of packed fma per scheduler when eight warps share it, so the fold hides as long as nothing in it waits. The
-// scales come from global memory (some 700 cycles away) and are therefore fetched kAhead blocks early. What is left is shared
-// memory: the copies write 48 KB per block and the products read 48 KB, 768 cycles at 128 bytes each (a copy of this kernel
-// that folds nothing runs at 2390 TFLOP/s). 4096 x 36864 x 7168: 1.11 ms, 1950 TFLOP/s; with 128-wide tiles, four fold warps
-// and the scales loaded where they are used it was 2.0 ms. 4096 x 18432 x 7168 gated + 4096 x 7168 x 18432 with their
-// quantisers (one dense feed-forward): 3.16 -> 2.0 ms.
+// What bounds it: a 128 x 256 x 128 block takes some 1080 cycles (4096 x 36864 x 7168: 1.11 ms, 1950 TFLOP/s), of which the tensor core
+// needs 512. Folding reads 128 KB of sums from TMEM, 256 cycles at the nominal 512 bytes, and takes 128 issue slots of packed fma per
+// scheduler when eight warps share it; copies and products write and read 48 KB of shared memory, 768 cycles at 128 bytes. Neither
+// alone explains it: a copy of this kernel that folds nothing takes 880 cycles (2390 TFLOP/s), and on pairs of SMs, which move a third
+// less through shared memory, the fold is no faster. What it waits for is not settled. The scales come from global memory (some 700
+// cycles away) and are therefore fetched kAhead blocks early. With 128-wide tiles, four fold warps and the scales loaded where they are
+// used the product above was 2.0 ms. 4096 x 18432 x 7168 gated + 4096 x 7168 x 18432 with their quantisers (one dense feed-forward):
+// 3.16 -> 2.0 ms.
 //
 // Also here: the dynamic per-token-group activation quantiser (reference fp8.py:354-552).
 #include <cuda_fp8.h>
