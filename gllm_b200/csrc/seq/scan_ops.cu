@@ -44,13 +44,17 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1,
 __device__ __forceinline__ float rcp(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
-// 2^t of both halves on the 2^x unit. Its results lie 1.5e-8 to 2e-8 below 2^t on average for t in (-1, 0), which adds up over the
-// tokens that a state remembers. The caller adds kBias = 1.9e-8 / ln 2 to t in the fma that forms it (states after 2048 tokens
-// against float64, steps of 0.001 to 0.1: 1.46e-7 with 2.2e-8, 1.41e-7 with 2.6e-8, 1.53e-7 with 3.4e-8; expf 1.43e-7).
+// 2^t of both halves on the 2^x unit. Its results lie below 2^t on average: by 0.5e-8 for t in (-0.004, 0), 1.6e-8 to 2.7e-8 in
+// (-0.5, -0.004), 2.5e-8 down to -1, 5e-8 below. That adds up over the tokens between two corrections of a state (`anchored`), so the
+// caller adds kBias = 2.1e-8 / ln 2 to t in the fma that forms it. Outputs of 2048 tokens against float64, decays around exp of
+// -0.001 / -0.005 / -0.01 / -0.02 / -0.05 / -0.1: 1.04e-6 / 4.3e-7 / 3.5e-7 / 3.1e-7 / 1.9e-7 / 1.3e-7 (with 2.7e-8: 9.5e-7 / 4.7e-7 /
+// 4.0e-7 / 3.6e-7 / 1.7e-7 / 1.3e-7, 3.3e-8: 1.13e-6 / 4.1e-7 / 3.3e-7 / 2.7e-7 / 2.0e-7 / 1.4e-7); chunks of 64 tokens with expf 9.7e-7 /
+// 3.9e-7 / 3.5e-7 / 3.2e-7 / 2.1e-7 / 1.5e-7. States: 8.8e-7 / 3.9e-7 / 3.1e-7 / 2.8e-7 / 1.7e-7 / 1.1e-7; 1.53e-6 / 4.6e-7 / 4.0e-7 / 3.3e-7 /
+// 2.0e-7 / 1.3e-7.
 // A single decay: A log2(e) is rounded before the product, so that decays of e^-5 and less have 1.4 times the rms error of expf(dt A),
-// of a value that is added to 150 times its size, and below 2^-126 they are 0. The states show nothing of it: steps of 0.1 to 2, A to
-// -24, 5.3e-8 against 5.4e-8 with expf.
-constexpr float kBias = 2.7e-8f;
+// of a value that is added to 150 times its size, and below 2^-126 they are 0. States that forget within a token or two, steps of 0.1
+// and A = -16: 6.7e-8, with expf 5.7e-8, a rounding of fp32 being 6e-8; steps of 0.1 to 2, A to -24: 5.3e-8, 5.2e-8.
+constexpr float kBias = 3.0e-8f;
 __device__ __forceinline__ f2 exp2_unit(f2 t) {
   float t0, t1;
   un(t, t0, t1);
@@ -119,7 +123,7 @@ __device__ __forceinline__ f2 silu2(f2 z) {
 constexpr float kMostF = 3.4028235e38f;
 // What a state lacks after steps of `Dt` in all from S0 on, decays whose product was P: the unit's errors have one sign for decays of
 // about the same size, and a state that keeps thousands of tokens adds them up. exp(A Dt), formed once in 64 tokens, does not. States
-// of 2048 tokens whose decays lie around 0.9999 / 0.999 / 0.99, against float64: 1.4e-6 / 8.4e-7 / 3.4e-7, without it 2.3e-5 / 1.0e-5 /
+// of 2048 tokens whose decays lie around 0.9999 / 0.999 / 0.99, against float64: 1.4e-6 / 8.8e-7 / 3.1e-7, without it 2.3e-5 / 1.0e-5 /
 // 5.5e-7, chunks of 64 tokens with expf 9e-7 / 1.5e-6 / 4.0e-7. It costs 8 % of the kernel.
 __device__ __forceinline__ float anchored(float a, float Dt, float P, float S0) {
   const float lack = (exp2f(a * Dt) - P) * S0;
