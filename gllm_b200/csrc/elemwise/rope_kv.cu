@@ -155,7 +155,8 @@ __global__ void rope_kv_kernel(const RopeParams p) {
 // earlier head's store), the rotation row read once for all of them. Memory-bound: every q / k element is read and
 // written once, v and the cache rows once more. The kernel above has one head per warp and re-reads its cos / sin row for
 // every head in 4-byte words. Cold L2, heads of 128, before and after: 4096 tokens x (32 + 8 + 8) heads 91 -> 43 us (2.7
-// TB/s), 8192 x (64 + 8 + 8) 290 -> 114 us, 256 x (32 + 8 + 8) 13 -> 11 us; heads of 64, 4096 x 48: 68 -> 26 us.
+// TB/s), 8192 x (64 + 8 + 8) 290 -> 114 us, 256 x (32 + 8 + 8) 13 -> 11 us; heads of 64, 4096 x 48: 68 -> 26 us. Whole NeoX heads of
+// 64 and 128 take the kernel below.
 template <int L, int NB>
 __global__ void __launch_bounds__(128) rope_kv_vec_kernel(const RopeParams p) {
   griddep_launch();
@@ -284,6 +285,131 @@ __global__ void __launch_bounds__(128) rope_kv_vec_kernel(const RopeParams p) {
   }
 }
 
+// NeoX rotation of whole heads (rot = D), the common form: a lane holds eight elements of the lower half and their partners of the
+// upper one, so that nothing is exchanged for the rotation (eight shuffles per eight elements above) and its row (read once for NB
+// heads) is half as long per lane. The projections come from L2, so the chain position -> row -> rotation and the issue slots bound it.
+// Heads of 128 with norms, in an attention block, kernel above and this one: 4096 tokens x (32 + 8 + 8) heads 38.6 -> 24.1 us (4.2
+// TB/s), 8192 x (64 + 8 + 8) without norms 106 -> 71 us, 256 x (32 + 8 + 8) 5.6 -> 3.6 us.
+template <int L, int NB>
+__global__ void __launch_bounds__(128) rope_kv_pair_kernel(const RopeParams p) {
+  griddep_launch();
+  griddep_wait();
+  constexpr int D = 16 * L, H = D / 2, kHeadsPerWarp = 32 / L, kStep = 4 * kHeadsPerWarp;
+  const int t = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int e0 = (lane % L) * 8;
+  const int n_qk = p.Hq + p.Hkv;
+  const int n_heads = n_qk + ((p.v != nullptr && p.slots != nullptr) ? p.Hkv : 0);
+  const int first = blockIdx.y * (kStep * NB) + warp * kHeadsPerWarp + lane / L;
+  const int pos = p.positions != nullptr ? p.positions[t] : 0, slot = p.slots != nullptr ? p.slots[t] : -1;
+
+  uint4 raw[NB][2];
+#pragma unroll
+  for (int n = 0; n < NB; ++n) {
+    const int hh = first + n * kStep;
+    raw[n][0] = raw[n][1] = make_uint4(0u, 0u, 0u, 0u);
+    if (hh < n_heads && (hh < n_qk || slot >= 0)) {
+      const __nv_bfloat16* src = hh < p.Hq ? p.q + t * p.q_ts + hh * p.q_hs
+                                 : hh < n_qk ? p.k + t * p.k_ts + (hh - p.Hq) * p.k_hs
+                                             : p.v + t * p.v_ts + (hh - n_qk) * p.v_hs;
+      raw[n][0] = *reinterpret_cast<const uint4*>(src + e0);
+      raw[n][1] = *reinterpret_cast<const uint4*>(src + H + e0);
+    }
+  }
+  float c[8], s[8];
+  const float* row = p.cos_sin + static_cast<size_t>(pos) * D + e0;
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    const float4 cv = *reinterpret_cast<const float4*>(row + 4 * g), sv = *reinterpret_cast<const float4*>(row + H + 4 * g);
+    c[4 * g] = cv.x; c[4 * g + 1] = cv.y; c[4 * g + 2] = cv.z; c[4 * g + 3] = cv.w;
+    s[4 * g] = sv.x; s[4 * g + 1] = sv.y; s[4 * g + 2] = sv.z; s[4 * g + 3] = sv.w;
+  }
+  const size_t slab = static_cast<size_t>(p.page_size) * 64;
+  size_t at = 0;                                           // of the lower eight elements in head 0 of the slot's page
+  if (slot >= 0) {
+    const int page = slot / p.page_size, off = slot - page * p.page_size;
+    at = static_cast<size_t>(page) * p.Hkv * (D / 64) * slab + static_cast<size_t>(off) * 64 + e0;
+  }
+  const size_t upper = D == 64 ? 32 : slab;                // ... and from there to the upper eight
+  const bool norm = p.q_norm_w != nullptr || p.k_norm_w != nullptr;
+#pragma unroll
+  for (int n = 0; n < NB; ++n) {
+    const int hh = first + n * kStep;
+    const bool is_q = hh < p.Hq;
+    float x[2][8];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t rw[4] = {raw[n][i].x, raw[n][i].y, raw[n][i].z, raw[n][i].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = unpack_bf16(rw[e]);
+        x[i][2 * e] = f.x;
+        x[i][2 * e + 1] = f.y;
+      }
+    }
+    if (norm) {
+      float ss = 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss += x[0][e] * x[0][e] + x[1][e] * x[1][e];
+#pragma unroll
+      for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const __nv_bfloat16* nw = is_q ? p.q_norm_w : p.k_norm_w;
+      if (hh < n_qk && nw != nullptr) {
+        const float inv = rsqrtf(ss / static_cast<float>(D) + p.eps);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const uint4 wv = *reinterpret_cast<const uint4*>(nw + i * H + e0);
+          const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = unpack_bf16(ww[e]);
+            // rounded to bf16 after the norm, as the unfused form does
+            x[i][2 * e] = __bfloat162float(__float2bfloat16(x[i][2 * e] * inv * f.x));
+            x[i][2 * e + 1] = __bfloat162float(__float2bfloat16(x[i][2 * e + 1] * inv * f.y));
+          }
+        }
+      }
+    }
+    if (hh >= n_heads) continue;
+    if (hh < n_qk) {
+      uint32_t w[2][4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float r[2][2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int i = 2 * e + j;
+          r[0][j] = x[0][i] * c[i] - x[1][i] * s[i];
+          r[1][j] = x[1][i] * c[i] + x[0][i] * s[i];
+        }
+        w[0][e] = pack_bf16(r[0][0], r[0][1]);
+        w[1][e] = pack_bf16(r[1][0], r[1][1]);
+      }
+      const uint4 a = make_uint4(w[0][0], w[0][1], w[0][2], w[0][3]), b = make_uint4(w[1][0], w[1][1], w[1][2], w[1][3]);
+      __nv_bfloat16* dst = is_q ? p.q + t * p.q_ts + hh * p.q_hs : p.k + t * p.k_ts + (hh - p.Hq) * p.k_hs;
+      *reinterpret_cast<uint4*>(dst + e0) = a;
+      *reinterpret_cast<uint4*>(dst + H + e0) = b;
+      if (!is_q && slot >= 0 && p.k_cache != nullptr) {
+        __nv_bfloat16* k = p.k_cache + at + (hh - p.Hq) * (D / 64) * slab;
+        *reinterpret_cast<uint4*>(k) = a;
+        *reinterpret_cast<uint4*>(k + upper) = b;
+      }
+    } else if (slot >= 0) {
+      __nv_bfloat16* v = p.v_cache + at + (hh - n_qk) * (D / 64) * slab;
+      *reinterpret_cast<uint4*>(v) = raw[n][0];
+      *reinterpret_cast<uint4*>(v + upper) = raw[n][1];
+    }
+  }
+}
+
+template <int L>
+static cudaError_t launch_rope_pair(const RopeParams& p, int n_heads, cudaStream_t st) {
+  constexpr int kStep = 4 * (32 / L);
+  if (static_cast<int64_t>(p.T) * n_heads >= static_cast<int64_t>(num_sms()) * 16 * kStep * 2)
+    return launch_pdl(rope_kv_pair_kernel<L, 2>, dim3(p.T, (n_heads + 2 * kStep - 1) / (2 * kStep)), dim3(128), 0, st, p);
+  return launch_pdl(rope_kv_pair_kernel<L, 1>, dim3(p.T, (n_heads + kStep - 1) / kStep), dim3(128), 0, st, p);
+}
+
 template <int L>
 static cudaError_t launch_rope_vec(const RopeParams& p, int n_heads, cudaStream_t st) {
   constexpr int kStep = 4 * (32 / L);
@@ -333,6 +459,10 @@ GLLM_EXPORT int gllm_rope_kv_write(void* q, int64_t q_ts, int64_t q_hs, int Hq, 
                    (rot == 0 || (neox ? rot % 16 == 0 : rot % 8 == 0));
   if (vec) {
     cudaStream_t vst = reinterpret_cast<cudaStream_t>(stream);
+    if (neox && rot == D && D <= 128 && sec0 == 0 && cos_sin != nullptr) {
+      CUDA_CHECK_RET(D == 64 ? launch_rope_pair<4>(p, n_heads, vst) : launch_rope_pair<8>(p, n_heads, vst));
+      return 0;
+    }
     CUDA_CHECK_RET(D == 64 ? launch_rope_vec<8>(p, n_heads, vst)
                            : D == 128 ? launch_rope_vec<16>(p, n_heads, vst) : launch_rope_vec<32>(p, n_heads, vst));
     return 0;

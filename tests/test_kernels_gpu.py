@@ -167,6 +167,37 @@ def test_rope_kv_write_edges(t, hq, hkv, d, rot, neox, shift):
     assert torch.equal(caches[1], caches[3])
 
 
+@pytest.mark.parametrize("t,hq,hkv", [(1, 5, 1), (3, 33, 8), (700, 19, 3), (2100, 32, 8)])   # one head per lane group, or two
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("norms,cached", [("qk", True), ("q", True), ("", True), ("k", False)])
+def test_rope_kv_write_whole_heads(t, hq, hkv, d, norms, cached):
+    """NeoX rotation of whole heads, both halves of a pair in one lane: lane groups without a head, one norm of the two, no cache;
+    tolerance as above (two roundings to bf16)."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(t + d)
+    page, pages = 16, (t + 15) // 16 + 2
+    buf = torch.randn(t, (hq + 2 * hkv) * d, device=_dev()).bfloat16()
+    ref_buf = buf.clone()
+    pos = torch.randint(0, 4000, (t,), device=_dev(), dtype=torch.int32)
+    slots = torch.randperm(pages * page, device=_dev())[:t].to(torch.int32)
+    slots[t // 2] = -1
+    cs = ref.build_cos_sin_cache(d, 4096, 10000.0).to(_dev())
+    qn, kn = ((1 + 0.1 * torch.randn(d, device=_dev())).bfloat16() if n in norms else None for n in "qk")
+    shape = ref.kv_cache_shape(pages, hkv, d, page)
+    caches = [torch.zeros(shape, device=_dev(), dtype=torch.bfloat16) if cached else None for _ in range(4)]
+
+    def views(b):
+        q, k, v = b.split([hq * d, hkv * d, hkv * d], 1)
+        return q.unflatten(1, (hq, d)), k.unflatten(1, (hkv, d)), v.unflatten(1, (hkv, d)) if cached else None
+
+    sm100.rope_kv_write(*views(buf), pos, cs, d, True, qn, kn, 1e-6, caches[0], caches[1], slots if cached else None)
+    ref.rope_kv_write(*views(ref_buf), pos, cs, d, True, qn, kn, 1e-6, caches[2], caches[3], slots if cached else None)
+    assert _rel_err(buf, ref_buf) < 8e-3
+    if cached:
+        assert _rel_err(caches[0], caches[2]) < 8e-3
+        assert torch.equal(caches[1], caches[3])
+
+
 @pytest.mark.parametrize("sec", [[16, 24, 24], [24, 20, 20, 1]])   # chunked (Qwen2.5-VL) / interleaved (Qwen3-VL)
 @pytest.mark.parametrize("strided", [False, True])
 def test_rope_mrope(sec, strided):
