@@ -59,7 +59,7 @@ struct TcAttnParams {
   const int32_t* block_table;
   const int32_t* seq_lens;
   const int32_t* q_start;
-  int max_blocks, Hq, Hkv, G, GP, page_size, seq_offset;
+  int max_blocks, Hq, Hkv, G, GP, page_size, seq_offset, num_seqs;
   float scale_log2;
   // score cap (kernel template CAP): a scaled score s becomes cap * tanh(s / cap); cap_log2 = cap * log2(e),
   // scale_over_cap = scale / cap. sink: one extra logit per query head in the softmax denominator that carries no
@@ -174,17 +174,21 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   volatile int* sees = reinterpret_cast<int*>(tmem_slot + 2);   // [2 tiles][low, end): keys that a query tile sees, from tile0 on
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int seq = blockIdx.y + p.seq_offset;
-  const int groups_per_kv = p.G / p.GP;
-  const int kvh = blockIdx.z / groups_per_kv;
-  const int hbase = kvh * p.G + (blockIdx.z % groups_per_kv) * p.GP;
+  // Head groups first, then sequences, then from the last query block of each to the first: the CTAs that start late are the
+  // ones with few keys. (One sequence of one head after the other left the last wave to the long blocks of the last head: expanded
+  // latent heads, 5 prompts of 4096 tokens in all, 169 us for 145; 19 prompts, 32 / 8 heads of 128, 65.6 for 63.9; 8192 tokens over
+  // 8192 cached, 64 / 8 heads, 2751 for 2703.)
+  const int groups_per_kv = p.G / p.GP, z = blockIdx.x % (p.Hkv * groups_per_kv), rest = blockIdx.x / (p.Hkv * groups_per_kv);
+  const int seq_in = rest % p.num_seqs, back = rest / p.num_seqs, seq = seq_in + p.seq_offset;
+  const int kvh = z / groups_per_kv;
+  const int hbase = kvh * p.G + (z % groups_per_kv) * p.GP;
   const int q_begin = p.q_start[seq], q_len = p.q_start[seq + 1] - q_begin;
-  if (DENSE && p.kv_row[blockIdx.y + 1] == p.kv_row[blockIdx.y]) return;      // no rows: not expanded
+  if (DENSE && p.kv_row[seq_in + 1] == p.kv_row[seq_in]) return;      // no rows: not expanded
   const int toks_per_tile = kTcRows / p.GP;
   const int toks_per_cta = toks_per_tile * p.q_tiles;
   const int n_blocks = (q_len + toks_per_cta - 1) / toks_per_cta;
-  if (static_cast<int>(blockIdx.x) >= n_blocks) return;
-  const int tok_cta = (n_blocks - 1 - blockIdx.x) * toks_per_cta;      // heaviest (last) queries first
+  if (back >= n_blocks) return;
+  const int tok_cta = (n_blocks - 1 - back) * toks_per_cta;
   const int seq_len = p.seq_lens[seq];
   const int ctx_len = seq_len - q_len;
   // KV tiles [tile0, tile0 + n): with a window the first query's oldest visible key decides where they start; pipeline
@@ -204,7 +208,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   const int j = lane % boxes, sl = lane / boxes;       // this lane's box and 64-wide slab
   const int32_t* bt = p.block_table + static_cast<size_t>(seq) * p.max_blocks;
   const int last_page = (seq_len - 1) / p.page_size;
-  const int row0 = DENSE ? p.kv_row[blockIdx.y] : 0;
+  const int row0 = DENSE ? p.kv_row[seq_in] : 0;
   auto page_of = [&](int tile) {                       // masked columns read the last page: keep the data finite
     return DENSE ? 0 : bt[min(((tile0 + tile) * KV + j * box) / p.page_size, last_page)];
   };
@@ -686,7 +690,13 @@ static int launch_prefill_tc(const CUtensorMap& tk, const CUtensorMap& tv, const
     fprintf(stderr, "[gllm_b200] query tensor-map encode failed (%d)\n", (int)r);
     return 1;
   }
-  dim3 grid((max_q_len + toks_per_cta - 1) / toks_per_cta, num_seqs, z);
+  p.num_seqs = num_seqs;
+  const int64_t ctas = static_cast<int64_t>((max_q_len + toks_per_cta - 1) / toks_per_cta) * num_seqs * z;
+  if (ctas > 0x7fffffff) {
+    fprintf(stderr, "[gllm_b200] prefill attention: %lld blocks\n", static_cast<long long>(ctas));
+    return 1;
+  }
+  const dim3 grid(static_cast<unsigned>(ctas));
   attn_prefill_tc_kernel<DK, DV, DENSE, CAP, BIAS><<<grid, kTcThreads, SM::kBytes, st>>>(tk, tv, tpe, tq, p);
   CUDA_CHECK_RET(cudaGetLastError());
   return 0;
