@@ -110,6 +110,8 @@ class MLAAttention(nn.Module):
         hl = self.num_heads
         h = tpc.materialize(h)
         qkv_a = self._qkv_a()
+        if kv_cache is not None and self._one_call(inp, h, qkv_a):
+            return self._forward_one_call(inp, h, qkv_a, kv_cache.k_cache[self.layer_id])
         if qkv_a is not None:
             both = Fn.linear(h, qkv_a)
             kv_a = both[:, self.q_lora:]
@@ -251,6 +253,21 @@ class MLAAttention(nn.Module):
             if hasattr(inp, "latent_plan"):
                 inp.latent_plan = plan
         return plan
+
+    def _one_call(self, inp, h, qkv_a) -> bool:
+        """Whether the block is the plain absorbed one on bf16 weights, which one native call launches as a whole."""
+        from gllm_b200.ops import sm100
+        return h.is_cuda and h.shape[0] > 0 and isinstance(qkv_a, torch.Tensor) and self.q_b_ws is None and self._expands() and \
+            self.q_lora <= 8192 and h.dtype == qkv_a.dtype == self.q_b_w.dtype == torch.bfloat16 and \
+            self.q_b_w.is_contiguous() and not sm100.gemm_forced() and not self._plan_on_device(inp, h.device)[0]
+
+    def _forward_one_call(self, inp, h, qkv_a, cache):
+        from gllm_b200.ops import sm100
+        pos = inp.positions if inp.positions.dim() == 1 else inp.positions[0]
+        w_uk, w_uv = self._absorbed_weights()
+        out = sm100.mla_block(h, self.num_heads, qkv_a, self.q_a_norm_w, self.kv_a_norm_w, self.eps, self.q_b_w, w_uk, w_uv,
+                              self.rope.cos_sin, pos, inp.slot_mapping, cache, inp.block_table, inp.tok_seq, self.scaling)
+        return out.view(h.shape[0], self.num_heads * self.v_dim)
 
     def _forward_absorbed(self, inp, q, kv_c, k_pe, cache):
         """sm_100a path: multi-query attention over the latent cache (csrc/attn/mla_attention.cu) for decoding sequences and

@@ -68,6 +68,8 @@ def _declare(lib):
     sig("gllm_attn_prefill_tc", [P, L, P, P, P, L, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P])
     sig("gllm_mla_attention", [P, P, P, L, P, P, P, P, P, P, I, I, I, I, I, F, I, P, P])
     sig("gllm_mla_rope_cache", [P, L, L, I, P, L, L, P, L, P, L, P, P, P, P, I, I, P])
+    sig("gllm_mla_block_scratch", [I, I, I, I], L)
+    sig("gllm_mla_block", [P, L, I, I, I, I, P, P, P, F, P, P, P, P, P, P, P, L, I, P, I, P, F, I, P, P, L, P, L, P, P, I, I, P])
     sig("gllm_mla_gather", [P, P, I, P, P, I, I, I, I, I, P, P, P, P])
     sig("gllm_attn_prefill_expanded", [P, L, P, L, P, P, L, P, P, P, I, I, I, I, I, F, P])
     sig("gllm_sample", [P, I, L, P, I, I, P, P, P, P, P, I, P, c_uint64, P, P, I, P])

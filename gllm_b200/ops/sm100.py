@@ -64,6 +64,11 @@ def _smallm_workspace(device):
     return ws
 
 
+def gemm_forced() -> bool:
+    """Whether a tuning switch overrides the choice between the GEMM kernels."""
+    return _FORCE_BN != 0 or _FORCE_SPLIT != 0
+
+
 def _linear_smallm(x, w, bias, out, silu: int):
     """`silu`: 0 plain, 1 SiLU-gate, 2 tanh-gelu-gate (gate / up rows interleaved per 128)."""
     m, k = x.shape
@@ -510,6 +515,35 @@ def mla_rope_cache(q_pe: torch.Tensor, q_full: Optional[torch.Tensor], k_pe: tor
                                 k_pe.stride(0), _p(kv_c), kv_c.stride(0), _p(cos_sin), _p(positions), _p(slots), _p(cache),
                                 cache.shape[3], t, stream_ptr()), "mla_rope_cache")
     _count()
+
+
+def mla_block(h: torch.Tensor, heads: int, qkv_a: torch.Tensor, q_norm_w: torch.Tensor, kv_norm_w: torch.Tensor, eps: float,
+              q_b: torch.Tensor, w_uk: torch.Tensor, w_uv: torch.Tensor, cos_sin: torch.Tensor, positions: torch.Tensor,
+              slots: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, tok_seq: Optional[torch.Tensor],
+              scale: float) -> torch.Tensor:
+    """Latent attention of h [T, width] in the absorbed form, every step from the projections to the heads' results [T, heads, 128]:
+    the kernels of `linear`, `rmsnorm_two`, `gemm_batched`, `mla_rope_cache` and `mla_attention` in one call
+    (csrc/attn/mla_block.cu). bf16 weights: qkv_a [q_rank + 576, width], q_b [heads * 192, q_rank]."""
+    t, width = h.shape
+    rank = q_b.shape[1]
+    pages, hkv, nslab, page_size, w = cache.shape
+    assert h.dtype == qkv_a.dtype == q_b.dtype == w_uk.dtype == w_uv.dtype == _BF16 and cos_sin.dtype == torch.float32
+    assert h.stride(1) == 1 and qkv_a.is_contiguous() and q_b.is_contiguous() and w_uk.is_contiguous() and w_uv.is_contiguous()
+    assert qkv_a.shape == (rank + 576, width) and q_b.shape[0] == heads * 192 and hkv == 1 and nslab == 9 and w == 64
+    assert w_uk.shape == (heads, 512, 128) and w_uv.shape == (heads, 128, 512)
+    L = _lib.load()
+    out = torch.empty(t, heads, 128, dtype=_BF16, device=h.device)
+    size = L.gllm_mla_block_scratch(t, heads, rank, NUM_SMS)
+    scratch = torch.empty(size, dtype=torch.uint8, device=h.device)
+    ws, cnt, tcnt = _smallm_workspace(h.device)
+    check(L.gllm_mla_block(h.data_ptr(), h.stride(0), t, width, heads, rank, qkv_a.data_ptr(), q_norm_w.data_ptr(),
+                           kv_norm_w.data_ptr(), eps, q_b.data_ptr(), w_uk.data_ptr(), w_uv.data_ptr(), cos_sin.data_ptr(),
+                           positions.data_ptr(), slots.data_ptr(), cache.data_ptr(), pages, page_size, block_table.data_ptr(),
+                           block_table.shape[1], None if tok_seq is None else tok_seq.data_ptr(), scale, NUM_SMS, out.data_ptr(),
+                           scratch.data_ptr(), size, ws.data_ptr(), _SMALLM_WS_FLOATS, cnt.data_ptr(), tcnt.data_ptr(),
+                           _SPLITK_MAX_TILES, _SMALLM_MAX, stream_ptr()), "mla_block")
+    _count(8)
+    return out
 
 
 def mla_expanded_attention(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, seq_lens: torch.Tensor,

@@ -1024,6 +1024,55 @@ def test_latent_attention_block_mixed_batches(decodes, q_lens, ctx, kv_rows, lat
             assert _rel_err(x[0][b:b + a], got[2][0][b:b + a]) < 1.2e-2
 
 
+@pytest.mark.parametrize("heads,width", [(1, 256), (5, 512), (16, 8192)])
+@pytest.mark.parametrize("q_lens,decodes", [([1], 1), ([1] * 33, 33), ([1] * 65 + [3, 7], 65), ([1] * 129, 129), ([20], 0)])
+def test_latent_attention_block_in_one_call(heads, width, q_lens, decodes, monkeypatch):
+    """The block launched by one native call is the block launched kernel by kernel, bit for bit: rows that take each of the GEMMs,
+    one head, strided hidden states, decoding sequences and short portions."""
+    from types import SimpleNamespace
+    from gllm_b200.layers.rotary import build_rope
+    from gllm_b200.models.decoder import ModelSpec
+    from gllm_b200.models.deepseek_v2 import MLAAttention
+    from gllm_b200.ops import sm100
+    torch.manual_seed(6)
+    dev, page = _dev(), 16
+    spec = ModelSpec(arch="DeepseekV3ForCausalLM", hidden_size=width, num_layers=1, num_heads=heads, num_kv_heads=heads, head_dim=192,
+                     intermediate_size=64, vocab_size=64, rms_eps=1e-6, dtype=torch.bfloat16, use_mla=True,
+                     extra={"qk_nope_head_dim": 128, "qk_rope_head_dim": 64, "v_head_dim": 128, "kv_lora_rank": 512,
+                            "q_lora_rank": 256})
+    att = MLAAttention(spec, 0, build_rope(64, 1024, 1e4, None, 64, False, device=dev), dev)
+    for p in att.parameters():
+        p.data.copy_(torch.randn(p.shape, device=dev) * p.shape[-1] ** -0.5 if p.dim() == 2 else 1 + 0.1 * torch.randn(p.shape, device=dev))
+    att.process_weights()
+    ctx = [(37 * i) % 150 for i in range(len(q_lens))]
+    lens = [a + b for a, b in zip(q_lens, ctx)]
+    need = [-(-n // page) for n in lens]
+    ids = torch.randperm(sum(need)).split(need)
+    bt = torch.zeros(len(lens), max(need), dtype=torch.int32)
+    for i, x in enumerate(ids):
+        bt[i, :len(x)] = x
+    qsl = np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32)
+    pos = torch.cat([torch.arange(a, a + b) for a, b in zip(ctx, q_lens)]).int()
+    seq = torch.repeat_interleave(torch.arange(len(q_lens)), torch.tensor(q_lens)).int()
+    slots = bt[seq.long(), pos.long() // page] * page + pos % page
+    inp = SimpleNamespace(num_decode_seqs=decodes, num_seqs=len(q_lens), padded_tokens=0, max_q_len=max(q_lens),
+                          batch=SimpleNamespace(query_start_loc=qsl, seq_lens=np.array(lens, np.int32)), positions=pos.to(dev),
+                          slot_mapping=slots.int().to(dev), block_table=bt.to(dev), seq_lens=torch.tensor(lens).int().to(dev),
+                          tok_seq=None if decodes == len(q_lens) else seq.to(dev), query_start_loc=torch.as_tensor(qsl).to(dev))
+    tpc = SimpleNamespace(materialize=lambda h: h)
+    cache0 = torch.randn(sum(need), 1, 9, page, 64, device=dev).bfloat16()
+    h = torch.randn(sum(q_lens), width + 64, device=dev).bfloat16()[:, 32:32 + width]
+    calls, got = [], []
+    one = sm100.mla_block
+    monkeypatch.setattr(sm100, "mla_block", lambda *a: calls.append(1) or one(*a))
+    for forced in (0, 1):
+        monkeypatch.setattr(sm100, "gemm_forced", lambda: bool(forced))
+        cache = cache0.clone()
+        got.append((att(inp, h, SimpleNamespace(k_cache=[cache]), tpc), cache))
+    assert len(calls) == 1
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 @pytest.mark.parametrize("m", [1, 2])
 @pytest.mark.parametrize("n,k", [(1, 8), (5, 264), (130, 1024), (4097, 1024), (4100, 2056), (257, 6144), (640, 8192)])
 def test_linear_few_rows(m, n, k):
