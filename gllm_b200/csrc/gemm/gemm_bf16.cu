@@ -18,6 +18,7 @@
 // and its GEMM -> NCCL all_reduce sequence (gllm/layers/linear.py:247-250).
 #include "../common/host_utils.h"
 #include "../common/ptx.cuh"
+#include "gemm_cluster.h"
 #include "gemm_pair.h"
 #include <string.h>
 
@@ -708,6 +709,13 @@ static int gemm_bf16_impl(const void* A, int64_t lda, const void* W, int64_t ldw
   const bool decode = ws != nullptr && tile_cnt != nullptr && ws_bytes > 0 && M <= g_max_split_m;   // pick_split's sizes
   // pairs, and gated tiles of 192 below, read gate and up rows that alternate in blocks of 128, as tiles of 256 do
   const bool free_bn = force_bn == (epi == kEpiSiluMul ? 256 : 0);
+  ClusterPlan plan;
+  if (comm == nullptr && decode && free_bn && g_force_split <= 0 && glu_limit <= 0.f && (epi != kEpiSiluMul || (N % 256 == 0 && bias == nullptr)) &&
+      plan_gemm_cluster(M, N, K, epi == kEpiSiluMul, &plan)) {
+    const ClusterGemm g{A, W, lda, ldw, reinterpret_cast<__nv_bfloat16*>(C), ldc, M, N, K,
+                        reinterpret_cast<const __nv_bfloat16*>(bias), epi == kEpiSiluMul, gelu};
+    return gemm_bf16_cluster(g, plan, reinterpret_cast<cudaStream_t>(stream));
+  }
   if (comm == nullptr && !decode && split == 1 && free_bn && pairs_are_faster(M, N, bn)) {
     const PairGemm g{A, W, lda, ldw, reinterpret_cast<__nv_bfloat16*>(C), ldc, M, N, K,
                      reinterpret_cast<const __nv_bfloat16*>(bias), epi == kEpiSiluMul, glu_limit, glu_alpha, gelu};

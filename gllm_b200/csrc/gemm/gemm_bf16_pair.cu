@@ -300,7 +300,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, PairParams p, cuda
   p.num_m = (p.g.M + 255) / 256;
   p.num_n = (p.g.N + kPBN - 1) / kPBN;
   const int tiles = p.num_m * p.num_n, all = num_sms() / 2;
-  CUDA_CHECK_RET(launch_pdl_pairs(kern, dim3(2 * (tiles < all ? tiles : all)), dim3(kPThreads), kPSmem, st, ta, tb, p));
+  CUDA_CHECK_RET(launch_pdl_cluster(kern, dim3(2 * (tiles < all ? tiles : all)), 2, dim3(kPThreads), kPSmem, st, ta, tb, p));
   return 0;
 }
 

@@ -12,12 +12,17 @@
 // workspace (L2 resident) and the last CTA to arrive for a tile reduces them in a fixed order
 // (deterministic), applies bias / SiLU-gate and stores bf16.
 //
+// Most products of a decode batch go to gemm_bf16_cluster.cu, which adds the parts of K up through distributed shared memory (the rule
+// and both sides' times stand there): what stays here are vocabulary heads, whose many tiles one persistent CTA per SM walks, and up
+// to eight rows on a few tiles, which up to sixteen parts of K draw faster.
+//
 // Same warp specialisation as gemm_bf16.cu: warp 0 TMA producer, warp 1 tcgen05.mma issuer,
 // warps 2-5 epilogue; TMEM accumulators double buffered.
 #include <string.h>
 
 #include "../common/host_utils.h"
 #include "../common/ptx.cuh"
+#include "gemm_cluster.h"
 
 namespace b200 {
 
@@ -318,6 +323,13 @@ GLLM_EXPORT int gllm_gemm_smallm(const void* A, int64_t lda, const void* W, int6
   if (force_split <= 0) {
     const int rc = gemv_bf16(A, lda, W, ldw, C, ldc, M, N, K, bias, silu, reinterpret_cast<cudaStream_t>(stream));
     if (rc >= 0) return rc;
+    ClusterPlan plan;
+    if (N % 8 == 0 && ldc % 8 == 0 && ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0 &&
+        (silu == 0 || (N % 256 == 0 && bias == nullptr)) && plan_gemm_cluster(M, N, K, silu != 0, &plan)) {
+      const ClusterGemm g{A, W, lda, ldw, reinterpret_cast<__nv_bfloat16*>(C), ldc, M, N, K,
+                          reinterpret_cast<const __nv_bfloat16*>(bias), silu != 0, silu == 2};
+      return gemm_bf16_cluster(g, plan, reinterpret_cast<cudaStream_t>(stream));
+    }
   }
   SmallMParams p;
   memset(&p, 0, sizeof(p));

@@ -256,10 +256,11 @@ class MLAAttention(nn.Module):
 
     def _one_call(self, inp, h, qkv_a) -> bool:
         """Whether the block is the plain absorbed one on bf16 weights, which one native call launches as a whole."""
+        if not (h.is_cuda and isinstance(qkv_a, torch.Tensor)) or h.shape[0] == 0 or self._plan_on_device(inp, h.device)[0]:
+            return False
         from gllm_b200.ops import sm100
-        return h.is_cuda and h.shape[0] > 0 and isinstance(qkv_a, torch.Tensor) and self.q_b_ws is None and self._expands() and \
-            self.q_lora <= 8192 and h.dtype == qkv_a.dtype == self.q_b_w.dtype == torch.bfloat16 and \
-            self.q_b_w.is_contiguous() and not sm100.gemm_forced() and not self._plan_on_device(inp, h.device)[0]
+        return self.q_b_ws is None and self._expands() and self.q_lora <= 8192 and self.q_b_w.is_contiguous() and \
+            h.dtype == qkv_a.dtype == self.q_b_w.dtype == torch.bfloat16 and not sm100.gemm_forced()
 
     def _forward_one_call(self, inp, h, qkv_a, cache):
         from gllm_b200.ops import sm100

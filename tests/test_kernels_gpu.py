@@ -1024,6 +1024,43 @@ def test_latent_attention_block_mixed_batches(decodes, q_lens, ctx, kv_rows, lat
             assert _rel_err(x[0][b:b + a], got[2][0][b:b + a]) < 1.2e-2
 
 
+@pytest.mark.parametrize("m,n,k,act", [(3, 128, 64, None), (17, 200, 520, None), (33, 256, 8, "silu"), (64, 1000, 776, None),
+                                       (100, 512, 4096, "gelu"), (129, 2112, 1024, None), (256, 384, 4104, None), (300, 136, 1536, None)])
+@pytest.mark.parametrize("parts", [1, 2, 3, 5, 8])
+@pytest.mark.parametrize("smem", [108, 220])
+def test_gemm_on_clusters(m, n, k, act, parts, smem):
+    """K over the CTAs of a cluster: parts without a row of their own, with one K block or a ragged one, tiles past the last column
+    and row, one and several tiles of rows, strided input and output, bias and both gates. fp32 sums of bf16 products, one rounding
+    to bf16; gated ones also __expf and a division (2^-8 relative in all)."""
+    from gllm_b200.ops import lib
+    if parts > -(-k // 64):
+        pytest.skip("no empty parts")
+    torch.manual_seed(m + n)
+    gated, n_out = act is not None, n // 2 if act else n
+    x = torch.randn(m, k + 16, device=_dev()).bfloat16()[:, 8:8 + k]
+    wide = torch.randn(n, k, device=_dev()).bfloat16() * k ** -0.5
+    w = torch.zeros(n, k + 8, device=_dev(), dtype=torch.bfloat16)[:, :k]
+    w.copy_(ref.interleave_gate_up(wide) if gated else wide)
+    b = None if gated else torch.randn(n, device=_dev()).bfloat16()
+    out = torch.full((m + 1, n_out + 8), 7.0, device=_dev()).bfloat16()
+    y = x.double() @ wide.double().t()
+    if gated:
+        g, u = y.chunk(2, -1)
+        want = (torch.nn.functional.silu(g) if act == "silu" else torch.nn.functional.gelu(g, approximate="tanh")) * u
+        tol = want.abs() * 2.0 ** -7 + 1e-3
+    else:
+        want = y + b.double()
+        tol = want.abs() * 2.0 ** -8 + (x.double().abs() @ wide.double().abs().t() + b.double().abs()) * k * 2.0 ** -24
+    rows = min(256, -(-m // 16) * 16)
+    for bt in {rows, max(16, -(-rows // 32) * 16)}:
+        out.fill_(7.0)
+        assert lib.load().gllm_gemm_bf16_cluster(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), m, n, k,
+                                                 None if b is None else b.data_ptr(), int(gated), int(act == "gelu"), bt, parts,
+                                                 smem * 1024, lib.stream_ptr()) == 0
+        assert bool((out[m] == 7.0).all()) and bool((out[:, n_out:] == 7.0).all())
+        assert bool(((out[:m, :n_out].double() - want).abs() <= tol).all())
+
+
 @pytest.mark.parametrize("heads,width", [(1, 256), (5, 512), (16, 8192)])
 @pytest.mark.parametrize("q_lens,decodes", [([1], 1), ([1] * 33, 33), ([1] * 65 + [3, 7], 65), ([1] * 129, 129), ([20], 0)])
 def test_latent_attention_block_in_one_call(heads, width, q_lens, decodes, monkeypatch):
