@@ -553,6 +553,13 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
   const int tiles = num_m * num_n * split;
   const int sms = (num_sms() / split) * split;  // split-K slices of a tile must run in the same round
   const int grid = tiles < sms ? tiles : sms;
+  if constexpr (MOE) {
+    // Not ahead of the kernel before: with every kernel of a routed feed-forward launched early, its CTAs wait on SMs that the one
+    // before still needs (48 tokens x 8 of 128 experts: 206 us, with the two products launched behind it 197).
+    kern<<<grid, kNumThreads, Cfg::kSmemBytes, stream>>>(ta, tb, moe, p);
+    CUDA_CHECK_RET(cudaGetLastError());
+    return 0;
+  }
   CUDA_CHECK_RET(launch_pdl(kern, dim3(grid), dim3(kNumThreads), Cfg::kSmemBytes, stream, ta, tb, moe, p));
   return 0;
 }

@@ -23,10 +23,10 @@
 // 3.16 -> 2.0 ms.
 //
 // Also here: the dynamic per-token-group activation quantiser (reference fp8.py:354-552).
-#include <cuda_fp8.h>
 #include <string.h>
 
 #include "../common/bounded.cuh"
+#include "../common/fp8_quant.cuh"
 #include "../common/host_utils.h"
 #include "../common/ptx.cuh"
 
@@ -343,25 +343,10 @@ fp8_quant_group_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_fp
 #pragma unroll
   for (int n = 0; n < 4; ++n) {
     const int pair = n * 16 + (threadIdx.x >> 4), row = row0 + (pair & 7), g = g0 + (pair >> 3);
-    const uint32_t w[4] = {raw[n].x, raw[n].y, raw[n].z, raw[n].w};
-    float f[8], amax = 0.f;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 a = unpack_bf16(w[e]);
-      f[2 * e] = a.x;
-      f[2 * e + 1] = a.y;
-      amax = fmaxf(amax, fmaxf(fabsf(a.x), fabsf(a.y)));
-    }
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    amax = fmaxf(amax, 1e-10f);
-    const float scale = amax / 448.f;
-    const float inv = 1.f / scale;
+    float scale;
+    const uint2 o8 = fp8_quant_lane(raw[n], scale);
     if (row >= rows || g >= groups) continue;
-    __align__(8) __nv_fp8_e4m3 o8[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) o8[e] = __nv_fp8_e4m3(f[e] * inv);
-    *reinterpret_cast<uint2*>(q + static_cast<size_t>(row) * K + g * 128 + lane * 8) = *reinterpret_cast<uint2*>(o8);
+    *reinterpret_cast<uint2*>(q + static_cast<size_t>(row) * K + g * 128 + lane * 8) = o8;
     if (lane == 0) scales[static_cast<size_t>(g) * M + row] = scale;
   }
 }

@@ -7,12 +7,13 @@
 //   moe_align         counting sort of the (token, k) slots by LOCAL expert into 128-row tiles:
 //                     expert_count -> padded offsets -> per-tile expert id, slot -> row position
 //                     (ref: moe_align_block_size, gllm/layers/moe/moe_align_block_size.py:10-78)
-//   moe_gather        xs[row] = x[token(row)]  (rows of padding are zero)
+//   moe_gather        xs[row] = x[token(row)], as it is or quantised to e4m3; up to 4096 slots in one launch with the sort
 //   moe_combine       out[t] = sum_j w[t,j] * y[pos[t,j]]   (ref: moe_sum, fused with the routing weight)
 //
 // The expert GEMMs themselves are the tcgen05 kernel in gemm/gemm_bf16.cu running in grouped mode
 // (per-M-tile expert id selects the weight slab; the tile count is read from device memory so the
 // whole MoE block is CUDA-graph capturable without a host sync).
+#include "../common/fp8_quant.cuh"
 #include "../common/host_utils.h"
 #include "../common/ptx.cuh"
 
@@ -171,63 +172,179 @@ __global__ void grouped_topk_kernel(const __nv_bfloat16* __restrict__ logits, in
 //                      [2+2E .. 2+3E+1) padded offsets
 // ---------------------------------------------------------------------------------------------
 // n_valid (optional device scalar): only the first *n_valid slots are live (EP receive pool, comm/ep_a2a.cu)
-__global__ void moe_count_kernel(const int32_t* __restrict__ ids, const int32_t* __restrict__ expert_map, int n_slots,
-                                 int E_local, int32_t* __restrict__ meta, const int32_t* __restrict__ n_valid) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_slots || (n_valid != nullptr && i >= *n_valid)) return;
-  int e = ids[i];
-  if (expert_map != nullptr) e = expert_map[e];
-  if (e >= 0 && e < E_local) atomicAdd(&meta[2 + e], 1);
+struct RouteParams {
+  const int32_t *ids, *expert_map, *n_valid;
+  int n_slots, top_k, E, max_tiles;
+  int32_t *meta, *tile_expert, *slot_pos;
+  const __nv_bfloat16* x;
+  int64_t ldx;
+  __nv_bfloat16* xs;        // rows as they are ...
+  __nv_fp8_e4m3* q;         // ... or quantised, scales [H / 128][rows]
+  float* scales;
+  int H, rows;
+};
+
+__device__ __forceinline__ int local_expert(const RouteParams& p, int slot, int valid) {
+  if (slot >= valid) return -1;
+  int e = p.ids[slot];
+  if (p.expert_map != nullptr) e = p.expert_map[e];
+  return e >= 0 && e < p.E ? e : -1;
 }
 
-__global__ void moe_offsets_kernel(int32_t* __restrict__ meta, int32_t* __restrict__ tile_expert, int E_local,
-                                   int max_tiles) {
-  // single thread block; E_local <= 1024
-  __shared__ int s_off[1025];
-  if (threadIdx.x == 0) {
-    int off = 0;
-    for (int e = 0; e < E_local; ++e) {
-      s_off[e] = off;
-      off += (meta[2 + e] + kTileM - 1) / kTileM * kTileM;
+// Row offsets of the experts, padded to whole tiles, from their counts (both in shared memory; s_off has E + 1 entries). All threads
+// of the block.
+__device__ __forceinline__ void expert_offsets(const int* s_cnt, int* s_off, int E, int* s_warp) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  int base = 0;
+  for (int e0 = 0; e0 < E; e0 += blockDim.x) {
+    const int e = e0 + static_cast<int>(threadIdx.x);
+    const int own = e < E ? (s_cnt[e] + kTileM - 1) / kTileM * kTileM : 0;
+    int sum = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += v;
     }
-    s_off[E_local] = off;
-    meta[0] = off / kTileM;
-    meta[1] = off;
+    if (lane == 31) s_warp[warp] = sum;
+    __syncthreads();
+    int before = base, all = 0;
+    for (int w = 0; w < nw; ++w) {
+      if (w < warp) before += s_warp[w];
+      all += s_warp[w];
+    }
+    if (e < E) s_off[e] = before + sum - own;
+    base += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) s_off[E] = base;
+  __syncthreads();
+}
+
+__device__ __forceinline__ void write_meta(const RouteParams& p, const int* s_cnt, const int* s_off) {
+  const int E = p.E, total = s_off[E];
+  for (int e = threadIdx.x; e <= E; e += blockDim.x) {
+    p.meta[2 + 2 * E + e] = s_off[e];
+    if (e == E) {
+      p.meta[0] = total / kTileM;
+      p.meta[1] = total;
+      continue;
+    }
+    p.meta[2 + e] = s_cnt[e];
+    for (int t = s_off[e] / kTileM; t < s_off[e + 1] / kTileM; ++t) p.tile_expert[t] = e;
+  }
+  for (int t = total / kTileM + threadIdx.x; t < p.max_tiles; t += blockDim.x) p.tile_expert[t] = -1;
+}
+
+// one warp: a token's row to its place in the expert's segment
+template <bool QUANT>
+__device__ __forceinline__ void gather_row(const RouteParams& p, int slot, int pos) {
+  const int lane = threadIdx.x & 31;
+  const __nv_bfloat16* src = p.x + static_cast<size_t>(slot / p.top_k) * p.ldx;
+  if constexpr (!QUANT) {
+    __nv_bfloat16* dst = p.xs + static_cast<size_t>(pos) * p.H;
+    for (int i = lane * 8; i < p.H; i += 256) *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(src + i);
+  } else {                                               // sixteen lanes per group of 128, four pairs of groups on their way
+    for (int i0 = 0; i0 < p.H; i0 += 1024) {
+      uint4 raw[4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const int i = i0 + n * 256 + lane * 8;
+        raw[n] = i < p.H ? *reinterpret_cast<const uint4*>(src + i) : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const int i = i0 + n * 256 + lane * 8;
+        float scale;
+        const uint2 o8 = fp8_quant_lane(raw[n], scale);
+        if (i >= p.H) continue;
+        *reinterpret_cast<uint2*>(p.q + static_cast<size_t>(pos) * p.H + i) = o8;
+        if ((lane & 15) == 0) p.scales[static_cast<size_t>(i / 128) * p.rows + pos] = scale;
+      }
+    }
+  }
+}
+
+// Up to kOneLaunch slots: every block counts the whole batch for itself (a few KB of ids), so that routing is one launch instead of
+// four with a memset; a slot's row is its rank among the slots of its expert. Then a warp per slot copies.
+// 48 tokens x 8 of 128 experts, 2048 wide: 8.1 us, where the four took 12.5 and their launches as much again; 4096 tokens x 8, 32 of 256
+// experts here, quantised on the way (the two kernels below): 33 us, with copies in bf16 and a quantiser behind them 68.
+static constexpr int kOneLaunch = 4096, kRouteThreads = 256;
+
+template <bool QUANT>
+__global__ void __launch_bounds__(kRouteThreads) moe_route_kernel(const RouteParams p) {
+  extern __shared__ int32_t s_route[];                   // counts [E], offsets [E + 1], then the slots' experts as 16 bits
+  __shared__ int s_warp[kRouteThreads / 32];
+  int *s_cnt = s_route, *s_off = s_route + p.E;
+  int16_t* s_e = reinterpret_cast<int16_t*>(s_off + p.E + 1);
+  griddep_launch();
+  for (int e = threadIdx.x; e < p.E; e += blockDim.x) s_cnt[e] = 0;
+  __syncthreads();
+  griddep_wait();
+  const int valid = p.n_valid != nullptr ? min(p.n_slots, *p.n_valid) : p.n_slots;
+  for (int i = threadIdx.x; i < p.n_slots; i += blockDim.x) {
+    const int e = local_expert(p, i, valid);
+    s_e[i] = static_cast<int16_t>(e);
+    if (e >= 0) atomicAdd(&s_cnt[e], 1);
   }
   __syncthreads();
-  for (int e = threadIdx.x; e <= E_local; e += blockDim.x) meta[2 + 2 * E_local + e] = s_off[e];
-  for (int e = threadIdx.x; e < E_local; e += blockDim.x) {
-    meta[2 + E_local + e] = 0;  // cursors
-    for (int t = s_off[e] / kTileM; t < s_off[e + 1] / kTileM; ++t) tile_expert[t] = e;
+  expert_offsets(s_cnt, s_off, p.E, s_warp);
+  if (blockIdx.x == 0) write_meta(p, s_cnt, s_off);
+  const int lane = threadIdx.x & 31;
+  for (int slot = blockIdx.x * (kRouteThreads / 32) + (threadIdx.x >> 5); slot < p.n_slots; slot += gridDim.x * (kRouteThreads / 32)) {
+    const int e = s_e[slot];
+    int pos = -1;
+    if (e >= 0) {
+      int rank = 0;
+      for (int i = lane; i < slot; i += 32) rank += s_e[i] == e;
+      pos = s_off[e] + __reduce_add_sync(0xffffffffu, rank);
+      gather_row<QUANT>(p, slot, pos);
+    }
+    if (lane == 0) p.slot_pos[slot] = pos;
   }
-  const int nt = s_off[E_local] / kTileM;
-  for (int t = nt + threadIdx.x; t < max_tiles; t += blockDim.x) tile_expert[t] = -1;
 }
 
-// one warp per slot: claim a row in the expert's segment, copy the token row there
-__global__ void moe_scatter_gather_kernel(const int32_t* __restrict__ ids, const int32_t* __restrict__ expert_map,
-                                          int n_slots, int top_k, int E_local, int32_t* __restrict__ meta,
-                                          int32_t* __restrict__ slot_pos, const __nv_bfloat16* __restrict__ x,
-                                          int64_t ldx, __nv_bfloat16* __restrict__ xs, int H,
-                                          const int32_t* __restrict__ n_valid) {
-  const int slot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (slot >= n_slots) return;
-  int e = (n_valid != nullptr && slot >= *n_valid) ? -1 : ids[slot];
-  if (expert_map != nullptr && e >= 0) e = expert_map[e];
-  int pos = -1;
-  if (e >= 0 && e < E_local) {
-    if (lane == 0) pos = meta[2 + 2 * E_local + e] + atomicAdd(&meta[2 + E_local + e], 1);
-    pos = __shfl_sync(0xffffffffu, pos, 0);
-    const __nv_bfloat16* src = x + static_cast<size_t>(slot / top_k) * ldx;
-    __nv_bfloat16* dst = xs + static_cast<size_t>(pos) * H;
-    for (int i = lane * 8; i < H; i += 256) *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(src + i);
+// More slots: one block counts, ranks and places the segments; slot_pos holds a slot's rank until the next kernel adds the offset
+__global__ void __launch_bounds__(1024) moe_align_kernel(const RouteParams p) {
+  __shared__ int s_cnt[1024], s_off[1025], s_warp[32];
+  griddep_launch();
+  for (int e = threadIdx.x; e < p.E; e += blockDim.x) s_cnt[e] = 0;
+  __syncthreads();
+  griddep_wait();
+  const int valid = p.n_valid != nullptr ? min(p.n_slots, *p.n_valid) : p.n_slots;
+  for (int i0 = threadIdx.x; i0 < p.n_slots; i0 += 4 * 1024) {
+    int e[4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) e[n] = i0 + n * 1024 < p.n_slots ? local_expert(p, i0 + n * 1024, valid) : -1;
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+      if (i0 + n * 1024 < p.n_slots) p.slot_pos[i0 + n * 1024] = e[n] >= 0 ? atomicAdd(&s_cnt[e[n]], 1) : -1;
   }
-  if (lane == 0) slot_pos[slot] = pos;
+  __syncthreads();
+  expert_offsets(s_cnt, s_off, p.E, s_warp);
+  write_meta(p, s_cnt, s_off);
+}
+
+// one warp per slot
+template <bool QUANT>
+__global__ void __launch_bounds__(256) moe_gather_kernel(const RouteParams p) {
+  griddep_launch();
+  griddep_wait();
+  const int slot = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (slot >= p.n_slots) return;
+  const int rank = p.slot_pos[slot];
+  if (rank < 0) return;
+  int e = p.ids[slot];
+  if (p.expert_map != nullptr) e = p.expert_map[e];
+  const int pos = p.meta[2 + 2 * p.E + e] + rank;
+  gather_row<QUANT>(p, slot, pos);
+  __syncwarp();                                          // every lane has read the rank
+  if (lane == 0) p.slot_pos[slot] = pos;
 }
 
 __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ slot_pos,
                                    const float* __restrict__ w, __nv_bfloat16* __restrict__ out, int top_k, int H) {
+  griddep_launch();
+  griddep_wait();
   const int t = blockIdx.x;
   for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -298,36 +415,70 @@ GLLM_EXPORT int gllm_moe_grouped_topk(const void* logits, int64_t ld, const void
   return 0;
 }
 
-// meta: int32[2 + 3*E_local + 1] scratch (zeroed here); tile_expert: int32[max_tiles]; slot_pos: int32[n_slots];
+static int route(const RouteParams& p, cudaStream_t st) {
+  if (p.n_slots <= 0) return 0;
+  if (p.E <= 0 || p.E > 1024) {
+    fprintf(stderr, "[gllm_b200] moe_align_gather: %d experts (1 to 1024)\n", p.E);
+    return 1;
+  }
+  const bool quant = p.q != nullptr;
+  if (p.n_slots <= kOneLaunch) {
+    const size_t smem = (2 * p.E + 1) * 4 + p.n_slots * 2;
+    const dim3 grid((p.n_slots + kRouteThreads / 32 - 1) / (kRouteThreads / 32));
+    CUDA_CHECK_RET(launch_pdl(quant ? moe_route_kernel<true> : moe_route_kernel<false>, grid, dim3(kRouteThreads), smem, st, p));
+    return 0;
+  }
+  CUDA_CHECK_RET(launch_pdl(moe_align_kernel, dim3(1), dim3(1024), 0, st, p));
+  CUDA_CHECK_RET(launch_pdl(quant ? moe_gather_kernel<true> : moe_gather_kernel<false>, dim3((p.n_slots + 7) / 8), dim3(256), 0, st, p));
+  return 0;
+}
+
+static RouteParams route_params(const void* ids, const void* expert_map, int T, int top_k, int E, void* meta, void* tile_expert,
+                                int max_tiles, void* slot_pos, const void* x, int64_t ldx, int H, const void* n_valid) {
+  RouteParams p = {};
+  p.ids = reinterpret_cast<const int32_t*>(ids);
+  p.expert_map = reinterpret_cast<const int32_t*>(expert_map);
+  p.n_valid = reinterpret_cast<const int32_t*>(n_valid);
+  p.n_slots = T * top_k; p.top_k = top_k; p.E = E; p.max_tiles = max_tiles;
+  p.meta = reinterpret_cast<int32_t*>(meta);
+  p.tile_expert = reinterpret_cast<int32_t*>(tile_expert);
+  p.slot_pos = reinterpret_cast<int32_t*>(slot_pos);
+  p.x = reinterpret_cast<const __nv_bfloat16*>(x);
+  p.ldx = ldx; p.H = H;
+  return p;
+}
+
+// meta: int32[2 + 3*E_local + 1] (written here); tile_expert: int32[max_tiles]; slot_pos: int32[n_slots];
 // xs: bf16 [max_tiles*128, H] (caller zero-fills padding rows once; stale finite rows are harmless).
 GLLM_EXPORT int gllm_moe_align_gather(const void* ids, const void* expert_map, int T, int top_k, int E_local,
                                       void* meta, void* tile_expert, int max_tiles, void* slot_pos, const void* x,
                                       int64_t ldx, void* xs, int H, const void* n_valid, void* stream) {
-  const int n_slots = T * top_k;
-  if (n_slots <= 0) return 0;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  CUDA_CHECK_RET(cudaMemsetAsync(meta, 0, sizeof(int32_t) * (2 + 3 * E_local + 1), st));
-  moe_count_kernel<<<(n_slots + 255) / 256, 256, 0, st>>>(reinterpret_cast<const int32_t*>(ids),
-                                                           reinterpret_cast<const int32_t*>(expert_map), n_slots,
-                                                           E_local, reinterpret_cast<int32_t*>(meta),
-                                                           reinterpret_cast<const int32_t*>(n_valid));
-  moe_offsets_kernel<<<1, 256, 0, st>>>(reinterpret_cast<int32_t*>(meta), reinterpret_cast<int32_t*>(tile_expert),
-                                        E_local, max_tiles);
-  moe_scatter_gather_kernel<<<(n_slots * 32 + 255) / 256, 256, 0, st>>>(
-      reinterpret_cast<const int32_t*>(ids), reinterpret_cast<const int32_t*>(expert_map), n_slots, top_k, E_local,
-      reinterpret_cast<int32_t*>(meta), reinterpret_cast<int32_t*>(slot_pos),
-      reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<__nv_bfloat16*>(xs), H,
-      reinterpret_cast<const int32_t*>(n_valid));
-  CUDA_CHECK_RET(cudaGetLastError());
-  return 0;
+  RouteParams p = route_params(ids, expert_map, T, top_k, E_local, meta, tile_expert, max_tiles, slot_pos, x, ldx, H, n_valid);
+  p.xs = reinterpret_cast<__nv_bfloat16*>(xs);
+  return route(p, reinterpret_cast<cudaStream_t>(stream));
+}
+
+// The same with the rows quantised on their way, as gllm_fp8_quant_group quantises them: q e4m3 [max_tiles*128, H], scales fp32
+// [H/128, max_tiles*128]. Rows that no token goes to are not written.
+GLLM_EXPORT int gllm_moe_align_gather_fp8(const void* ids, const void* expert_map, int T, int top_k, int E_local, void* meta,
+                                          void* tile_expert, int max_tiles, void* slot_pos, const void* x, int64_t ldx, void* q,
+                                          void* scales, int H, void* stream) {
+  if (H % 128 != 0 || ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0) {
+    fprintf(stderr, "[gllm_b200] moe_align_gather_fp8: H %% 128 and rows on 16-byte boundaries required\n");
+    return 1;
+  }
+  RouteParams p = route_params(ids, expert_map, T, top_k, E_local, meta, tile_expert, max_tiles, slot_pos, x, ldx, H, nullptr);
+  p.q = reinterpret_cast<__nv_fp8_e4m3*>(q);
+  p.scales = reinterpret_cast<float*>(scales);
+  p.rows = max_tiles * kTileM;
+  return route(p, reinterpret_cast<cudaStream_t>(stream));
 }
 
 GLLM_EXPORT int gllm_moe_combine(const void* y, const void* slot_pos, const void* w, void* out, int T, int top_k,
                                  int H, void* stream) {
   if (T <= 0) return 0;
-  moe_combine_kernel<<<T, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(y), reinterpret_cast<const int32_t*>(slot_pos),
-      reinterpret_cast<const float*>(w), reinterpret_cast<__nv_bfloat16*>(out), top_k, H);
-  CUDA_CHECK_RET(cudaGetLastError());
+  CUDA_CHECK_RET(launch_pdl(moe_combine_kernel, dim3(T), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
+                            reinterpret_cast<const __nv_bfloat16*>(y), reinterpret_cast<const int32_t*>(slot_pos),
+                            reinterpret_cast<const float*>(w), reinterpret_cast<__nv_bfloat16*>(out), top_k, H));
   return 0;
 }

@@ -84,6 +84,7 @@ def _declare(lib):
     sig("gllm_moe_grouped_gemm_glu", [P, L, P, P, L, I, I, I, I, P, P, F, F, P])
     sig("gllm_gemm_bf16_glu", [P, L, P, L, P, L, I, I, I, F, F, P, L, P, I, P])
     sig("gllm_gemm_bf16_gelu", [P, L, P, L, P, L, I, I, I, P, L, P, I, P])
+    sig("gllm_moe_align_gather_fp8", [P, P, I, I, I, P, P, I, P, P, L, P, P, I, P])
     sig("gllm_moe_combine", [P, P, P, P, I, I, I, P])
     sig("gllm_fp8_quant_group", [P, L, P, P, I, I, P, P])
     sig("gllm_moe_grouped_gemm_fp8", [P, P, P, P, P, L, I, I, I, I, I, P, P, I, P])

@@ -114,13 +114,13 @@ def fused_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, topk_w: 
         row_dest = row_dest_fn(slot_pos, rows)
         check(L.gllm_moe_grouped_gemm(_p(hbuf), inter, _p(w2), _p(hbuf), h, max_tiles, h, inter, e_local,
                                       _p(tile_expert), _p(meta), 0, _p(row_dest), st), "moe_grouped_gemm2_push")
-        _count(6)
+        _count(5)
         return None
     ybuf = _buf("y", (rows, h), _BF16, dev)
     check(L.gllm_moe_grouped_gemm(_p(hbuf), inter, _p(w2), _p(ybuf), h, max_tiles, h, inter, e_local,
                                   _p(tile_expert), _p(meta), 0, None, st), "moe_grouped_gemm2")
     check(L.gllm_moe_combine(_p(ybuf), _p(slot_pos), _p(topk_w), _p(out), t, k, h, st), "moe_combine")
-    _count(7)
+    _count(4 if t * k <= 4096 else 5)
     return out
 
 
@@ -130,7 +130,7 @@ def fused_experts_fp8(x: torch.Tensor, w13: torch.Tensor, w13_s: torch.Tensor, w
     """Block-scaled fp8 experts (DeepSeek-V3 / Qwen3-FP8 checkpoints; reference: Fp8MoEMethod,
     gllm/layers/moe/fused_moe_triton/layer.py:99-194). w13 [E_local, 2I, H] e4m3 with gate/up rows interleaved
     per 64, w13_s fp32 [E_local, 2I/64, H/128]; w2 [E_local, H, I] e4m3, w2_s [E_local, H/64, I/128].
-    align+gather (bf16) -> per-token-group quant -> grouped fp8 GEMM1 (SiLU gate) -> quant -> grouped fp8
+    align+gather with per-token-group quant -> grouped fp8 GEMM1 (SiLU gate) -> quant -> grouped fp8
     GEMM2 -> combine."""
     assert x.dtype == _BF16 and x.stride(1) == 1 and w13.dtype == torch.float8_e4m3fn
     t, h = x.shape
@@ -148,7 +148,6 @@ def fused_experts_fp8(x: torch.Tensor, w13: torch.Tensor, w13_s: torch.Tensor, w
     meta = _buf("meta", (2 + 3 * e_local + 1,), torch.int32, dev)
     tile_expert = _buf("tile_expert", (max_tiles,), torch.int32, dev)
     slot_pos = _buf("slot_pos", (t * k,), torch.int32, dev)
-    xs = _buf("xs", (rows, h), _BF16, dev, zero=True)
     xs8 = _buf("xs8", (rows, h), torch.uint8, dev)
     xs_s = _buf("xs_s", (h // 128, rows), torch.float32, dev)
     hbuf = _buf("h", (rows, inter), _BF16, dev)
@@ -157,14 +156,15 @@ def fused_experts_fp8(x: torch.Tensor, w13: torch.Tensor, w13_s: torch.Tensor, w
     ybuf = _buf("y", (rows, h), _BF16, dev)
     L = _lib.load()
     st = stream_ptr()
-    check(L.gllm_moe_align_gather(_p(topk_ids), _p(expert_map), t, k, e_local, _p(meta), _p(tile_expert), max_tiles,
-                                  _p(slot_pos), _p(x), x.stride(0), _p(xs), h, None, st), "moe_align_gather")
-    check(L.gllm_fp8_quant_group(_p(xs), h, _p(xs8), _p(xs_s), rows, h, _p(meta), st), "fp8_quant(xs)")   # meta[0]: live tiles
+    if x.stride(0) % 8 or x.data_ptr() % 16:
+        x = x.clone(memory_format=torch.contiguous_format)
+    check(L.gllm_moe_align_gather_fp8(_p(topk_ids), _p(expert_map), t, k, e_local, _p(meta), _p(tile_expert), max_tiles,
+                                      _p(slot_pos), _p(x), x.stride(0), _p(xs8), _p(xs_s), h, st), "moe_align_gather_fp8")
     check(L.gllm_moe_grouped_gemm_fp8(_p(xs8), _p(xs_s), _p(w13), _p(w13_s), _p(hbuf), inter, max_tiles, max_live, two_i, h,
                                       e_local, _p(tile_expert), _p(meta), 1, st), "moe_grouped_gemm_fp8(1)")
     check(L.gllm_fp8_quant_group(_p(hbuf), inter, _p(h8), _p(h_s), rows, inter, _p(meta), st), "fp8_quant(h)")
     check(L.gllm_moe_grouped_gemm_fp8(_p(h8), _p(h_s), _p(w2), _p(w2_s), _p(ybuf), h, max_tiles, max_live, h, inter, e_local,
                                       _p(tile_expert), _p(meta), 0, st), "moe_grouped_gemm_fp8(2)")
     check(L.gllm_moe_combine(_p(ybuf), _p(slot_pos), _p(topk_w), _p(out), t, k, h, st), "moe_combine")
-    _count(9)
+    _count(6 if t * k <= 4096 else 7)
     return out

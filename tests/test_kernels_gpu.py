@@ -1061,6 +1061,68 @@ def test_gemm_on_clusters(m, n, k, act, parts, smem):
         assert bool(((out[:m, :n_out].double() - want).abs() <= tol).all())
 
 
+@pytest.mark.parametrize("t,k,experts,held,valid", [(1, 1, 1, 1, None), (3, 8, 16, 16, None), (512, 8, 128, 128, None),
+                                                    (513, 8, 256, 32, None), (2048, 2, 1024, 1024, None), (2049, 2, 1024, 700, None),
+                                                    (600, 1, 8, 8, 37), (5000, 1, 8, 8, 4097), (40, 4, 300, 0, None)])
+@pytest.mark.parametrize("quant", [False, True])
+def test_moe_routing_and_gather(t, k, experts, held, valid, quant):
+    """Counts, padded offsets, tiles, places and rows of both forms of the routing (up to 4096 slots in one launch), and quantised on
+    the way the same bytes and scales as by the quantiser."""
+    from gllm_b200.ops import lib
+    torch.manual_seed(t + experts)
+    dev, h, E = _dev(), 384, max(held, 1)
+    ids = torch.randint(0, experts, (t, k), device=dev, dtype=torch.int32)
+    ids[: t // 3] = ids[0, 0]                              # a liked expert: several tiles
+    emap = None
+    if held < experts:
+        emap = torch.full((experts,), -1, dtype=torch.int32, device=dev)
+        emap[torch.randperm(experts, device=dev)[:held]] = torch.arange(held, dtype=torch.int32, device=dev)
+    x = torch.randn(t, h + 8, device=dev).bfloat16()[:, :h]
+    if valid is not None:
+        ids[valid:] = 10 ** 6                              # never looked at
+    tiles = (t * k + 127) // 128 + E
+    new = lambda *s, dtype=torch.int32: torch.full(s, -77, dtype=dtype, device=dev)   # noqa: E731
+    meta, tile_expert, pos = new(2 + 3 * E + 1), new(tiles), new(t * k)
+    nv = None if valid is None else torch.tensor([valid], dtype=torch.int32, device=dev)
+    p = lambda v: None if v is None else v.data_ptr()      # noqa: E731
+    L = lib.load()
+    if quant:
+        if nv is not None:
+            pytest.skip("the quantised form takes every row")
+        rows, scales = torch.zeros(tiles * 128, h, dtype=torch.uint8, device=dev), torch.zeros(h // 128, tiles * 128, device=dev)
+        rc = L.gllm_moe_align_gather_fp8(p(ids), p(emap), t, k, E, p(meta), p(tile_expert), tiles, p(pos), p(x), x.stride(0), p(rows),
+                                         p(scales), h, lib.stream_ptr())
+    else:
+        rows = torch.zeros(tiles * 128, h, dtype=torch.bfloat16, device=dev)
+        rc = L.gllm_moe_align_gather(p(ids), p(emap), t, k, E, p(meta), p(tile_expert), tiles, p(pos), p(x), x.stride(0), p(rows), h,
+                                     p(nv), lib.stream_ptr())
+    assert rc == 0
+    e = ids.flatten().long() if valid is None else ids.flatten().clamp(max=experts - 1).long()
+    e = e if emap is None else emap[e].long()
+    if valid is not None:
+        e[valid:] = -1
+    live = e >= 0
+    cnt = torch.bincount(e[live], minlength=E)
+    off = torch.cat([torch.zeros(1, dtype=torch.long, device=dev), ((cnt + 127) // 128 * 128).cumsum(0)])
+    assert torch.equal(meta[2:2 + E].long(), cnt) and torch.equal(meta[2 + 2 * E:].long(), off)
+    assert meta[0] == off[-1] // 128 and meta[1] == off[-1]
+    want = torch.full((tiles,), -1, dtype=torch.int32, device=dev)
+    want[: int(off[-1]) // 128] = torch.repeat_interleave(torch.arange(E, device=dev), (cnt + 127) // 128).int()
+    assert torch.equal(tile_expert, want)
+    assert bool((pos[~live] == -1).all())
+    place, which = pos[live].long(), e[live]
+    assert torch.equal(place.sort().values, torch.cat([torch.arange(int(o), int(o + c), device=dev) for o, c in zip(off, cnt)] or [place[:0]]))
+    assert bool((place >= off[which]).all()) and bool((place < off[which] + cnt[which]).all())
+    src = x.repeat_interleave(k, 0)[live]
+    if not quant:
+        assert torch.equal(rows[place], src)
+    elif len(place):
+        src = src.contiguous()
+        q, s = torch.empty(len(place), h, dtype=torch.uint8, device=dev), torch.empty(h // 128, len(place), device=dev)
+        assert L.gllm_fp8_quant_group(p(src), h, p(q), p(s), len(place), h, None, lib.stream_ptr()) == 0
+        assert torch.equal(rows[place], q) and torch.equal(scales[:, place], s)
+
+
 @pytest.mark.parametrize("heads,width", [(1, 256), (5, 512), (16, 8192)])
 @pytest.mark.parametrize("q_lens,decodes", [([1], 1), ([1] * 33, 33), ([1] * 65 + [3, 7], 65), ([1] * 129, 129), ([20], 0)])
 def test_latent_attention_block_in_one_call(heads, width, q_lens, decodes, monkeypatch):
