@@ -275,7 +275,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTcRegsIssue));
     if (warp == kTcSoftmaxWarps) {
       // ------------------------------------------------------------------ TMA producer
-      auto after_step = [&](int j) { return j < 0 || guard.wait(&step[j & 3], (j >> 2) & 1); };
+      auto after_step = [&](int j) { return j < 0 || guard.wait<true>(&step[j & 3], (j >> 2) & 1); };
       int tk = n_max > 0 ? 1 : 0, tv = 0;                  // tiles issued
       bool ok = true;
       int page_v = page;
@@ -340,8 +340,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       };
       bool ok = n_max > 0 && guard.first(&k_full[0]);
       for (int t = 0; t < 2; ++t)
-        if (t ? n1 : n0) ok = ok && guard.wait(&q_full[t], 0);
-      ok = ok && guard.wait(&k_full[0], 0);
+        if (t ? n1 : n0) ok = ok && guard.wait<true>(&q_full[t], 0);
+      ok = ok && guard.wait<true>(&k_full[0], 0);
       if (ok) {
         tc_fence_after();
         if (n0 > 0) { issue_s(0, 0); umma_commit(s_full); }
@@ -349,13 +349,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         umma_commit(&step[0]);
       }
       for (int tile = 0; tile < n_max && ok; ++tile) {
-        if (tile + 1 < n_max) ok = guard.wait(&k_full[(tile + 1) % SM::kKStages], ((tile + 1) / SM::kKStages) & 1);
-        ok = ok && guard.wait(&v_full[tile % SM::kVStages], (tile / SM::kVStages) & 1);
+        if (tile + 1 < n_max) ok = guard.wait<true>(&k_full[(tile + 1) % SM::kKStages], ((tile + 1) / SM::kKStages) & 1);
+        ok = ok && guard.wait<true>(&v_full[tile % SM::kVStages], (tile / SM::kVStages) & 1);
         for (int t = 0; t < 2 && ok; ++t) {
           const int n = t ? n1 : n0;
           if (tile < n) {
             const int low = DENSE ? -tile : sees[2 * t] - tile * KV, end = DENSE ? KV : sees[2 * t + 1] - tile * KV;
-            ok = guard.wait(&p_full[t], tile & 1);
+            ok = guard.wait<true>(&p_full[t], tile & 1);
             if (!ok) break;
             tc_fence_after();
             issue_pv(t, tile, low, end);
@@ -405,8 +405,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       float m_run = -INFINITY, l_run = 0.f;
       // phase j of the query tile: S_j is there and PV_j-1 is in O
       auto await = [&](int j) {
-        if (qt == 0) guard.wait(s_full, j & 1);
-        else guard.wait(&step[j & 3], (j >> 2) & 1);
+        if (qt == 0) guard.wait<true>(s_full, j & 1);
+        else guard.wait<true>(&step[j & 3], (j >> 2) & 1);
         tc_fence_after();
       };
       const uint32_t t_s = tmem + lane_base + qt * KV, t_o = tmem_o + lane_base;

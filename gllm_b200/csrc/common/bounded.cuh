@@ -29,10 +29,11 @@ struct WaitGuard {
 
   __device__ __forceinline__ bool gave_up() const { return *dead != 0; }
 
-  // true: the phase completed. try_wait suspends the thread in hardware, so the clock is read rarely
+  // true: the phase completed. try_wait suspends the thread in hardware, so the clock is read rarely. SOON: it polls
+  template <bool SOON = false>
   __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity) const {
-    if (mbar_try_wait(bar, parity)) return true;
-    return wait_on(bar, parity);
+    if (look<SOON>(bar, parity)) return true;
+    return wait_on<SOON>(bar, parity);
   }
 
   // a role's first wait, looked at once: with a limit of 0 (tests) it is given up unless the phase has completed already
@@ -54,6 +55,10 @@ struct WaitGuard {
   }
 
  private:
+  template <bool SOON>
+  __device__ __forceinline__ static bool look(uint64_t* bar, uint32_t parity) {
+    return SOON ? mbar_try_wait_soon(bar, parity) : mbar_try_wait(bar, parity);
+  }
   __device__ __forceinline__ void give_up() const {
     *dead = 1;
     if (cfg.word != nullptr) {
@@ -62,6 +67,7 @@ struct WaitGuard {
     }
   }
   // the clock and the flag are looked at every 64 tries: in front of each, they cost the fp8 GEMM of one or two rows 3 %
+  template <bool SOON>
   __device__ __forceinline__ bool wait_on(uint64_t* bar, uint32_t parity) const {
     if (cfg.limit_ns == 0) {
       give_up();
@@ -71,7 +77,7 @@ struct WaitGuard {
     for (bool again = false;; again = true) {
 #pragma unroll 1
       for (int n = 0; n < 64; ++n)
-        if (mbar_try_wait(bar, parity)) return true;
+        if (look<SOON>(bar, parity)) return true;
       if (*dead != 0) return false;
       const uint32_t now = global_ns();
       if (!again) t0 = now;

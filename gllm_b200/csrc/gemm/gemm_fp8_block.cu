@@ -13,11 +13,13 @@
 // TMEM buffers ping-pong per K block so the tensor core runs block kb+1 while the CUDA cores fold
 // block kb. Same TMA (SWIZZLE_128B, 128 fp8 = one 128-byte row) / mbarrier ring as gemm_bf16.cu.
 //
-// What bounds it: a 128 x 256 x 128 block takes some 1080 cycles (4096 x 36864 x 7168: 1.11 ms, 1950 TFLOP/s), of which the tensor core
-// needs 512. Folding reads 128 KB of sums from TMEM, 256 cycles at the nominal 512 bytes, and takes 128 issue slots of packed fma per
-// scheduler when eight warps share it; copies and products write and read 48 KB of shared memory, 768 cycles at 128 bytes. Neither
-// alone explains it: a copy of this kernel that folds nothing takes 880 cycles (2390 TFLOP/s), and on pairs of SMs, which move a third
-// less through shared memory, the fold is no faster. What it waits for is not settled. The scales come from global memory (some 700
+// What bounds it: power. With operands of random bits the clock falls to 1.42 GHz when the product is repeated (4096 x 36864 x 7168: 1.22 ms,
+// 1770 TFLOP/s; all zeros run at 1.89 GHz, 0.98 ms), so that a cycle less costs clock: a 128 x 256 x 128 block takes 965 cycles, without the fold 880 and
+// 1.07 ms. The tensor core needs 512 of them, copies and products write and read 48 KB of shared memory, 768 at 128 bytes; a bare
+// hand-over of products, fold (376 to 440 cycles of its own) and copies reaches 677. What mattered besides is who polls: threads that wait
+// for a barrier without a suspend time took issue slots from the fold (1030 cycles a block). Sixteen fold warps 1290 us for 1110, scales
+// copied by cp.async behind a barrier of their own 1230, boxes of 128 or 256 weight rows, tensor memory handed back before the last sums are added, and
+// pairs of SMs no faster. The scales come from global memory (some 700
 // cycles away) and are therefore fetched kAhead blocks early. With 128-wide tiles, four fold warps and the scales loaded where they are
 // used the product above was 2.0 ms. 4096 x 18432 x 7168 gated + 4096 x 7168 x 18432 with their quantisers (one dense feed-forward):
 // 3.16 -> 2.0 ms.
