@@ -31,6 +31,10 @@ struct GemvParams {
   const __nv_bfloat16* bias;
   int64_t lda, ldw, ldc;
   int N, K, units;
+  // NORM: the rows of A are rmsnorm(a + residual) * norm_w; the sums go to residual_out ([M, K], as residual)
+  const __nv_bfloat16 *residual, *norm_w;
+  __nv_bfloat16* residual_out;
+  float eps;
 };
 
 __device__ __forceinline__ uint4 ldg_stream(const __nv_bfloat16* p) {
@@ -54,7 +58,9 @@ static constexpr int64_t kMostOneRow = 560 * 1024, kMostTwoRows = 140 * 1024;
 
 // MT: rows of A; R weight rows per warp, U 16-byte loads per lane and row at a time.
 // ACT 0: plain (+ bias); 1: silu(gate) * up; 2: tanh gelu. Gated weights are interleaved per 128 rows (128 gate, 128 up), R = 2.
-template <int MT, int R, int U, int ACT>
+// NORM: every block forms the normed rows for itself (6 KB of reads at K = 1024), so that a decoding layer's norms are no launches of their
+// own: decode step of one sequence, 8 layers of the 0.6B shape, 282 -> 270 us (sixteen launches of 1.8 less, the products 0.2 longer).
+template <int MT, int R, int U, int ACT, bool NORM>
 __global__ void __launch_bounds__(128) gemv_kernel(const GemvParams p) {
   extern __shared__ __align__(16) uint8_t gemv_smem[];
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(gemv_smem);      // [MT][K]
@@ -78,9 +84,53 @@ __global__ void __launch_bounds__(128) gemv_kernel(const GemvParams p) {
   int u = wid, c = 0;
   if (u < p.units) load(u, 0, cur);
   griddep_wait();
-  for (int i = threadIdx.x; i < MT * (p.K / 8); i += 128) {
-    const int m = i / (p.K / 8), k = (i - m * (p.K / 8)) * 8;
-    *reinterpret_cast<uint4*>(xs + m * p.K + k) = __ldcg(reinterpret_cast<const uint4*>(p.a + m * p.lda + k));
+  if constexpr (NORM) {
+    __shared__ float red[MT][4];
+    float ss[MT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      ss[m] = 0.f;
+      for (int k = threadIdx.x * 8; k < p.K; k += 128 * 8) {
+        const uint4 a = __ldcg(reinterpret_cast<const uint4*>(p.a + m * p.lda + k));
+        const uint4 b = __ldcg(reinterpret_cast<const uint4*>(p.residual + static_cast<size_t>(m) * p.K + k));
+        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 x = unpack_bf16(aw[e]), y = unpack_bf16(bw[e]);
+          o[e] = pack_bf16(x.x + y.x, x.y + y.y);
+          const float2 z = unpack_bf16(o[e]);              // the norm is of the rounded sum
+          ss[m] += z.x * z.x + z.y * z.y;
+        }
+        const uint4 v = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4*>(xs + m * p.K + k) = v;
+        if (blockIdx.x == 0) *reinterpret_cast<uint4*>(p.residual_out + static_cast<size_t>(m) * p.K + k) = v;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss[m] += __shfl_xor_sync(0xffffffffu, ss[m], o);
+      if (lane == 0) red[m][threadIdx.x >> 5] = ss[m];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      const float inv = rsqrtf((red[m][0] + red[m][1] + red[m][2] + red[m][3]) / static_cast<float>(p.K) + p.eps);
+      for (int k = threadIdx.x * 8; k < p.K; k += 128 * 8) {          // this thread's own values
+        const uint4 v = *reinterpret_cast<const uint4*>(xs + m * p.K + k), g = *reinterpret_cast<const uint4*>(p.norm_w + k);
+        const uint32_t vw[4] = {v.x, v.y, v.z, v.w}, gw[4] = {g.x, g.y, g.z, g.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 x = unpack_bf16(vw[e]), y = unpack_bf16(gw[e]);
+          o[e] = pack_bf16(x.x * inv * y.x, x.y * inv * y.y);
+        }
+        *reinterpret_cast<uint4*>(xs + m * p.K + k) = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+    }
+  } else {
+    for (int i = threadIdx.x; i < MT * (p.K / 8); i += 128) {
+      const int m = i / (p.K / 8), k = (i - m * (p.K / 8)) * 8;
+      *reinterpret_cast<uint4*>(xs + m * p.K + k) = __ldcg(reinterpret_cast<const uint4*>(p.a + m * p.lda + k));
+    }
   }
   __syncthreads();
   uint64_t acc[R][MT];
@@ -146,32 +196,33 @@ __global__ void __launch_bounds__(128) gemv_kernel(const GemvParams p) {
   }
 }
 
-template <int MT, int R, int U, int ACT>
+template <int MT, int R, int U, int ACT, bool NORM>
 static int launch_gemv(GemvParams p, cudaStream_t st) {
   p.units = ACT != 0 ? p.N / 2 : (p.N + R - 1) / R;
   const int want = (p.units + 3) / 4, sms = num_sms(), grid = want < 4 * sms ? want : 4 * sms;
   // what the busiest SM streams: whole rounds of its warps, the last one included
   const int64_t rounds = (p.units + 4 * grid - 1) / (4 * grid), warps = (grid + sms - 1) / sms * 4;
   if (rounds * warps * R * p.K * 2 > (MT == 1 ? kMostOneRow : kMostTwoRows)) return -1;
-  CUDA_CHECK_RET(launch_pdl(gemv_kernel<MT, R, U, ACT>, dim3(grid), dim3(128), MT * p.K * 2, st, p));
+  CUDA_CHECK_RET(launch_pdl(gemv_kernel<MT, R, U, ACT, NORM>, dim3(grid), dim3(128), MT * p.K * 2, st, p));
   return 0;
 }
 
-template <int MT>
+template <int MT, bool NORM>
 static int launch_gemv_rows(const GemvParams& p, int act, cudaStream_t st) {
-  if (act == 1) return launch_gemv<MT, 2, 4, 1>(p, st);
-  if (act == 2) return launch_gemv<MT, 2, 4, 2>(p, st);
+  if (act == 1) return launch_gemv<MT, 2, 4, 1, NORM>(p, st);
+  if (act == 2) return launch_gemv<MT, 2, 4, 2, NORM>(p, st);
   // two short rows at a time share the reads of A; one row at a time while two would leave SMs without work
-  if (p.K <= 1024 && p.N >= 4096) return launch_gemv<MT, 2, 4, 0>(p, st);
-  return launch_gemv<MT, 1, 8, 0>(p, st);
+  if (p.K <= 1024 && p.N >= 4096) return launch_gemv<MT, 2, 4, 0, NORM>(p, st);
+  return launch_gemv<MT, 1, 8, 0, NORM>(p, st);
 }
 
-// Called by gllm_gemm_smallm. Returns -1 for what this kernel does not take.
-int gemv_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int M, int N, int K, const void* bias,
-              int act, cudaStream_t st) {
-  if (M > 2 || K <= 0 || (act != 0 && N % 256 != 0)) return -1;
-  if (((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) != 0) return -1;
-  if (M * K * 2 > 48 * 1024) return -1;                // the rows of A in shared memory
+static bool gemv_takes(const void* A, const void* W, int M, int N, int K, int act) {
+  return M <= 2 && K > 0 && (act == 0 || N % 256 == 0) && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0 &&
+         M * K * 2 <= 48 * 1024;                           // the rows of A in shared memory
+}
+
+static GemvParams gemv_params(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int N, int K,
+                              const void* bias) {
   GemvParams p = {};
   p.a = reinterpret_cast<const __nv_bfloat16*>(A);
   p.w = reinterpret_cast<const __nv_bfloat16*>(W);
@@ -179,7 +230,36 @@ int gemv_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, i
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.lda = lda; p.ldw = ldw; p.ldc = ldc;
   p.N = N; p.K = K;
-  return M == 1 ? launch_gemv_rows<1>(p, act, st) : launch_gemv_rows<2>(p, act, st);
+  return p;
+}
+
+// Called by gllm_gemm_smallm. Returns -1 for what this kernel does not take.
+int gemv_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int M, int N, int K, const void* bias,
+              int act, cudaStream_t st) {
+  if (!gemv_takes(A, W, M, N, K, act)) return -1;
+  const GemvParams p = gemv_params(A, lda, W, ldw, C, ldc, N, K, bias);
+  return M == 1 ? launch_gemv_rows<1, false>(p, act, st) : launch_gemv_rows<2, false>(p, act, st);
 }
 
 }  // namespace b200
+
+using namespace b200;
+
+// C[M, N] = (rmsnorm(y + residual) * norm_w) · W[N, K]^T (+ bias, or gated by `act` as in gllm_gemm_smallm); residual_out = y + residual.
+// residual, residual_out [M, K] contiguous and not the same. Returns 2 for what the kernel of one or two rows does not take.
+GLLM_EXPORT int gllm_norm_gemv(const void* y, int64_t ldy, const void* residual, void* residual_out, const void* norm_w, float eps,
+                               const void* W, int64_t ldw, void* C, int64_t ldc, int M, int N, int K, const void* bias, int act,
+                               void* stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K % 8 != 0 || ldy % 8 != 0 || ldw % 8 != 0 || !gemv_takes(y, W, M, N, K, act) ||
+      ((reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(residual_out) | reinterpret_cast<uintptr_t>(norm_w)) & 15) != 0)
+    return 2;
+  GemvParams p = gemv_params(y, ldy, W, ldw, C, ldc, N, K, bias);
+  p.residual = reinterpret_cast<const __nv_bfloat16*>(residual);
+  p.residual_out = reinterpret_cast<__nv_bfloat16*>(residual_out);
+  p.norm_w = reinterpret_cast<const __nv_bfloat16*>(norm_w);
+  p.eps = eps;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const int rc = M == 1 ? launch_gemv_rows<1, true>(p, act, st) : launch_gemv_rows<2, true>(p, act, st);
+  return rc < 0 ? 2 : rc;
+}

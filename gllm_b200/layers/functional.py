@@ -42,6 +42,32 @@ def linear_silu_mul(x, w_interleaved, out=None, act="silu"):
     return y if out is None else out.copy_(y)
 
 
+class NormedSum:
+    """rmsnorm(y + residual) * w of one or two rows, formed by the product that reads it (ops.sm100.norm_linear) or, where that
+    kernel does not apply, by the norm's. `residual`, the sum, holds its value once either has run."""
+    __slots__ = ("y", "before", "residual", "w", "eps")
+
+    def __init__(self, y, before, w, eps):
+        self.y, self.before, self.w, self.eps = y, before, w, eps
+        self.residual = torch.empty_like(before)
+
+    @staticmethod
+    def takes(y, residual):
+        return y.is_cuda and y.shape[0] <= 2 and y.dtype == residual.dtype == torch.bfloat16 and y.shape[1] % 8 == 0 and \
+            residual.is_contiguous()
+
+    def tensor(self):
+        return _sm().rmsnorm(self.y, self.w, self.eps, self.before, residual_out=self.residual)[0]
+
+    def linear(self, w, bias=None):
+        out = None if isinstance(w, tuple) else _sm().norm_linear(self.y, self.before, self.residual, self.w, self.eps, w, bias)
+        return linear(self.tensor(), w, bias) if out is None else out
+
+    def linear_silu_mul(self, w):
+        out = None if isinstance(w, tuple) else _sm().norm_linear(self.y, self.before, self.residual, self.w, self.eps, w, act=1)
+        return linear_silu_mul(self.tensor(), w) if out is None else out
+
+
 def rmsnorm_two(x1, w1, x2, w2, eps):
     """(rmsnorm(x1) * w1, rmsnorm(x2) * w2) of two column ranges of the same rows."""
     if x1.is_cuda and all(x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and x.shape[1] % 8 == 0 and x.shape[1] <= 8192

@@ -238,13 +238,15 @@ class DecoderLayer(nn.Module):
             self.mlp = DenseMLP(h, spec.intermediate_size, dt, device, spec=spec)
 
     def forward(self, inp, h: torch.Tensor, residual: torch.Tensor, kv_cache, tpc: TPComm,
-                next_norm_w: Optional[torch.Tensor], qkv: Optional[torch.Tensor] = None):
-        """h = RMSNorm'ed block input, residual = running residual stream.
+                next_norm_w: Optional[torch.Tensor], qkv: Optional[torch.Tensor] = None, defer: bool = False):
+        """h = RMSNorm'ed block input, residual = running residual stream. `defer`: the next block is one like this, so the norm in
+        front of it may be left to its first product.
         Returns (normed input of the next block, residual) — or (un-normed block output, residual)
         when `next_norm_w` is None (last layer of a non-final pipeline stage)."""
         eps = self.spec.rms_eps
         a = self.attn(inp, h, kv_cache, tpc, qkv=qkv)
-        h, residual = tpc.row_linear_add_norm(a, _qw(self.attn.o_w, self.attn.o_ws), residual, self.post_norm_w, eps, self.attn.o_b)
+        h, residual = tpc.row_linear_add_norm(a, _qw(self.attn.o_w, self.attn.o_ws), residual, self.post_norm_w, eps, self.attn.o_b,
+                                              defer=not self.is_moe and self.mlp.fused_act)
         if self.is_moe:
             if next_norm_w is None:
                 return tpc.all_reduce(self.mlp(tpc.materialize(h), tpc)), residual
@@ -252,7 +254,7 @@ class DecoderLayer(nn.Module):
         act = self.mlp.act(h, tpc)
         if next_norm_w is None:
             return tpc.row_linear(act, self.mlp.down_weight()), residual
-        return tpc.row_linear_add_norm(act, self.mlp.down_weight(), residual, next_norm_w, eps)
+        return tpc.row_linear_add_norm(act, self.mlp.down_weight(), residual, next_norm_w, eps, defer=defer)
 
 
 class CausalLM(nn.Module):
@@ -374,7 +376,8 @@ class CausalLM(nn.Module):
             elif i == 0 and qkv0 is not None:
                 h, residual = layer(inp, h, residual, kv_cache, tpc, nxt, qkv=qkv0)
             else:
-                h, residual = layer(inp, h, residual, kv_cache, tpc, nxt)
+                more = {"defer": True} if i + 1 < n and type(layer) is type(self.layers[i + 1]) is DecoderLayer else {}
+                h, residual = layer(inp, h, residual, kv_cache, tpc, nxt, **more)
         if nvtx and n:
             torch.cuda.nvtx.range_pop()
         if not self.is_last:

@@ -57,6 +57,7 @@ def _declare(lib):
     sig("gllm_gemm_bf16_batched", [P, L, L, P, P, L, L, I, I, I, I, P])
     sig("gllm_gemm_smallm", [P, L, P, L, P, L, I, I, I, P, I, I, P, L, P, P])
     sig("gllm_gemm_bf16_cluster", [P, L, P, L, P, L, I, I, I, P, I, I, I, I, I, P])
+    sig("gllm_norm_gemv", [P, L, P, P, P, F, P, L, P, L, I, I, I, P, I, P])
     sig("gllm_rmsnorm", [P, P, P, P, P, I, I, L, F, P])
     sig("gllm_rmsnorm_two", [P, L, P, P, I, P, L, P, P, I, I, F, P])
     sig("gllm_silu_and_mul", [P, P, I, I, L, P])

@@ -164,6 +164,24 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, residual: Optional[tor
     return out, residual_out
 
 
+def norm_linear(y: torch.Tensor, residual: torch.Tensor, residual_out: torch.Tensor, norm_w: torch.Tensor, eps: float,
+                w: torch.Tensor, bias: Optional[torch.Tensor] = None, act: int = 0) -> Optional[torch.Tensor]:
+    """(rmsnorm(y + residual) * norm_w) @ w.T (+ bias; `act` 1: the gated form of `linear_silu_mul`) of one or two rows in one launch,
+    the sum into residual_out; None where the kernel does not take the product."""
+    m, k = y.shape
+    n = w.shape[0]
+    if gemm_forced() or not (m <= 2 and m <= _SMALLM_MAX and y.dtype == w.dtype == _BF16 and y.stride(1) == 1 and w.stride(1) == 1):
+        return None
+    out = torch.empty(m, n // 2 if act else n, dtype=_BF16, device=y.device)
+    rc = _lib.load().gllm_norm_gemv(_p(y), y.stride(0), _p(residual), _p(residual_out), _p(norm_w), float(eps), _p(w), w.stride(0),
+                                    _p(out), out.stride(0), m, n, k, _p(bias), act, stream_ptr())
+    if rc == 2:
+        return None
+    check(rc, "norm_gemv")
+    _count()
+    return out
+
+
 def rmsnorm_two(x1: torch.Tensor, w1: torch.Tensor, x2: torch.Tensor, w2: torch.Tensor, eps: float):
     """(rmsnorm(x1) * w1, rmsnorm(x2) * w2) in one launch: column ranges of the same rows, say. Rows on 16-byte boundaries."""
     t = x1.shape[0]

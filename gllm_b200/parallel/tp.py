@@ -41,18 +41,18 @@ class TPComm:
         return h, x
 
     def materialize(self, h: torch.Tensor) -> torch.Tensor:
-        """Make `h` safe to read by kernels that are not collective-aware (no-op here)."""
-        return h
+        """Make `h` safe to read by kernels that are not collective-aware (here only a deferred norm is anything but a tensor)."""
+        return h.tensor() if isinstance(h, Fn.NormedSum) else h
 
     def stage_exit(self, residual: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
         """Residual stream in the replicated [T, H] form a pipeline stage boundary ships (no-op here)."""
         return residual
 
     def col_linear(self, x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
-        return Fn.linear(x, w, bias)
+        return x.linear(w, bias) if isinstance(x, Fn.NormedSum) else Fn.linear(x, w, bias)
 
     def col_linear_silu_mul(self, x: torch.Tensor, w_interleaved: torch.Tensor) -> torch.Tensor:
-        return Fn.linear_silu_mul(x, w_interleaved)
+        return x.linear_silu_mul(w_interleaved) if isinstance(x, Fn.NormedSum) else Fn.linear_silu_mul(x, w_interleaved)
 
     def all_reduce(self, x: torch.Tensor) -> torch.Tensor:
         return ps.tp_all_reduce(x)
@@ -75,9 +75,13 @@ class TPComm:
         return self.reduce_add_norm(partial, residual, norm_w, eps)
 
     def row_linear_add_norm(self, x: torch.Tensor, w: torch.Tensor, residual: Optional[torch.Tensor],
-                            norm_w: torch.Tensor, eps: float, bias: Optional[torch.Tensor] = None):
+                            norm_w: torch.Tensor, eps: float, bias: Optional[torch.Tensor] = None, defer: bool = False):
+        """`defer`: what comes back first may be a `NormedSum`, for a caller that hands it to this object's methods only."""
         # bias is added once (rank 0) like the reference (gllm/layers/linear.py:230-258)
         partial = Fn.linear(x, w, bias if self.tp_rank == 0 else None)
+        if defer and self.tp_size == 1 and residual is not None and Fn.NormedSum.takes(partial, residual):
+            h = Fn.NormedSum(partial, residual, norm_w, eps)
+            return h, h.residual
         return self.reduce_add_norm(partial, residual, norm_w, eps)
 
     def row_linear(self, x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -1173,6 +1173,41 @@ def test_latent_attention_block_in_one_call(heads, width, q_lens, decodes, monke
 
 
 @pytest.mark.parametrize("m", [1, 2])
+@pytest.mark.parametrize("n,k,act", [(8, 8, 0), (5, 264, 0), (4100, 1024, 0), (640, 6144, 0), (512, 1032, 1), (6144, 1024, 1)])
+def test_norm_with_the_product_behind_it(m, n, k, act):
+    """rmsnorm(y + residual) formed by the one-or-two-row product: the sum bit for bit that of the norm kernel, the product within the
+    roundings of fp32 sums of bf16 products and of normed values that may round to the other neighbour (2^-8 each, not all one way)."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(n + k)
+    y = torch.randn(m, k + 16, device=_dev()).bfloat16()[:, 8:8 + k]
+    res, w = torch.randn(m, k, device=_dev()).bfloat16(), (1 + 0.2 * torch.randn(k, device=_dev())).bfloat16()
+    wt = torch.randn(n, k + 8, device=_dev()).bfloat16()[:, :k] * k ** -0.5
+    b = None if act else torch.randn(n, device=_dev()).bfloat16()
+    out = torch.full_like(res, 7.0)
+    got = sm100.norm_linear(y, res, out, w, 1e-6, wt, b, act)
+    want_res = res.clone()
+    normed, _ = sm100.rmsnorm(y, w, 1e-6, want_res)
+    assert got is not None and torch.equal(out, want_res)
+    want = sm100.linear_silu_mul(normed, wt) if act else sm100.linear(normed, wt, b)
+    assert got.shape == want.shape and _rel_err(got, want) < 6e-3
+
+
+def test_norm_that_no_product_takes():
+    """A deferred norm whose product is too large for the kernel (rows beyond its shared memory) is formed by the norm's own."""
+    from gllm_b200.layers import functional as Fn
+    torch.manual_seed(3)
+    k = 24584
+    y, res = torch.randn(1, k, device=_dev()).bfloat16(), torch.randn(1, k, device=_dev()).bfloat16()
+    w, wt = torch.ones(k, device=_dev()).bfloat16(), torch.randn(64, k, device=_dev()).bfloat16() * k ** -0.5
+    h = Fn.NormedSum(y, res, w, 1e-6)
+    got = h.linear(wt)
+    want_res = res.clone()
+    normed, _ = Fn.rmsnorm(y, w, 1e-6, want_res)
+    assert torch.equal(h.residual, want_res) and torch.equal(got, Fn.linear(normed, wt))
+    assert torch.equal(Fn.NormedSum(y, res, w, 1e-6).tensor(), normed)
+
+
+@pytest.mark.parametrize("m", [1, 2])
 @pytest.mark.parametrize("n,k", [(1, 8), (5, 264), (130, 1024), (4097, 1024), (4100, 2056), (257, 6144), (640, 8192)])
 def test_linear_few_rows(m, n, k):
     """One and two rows: a warp per weight row with the whole of K. Rows and columns beyond the last block, K below one 16-byte
