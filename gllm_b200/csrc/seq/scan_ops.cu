@@ -34,16 +34,6 @@ constexpr int kThreads = 128;
 constexpr int kTile = 16;                           // tokens between two barriers
 constexpr int kAnchor = 4;                          // tiles between two corrections of the states' decay
 
-// ---- pairs of fp32 ----
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 pk(float a, float b) { f2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
-__device__ __forceinline__ void un(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
-__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ float rcp(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-
 // 2^t of both halves on the 2^x unit. Its results lie below 2^t on average: by 0.5e-8 for t in (-0.004, 0), 1.6e-8 to 2.7e-8 in
 // (-0.5, -0.004), 2.5e-8 down to -1, 5e-8 below. That adds up over the tokens between two corrections of a state (`anchored`), so the
 // caller adds kBias = 2.1e-8 / ln 2 to t in the fma that forms it. Outputs of 2048 tokens against float64, decays around exp of

@@ -34,14 +34,15 @@ template <int NT> __device__ __forceinline__ float block_sum(float v, float* scr
   for (int i = 0; i < NT / 32; ++i) t += scratch[i];
   return t;
 }
-// 1 / (1 + e^-v) from the 2^x and 1/x units: __fdividef(1, 1 + __expf(-v)) without the handling of denormals. Within 2^-21 of it, and
-// within |v| 2^-24 + 2^-21 of it relative to the value, for the exponent is rounded to one fp32.
-__device__ __forceinline__ float sigmoid_unit(float v) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * v));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-  return r;
-}
+// ---- pairs of fp32 ----
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk(float a, float b) { f2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b)); return d; }
+__device__ __forceinline__ void un(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ float rcp(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 // sequence that owns batch row t: largest s with qsl[s] <= t
 __device__ __forceinline__ int find_seq(const int* __restrict__ qsl, int nseq, int t) {
   if (t < nseq && qsl[t] <= t && t < qsl[t + 1]) return t;   // single-token sequences lead the batch: row t is theirs

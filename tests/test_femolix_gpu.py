@@ -213,6 +213,31 @@ def test_conv_rows_fetched_ahead(qlens, taps):
     assert close(c1, c2, 1e-2) and torch.equal(st1, st2)
 
 
+@pytest.mark.parametrize("act", ["silu", "none"])
+@pytest.mark.parametrize("taps", [1, 3, 4])
+def test_conv_groups_without_a_border(taps, act):
+    """Groups of four rows that lie inside one sequence go side by side, the others row by row: sequences that end at each place of a
+    group, single tokens between them, the block's last group cut short, an input bias. The sum of at most 5 terms and the sigmoid
+    are fp32: their errors are far below the rounding to bf16 of the result, 2^-8 of it or of its terms where they cancel."""
+    from gllm_b200.ops import ref, sm100_seq as S
+    torch.manual_seed(taps)
+    qlens = [1, 4, 5, 6, 7, 8, 1, 9, 2100, 2, 3, 1, 17]
+    ns, t, C = len(qlens), sum(qlens), 1028
+    ctx = [3 * (i % 2) for i in range(ns)]
+    qsl = torch.tensor([0] + qlens, device=DEV).cumsum(0).to(torch.int32)
+    sl = torch.tensor([c + q for c, q in zip(ctx, qlens)], dtype=torch.int32, device=DEV)
+    rs = torch.randperm(ns + 1, device=DEV)[:ns].to(torch.int32)
+    xz = torch.randn(t, C + 4, device=DEV).bfloat16()
+    w, b, ib = torch.randn(C, taps, device=DEV), torch.randn(C, device=DEV), torch.randn(C, device=DEV)
+    st1 = torch.randn(ns + 1, max(taps - 1, 1), C, device=DEV).bfloat16()
+    st2 = st1.clone()
+    got = S.causal_conv_silu(xz, C, w, b, st1, rs, sl, qsl, act=act, in_bias=ib)
+    want = ref.causal_conv_silu(xz.float(), C, w, b, st2.float(), rs, sl, qsl, act=act, in_bias=ib)
+    ref.causal_conv_silu(xz, C, w, b, st2, rs, sl, qsl, act=act, in_bias=ib)
+    assert torch.equal(st1, st2)
+    assert bool(((got.float() - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -16).all())
+
+
 @pytest.mark.parametrize("C", [5120, 10240])
 @pytest.mark.parametrize("qlens", [[4100], [1, 1, 700, 13, 1500, 18, 1, 1866]])
 def test_conv_rows_beyond_the_ring(C, qlens):
