@@ -19,16 +19,22 @@ using namespace seqk;
 
 __device__ __forceinline__ float sigmoid_f(float v) { return 1.0f / (1.0f + expf(-v)); }
 __device__ __forceinline__ float silu_f(float v) { return v / (1.0f + expf(-v)); }
-// sigmoid_f from the 2^x and 1/x units, within 2^-21 of it relative to the value: e = 2^(-|v| log2 e) with the exponent in two parts
-// (rounded to one it would cost |v| 2^-24), then 1 / (1 + e) or e / (1 + e). Denormals of e are kept.
-__device__ __forceinline__ float sigmoid_parts(float v) {
-  const float m = fabsf(v) > 200.f ? 200.f : fabsf(v);                     // finite, or NaN
-  const float t = m * 1.4426950216293335f, rest = fmaf(m, -1.925963033500011e-8f, fmaf(m, -1.4426950216293335f, t));
-  float e, r;
-  asm("ex2.approx.f32 %0, %1;" : "=f"(e) : "f"(-t));
-  e = fmaf(e, 0.6931472f * rest, e);
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-  return v < 0.f ? e * r : r;
+// sigmoid_f of both halves from the 2^x and 1/x units, within 2^-21 of it relative to the value: e = 2^(-|v| log2 e) with the exponent
+// in two parts (rounded to one it would cost |v| 2^-24), then 1 / (1 + e) or e / (1 + e). Denormals of e are kept.
+__device__ __forceinline__ f2 sigmoid_parts2(float v0, float v1) {
+  const float m0 = fabsf(v0), m1 = fabsf(v1);
+  const f2 m = pk(m0 > 200.f ? 200.f : m0, m1 > 200.f ? 200.f : m1);        // finite, or NaN
+  const f2 t = mul2(m, pk(-1.4426950216293335f, -1.4426950216293335f));
+  const f2 rest = fma2(m, pk(-1.925963033500011e-8f, -1.925963033500011e-8f), fma2(m, pk(-1.4426950216293335f, -1.4426950216293335f), t ^ 0x8000000080000000ull));
+  float t0, t1, e0, e1;
+  un(t, t0, t1);
+  asm("ex2.approx.f32 %0, %1;" : "=f"(e0) : "f"(t0));
+  asm("ex2.approx.f32 %0, %1;" : "=f"(e1) : "f"(t1));
+  f2 e = pk(e0, e1);
+  e = fma2(e, mul2(rest, pk(0.6931472f, 0.6931472f)), e);
+  un(e, e0, e1);
+  un(add2(e, pk(1.f, 1.f)), t0, t1);
+  return mul2(pk(v0 < 0.f ? e0 : 1.f, v1 < 0.f ? e1 : 1.f), pk(rcp(t0), rcp(t1)));
 }
 
 // x <- rms(alpha * x + y) * w (fp32 stream, in place); out = the same row in the compute dtype (optional)
@@ -450,7 +456,9 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ o, int n, cons
 
 // The same for bf16 rows whose groups are 128 or 256 wide and lie on 8-byte boundaries (o: 16): 16- and 8-byte accesses, and a
 // warp has the loads of 4 x 128 columns in flight, where 4-byte loads of one group at a time were bound by their latency.
-// 6000 tokens x 32 groups of 128: 97 -> 61 us, with the gate from the 2^x and 1/x units instead of expf and a division 51. Where the
+// 6000 tokens x 32 groups of 128: 97 -> 61 us, with the gate from the 2^x and 1/x units instead of expf and a division 51. What bounds
+// it then is the issue slots (73 % of the cycles): two columns to an instruction, and one tree of sums and one root for the warp's
+// four groups, 53 -> 43 (3.4 TB/s; 8192 tokens 70 -> 54; groups of 256, 8192 tokens: 61 -> 54). Where the
 // groups do not fill the machine, four in a row only make a warp slower (one token, 32 groups of 128: 3.2 us element-wise, 4.1 with
 // four): one group per warp there.
 template <int NCH, int kRows>
@@ -479,27 +487,49 @@ __global__ void __launch_bounds__(128) gated_group_norm_vec_kernel(
       }
     }
   }
+  float ss[kRows];
 #pragma unroll
   for (int i = 0; i < kRows; ++i) {
-    if (i >= count) break;
-    float ss = 0.f;
+    ss[i] = 0.f;
+    if (i < count)
 #pragma unroll
-    for (int c = 0; c < NCH; ++c)
-      ss += v[i][c].x * v[i][c].x + v[i][c].y * v[i][c].y + v[i][c].z * v[i][c].z + v[i][c].w * v[i][c].w;
-    ss = warp_sum(ss);
-    const float r = 1.0f / sqrtf(ss / (float)kGroup + eps);
+      for (int c = 0; c < NCH; ++c)
+        ss[i] += v[i][c].x * v[i][c].x + v[i][c].y * v[i][c].y + v[i][c].z * v[i][c].z + v[i][c].w * v[i][c].w;
+  }
+  // the groups' sums in one tree: at each of its first steps half the lanes hand over half of the groups they hold, so that a
+  // lane ends with one group's sum (of the same pairs as warp_sum's) and the root and the division are formed once
+#pragma unroll
+  for (int h = kRows / 2, bit = 16; h > 0; h >>= 1, bit >>= 1)
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const bool up = lane & bit;
+      const float give = up ? ss[i] : ss[i + h];
+      ss[i] = (up ? ss[i + h] : ss[i]) + __shfl_xor_sync(0xffffffffu, give, bit);
+    }
+#pragma unroll
+  for (int bit = 16 / kRows; bit > 0; bit >>= 1) ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], bit);
+  const float rr = 1.0f / sqrtf(ss[0] / (float)kGroup + eps);
+  const f2 scale = pk(out_scale, out_scale);
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    const float ri = __shfl_sync(0xffffffffu, rr, i * (32 / kRows));       // where group i's sum is
+    if (i >= count) continue;
+    const f2 r = pk(ri, ri);
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
-      const float2 g01 = b200::unpack_bf16(gt[i][c].x), g23 = b200::unpack_bf16(gt[i][c].y);
-      const uint2 wr = *reinterpret_cast<const uint2*>(w + (col[i] + c * 128) % wlen);
-      const float2 w01 = b200::unpack_bf16(wr.x), w23 = b200::unpack_bf16(wr.y);
-      auto one = [&](float x, float wt, float g) {
-        const float sg = sigmoid_parts(g);
-        return x * r * wt * (act ? sg : g * sg) * out_scale;
+      const int k = col[i] + c * 128, wc = wlen == kGroup ? lane * 4 + c * 128 : wlen == n ? k : k % wlen;
+      const uint2 wr = *reinterpret_cast<const uint2*>(w + wc);
+      auto two = [&](float x0, float x1, uint32_t wt, uint32_t g) {
+        const float g0 = __uint_as_float(g << 16), g1 = __uint_as_float(g & 0xffff0000u);
+        f2 sg = sigmoid_parts2(g0, g1);
+        if (!act) sg = mul2(pk(g0, g1), sg);
+        const f2 xw = mul2(mul2(pk(x0, x1), r), pk(__uint_as_float(wt << 16), __uint_as_float(wt & 0xffff0000u)));
+        float y0, y1;
+        un(mul2(mul2(xw, sg), scale), y0, y1);
+        return b200::pack_bf16(y0, y1);
       };
-      *reinterpret_cast<uint2*>(out + (size_t)tok[i] * ldo + col[i] + c * 128) =
-          make_uint2(b200::pack_bf16(one(v[i][c].x, w01.x, g01.x), one(v[i][c].y, w01.y, g01.y)),
-                     b200::pack_bf16(one(v[i][c].z, w23.x, g23.x), one(v[i][c].w, w23.y, g23.y)));
+      *reinterpret_cast<uint2*>(out + (size_t)tok[i] * ldo + k) =
+          make_uint2(two(v[i][c].x, v[i][c].y, wr.x, gt[i][c].x), two(v[i][c].z, v[i][c].w, wr.y, gt[i][c].y));
     }
   }
 }

@@ -171,6 +171,23 @@ def test_gated_group_norm_wide_rows(group, ngroups, ntok, pad, act):
         assert out[:, n:].abs().sum().item() == 0
 
 
+@pytest.mark.parametrize("group,ngroups,ntok", [(128, 3, 7001), (256, 3, 5001), (128, 8, 3000)])
+def test_gated_group_norm_groups_of_a_warp(group, ngroups, ntok):
+    """As many groups as a warp takes four (two of 256) at a time, the last warp with fewer, groups of very different size so that one's
+    root cannot stand for another's; weights of a group, of a row, and of a length that neither is. One bf16 rounding."""
+    from gllm_b200.ops import ref, sm100_seq as S
+    torch.manual_seed(ntok)
+    n = group * ngroups
+    o = (torch.randn(ntok, ngroups, group, device=DEV) * torch.exp(torch.randn(ntok, ngroups, 1, device=DEV) * 3)).view(ntok, n)
+    gate = torch.randn(ntok, n, device=DEV).bfloat16()
+    out = torch.empty(ntok, n, device=DEV).bfloat16()
+    for w in (torch.randn(group, device=DEV).bfloat16(), torch.randn(n, device=DEV).bfloat16(), torch.randn(64, device=DEV).bfloat16()):
+        got = S.gated_group_norm(o, gate, w, group, 1e-5, "silu", 1.0, out)
+        full = w.float().repeat(n // w.shape[0])
+        want = ref.gated_group_norm(o, gate.float(), full, group, 1e-5, "silu", 1.0, None, torch.float32)
+        assert bool(((got.float() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-6).all())
+
+
 @pytest.mark.parametrize("act", ["silu", "sigmoid"])
 def test_gated_group_norm_gates_one_by_one(act):
     """Unit rows (norm exactly 1) and gates from -100 to 100: the product before the bf16 rounding is within 2^-20 of float64 at any
