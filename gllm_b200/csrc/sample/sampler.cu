@@ -16,6 +16,7 @@
 namespace b200 {
 
 static constexpr int kSampleThreads = 1024;
+static constexpr int kSampleParts = 8;       // CTAs that may share a row
 
 __device__ __forceinline__ uint32_t f2key(float f) {
   // order-preserving map float -> uint32 (larger float => larger key)
@@ -127,9 +128,10 @@ struct GlobalRow {
   }
   __device__ __forceinline__ int token(int i) const { return i + vocab_offset; }
 
-  // This thread's largest value and its first index, over elements spread across the block. Bound by the latency of one block's
-  // loads: 16 bytes each and four in flight on aligned rows (151,936 bf16 logits: 38 -> 9 us against one element at a time).
-  __device__ __forceinline__ void argmax(int V, float& vmax, int& imax) const {
+  // This thread's largest value and its first index, over elements spread across the block, part `part` of `parts` equal ones of
+  // the row. Bound by the latency of one block's loads: 16 bytes each and four in flight on aligned rows (151,936 bf16 logits:
+  // 38 -> 9 us against one element at a time).
+  __device__ __forceinline__ void argmax(int V, int part, int parts, float& vmax, int& imax) const {
     constexpr int kVec = 16 / static_cast<int>(sizeof(T)), kUnroll = 4;
     vmax = -INFINITY;
     imax = 0x7fffffff;
@@ -138,9 +140,11 @@ struct GlobalRow {
     };
     int done = 0;
     if ((reinterpret_cast<uintptr_t>(lr) & 15) == 0) {
-      const int chunks = V / kVec, step = blockDim.x;
-      done = chunks * kVec;
-      for (int c0 = threadIdx.x; c0 < chunks; c0 += kUnroll * step) {
+      const int all = V / kVec, step = blockDim.x;
+      const int first = static_cast<int>(static_cast<int64_t>(all) * part / parts);
+      const int chunks = static_cast<int>(static_cast<int64_t>(all) * (part + 1) / parts);
+      done = all * kVec;
+      for (int c0 = first + threadIdx.x; c0 < chunks; c0 += kUnroll * step) {
         uint4 raw[kUnroll];
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u)
@@ -157,7 +161,7 @@ struct GlobalRow {
         }
       }
     }
-    for (int i = done + threadIdx.x; i < V; i += blockDim.x) take(val(i), i);
+    for (int i = done + part * blockDim.x + threadIdx.x; i < V; i += parts * blockDim.x) take(val(i), i);
   }
 };
 
@@ -272,15 +276,19 @@ __device__ __forceinline__ void select_and_draw(const Row& R, int V, int k, floa
   tok_out = besti;
 }
 
+// `parts` CTAs, a cluster, share a row's argmax pass: each hands its winner to the first, which goes on alone.
 template <typename T>
 __global__ void __launch_bounds__(kSampleThreads)
-sample_kernel(const T* __restrict__ logits, int64_t ld, int V, const float* __restrict__ temperature,
+sample_kernel(int parts, const T* __restrict__ logits, int64_t ld, int V, const float* __restrict__ temperature,
               const int32_t* __restrict__ top_k, const float* __restrict__ top_p,
               const float* __restrict__ rep_penalty, const uint32_t* __restrict__ seen, int seen_words,
               const int32_t* __restrict__ slot_idx, uint64_t seed, const int64_t* __restrict__ step_ptr, int32_t* __restrict__ out_tokens,
               float* __restrict__ out_max, int vocab_offset) {
   __shared__ BlockScratch S;
-  const int row = blockIdx.x;
+  __shared__ uint2 winners[kSampleParts];         // of the cluster's CTAs, in the first one's memory
+  const int row = blockIdx.x / parts, part = blockIdx.x % parts;
+  if (parts > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  griddep_wait();
   const uint32_t* seen_row =
       seen != nullptr ? seen + static_cast<size_t>(slot_idx != nullptr ? slot_idx[row] : row) * seen_words : nullptr;
   const float temp = temperature != nullptr ? temperature[row] : 1.0f;
@@ -297,8 +305,22 @@ sample_kernel(const T* __restrict__ logits, int64_t ld, int V, const float* __re
   // ---- pass A: max / argmax ----
   float vmax;
   int imax;
-  R.argmax(V, vmax, imax);
+  R.argmax(V, part, parts, vmax, imax);
   block_argmax(vmax, imax, S);
+  if (parts > 1) {
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");            // every CTA of the cluster has begun: its memory is there
+    if (threadIdx.x == 0)
+      asm volatile("st.shared::cluster.v2.b32 [%0], {%1, %2};" ::"r"(cluster_addr(&winners[part], 0)), "r"(__float_as_uint(vmax)),
+                   "r"(imax) : "memory");
+    cluster_sync();
+    if (part != 0) return;
+    for (int i = 0; i < parts; ++i) {
+      const uint2 w = winners[i];
+      const float ov = __uint_as_float(w.x);
+      const int oi = static_cast<int>(w.y);
+      if (i == 0 || ov > vmax || (ov == vmax && oi < imax)) { vmax = ov; imax = oi; }
+    }
+  }
   if (k == 1) {
     if (threadIdx.x == 0) {
       out_tokens[row] = imax + vocab_offset;
@@ -367,7 +389,7 @@ vp_candidates_kernel(const T* __restrict__ logits, int64_t ld, int V, int V_full
   }
   float vmax;
   int imax;
-  R.argmax(V, vmax, imax);
+  R.argmax(V, 0, 1, vmax, imax);
   block_argmax(vmax, imax, S);
   const float m = vmax;
   float z = 0.f;
@@ -504,23 +526,25 @@ GLLM_EXPORT int gllm_sample(const void* logits, int dtype, int64_t ld, void* out
                             const void* step_ptr, void* out_max, int vocab_offset, void* stream) {
   if (B <= 0) return 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (dtype == 0) {
-    sample_kernel<__nv_bfloat16><<<B, kSampleThreads, 0, st>>>(
-        reinterpret_cast<const __nv_bfloat16*>(logits), ld, V, reinterpret_cast<const float*>(temperature),
-        reinterpret_cast<const int32_t*>(top_k), reinterpret_cast<const float*>(top_p),
-        reinterpret_cast<const float*>(rep_penalty), reinterpret_cast<const uint32_t*>(seen), seen_words,
-        reinterpret_cast<const int32_t*>(slot_idx), seed,
-        reinterpret_cast<const int64_t*>(step_ptr), reinterpret_cast<int32_t*>(out_tokens),
-        reinterpret_cast<float*>(out_max), vocab_offset);
-  } else {
-    sample_kernel<float><<<B, kSampleThreads, 0, st>>>(
-        reinterpret_cast<const float*>(logits), ld, V, reinterpret_cast<const float*>(temperature),
-        reinterpret_cast<const int32_t*>(top_k), reinterpret_cast<const float*>(top_p),
-        reinterpret_cast<const float*>(rep_penalty), reinterpret_cast<const uint32_t*>(seen), seen_words,
-        reinterpret_cast<const int32_t*>(slot_idx), seed,
-        reinterpret_cast<const int64_t*>(step_ptr), reinterpret_cast<int32_t*>(out_tokens),
-        reinterpret_cast<float*>(out_max), vocab_offset);
-  }
+  // CTAs of a row: up to eight, as long as all clusters run at once (a cluster lies inside a processing cluster of the chip, which
+  // leaves some SMs over: 16 clusters of eight and 37 of four took two rounds, 8.1 and 9.6 us for 151,936 bf16 logits against 9.0 and
+  // 9.2 with one CTA a row; 17 and 32 of four 5.3 and 5.5, 64 of two 7.3), and for rows so long that the pass costs more than the
+  // cluster's two barriers. One row, one CTA / eight, bf16: 32,000 logits 3.6 / 3.8 us, 50,000 4.6 / 3.9, 151,936 8.8 / 4.4; fp32:
+  // 4.4 / 3.8, 5.8 / 4.0, 11.2 / 4.9.
+  int parts = 1;
+  while (static_cast<int64_t>(V) * (dtype == 0 ? 2 : 4) >= 98304 && parts < kSampleParts &&
+         (static_cast<int64_t>(B) + 5) * parts * 2 <= num_sms())
+    parts *= 2;
+  auto run = [&](auto* row0) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(row0)>>;
+    return launch_pdl_cluster(sample_kernel<T>, dim3(B * parts), parts, dim3(kSampleThreads), 0, st, parts, row0, ld, V,
+                              reinterpret_cast<const float*>(temperature), reinterpret_cast<const int32_t*>(top_k),
+                              reinterpret_cast<const float*>(top_p), reinterpret_cast<const float*>(rep_penalty),
+                              reinterpret_cast<const uint32_t*>(seen), seen_words, reinterpret_cast<const int32_t*>(slot_idx), seed,
+                              reinterpret_cast<const int64_t*>(step_ptr), reinterpret_cast<int32_t*>(out_tokens),
+                              reinterpret_cast<float*>(out_max), vocab_offset);
+  };
+  CUDA_CHECK_RET(dtype == 0 ? run(reinterpret_cast<const __nv_bfloat16*>(logits)) : run(reinterpret_cast<const float*>(logits)));
   CUDA_CHECK_RET(cudaGetLastError());
   return 0;
 }

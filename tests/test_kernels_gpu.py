@@ -487,6 +487,31 @@ def test_sampler_greedy_edges(v, dt):
     assert sm100.sample(z, rep_penalty=pen, seen_bits=seen).tolist() == [int((r == r.max()).nonzero()[0, 0]) for r in want]
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("b,v", [(1, 24575), (1, 24576), (3, 49159), (13, 50001), (14, 50000), (32, 49152), (33, 49156), (69, 49152), (70, 49151)])
+def test_sampler_rows_shared_by_a_cluster(b, v, dt):
+    """Rows whose argmax pass eight, four, two CTAs or one share: ties within and across their parts, an unaligned row, rows that draw
+    beside greedy ones, whose tokens do not depend on how many CTAs share the row."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(b + v)
+    base = torch.randn(b, v + 3, device=_dev()).to(dt)
+    for off in (0, 3):
+        z = base[:, off:off + v]
+        z[0] = z[0].clamp(max=z[0].float().quantile(0.999).item())             # some ties, in all parts
+        z[b - 1, v - 1] = 9.0                                                  # the row's end
+        top = torch.empty(b, device=_dev())
+        want = [int((r == r.max()).nonzero()[0, 0]) for r in z]
+        assert sm100.sample(z, out_max=top).tolist() == want
+        assert torch.equal(top, z.float().amax(-1))
+    k = torch.tensor([1 if i % 2 else 40 for i in range(b)], dtype=torch.int32, device=_dev())
+    temp, p = torch.full((b,), 0.7, device=_dev()), torch.full((b,), 0.9, device=_dev())
+    got = sm100.sample(z, temp, k, p, seed=11).tolist()
+    many = torch.cat([z, z.new_zeros(150, v)])                                 # one CTA to a row
+    pad = lambda t, fill: torch.cat([t, torch.full((150,), fill, dtype=t.dtype, device=_dev())])
+    assert sm100.sample(many, pad(temp, 1.0), pad(k, 1), pad(p, 1.0), seed=11).tolist()[:b] == got
+    assert all(got[i] == want[i] for i in range(1, b, 2))
+
+
 def test_sampler_distribution():
     from gllm_b200.ops import sm100
     torch.manual_seed(7)
