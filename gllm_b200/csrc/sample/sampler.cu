@@ -312,6 +312,7 @@ sample_kernel(int parts, const T* __restrict__ logits, int64_t ld, int V, const 
     if (threadIdx.x == 0)
       asm volatile("st.shared::cluster.v2.b32 [%0], {%1, %2};" ::"r"(cluster_addr(&winners[part], 0)), "r"(__float_as_uint(vmax)),
                    "r"(imax) : "memory");
+    __syncwarp();
     cluster_sync();
     if (part != 0) return;
     for (int i = 0; i < parts; ++i) {
