@@ -3,7 +3,7 @@
 // The reference does this with ~15 PyTorch ops including a full-vocabulary sort
 // (gllm/layers/sampler.py:8-54). Here one CTA per sequence makes a handful of passes over its
 // logits row (L2-resident) and never sorts:
-//   pass A : transformed logit t(x) = penalty(x) / temperature, row max m, Z = sum exp(t - m)
+//   pass A : transformed logit t(x) = penalty(x) / temperature, row max m (few long rows: by a cluster), Z = sum exp(t - m)
 //   top-k  : 4-pass MSB radix select on the order-preserving integer key of t  -> threshold key
 //   top-p  : 4-pass radix select on probability mass among the top-k survivors -> threshold key
 //   draw   : exponential race  argmax_i  exp(t_i - m) / E_i ,  E_i ~ Exp(1)   (== Gumbel-max,
