@@ -68,7 +68,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // 1268 -> 1222 us at the power limit).
 static constexpr uint32_t kSuspendNs = 100000;
 
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity, uint32_t suspend_ns = kSuspendNs) {
   uint32_t ok;
   asm volatile(
       "{\n\t"
@@ -77,7 +77,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       "selp.u32 %0, 1, 0, P;\n\t"
       "}\n"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendNs)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(suspend_ns)
       : "memory");
   return ok != 0;
 }

@@ -395,8 +395,8 @@ def test_wait_that_gives_up_reaches_the_caller(family):
 
 @pytest.mark.parametrize("m,n,k", [(600, 6144, 64), (600, 6144, 1024), (4200, 4104, 4096)])
 def test_gemm_on_pairs_that_gives_up_ends_soon(m, n, k):
-    """Limits of nothing and of 2 us: the two CTAs of a pair give up at different stages, and still no copy is waited for that was
-    never issued (two seconds each)."""
+    """Limits of nothing, 1 ns and 2 us: the two CTAs of a pair give up at different stages, and still no copy is waited for that was
+    never issued (two seconds each). The sums of 64 K blocks are waited for longer than that."""
     import time
     from gllm_b200.ops import lib, sm100
     torch.manual_seed(k)
@@ -404,14 +404,14 @@ def test_gemm_on_pairs_that_gives_up_ends_soon(m, n, k):
     want = sm100.linear(x, w)
     torch.cuda.synchronize()
     try:
-        for limit in (0, 2000):
+        for limit in (0, 1, 2000):
             lib.watch_waits(limit_ns=limit)
             for _ in range(5):
                 t0 = time.monotonic()
                 sm100.linear(x, w)
                 torch.cuda.synchronize()
                 assert time.monotonic() - t0 < 0.5, limit
-            assert limit or lib.waits_gave_up()
+            assert lib.waits_gave_up(clear=True) or (limit == 2000 and k < 4096), limit
     finally:
         lib.watch_waits()
         lib.waits_gave_up(clear=True)
@@ -420,7 +420,8 @@ def test_gemm_on_pairs_that_gives_up_ends_soon(m, n, k):
 
 def test_wait_limit_does_not_count_the_kernel_before():
     """A GEMM on pairs of SMs starts while ten CTAs of the kernel before it still have a long product to sum up: what it waits for
-    there is not a wait of its own."""
+    there is not a wait of its own. A wait ends within a suspension (as long as the limit here) of its limit, so the kernel before has to
+    take longer than twice the limit."""
     from gllm_b200.ops import lib, sm100
     torch.manual_seed(1)
     x0, w0 = torch.randn(600, 1 << 17, device=_dev()).bfloat16(), torch.randn(256, 1 << 17, device=_dev()).bfloat16()
@@ -428,6 +429,10 @@ def test_wait_limit_does_not_count_the_kernel_before():
     want = x.float() @ w.float().t()
     sm100.linear(x0, w0), sm100.linear(x, w)
     assert sm100.waits_given_up() == 0
+    start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    start.record(), sm100.linear(x0, w0), end.record()
+    torch.cuda.synchronize()
+    assert start.elapsed_time(end) > 0.3
     try:
         lib.watch_waits(limit_ns=100_000)
         for _ in range(3):
