@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(128) gemv_kernel(const GemvParams p) {
   if (u < p.units) load(u, 0, cur);
   griddep_wait();
   if constexpr (NORM) {
-    __shared__ float red[MT][4];
+    __shared__ float red[MT][4];                           // counted by gemv_takes
     float ss[MT];
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
@@ -216,9 +216,9 @@ static int launch_gemv_rows(const GemvParams& p, int act, cudaStream_t st) {
   return launch_gemv<MT, 1, 8, 0, NORM>(p, st);
 }
 
-static bool gemv_takes(const void* A, const void* W, int M, int N, int K, int act) {
+static bool gemv_takes(const void* A, const void* W, int M, int N, int K, int act, bool norm) {
   return M <= 2 && K > 0 && (act == 0 || N % 256 == 0) && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0 &&
-         M * K * 2 <= 48 * 1024;                           // the rows of A in shared memory
+         M * K * 2 + (norm ? M * 16 : 0) <= 48 * 1024;     // shared memory: the rows of A and, normed, the warps' sums
 }
 
 static GemvParams gemv_params(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int N, int K,
@@ -236,7 +236,7 @@ static GemvParams gemv_params(const void* A, int64_t lda, const void* W, int64_t
 // Called by gllm_gemm_smallm. Returns -1 for what this kernel does not take.
 int gemv_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int M, int N, int K, const void* bias,
               int act, cudaStream_t st) {
-  if (!gemv_takes(A, W, M, N, K, act)) return -1;
+  if (!gemv_takes(A, W, M, N, K, act, false)) return -1;
   const GemvParams p = gemv_params(A, lda, W, ldw, C, ldc, N, K, bias);
   return M == 1 ? launch_gemv_rows<1, false>(p, act, st) : launch_gemv_rows<2, false>(p, act, st);
 }
@@ -251,7 +251,7 @@ GLLM_EXPORT int gllm_norm_gemv(const void* y, int64_t ldy, const void* residual,
                                const void* W, int64_t ldw, void* C, int64_t ldc, int M, int N, int K, const void* bias, int act,
                                void* stream) {
   if (M <= 0 || N <= 0) return 0;
-  if (K % 8 != 0 || ldy % 8 != 0 || ldw % 8 != 0 || !gemv_takes(y, W, M, N, K, act) ||
+  if (K % 8 != 0 || ldy % 8 != 0 || ldw % 8 != 0 || !gemv_takes(y, W, M, N, K, act, true) ||
       ((reinterpret_cast<uintptr_t>(residual) | reinterpret_cast<uintptr_t>(residual_out) | reinterpret_cast<uintptr_t>(norm_w)) & 15) != 0)
     return 2;
   GemvParams p = gemv_params(y, ldy, W, ldw, C, ldc, N, K, bias);

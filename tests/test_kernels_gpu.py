@@ -1203,7 +1203,7 @@ def test_latent_attention_block_in_one_call(heads, width, q_lens, decodes, monke
 
 
 @pytest.mark.parametrize("m", [1, 2])
-@pytest.mark.parametrize("n,k,act", [(8, 8, 0), (5, 264, 0), (4100, 1024, 0), (640, 6144, 0), (512, 1032, 1), (6144, 1024, 1)])
+@pytest.mark.parametrize("n,k,act", [(8, 8, 0), (5, 264, 0), (4100, 1024, 0), (640, 6144, 0), (512, 1032, 1), (6144, 1024, 1), (64, 12280, 0)])
 def test_norm_with_the_product_behind_it(m, n, k, act):
     """rmsnorm(y + residual) formed by the one-or-two-row product: the sum bit for bit that of the norm kernel, the product within the
     roundings of fp32 sums of bf16 products and of normed values that may round to the other neighbour (2^-8 each, not all one way)."""
@@ -1222,12 +1222,13 @@ def test_norm_with_the_product_behind_it(m, n, k, act):
     assert got.shape == want.shape and _rel_err(got, want) < 6e-3
 
 
-def test_norm_that_no_product_takes():
-    """A deferred norm whose product is too large for the kernel (rows beyond its shared memory) is formed by the norm's own."""
+@pytest.mark.parametrize("m,k", [(1, 24584), (1, 24576), (2, 12288), (2, 12296)])
+def test_norm_that_no_product_takes(m, k):
+    """A deferred norm whose product is too large for the kernel is formed by the norm's own: rows beyond its shared memory, or rows
+    that fill it to the last byte and leave nothing for the sums of squares."""
     from gllm_b200.layers import functional as Fn
     torch.manual_seed(3)
-    k = 24584
-    y, res = torch.randn(1, k, device=_dev()).bfloat16(), torch.randn(1, k, device=_dev()).bfloat16()
+    y, res = torch.randn(m, k, device=_dev()).bfloat16(), torch.randn(m, k, device=_dev()).bfloat16()
     w, wt = torch.ones(k, device=_dev()).bfloat16(), torch.randn(64, k, device=_dev()).bfloat16() * k ** -0.5
     h = Fn.NormedSum(y, res, w, 1e-6)
     got = h.linear(wt)
