@@ -417,8 +417,8 @@ GLLM_EXPORT int gllm_moe_grouped_topk(const void* logits, int64_t ld, const void
 
 static int route(const RouteParams& p, cudaStream_t st) {
   if (p.n_slots <= 0) return 0;
-  if (p.E <= 0 || p.E > 1024) {
-    fprintf(stderr, "[gllm_b200] moe_align_gather: %d experts (1 to 1024)\n", p.E);
+  if (p.E < 0 || p.E > 1024) {                           // none: zero counts, no tile, no slot placed
+    fprintf(stderr, "[gllm_b200] moe_align_gather: %d experts (0 to 1024)\n", p.E);
     return 1;
   }
   const bool quant = p.q != nullptr;
