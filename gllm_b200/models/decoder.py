@@ -240,7 +240,7 @@ class DecoderLayer(nn.Module):
     def forward(self, inp, h: torch.Tensor, residual: torch.Tensor, kv_cache, tpc: TPComm,
                 next_norm_w: Optional[torch.Tensor], qkv: Optional[torch.Tensor] = None, defer: bool = False):
         """h = RMSNorm'ed block input, residual = running residual stream. `defer`: the next block is one like this, so the norm in
-        front of it may be left to its first product.
+        front of it may be left to its first product: then what comes back may be a `NormedSum`, whose residual is only there behind it.
         Returns (normed input of the next block, residual) — or (un-normed block output, residual)
         when `next_norm_w` is None (last layer of a non-final pipeline stage)."""
         eps = self.spec.rms_eps
@@ -255,6 +255,18 @@ class DecoderLayer(nn.Module):
         if next_norm_w is None:
             return tpc.row_linear(act, self.mlp.down_weight()), residual
         return tpc.row_linear_add_norm(act, self.mlp.down_weight(), residual, next_norm_w, eps, defer=defer)
+
+
+def _hooked(module: nn.Module) -> bool:
+    m = nn.modules.module
+    return bool(module._forward_hooks or module._forward_pre_hooks or m._global_forward_hooks or m._global_forward_pre_hooks)
+
+
+def _defers(layer: nn.Module, behind: nn.Module) -> bool:
+    """Whether `layer` may leave the norm behind it to the first product of `behind`: nobody but these two sees what lies between them,
+    which is no tensor, and a residual stream that is not there yet. A hook would."""
+    return type(layer) is type(behind) is DecoderLayer and type(behind.attn) is Attention and \
+        not (_hooked(layer) or _hooked(behind) or _hooked(behind.attn))
 
 
 class CausalLM(nn.Module):
@@ -376,7 +388,7 @@ class CausalLM(nn.Module):
             elif i == 0 and qkv0 is not None:
                 h, residual = layer(inp, h, residual, kv_cache, tpc, nxt, qkv=qkv0)
             else:
-                more = {"defer": True} if i + 1 < n and type(layer) is type(self.layers[i + 1]) is DecoderLayer else {}
+                more = {"defer": True} if i + 1 < n and _defers(layer, self.layers[i + 1]) else {}
                 h, residual = layer(inp, h, residual, kv_cache, tpc, nxt, **more)
         if nvtx and n:
             torch.cuda.nvtx.range_pop()

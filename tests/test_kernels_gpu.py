@@ -1239,6 +1239,49 @@ def test_norm_that_no_product_takes(m, k):
     assert torch.equal(Fn.NormedSum(y, res, w, 1e-6).tensor(), normed)
 
 
+@pytest.mark.parametrize("where", ["layer", "layer behind", "attention", "all modules", None])
+def test_hooks_see_tensors_between_layers(where, monkeypatch):
+    """A hook between two layers sees the normed input and the residual stream as tensors that are there: the norm is not left to the
+    next layer's first product then. Both forms round alike but for the order of the fp32 sums."""
+    from types import SimpleNamespace
+    from gllm_b200.layers import functional as Fn
+    from gllm_b200.models.decoder import CausalLM, ModelSpec
+    from gllm_b200.parallel.tp import TPComm
+    torch.manual_seed(11)
+    spec = ModelSpec(arch="Qwen3ForCausalLM", hidden_size=512, num_layers=3, num_heads=4, num_kv_heads=2, head_dim=128,
+                     intermediate_size=1024, vocab_size=128, max_position=64)
+    model = CausalLM(spec, _dev())
+    for w in model.parameters():
+        w.data.copy_(torch.randn_like(w) * (0.05 if w.dim() > 1 else 1.0))
+    inp = SimpleNamespace(tokens=torch.tensor([5, 77], dtype=torch.int32, device=_dev()))
+    deferred, made = [], Fn.NormedSum.__init__
+    monkeypatch.setattr(Fn.NormedSum, "__init__", lambda self, *a: deferred.append(1) or made(self, *a))
+
+    def run():
+        seen = []
+
+        def keep(module, args, out=None):
+            values = args if out is None or module is model.layers[1].attn else out if isinstance(out, tuple) else (out,)
+            seen.extend(x.clone() for x in values if isinstance(x, (torch.Tensor, Fn.NormedSum)))
+        hook = {"layer": lambda: model.layers[0].register_forward_hook(keep),
+                "layer behind": lambda: model.layers[1].register_forward_pre_hook(keep),
+                "attention": lambda: model.layers[1].attn.register_forward_hook(keep),
+                "all modules": lambda: torch.nn.modules.module.register_module_forward_hook(keep), None: lambda: None}[where]()
+        try:
+            return [*model(inp, None, TPComm()), *seen]
+        finally:
+            if hook is not None:
+                hook.remove()
+
+    got = run()
+    between = {"layer behind": 2, "all modules": 2, None: 0}.get(where, 1)    # the middle layer's hook speaks for both its sides
+    assert len(deferred) == 5 - between                     # three norms inside layers, two between them
+    monkeypatch.setattr(Fn.NormedSum, "takes", staticmethod(lambda *a: False))
+    want = run()
+    assert len(got) == len(want) and (len(got) == 2) == (where is None)
+    assert all(_rel_err(a, b) < 2e-2 for a, b in zip(got, want))
+
+
 @pytest.mark.parametrize("m", [1, 2])
 @pytest.mark.parametrize("n,k", [(1, 8), (5, 264), (130, 1024), (4097, 1024), (4100, 2056), (257, 6144), (640, 8192)])
 def test_linear_few_rows(m, n, k):
