@@ -170,6 +170,7 @@ def norm_linear(y: torch.Tensor, residual: torch.Tensor, residual_out: torch.Ten
     the sum into residual_out; None where the kernel does not take the product."""
     m, k = y.shape
     n = w.shape[0]
+    assert w.shape == (n, k) and residual.shape == residual_out.shape == (m, k), (y.shape, residual.shape, w.shape)
     if gemm_forced() or not (m <= 2 and m <= _SMALLM_MAX and y.dtype == w.dtype == _BF16 and y.stride(1) == 1 and w.stride(1) == 1):
         return None
     out = torch.empty(m, n // 2 if act else n, dtype=_BF16, device=y.device)

@@ -815,3 +815,16 @@ def test_a_load_that_raises_leaves_nothing_for_the_next(monkeypatch):
     for pair, want in ((inp._tokens, 500 + np.arange(9)), (inp._seq_lens, 500 + np.arange(2)), (inp._block_table, 500 + np.arange(6))):
         p = at[pair[1].data_ptr()]
         assert np.array_equal(block.numpy()[p[2]:p[2] + p[3] * p[4]], want)
+
+
+@pytest.mark.parametrize("act", [0, 1])
+def test_deferred_norm_refuses_a_weight_of_another_width(act):
+    """A product behind a norm that is formed with it checks its shapes as the product alone does: nothing is launched on a weight whose
+    rows are shorter or longer than the normed ones."""
+    import torch
+    from gllm_b200.layers import functional as Fn
+    y, w = torch.zeros(1, 64).bfloat16(), torch.ones(64).bfloat16()
+    for k in (56, 72):
+        h = Fn.NormedSum(y, torch.zeros(1, 64).bfloat16(), w, 1e-6)
+        with pytest.raises(AssertionError):
+            (h.linear_silu_mul if act else h.linear)(torch.zeros(256, k).bfloat16())
