@@ -1094,11 +1094,13 @@ def test_gemm_on_clusters(m, n, k, act, parts, smem):
 @pytest.mark.parametrize("t,k,experts,held,valid", [(1, 1, 1, 1, None), (3, 8, 16, 16, None), (512, 8, 128, 128, None),
                                                     (513, 8, 256, 32, None), (2048, 2, 1024, 1024, None), (2049, 2, 1024, 700, None),
                                                     (600, 1, 8, 8, 37), (5000, 1, 8, 8, 4097), (40, 4, 300, 0, None),
-                                                    (5000, 1, 8, 0, None)])
+                                                    (5000, 1, 8, 0, None), (16384, 1, 5, 5, None), (16385, 1, 5, 5, None),
+                                                    (5000, 8, 256, 31, None), (17000, 8, 1024, 1024, None), (20000, 1, 8, 8, 37),
+                                                    (40000, 1, 8, 8, 17001), (20000, 1, 8, 8, 0)])
 @pytest.mark.parametrize("quant", [False, True])
 def test_moe_routing_and_gather(t, k, experts, held, valid, quant):
-    """Counts, padded offsets, tiles, places and rows of both forms of the routing (up to 4096 slots in one launch), a rank that holds
-    no expert among them, and quantised on the way the same bytes and scales as by the quantiser."""
+    """Counts, padded offsets, tiles, places and rows of the forms of the routing (up to 4096 slots in one launch, up to 16,384 by one
+    block, beyond by the CTAs of a cluster, the last of them in several steps), a rank that holds no expert among them, and quantised on the way the same bytes and scales as by the quantiser."""
     from gllm_b200.ops import lib
     torch.manual_seed(t + experts)
     dev, h, E = _dev(), 384, held
