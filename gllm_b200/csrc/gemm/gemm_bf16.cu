@@ -718,7 +718,7 @@ static int gemm_bf16_impl(const void* A, int64_t lda, const void* W, int64_t ldw
   const bool free_bn = force_bn == (epi == kEpiSiluMul ? 256 : 0);
   ClusterPlan plan;
   if (comm == nullptr && decode && free_bn && g_force_split <= 0 && glu_limit <= 0.f && (epi != kEpiSiluMul || (N % 256 == 0 && bias == nullptr)) &&
-      plan_gemm_cluster(M, N, K, epi == kEpiSiluMul, &plan)) {
+      plan_gemm_cluster(M, N, K, epi == kEpiSiluMul, bn, split, &plan)) {
     const ClusterGemm g{A, W, lda, ldw, reinterpret_cast<__nv_bfloat16*>(C), ldc, M, N, K,
                         reinterpret_cast<const __nv_bfloat16*>(bias), epi == kEpiSiluMul, gelu};
     return gemm_bf16_cluster(g, plan, reinterpret_cast<cudaStream_t>(stream));

@@ -325,7 +325,7 @@ GLLM_EXPORT int gllm_gemm_smallm(const void* A, int64_t lda, const void* W, int6
     if (rc >= 0) return rc;
     ClusterPlan plan;
     if (N % 8 == 0 && ldc % 8 == 0 && ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0 &&
-        (silu == 0 || (N % 256 == 0 && bias == nullptr)) && plan_gemm_cluster(M, N, K, silu != 0, &plan)) {
+        (silu == 0 || (N % 256 == 0 && bias == nullptr)) && plan_gemm_cluster(M, N, K, silu != 0, 0, 0, &plan)) {
       const ClusterGemm g{A, W, lda, ldw, reinterpret_cast<__nv_bfloat16*>(C), ldc, M, N, K,
                           reinterpret_cast<const __nv_bfloat16*>(bias), silu != 0, silu == 2};
       return gemm_bf16_cluster(g, plan, reinterpret_cast<cudaStream_t>(stream));

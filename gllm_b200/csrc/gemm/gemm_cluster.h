@@ -26,8 +26,9 @@ struct ClusterPlan {
   int smem;                                  // shared memory per CTA that the ring may fill
 };
 
-// whether this kernel is the faster one for a product of this size, and how
-bool plan_gemm_cluster(int M, int N, int K, bool gated, ClusterPlan* plan);
+// Whether this kernel is the faster one for a product of this size, and how. `bn`, `split`: the tile width and K split that gemm_bf16.cu
+// would take instead (0: not that kernel).
+bool plan_gemm_cluster(int M, int N, int K, bool gated, int bn, int split, ClusterPlan* plan);
 
 // 0: launched
 int gemm_bf16_cluster(const ClusterGemm& g, const ClusterPlan& plan, cudaStream_t st);

@@ -1091,6 +1091,20 @@ def test_gemm_on_clusters(m, n, k, act, parts, smem):
         assert bool(((out[:m, :n_out].double() - want).abs() <= tol).all())
 
 
+@pytest.mark.parametrize("m,n,k", [(32, 16512, 72), (32, 19072, 72), (128, 12800, 264), (80, 12800, 264), (79, 12800, 264), (256, 10496, 1544),
+                                   (128, 4608, 2368), (111, 4608, 2368), (384, 3072, 4416), (384, 3072, 4424), (128, 11008, 1536),
+                                   (128, 11008, 1544), (128, 5760, 1032), (200, 3328, 2056)])
+def test_linear_where_the_kernels_meet(m, n, k):
+    """Sizes on both sides of the rules that choose between clusters and the other tiles, and tiles that fill the clusters of three and five
+    that run at once to the last. fp32 sums of bf16 products in any order, one rounding."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(n + k)
+    x, w = torch.randn(m, k, device=_dev()).bfloat16(), torch.randn(n, k, device=_dev()).bfloat16()
+    want = x.double() @ w.double().t()
+    tol = want.abs() * 2.0 ** -8 + (x.double().abs() @ w.double().abs().t()) * k * 2.0 ** -24
+    assert bool(((sm100.linear(x, w).double() - want).abs() <= tol).all())
+
+
 @pytest.mark.parametrize("t,k,experts,held,valid", [(1, 1, 1, 1, None), (3, 8, 16, 16, None), (512, 8, 128, 128, None),
                                                     (513, 8, 256, 32, None), (2048, 2, 1024, 1024, None), (2049, 2, 1024, 700, None),
                                                     (600, 1, 8, 8, 37), (5000, 1, 8, 8, 4097), (40, 4, 300, 0, None),
