@@ -1,6 +1,8 @@
 """sm_100a kernels vs the PyTorch fp32 oracle (runs on the B200 box: `pytest -m gpu`)."""
+import contextlib
 import math
 import os
+import time
 
 import numpy as np
 import pytest
@@ -350,7 +352,7 @@ def test_prefill_value_that_is_no_number(window, bad, clean, seqs):
     assert bool(torch.isnan(got[sees]).all())
 
 
-@pytest.mark.parametrize("family", ["fp8", "attn", "mla", "gemm"])
+@pytest.mark.parametrize("family", ["fp8", "attn", "mla", "gemm", "clusters", "gated clusters"])
 def test_wait_that_gives_up_reaches_the_caller(family):
     """A wait limit of zero: whatever is not there at the first look is given up. The kernel returns, the engine's check raises,
     and the next call is right again."""
@@ -366,6 +368,14 @@ def test_wait_that_gives_up_reaches_the_caller(family):
         x, w = torch.randn(600, 1024, device=_dev()).bfloat16(), torch.randn(6144, 1024, device=_dev()).bfloat16()
         call = lambda: sm100.linear(x, w)
         want = x.float() @ w.float().t()
+    elif "clusters" in family:                                # 192 K blocks: every part of a cluster fills its ring more than once
+        x, w = torch.randn(64, 12288, device=_dev()).bfloat16(), torch.randn(4096, 12288, device=_dev()).bfloat16() * 12288 ** -0.5
+        call = lambda: sm100.linear(x, w)
+        want = x.float() @ w.float().t()
+        if family != "clusters":
+            wi = ref.interleave_gate_up(w, 128)
+            call = lambda: sm100.linear_silu_mul(x, wi)
+            want = torch.nn.functional.silu(want[:, :2048]) * want[:, 2048:]
     elif family == "attn":
         lens = [300, 129]
         a = _make_paged(lens, lens, 8, 2, 128, 16, _dev(), seed=1)
@@ -382,8 +392,10 @@ def test_wait_that_gives_up_reaches_the_caller(family):
     done = StepResult(tokens=torch.zeros(1, dtype=torch.int32), num_emit=1)
     try:
         lib.watch_waits(limit_ns=0)
+        t0 = time.monotonic()
         call()
         torch.cuda.synchronize()
+        assert time.monotonic() - t0 < 0.5                   # nothing waits for what was never issued (two seconds)
         with pytest.raises(RuntimeError, match="bounded wait"):
             done.tokens_list()
     finally:
@@ -397,7 +409,6 @@ def test_wait_that_gives_up_reaches_the_caller(family):
 def test_gemm_on_pairs_that_gives_up_ends_soon(m, n, k):
     """Limits of nothing, 1 ns and 2 us: the two CTAs of a pair give up at different stages, and still no copy is waited for that was
     never issued (two seconds each). The sums of 64 K blocks are waited for longer than that."""
-    import time
     from gllm_b200.ops import lib, sm100
     torch.manual_seed(k)
     x, w = torch.randn(m, k, device=_dev()).bfloat16(), torch.randn(n, k, device=_dev()).bfloat16()
@@ -771,23 +782,36 @@ def test_gemm_fp8_block(m, n, k):
     assert _rel_err(q.float(), q_r.float()) < 3e-2
 
 
+@contextlib.contextmanager
+def _forced_split(parts):
+    """A forced K split of the tiles on single SMs, which products of these sizes would otherwise leave to clusters (0: nothing forced)."""
+    from gllm_b200.ops import lib
+    lib.load().gllm_gemm_tune(parts, 512)
+    try:
+        yield
+    finally:
+        lib.load().gllm_gemm_tune(0, 512)
+
+
+@pytest.mark.parametrize("split", [0, 2, 4])
 @pytest.mark.parametrize("m", [64, 128, 200, 256, 384, 512])
 @pytest.mark.parametrize("n,k", [(4096, 4096), (4096, 12288), (6144, 4096), (1000, 1536)])
-def test_gemm_splitk_decode_shapes(m, n, k):
-    """Decode-sized M takes the wide-tile split-K path (fp32 partials, last-arriver sum): exact shape sweep,
-    bias, and back-to-back launches (tile counters re-arm themselves)."""
+def test_gemm_splitk_decode_shapes(m, n, k, split):
+    """Decode-sized M as the dispatch has it (mostly clusters), and on the wide-tile split-K path (fp32 partials, last-arriver sum): exact
+    shape sweep, bias, and back-to-back launches (tile counters re-arm themselves)."""
     from gllm_b200.ops import sm100
     torch.manual_seed(m + n + k)
     x = (torch.randn(m, k, device=_dev()) * 0.5).bfloat16()
     w = (torch.randn(n, k, device=_dev()) * 0.05).bfloat16()
     b = torch.randn(n, device=_dev()).bfloat16()
-    for bias in (None, b):
-        y = sm100.linear(x, w, bias)
-        yr = x.float() @ w.float().t() + (bias.float() if bias is not None else 0)
-        assert _rel_err(y, yr) < 6e-3, _rel_err(y, yr)
-    y2 = sm100.linear(x, w, None)
-    for _ in range(3):
-        assert torch.equal(y2, sm100.linear(x, w, None))   # deterministic slice-ordered reduction
+    with _forced_split(split):
+        for bias in (None, b):
+            y = sm100.linear(x, w, bias)
+            yr = x.float() @ w.float().t() + (bias.float() if bias is not None else 0)
+            assert _rel_err(y, yr) < 6e-3, _rel_err(y, yr)
+        y2 = sm100.linear(x, w, None)
+        for _ in range(3):
+            assert torch.equal(y2, sm100.linear(x, w, None))   # deterministic slice-ordered reduction
 
 
 @pytest.mark.parametrize("m", [64, 256, 384])
@@ -1379,7 +1403,8 @@ def test_gemm_smallm_any_output(m, ldc, shift):
 @pytest.mark.parametrize("act", ["silu", "gelu", "glu"])
 @pytest.mark.parametrize("m,f,k", [(64, 1536, 4096), (100, 2048, 7168), (128, 1792, 4096)])
 def test_gemm_gated_split_in_eight(m, f, k, act):
-    """K in eight parts, each of whose CTAs gates 16 columns of a tile. fp32 sums in the order of the parts, one rounding."""
+    """K in eight parts, each of whose CTAs gates 16 columns of a tile: what the rule of that kernel chooses here, though clusters take the
+    silu and gelu forms if nothing is forced. fp32 sums in the order of the parts, one rounding."""
     from gllm_b200.ops import lib, ref, sm100, sm100_latent
     torch.manual_seed(f)
     x, w = torch.randn(m, k, device=_dev()).bfloat16(), (torch.randn(2 * f, k, device=_dev()) * k ** -0.5).bfloat16()
@@ -1393,8 +1418,9 @@ def test_gemm_gated_split_in_eight(m, f, k, act):
     else:
         want = (torch.nn.functional.silu(g) if act == "silu" else torch.nn.functional.gelu(g, approximate="tanh")) * u
         call = lambda: sm100.linear_silu_mul(x, wi, act=act)  # noqa: E731
-    for _ in range(3):                                       # the counters of a tile are set back behind each product
-        got = call()
+    for split in (8, 8, 8, 0):                               # the counters of a tile are set back behind each product; as dispatched
+        with _forced_split(split):
+            got = call()
         assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 2.0 ** -16 * (1 + want.abs())).all())
 
 
