@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Headline benchmark: offline serving throughput (output tokens/s) of Qwen3-8B bf16 with TP=N on N
-B200s, on synthetic ShareGPT-shaped requests with random-init weights (BASELINE.json metric;
-workload definition = the reference's benchmarks/benchmark_throughput.py: all requests submitted at
+B200s, on synthetic ShareGPT-shaped requests with random-init weights
+(workload definition = the reference's benchmarks/benchmark_throughput.py: all requests submitted at
 t=0, prompt <= 1024, prompt+output <= 2048, greedy, ignore_eos).
 
 One *step* = one complete pass over the request set (`--num-prompts` requests, all prompt and output
@@ -26,7 +26,7 @@ import time
 sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
 
 
-# BASELINE.json configurations: model preset, pipeline stages (tp = gpus / pp), schedule policy, metric label
+# named configurations: model preset, pipeline stages (tp = gpus / pp), schedule policy, metric label
 CONFIGS = {
     "qwen3-8b-tp": dict(model="qwen3-8b", pp=1, method="chunked_prefill", label="Qwen3-8B TP"),
     "mixtral-8x7b-ep": dict(model="mixtral-8x7b", pp=1, method="chunked_prefill", label="Mixtral-8x7B EP"),
@@ -53,7 +53,7 @@ def parse():
     ap.add_argument("--schedule-method", default="chunked_prefill")
     ap.add_argument("--pp", type=int, default=1)
     ap.add_argument("--config", default="qwen3-8b-tp", choices=sorted(CONFIGS),
-                    help="named BASELINE.json configuration (model + parallel layout + schedule policy)")
+                    help="named configuration (model + parallel layout + schedule policy)")
     ap.add_argument("--layers", type=int, default=0, help="override num_hidden_layers (0 = the model's own); a "
                     "reduced depth is reported in `config.model` and is NOT the named model")
     ap.add_argument("--seed", type=int, default=0)
@@ -74,7 +74,7 @@ def reference_arm(args):
     """Run the unmodified reference (baseline/install_reference.sh -> baseline/_ref) through its own public API in
     a subprocess (baseline/run_reference.py) and forward its JSON line. The reference pins vLLM 0.11 / torch 2.8 /
     transformers < 5, this image has vLLM 0.22 / torch 2.11 / transformers 5: if its native ops or imports do not
-    line up on the box, the arm reports {"impl": "reference", "unavailable": <why>} and exits 0 (DESIGN.md)."""
+    line up on the box, the arm reports {"impl": "reference", "unavailable": <why>} and exits 0."""
     if int(os.environ.get("RANK", "0")) != 0:
         return 0          # the reference spawns its own per-GPU workers: only one front-end process
     root = os.path.dirname(os.path.abspath(__file__))
@@ -86,7 +86,7 @@ def reference_arm(args):
 
     if not os.path.isfile(os.path.join(ref_root, "gllm", "llm_engine.py")):
         return unavailable("baseline/_ref is not populated (run baseline/install_reference.sh; the reference's "
-                           "setup.py needs a vLLM wheel for its native kernels, see DESIGN.md)")
+                           "setup.py needs a vLLM wheel for its native kernels)")
     env = dict(os.environ)
     for k in ("RANK", "LOCAL_RANK", "WORLD_SIZE", "MASTER_ADDR", "MASTER_PORT", "TORCHELASTIC_USE_AGENT_STORE",
               "GROUP_RANK", "ROLE_RANK", "LOCAL_WORLD_SIZE", "TORCHELASTIC_RUN_ID", "OMP_NUM_THREADS"):

@@ -3,7 +3,7 @@
 # benchmark_serving client with ShareGPT-shaped synthetic prompts, Poisson arrivals.
 #   run_serving_gpu.sh [tp] [rate] [num_prompts]          IMPL=ours (default) | reference ; STAGES=n for staged arrivals
 # IMPL=reference starts the UNMODIFIED reference's own server (baseline/_ref, `python -m gllm.entrypoints.api_server`)
-# on the same model shape, flags and client: the p50 TTFT / TPOT pair of BASELINE.json's metric for both arms.
+# on the same model shape, flags and client: the p50 TTFT / TPOT pair for both arms.
 TP=${1:-1}; RATE=${2:-16}; N=${3:-300}; PORT=${PORT:-18000}; IMPL=${IMPL:-ours}; STAGES=${STAGES:-1}
 cd "$(dirname "$0")/.."
 OUT=${OUT:-/tmp/serving}

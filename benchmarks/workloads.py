@@ -1,5 +1,4 @@
-"""Synthetic workloads shaped like the reference's datasets (no network: BASELINE.json asks for
-"synthetic ShareGPT-shaped requests"). Optionally reads a local ShareGPT json with --dataset."""
+"""Synthetic workloads shaped like the reference's datasets (ShareGPT-shaped requests; no network). Optionally reads a local ShareGPT json with --dataset."""
 import json
 from typing import List, Optional, Tuple
 

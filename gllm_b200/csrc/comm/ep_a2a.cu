@@ -1,4 +1,4 @@
-// Expert-parallel all-to-all over NVLink peer memory (SURVEY §2.4 X3).
+// Expert-parallel all-to-all over NVLink peer memory.
 //
 // Activations are token-sharded (the fused TP layout, comm/tp_fused.cu). Per MoE block:
 //

@@ -557,7 +557,7 @@ GLLM_EXPORT int gllm_rs_reduce_norm(const ReduceNormArgs* a, void* stream) {
   const int grid = p.rows_per_rank > 0 ? p.rows_per_rank : 1;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   // (plain launch: measured slower with programmatic dependent launch — the gated consumer GEMM then polls
-  // system-scope flags next to the reduction, profiles/tp_fused.md)
+  // system-scope flags next to the reduction)
   if (nv == 1) rs_reduce_norm_kernel<1><<<grid, threads, 0, st>>>(p);
   else if (nv == 2) rs_reduce_norm_kernel<2><<<grid, threads, 0, st>>>(p);
   else if (nv == 4) rs_reduce_norm_kernel<4><<<grid, threads, 0, st>>>(p);

@@ -8,7 +8,7 @@
 //     main loop of tile i+1,
 //   * four epilogue warps drain TMEM with tcgen05.ld and apply the fused epilogue
 //     (bias, SiLU-gate for the merged gate/up projection),
-//   * optional fused collectives over NVLink peer memory (SURVEY §2.4 X1/X2):
+//   * optional fused collectives over NVLink peer memory:
 //       - all-gather ⊕ GEMM: the TMA producer gates each M tile on per-row-block
 //         "ready" flags that peer ranks set after pushing their activation shard,
 //       - GEMM ⊕ reduce-scatter: the epilogue stores each partial tile straight into the
@@ -60,7 +60,7 @@ struct GemmParams {
   // batched mode (batch > 0): `batch` independent [rows_per_batch, K] x [N, K]^T products over strided operands —
   // A is a 3-D tensor map (k, row, batch), batch b uses the weight slab b ([batch, N, K] contiguous) and writes
   // C + row * ldc + b * c_batch_stride. MLA weight absorption (q_nope·W_UK, out_lat·W_UV per head) runs on it
-  // instead of a cuBLAS bmm (SURVEY §2.3 K13; reference: gllm/layers/attention.py:463-484).
+  // instead of a cuBLAS bmm (reference: gllm/layers/attention.py:463-484).
   int batch, rows_per_batch;
   int64_t c_batch_stride;
   // gated epilogue variant (kEpiSiluMul with glu_limit > 0): g = min(gate, limit), u = clamp(up, +-limit),
@@ -602,7 +602,7 @@ static bool pairs_are_faster(int M, int N, int bn) {
 }
 
 // Decode-sized M: few output tiles, so tile shape and a K split are chosen together. Cost model in SM clocks,
-// calibrated on B200 (profiles/gemm_splitk.md): a 64-deep k-block costs ~650 clk for BN=256 and ~420 clk for
+// calibrated on B200: a 64-deep k-block costs ~650 clk for BN=256 and ~420 clk for
 // BN<=128 (SMEM fill bound: 16 KB of A per k-block regardless of BN), a split-K round adds ~2000 + 24*BN.
 static void pick_split(int M, int N, int K, int epi, int forced_bn, int64_t ws_bytes, int max_tiles, int* bn_out,
                        int* split_out) {
@@ -616,7 +616,7 @@ static void pick_split(int M, int N, int K, int epi, int forced_bn, int64_t ws_b
     if (forced_bn > 0 && bn != forced_bn) continue;
     if (epi == kEpiSiluMul && bn < 64) continue;
     const int tiles = num_m * ((N + bn - 1) / bn);
-    // measured per-k-block time in SM clocks (benchmarks/gemm_tune.py, profiles/gemm_splitk.md)
+    // measured per-k-block time in SM clocks (benchmarks/gemm_tune.py)
     const double t_kb = bn >= 256 ? 650.0 : 420.0;
     for (int split = 1; split <= 8; split *= 2) {
       const int kpb = (num_kb + split - 1) / split;

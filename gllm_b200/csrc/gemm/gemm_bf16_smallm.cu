@@ -2,7 +2,7 @@
 //
 //     C[M, N] = A[M, K] · W[N, K]^T        with M <= 256 (a decode micro-batch)
 //
-// ncu on the 128xBN kernel (profiles/gemm_small_m_before.md) showed that for M << 128 the SM's
+// ncu on the 128xBN kernel showed that for M << 128 the SM's
 // L2->SMEM fill bandwidth (~64 B/clk/SM) is spent on the 128-row activation tile that every CTA
 // re-reads, not on weights. Here the operands are swapped: the *weights* fill the 128-row MMA M
 // slot (every byte fetched is a weight byte that must come from HBM anyway) and the tokens sit in

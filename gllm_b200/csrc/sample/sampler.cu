@@ -9,7 +9,7 @@
 //   draw   : exponential race  argmax_i  exp(t_i - m) / E_i ,  E_i ~ Exp(1)   (== Gumbel-max,
 //            the same distribution the reference draws with `probs / Exp(1)` then argmax)
 // Greedy rows (top_k == 1) take a single argmax pass. A vocab-parallel variant returns the
-// per-rank (max, index) pair so TP ranks only exchange B x 2 scalars (SURVEY §2.4 X4).
+// per-rank (max, index) pair so TP ranks only exchange B x 2 scalars.
 #include "../common/host_utils.h"
 #include "../common/ptx.cuh"
 
@@ -344,7 +344,7 @@ sample_kernel(int parts, const T* __restrict__ logits, int64_t ld, int V, const 
 }
 
 // ------------------------------------------------------------------------------------------------------------------
-// Vocab-parallel sampling (SURVEY §2.4 X4): the [B, V] logits are never gathered. Every TP rank reduces its own
+// Vocab-parallel sampling: the [B, V] logits are never gathered. Every TP rank reduces its own
 // vocab shard to a fixed-size record per row — its C best candidates after penalty and temperature (value + token
 // id), the shard's softmax statistics (max, sum exp) and, for rows that sample from the whole vocabulary, the
 // shard's exponential-race winner — the ranks all-gather these records (B x (2C+4) floats per rank instead of

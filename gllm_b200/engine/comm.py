@@ -86,8 +86,8 @@ class Comm:
             if bind:
                 # Bind on the master's own address, not on every interface: the frames on these sockets are pickled
                 # Python objects (control messages, token lists), so whoever can connect can execute code in the
-                # engine. The trust boundary is the cluster network the master address lives on ("Trust
-                # boundary of the control plane"); `--host 0.0.0.0` restores the reference's bind-everywhere.
+                # engine. The trust boundary is the cluster network the master address lives on;
+                # `--host 0.0.0.0` restores the reference's bind-everywhere.
                 wide = self.tcp_host in ("", "0.0.0.0", "*")
                 return f"tcp://{'*' if wide else (self.tcp_host or self.master_addr)}:{port}"
             return f"tcp://{self.master_addr}:{port}"

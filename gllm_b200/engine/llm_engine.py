@@ -233,7 +233,7 @@ class LLM:
 
     # The three inboxes below are filled from request handlers (event-loop thread of the API server) while the
     # engine tick runs in a worker thread: every append and the swap in `_send` hold `_inbox_lock`, so a request
-    # can never land in a list the tick has already shipped (the reference has this race, SURVEY §5.2).
+    # can never land in a list the tick has already shipped (the reference has this race).
     def add_requests(self, seqs: List[Sequence]):
         with self._inbox_lock:
             self.wait_lists.extend(seqs)

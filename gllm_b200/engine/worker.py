@@ -275,7 +275,7 @@ class Worker(ProfilerMixin):
     def _pp_send(self, res: StepResult):
         tensors = [res.hidden, res.residual] if self.runner.model.ret_residual else [res.hidden]
         # clone: the static output buffers are overwritten by the next micro-batch while the send is
-        # still in flight (latent race in the reference, SURVEY §5.2)
+        # still in flight (latent race in the reference)
         tensors = [t.clone() for t in tensors]
         handles = ps.pp_send_tiled(tensors)
         self.inflight_sends.append((handles, tensors))

@@ -190,7 +190,7 @@ class SparseMoeBlock(nn.Module):
         out = self.experts(h, tpc)
         if self.shared is not None:
             # partial (un-reduced) shared-expert output: reduced together with the routed experts —
-            # the reference double-reduces here on Qwen2-MoE (SURVEY §2.2 C23); we do it once.
+            # the reference double-reduces here on Qwen2-MoE; we do it once.
             s = Fn.linear(self.shared.act(h, tpc), self.shared.down_weight())
             if self.shared_gate_w is not None:
                 g = torch.sigmoid(torch.nn.functional.linear(h.float(), self.shared_gate_w.float()))

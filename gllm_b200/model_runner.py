@@ -419,7 +419,7 @@ class ModelRunner:
     VP_CANDIDATES = 256   # per rank and row; top_k <= this is exact (csrc/sample/sampler.cu)
 
     def _vp_sample(self, shard: torch.Tensor, seen: Optional[torch.Tensor]) -> torch.Tensor:
-        """Vocab-parallel top-k / top-p / penalty sampling (SURVEY §2.4 X4): every rank reduces its vocab shard to
+        """Vocab-parallel top-k / top-p / penalty sampling: every rank reduces its vocab shard to
         a [E, 2C+4] record (C best candidates, softmax statistics, race winner), the ranks all-gather the records —
         ~2 KB per row and rank instead of V/tp logits — and finish on the tp x C candidates with the exact global
         normalisation. The [E, V] logits are never materialised (the reference all-gathers them and sorts the full
@@ -463,7 +463,7 @@ class ModelRunner:
         return ref.vp_final(allr, c, v_full, inp.top_k[:e], inp.top_p[:e], generator=g)
 
     def _vp_greedy(self, shard: torch.Tensor) -> torch.Tensor:
-        """Vocab-parallel greedy sampling (SURVEY §2.4 X4): every rank takes the argmax of its own vocab shard
+        """Vocab-parallel greedy sampling: every rank takes the argmax of its own vocab shard
         with the sampler kernel, the ranks exchange (value, global index) pairs — 8 bytes per row instead of the
         [E, V] logits — and pick the winner (lowest rank on ties == lowest token id)."""
         import torch.distributed as dist

@@ -352,7 +352,7 @@ class CausalLM(nn.Module):
                 h, residual = tpc.first_norm(res_full, self.layers[0].input_norm_w, eps)
             elif recv_tiles and len(recv_tiles) > 1 and hasattr(self.layers[0].attn, "qkv_proj"):
                 # tile-streamed pipeline input: add+RMSNorm and the QKV GEMM run per row tile as the tiles
-                # land, overlapping the NCCL transfer of the following tiles (SURVEY §2.4 X5)
+                # land, overlapping the NCCL transfer of the following tiles
                 h = torch.empty_like(hidden)
                 at = self.layers[0].attn
                 for r0, r1, works in recv_tiles:

@@ -11,7 +11,7 @@ On sm_100a the attention runs in the *absorbed* form: q_nope·W_UK per head (bat
 views, written straight into the 576-wide query), fused RoPE + latent-cache write, split-KV multi-query attention
 over the paged latent cache (csrc/attn/mla_attention.cu), then out_lat·W_UV per head (the same batched GEMM,
 written in the [T, heads·v] layout o_proj reads). No cuBLAS and no host synchronisation on that path, so decode
-batches run inside CUDA graphs (SURVEY §2.3 K11/K13). Prompt portions of 32 tokens and more take the
+batches run inside CUDA graphs. Prompt portions of 32 tokens and more take the
 *expanded* form instead: the cached latents are gathered, a GEMM makes every head's keys and values, and the tcgen05
 prefill attention runs on them. The CPU / odd-shape path below evaluates the expanded form with PyTorch ops per sequence
 (the numerical oracle of the GPU path).

@@ -1,6 +1,6 @@
 """Built-in HF `config.json` equivalents for the benchmark models, so `--load-format dummy` runs
 need no checkpoint directory (there is no network in the build/bench environment).
-Use as `model_path="preset:qwen3-8b"`. Shapes follow the public HF configs (SURVEY Appendix A).
+Use as `model_path="preset:qwen3-8b"`. Shapes follow the public HF configs.
 """
 PRESETS = {
     "qwen3-8b": {

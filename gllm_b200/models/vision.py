@@ -1,7 +1,7 @@
 """Vision towers of the Qwen-VL families (Qwen2.5-VL windowed ViT, Qwen3-VL ViT with DeepStack).
 
 Runs once per image on the first pipeline stage; not on the serving hot path, so it uses PyTorch
-library ops (SDPA per attention segment) — SURVEY §7 P8. Parameter names mirror the HF checkpoints
+library ops (SDPA per attention segment). Parameter names mirror the HF checkpoints
 (`visual.*`), so loading is a name walk. Every TP rank holds the full tower (the reference shards its QKV
 and re-interleaves with an all-gather, gllm/models/qwen2_5_vl.py:160-239; at <1 B parameters replication is
 cheaper than the extra collectives).
@@ -32,7 +32,7 @@ def _apply_rope(q, k, cos, sin):
 
 # ------------------------------------------------------------------------------------------------
 # tensor parallelism inside the towers (reference: QKVParallel + all_gather_interleave in
-# gllm/models/qwen2_5_vl.py:160-239, SURVEY §2.4 P2c). Here: attention heads and the MLP intermediate dimension
+# gllm/models/qwen2_5_vl.py:160-239). Here: attention heads and the MLP intermediate dimension
 # are split over the TP group, the two row-parallel projections of a block end in an all-reduce; patch embedding,
 # position tables and the mergers stay replicated (small). `GLLM_VISION_TP=0` keeps the whole tower replicated.
 # ------------------------------------------------------------------------------------------------

@@ -47,7 +47,7 @@ def waits_given_up() -> int:
 # ----------------------------------------------------------------------------------------------
 _FORCE_BN = int(os.environ.get("GLLM_GEMM_BN", "0"))
 _SMALLM_MAX = int(os.environ.get("GLLM_GEMM_SMALLM_MAX", "32"))   # M <= this -> swap-AB split-K kernel
-# (measured crossover vs the 128xBN kernel on B200: profiles/gemm_smallm.md)
+# (the crossover with the 128-row kernel, measured)
 _FORCE_SPLIT = int(os.environ.get("GLLM_GEMM_SPLIT", "0"))
 _SMALLM_WS_FLOATS = 24 << 20   # fp32 partial-sum workspace shared by the swap-AB and the split-K kernels
 _SPLITK_MAX_TILES = 4096
@@ -287,7 +287,7 @@ def rope_kv_write(q: torch.Tensor, k: torch.Tensor, v: Optional[torch.Tensor], p
 _attn_ws = {}
 _FUSED_MERGE = os.environ.get("GLLM_ATTN_FUSED_MERGE", "0") == "1"
 # tcgen05 / TMEM prefill attention (csrc/attn/prefill_attention_tc.cu) is the default prefill kernel (validated on
-# B200: profiles/attn_prefill_tc.md; 1.3-2.1x the mma.sync kernel); GLLM_ATTN_TC=0 selects the mma.sync kernel, which
+# B200; 1.3-2.1x the mma.sync kernel); GLLM_ATTN_TC=0 selects the mma.sync kernel, which
 # also serves the shapes outside the tcgen05 kernel's envelope. ATTN_TC_KV (64 or 128) bounds the page size that it takes, and
 # nothing else: it walks 128 keys at a time whatever the pages. The other paged kernels end at pages of 64, hence the default.
 # Module attributes so tests / benches can flip them.

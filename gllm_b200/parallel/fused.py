@@ -73,7 +73,7 @@ MAX_BLOCKS = 256   # kMaxBlocks in csrc/comm/tp_fused.cu (128-row blocks per gat
 # replicated rows + the one-kernel all-reduce⊕add⊕norm instead of the token-sharded GEMM⊕RS / AG⊕GEMM dataflow (see
 # begin_forward). GLLM_TP_SMALL_T=<n> sets both; GLLM_TP_SMALL_T=auto
 # keeps the 64-row buffers and scales the threshold with the LL variant's incoming traffic, (tp-1)*T rows
-# (measured on 8xB200: a 64-token LL step costs 1.8x the 128-token sharded step at TP8, profiles/tp_scaling.md).
+# (measured on 8xB200: a 64-token LL step costs 1.8x the 128-token sharded step at TP8).
 _SMALL_T_ENV = os.environ.get("GLLM_TP_SMALL_T", "64")
 SMALL_T = 64 if _SMALL_T_ENV == "auto" else int(_SMALL_T_ENV)
 

@@ -216,7 +216,7 @@ def divide(a: int, b: int) -> int:
 
 
 # ------------------------------------------------------------------------------------------------
-# tile-streamed PP p2p (SURVEY §2.4 X5): the activation travels as row tiles over NCCL p2p; the receiver
+# tile-streamed PP p2p: the activation travels as row tiles over NCCL p2p; the receiver
 # posts every tile's irecv up front and lets its compute stream wait per tile, so the first layer's
 # add+RMSNorm and QKV GEMM of tile i overlap the transfer of tiles i+1.. (the reference blocks on the
 # whole tensor, gllm/worker.py:141-157).
@@ -232,7 +232,7 @@ def pp_row_tiles(num_rows: int, min_rows: Optional[int] = None, max_tiles: int =
 
 def _pp_shard_rows(r0: int, r1: int):
     """TP>1: instead of every TP rank of a stage shipping the same replicated [rows, H] tile to its peer in the
-    next stage (what the reference does: tp_size redundant copies, SURVEY §2.4 P1), rank k ships only the k-th
+    next stage (what the reference does: tp_size redundant copies), rank k ships only the k-th
     1/tp slice of the tile and the receiving stage re-assembles it with one all-gather over its own TP group
     (NVLink) — tp x fewer bytes on the inter-stage link, which is the slow one when stages sit on different nodes.
     Small tiles (decode) keep the replicated send: one more collective would cost more than the bytes saved.

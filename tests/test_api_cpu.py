@@ -217,7 +217,7 @@ def test_disable_thinking_reaches_the_chat_template():
 
 
 def test_disconnect_mid_chunked_prefill_and_penalty_flood_do_not_kill_the_engine():
-    """ADVICE r1 (high + medium): (1) a client that goes away while its prompt is between two prefill chunks used to
+    """(1) a client that goes away while its prompt is between two prefill chunks used to
     leave a freed sequence at the head of the prefill queue -> double free of its id -> engine loop dead for good;
     (2) more queued repetition-penalty requests than max_running_seqs exhausted the penalty-state pool on arrival."""
     import asyncio

@@ -141,7 +141,7 @@ def test_prefix_cache_decode_page_registered():
 
 
 def test_prefix_cache_never_serves_pages_that_were_not_computed():
-    """a sequence aborted (or stall-broken) between two prefill chunks left the hashes of pages it had only
+    """A sequence aborted (or stall-broken) between two prefill chunks left the hashes of pages it had only
     allocated; a retry of the same prompt then skipped tokens whose KV was never written."""
     ps = 16
     mm = PrefixMemoryManager(64, ps, reserve_dummy_page=True)
@@ -164,7 +164,7 @@ def test_prefix_cache_never_serves_pages_that_were_not_computed():
 
 
 def test_abort_between_prefill_chunks_reports_once_and_leaves_no_stale_id():
-    """ADVICE r1: (a) a sequence flagged while its chunk is in flight is freed and reported exactly once and never
+    """(a) a sequence flagged while its chunk is in flight is freed and reported exactly once and never
     scheduled again; (b) an abort id that matches nothing alive is dropped instead of lingering (it disabled
     lookahead scheduling and hit the next request re-using the id)."""
     ps = 16
@@ -648,7 +648,7 @@ def test_incremental_detokenizer_streams_exactly_the_final_text():
 
 
 def test_vocab_parallel_sampling_model_matches_the_full_vocab_filter():
-    """per-shard candidates + (max, sum-exp) statistics are enough to finish top-k / top-p / penalty
+    """Per-shard candidates + (max, sum-exp) statistics are enough to finish top-k / top-p / penalty
     sampling exactly — every draw lies in the support of the full-vocabulary filter, greedy rows give the argmax, and
     the empirical distribution of a row matches the filtered distribution."""
     import torch

@@ -52,7 +52,7 @@ def test_mixtral_ep2_matches_single():
 
 def test_pp2_tile_streamed_recv_matches_single(single, monkeypatch):
     """Force tiny row tiles so the stage-1 input really arrives as several NCCL/gloo p2p tiles and the
-    first layer's add+norm / QKV projection run per tile (SURVEY §2.4 X5)."""
+    first layer's add+norm / QKV projection run per tile."""
     monkeypatch.setenv("GLLM_PP_TILE_ROWS", "8")
     assert _run(2, 1, port=29871) == single
 
@@ -80,7 +80,7 @@ def test_pp2_tp2_sharded_stage_transfer_matches_single(single, monkeypatch):
 
 @pytest.mark.parametrize("which", ["qwen2_5", "qwen3"])
 def test_vision_tower_tp2_matches_replicated(which):
-    """Heads / MLP-intermediate sharded vision towers (SURVEY §2.4 P2c) == the replicated tower, on both ranks."""
+    """Heads / MLP-intermediate sharded vision towers == the replicated tower, on both ranks."""
     out = os.path.join(scratch_dir("gllm_b200_f_"), "vision.json")
     env = dict(os.environ, PYTHONPATH=ROOT, GLLM_B200_LOG="WARNING")
     port = 29901 if which == "qwen2_5" else 29911
@@ -125,7 +125,7 @@ def test_mixtral_tp2_without_expert_parallelism_matches_single(monkeypatch):
 
 
 def test_tp2_vocab_parallel_sampling_runs_and_keeps_greedy_rows_exact(monkeypatch):
-    """SURVEY §2.4 X4 under gloo: a batch mixing greedy, top-k/top-p + repetition-penalty and unfiltered temperature
+    """Under gloo: a batch mixing greedy, top-k/top-p + repetition-penalty and unfiltered temperature
     rows never gathers the [E, V] logits at TP2 (the runner counts vocab-parallel sampling steps); its greedy rows
     — one of them with a repetition penalty — reproduce the single-process tokens."""
     monkeypatch.setenv("GLLM_TEST_SAMPLED", "1")

@@ -1,5 +1,5 @@
 """Property tests (hypothesis): random request streams through the real Scheduler + PrefixMemoryManager must
-keep the paged-KV bookkeeping consistent at every step (SURVEY §4.2: allocator / prefix-cache refcount and
+keep the paged-KV bookkeeping consistent at every step (allocator / prefix-cache refcount and
 eviction invariants; scheduler budgets; abort and preemption paths)."""
 import random
 
@@ -41,7 +41,7 @@ def check_invariants(mm: PrefixMemoryManager, live):
                 assert i == j and o.token_ids[:(i + 1) * PAGE] == s.token_ids[:(i + 1) * PAGE]
             owner.setdefault(p, (s, i))
     # a cache entry is never ahead of the computation: a page that only this sequence holds and that did not come
-    # from a prefix-cache hit is published only once its whole token range has been computed (ADVICE r1: hashes were
+    # from a prefix-cache hit is published only once its whole token range has been computed (hashes were
     # registered at allocation; an abort / stall-break between two chunks then left entries for unwritten KV)
     for s in live:
         hit_pages = s.num_cached_tokens // mm.page_size

@@ -566,7 +566,7 @@ def test_gemm_batched_strided_views(t, b, n, k):
 
 @pytest.mark.parametrize("tp", [2, 8])
 def test_vocab_parallel_sampling_equals_the_full_vocab_kernel(tp):
-    """SURVEY §2.4 X4: vp_candidates_kernel on each vocab shard + vp_final_kernel on the gathered records draw the
+    """vp_candidates_kernel on each vocab shard + vp_final_kernel on the gathered records draw the
     SAME token as sample_kernel on the full [B, V] row (the race's random numbers are keyed by token id) for greedy,
     top-k, top-k + top-p, nucleus-only, penalised and unfiltered rows — without ever holding the full logits."""
     from gllm_b200.ops import sm100

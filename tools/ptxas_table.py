@@ -3,7 +3,7 @@
     python tools/ptxas_table.py > profiles/ptxas_resources.md
 
 Same flags as gllm_b200/build.py. A spill or a register count near the launch bound is the first thing to check
-before spending GPU time on a kernel change (B200_PROFILING.md)."""
+before spending GPU time on a kernel change."""
 import os
 import re
 import subprocess
