@@ -348,9 +348,13 @@ __global__ void __launch_bounds__(128) rope_kv_pair_kernel(const RopeParams p) {
       }
     }
     if (norm) {
-      float ss = 0.f;
+      float ss = 0.f, upper_ss = 0.f;                    // apart: the order of the sums is the kernel's above, and so are the bits
 #pragma unroll
-      for (int e = 0; e < 8; ++e) ss += x[0][e] * x[0][e] + x[1][e] * x[1][e];
+      for (int e = 0; e < 8; ++e) {
+        ss += x[0][e] * x[0][e];
+        upper_ss += x[1][e] * x[1][e];
+      }
+      ss += upper_ss;
 #pragma unroll
       for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
       const __nv_bfloat16* nw = is_q ? p.q_norm_w : p.k_norm_w;

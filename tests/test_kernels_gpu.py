@@ -200,6 +200,29 @@ def test_rope_kv_write_whole_heads(t, hq, hkv, d, norms, cached):
         assert torch.equal(caches[1], caches[3])
 
 
+@pytest.mark.parametrize("d,sec", [(64, [8, 12, 12]), (128, [16, 24, 24])])
+@pytest.mark.parametrize("t", [300, 4099])                          # one head per lane group, or two
+def test_rope_kv_write_both_forms_give_the_same_bits(d, sec, t):
+    """Three equal rows of positions take the form with a lane per eight elements, one row the one with both halves of a pair in a lane:
+    sums, roundings and rotations are the same, and so is every bit."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(d)
+    hq, hkv = 24, 8
+    pos = torch.randint(0, 4000, (t,), device=_dev(), dtype=torch.int32)
+    slots = torch.randperm(t + 16, device=_dev())[:t].to(torch.int32)
+    cs = ref.build_cos_sin_cache(d, 4096, 10000.0).to(_dev())
+    qn, kn = ((1 + 0.1 * torch.randn(d, device=_dev())).bfloat16() for _ in range(2))
+    src, got = torch.randn(t, (hq + 2 * hkv) * d, device=_dev()).bfloat16(), []
+    for p, section in ((pos, None), (pos.repeat(3, 1), sec)):
+        buf = src.clone()
+        q, k, v = buf.split([hq * d, hkv * d, hkv * d], 1)
+        caches = [torch.zeros(ref.kv_cache_shape(t // 16 + 2, hkv, d, 16), device=_dev(), dtype=torch.bfloat16) for _ in range(2)]
+        sm100.rope_kv_write(q.unflatten(1, (hq, d)), k.unflatten(1, (hkv, d)), v.unflatten(1, (hkv, d)), p, cs, d, True, qn, kn, 1e-6,
+                            *caches, slots, section)
+        got.append((buf, *caches))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 @pytest.mark.parametrize("sec", [[16, 24, 24], [24, 20, 20, 1]])   # chunked (Qwen2.5-VL) / interleaved (Qwen3-VL)
 @pytest.mark.parametrize("strided", [False, True])
 def test_rope_mrope(sec, strided):
