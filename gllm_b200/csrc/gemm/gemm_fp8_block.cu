@@ -13,16 +13,17 @@
 // TMEM buffers ping-pong per K block so the tensor core runs block kb+1 while the CUDA cores fold
 // block kb. Same TMA (SWIZZLE_128B, 128 fp8 = one 128-byte row) / mbarrier ring as gemm_bf16.cu.
 //
-// What bounds it: power. With operands of random bits the clock falls to 1.42 GHz when the product is repeated (4096 x 36864 x 7168: 1.22 ms,
-// 1770 TFLOP/s; all zeros run at 1.89 GHz, 0.98 ms), so that a cycle less costs clock: a 128 x 256 x 128 block takes 965 cycles, without the fold 880 and
-// 1.07 ms. The tensor core needs 512 of them, copies and products write and read 48 KB of shared memory, 768 at 128 bytes; a bare
-// hand-over of products, fold (376 to 440 cycles of its own) and copies reaches 677. What mattered besides is who polls: threads that wait
-// for a barrier without a suspend time took issue slots from the fold (1030 cycles a block). Sixteen fold warps 1290 us for 1110, scales
-// copied by cp.async behind a barrier of their own 1230, boxes of 128 or 256 weight rows, tensor memory handed back before the last sums are added, and
-// pairs of SMs no faster. The scales come from global memory (some 700
-// cycles away) and are therefore fetched kAhead blocks early. With 128-wide tiles, four fold warps and the scales loaded where they are
-// used the product above was 2.0 ms. 4096 x 18432 x 7168 gated + 4096 x 7168 x 18432 with their quantisers (one dense feed-forward):
-// 3.16 -> 2.0 ms.
+// What bounds it: its cycles, at a clock that power sets. 4096 x 36,864 x 7168 repeated for seconds takes 1.20 ms (1810 TFLOP/s) at the
+// power limit, with the clock at 1.50 GHz; all-zero operands run at 1.965 GHz, 0.90 ms. Both are some 990 cycles per 128 x 256 x 128
+// block, so what a change saves in cycles it may pay back in part in clock: without the fold a block took 880, where the product took 1.07
+// ms for 1.22. The tensor core needs 512 of them; copies and products write and read 48 KB of shared memory, 768 at 128 bytes; a bare
+// hand-over of products, fold (376 to 440 cycles of its own) and copies reaches 677. What mattered besides is who polls: threads that
+// wait for a barrier without a suspend time took issue slots from the fold (some 65 cycles a block).
+// No faster, each timed in a short loop, ahead of the power limit, in which this kernel with polling waits took 1110 us: sixteen fold warps (1290),
+// scales copied by cp.async behind a barrier of their own (1230), boxes of 128 or 256 weight rows, tensor memory handed back before the last sums
+// are added, pairs of SMs. The scales come from global memory (some 700 cycles away) and are therefore fetched kAhead blocks early. With
+// 128-wide tiles, four fold warps and the scales loaded where they are used the product was 2.0 ms. 4096 x 18432 x 7168 gated + 4096 x
+// 7168 x 18432 with their quantisers (one dense feed-forward): 3.16 -> 1.93 ms.
 //
 // Also here: the dynamic per-token-group activation quantiser (reference fp8.py:354-552).
 #include <string.h>
@@ -186,7 +187,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kFRegsFold));
     const int q = warp & 3, h = (warp - 4) >> 2;
     constexpr int kHalf = T::kCols / 2;                   // columns of one run
-    constexpr int kLd = 16;                               // columns of one TMEM load (32 at a time: 1390 us for 1110)
+    constexpr int kLd = 16;                               // columns of one TMEM load (32 at a time: 1390 us in the short loop)
     const int c_lo = T::lo(h), c_hi = T::hi(h);
     uint32_t it = 0;
     bool ok = true;
