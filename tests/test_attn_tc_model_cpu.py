@@ -26,7 +26,7 @@ def emulate_prefill_tc(q, kc, vc, bt, seq_lens, q_start, hq, hkv, d, page, scale
     num_seqs = seq_lens.shape[0] - seq_offset
     max_q = int((q_start[1:] - q_start[:-1]).max())
     groups = g_all // gp
-    for block in range((max_q + toks_per_tile - 1) // toks_per_tile * num_seqs * hkv * groups):   # blockIdx.x
+    for block in range((max_q + toks_per_tile - 1) // toks_per_tile * num_seqs * hkv * groups):   # flat: x, y, z of the grid in this order
         # head groups first, then sequences, then from the last query block of each to the first
         z, rest = block % (hkv * groups), block // (hkv * groups)
         seq, back = rest % num_seqs + seq_offset, rest // num_seqs

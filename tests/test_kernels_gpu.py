@@ -356,6 +356,25 @@ def test_prefill_attention_tc_edges(hq, hkv, d, page, many, monkeypatch):
     assert sm100.waits_given_up() == 0
 
 
+def test_prefill_attention_of_more_sequences_than_a_grid_dimension():
+    """65,600 sequences of one or two tokens: the blocks are counted in one dimension then."""
+    from gllm_b200.ops import sm100
+    torch.manual_seed(4)
+    n, d = 65600, 64
+    two = torch.arange(n) % 3 == 0
+    lens = 1 + two.int()
+    qsl = torch.cat([torch.zeros(1, dtype=torch.int32), lens.cumsum(0).int()]).to(_dev())
+    q = torch.randn(int(lens.sum()), d, device=_dev()).bfloat16()
+    kc, vc = (torch.randn(n, 1, 1, 8, d, device=_dev()).bfloat16() for _ in range(2))
+    bt = torch.randperm(n, device=_dev()).int().view(n, 1)
+    o = sm100.paged_attention(q, kc, vc, bt, lens.to(_dev()).int(), qsl, d ** -0.5, 1, d, 0, n, 2, 2).float()
+    k, v = (x[bt[:, 0].long(), 0, 0].float() for x in (kc, vc))
+    first, at = qsl[:-1].long(), two.to(_dev())
+    assert _rel_err(o[first], v[:, 0]) < 1e-2
+    s = torch.einsum("nd,nkd->nk", q[first[at] + 1].float(), k[at, :2]) * d ** -0.5
+    assert _rel_err(o[first[at] + 1], torch.einsum("nk,nkd->nd", s.softmax(-1), v[at, :2])) < 1e-2
+
+
 @pytest.mark.parametrize("window,bad,clean", [(None, 180, (40, 168)), (100, 60, (168, 340))])
 @pytest.mark.parametrize("seqs", [1, 12])                   # one query tile per CTA, or two
 def test_prefill_value_that_is_no_number(window, bad, clean, seqs):
