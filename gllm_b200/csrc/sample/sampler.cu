@@ -276,18 +276,18 @@ __device__ __forceinline__ void select_and_draw(const Row& R, int V, int k, floa
   tok_out = besti;
 }
 
-// `parts` CTAs, a cluster, share a row's argmax pass: each hands its winner to the first, which goes on alone.
-template <typename T>
+// SHARED: `shared_by` CTAs, a cluster, share a row's argmax pass: each hands its winner to the first, which goes on alone.
+template <typename T, bool SHARED>
 __global__ void __launch_bounds__(kSampleThreads)
-sample_kernel(int parts, const T* __restrict__ logits, int64_t ld, int V, const float* __restrict__ temperature,
+sample_kernel(int shared_by, const T* __restrict__ logits, int64_t ld, int V, const float* __restrict__ temperature,
               const int32_t* __restrict__ top_k, const float* __restrict__ top_p,
               const float* __restrict__ rep_penalty, const uint32_t* __restrict__ seen, int seen_words,
               const int32_t* __restrict__ slot_idx, uint64_t seed, const int64_t* __restrict__ step_ptr, int32_t* __restrict__ out_tokens,
               float* __restrict__ out_max, int vocab_offset) {
   __shared__ BlockScratch S;
-  __shared__ uint2 winners[kSampleParts];         // of the cluster's CTAs, in the first one's memory
-  const int row = blockIdx.x / parts, part = blockIdx.x % parts;
-  if (parts > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  __shared__ uint2 winners[SHARED ? kSampleParts : 1];    // of the cluster's CTAs, in the first one's memory
+  const int parts = SHARED ? shared_by : 1, row = blockIdx.x / parts, part = blockIdx.x % parts;
+  if (SHARED) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   griddep_wait();
   const uint32_t* seen_row =
       seen != nullptr ? seen + static_cast<size_t>(slot_idx != nullptr ? slot_idx[row] : row) * seen_words : nullptr;
@@ -307,7 +307,7 @@ sample_kernel(int parts, const T* __restrict__ logits, int64_t ld, int V, const 
   int imax;
   R.argmax(V, part, parts, vmax, imax);
   block_argmax(vmax, imax, S);
-  if (parts > 1) {
+  if constexpr (SHARED) {
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");            // every CTA of the cluster has begun: its memory is there
     if (threadIdx.x == 0)
       asm volatile("st.shared::cluster.v2.b32 [%0], {%1, %2};" ::"r"(cluster_addr(&winners[part], 0)), "r"(__float_as_uint(vmax)),
@@ -538,12 +538,18 @@ GLLM_EXPORT int gllm_sample(const void* logits, int dtype, int64_t ld, void* out
     parts *= 2;
   auto run = [&](auto* row0) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(row0)>>;
-    return launch_pdl_cluster(sample_kernel<T>, dim3(B * parts), parts, dim3(kSampleThreads), 0, st, parts, row0, ld, V,
-                              reinterpret_cast<const float*>(temperature), reinterpret_cast<const int32_t*>(top_k),
-                              reinterpret_cast<const float*>(top_p), reinterpret_cast<const float*>(rep_penalty),
-                              reinterpret_cast<const uint32_t*>(seen), seen_words, reinterpret_cast<const int32_t*>(slot_idx), seed,
-                              reinterpret_cast<const int64_t*>(step_ptr), reinterpret_cast<int32_t*>(out_tokens),
-                              reinterpret_cast<float*>(out_max), vocab_offset);
+    auto launch = [&](auto kern, auto go) {
+      return go(kern, parts, row0, ld, V, reinterpret_cast<const float*>(temperature), reinterpret_cast<const int32_t*>(top_k),
+                reinterpret_cast<const float*>(top_p), reinterpret_cast<const float*>(rep_penalty),
+                reinterpret_cast<const uint32_t*>(seen), seen_words, reinterpret_cast<const int32_t*>(slot_idx), seed,
+                reinterpret_cast<const int64_t*>(step_ptr), reinterpret_cast<int32_t*>(out_tokens), reinterpret_cast<float*>(out_max),
+                vocab_offset);
+    };
+    if (parts == 1)
+      return launch(sample_kernel<T, false>, [&](auto kern, auto... a) { return launch_pdl(kern, dim3(B), dim3(kSampleThreads), 0, st, a...); });
+    return launch(sample_kernel<T, true>, [&](auto kern, auto... a) {
+      return launch_pdl_cluster(kern, dim3(B * parts), parts, dim3(kSampleThreads), 0, st, a...);
+    });
   };
   CUDA_CHECK_RET(dtype == 0 ? run(reinterpret_cast<const __nv_bfloat16*>(logits)) : run(reinterpret_cast<const float*>(logits)));
   CUDA_CHECK_RET(cudaGetLastError());
