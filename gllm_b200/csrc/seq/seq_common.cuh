@@ -2,6 +2,7 @@
 // row -> sequence lookup, paged-cache indexing. Each .cu file pulls them in with `using namespace seqk`.
 #pragma once
 #include <cuda_bf16.h>
+#include <type_traits>
 
 namespace seqk {
 
@@ -41,6 +42,15 @@ __device__ __forceinline__ void un(f2 v, float& a, float& b) { asm("mov.b64 {%0,
 __device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
 __device__ __forceinline__ f2 add2(f2 a, f2 b) { f2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+// the same, one float to an instruction
+template <typename V> __device__ __forceinline__ V pair(float a, float b) {
+  if constexpr (std::is_same_v<V, f2>) return pk(a, b);
+  else return make_float2(a, b);
+}
+__device__ __forceinline__ void un(float2 v, float& a, float& b) { a = v.x; b = v.y; }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)); }
 __device__ __forceinline__ float rcp(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 // sequence that owns batch row t: largest s with qsl[s] <= t

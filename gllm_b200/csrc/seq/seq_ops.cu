@@ -369,10 +369,12 @@ __global__ void conv_silu_kernel(const T* __restrict__ xz, long ldxz, int C, con
 // issue slots and a row's own chain (sum, 2^x, 1/x), hence the sigmoid from the units, two channels to an instruction, and groups of
 // four rows without a border that carry no branch, so that the rows' chains overlap (two channels to an instruction alone gained
 // nothing). With the state's update, 6000 rows of 8192 channels: 71 -> 60 us; 8192 rows: 87 -> 71; 40000: 343 -> 269 (4.9 TB/s);
-// 8192 rows of 2560: 38 -> 34. Of 8192 channels, blocks of 48 to 128 rows lie within 9 % of 64, blocks of 16 up to 18 % above.
+// 8192 rows of 2560: 38 -> 34. Blocks of one row wait for their first loads and are done sooner with a channel to an instruction (not
+// PAIRS): 500 rows of 8192 channels 20.1 us, in pairs 22.8; blocks of eight rows are not (2000 of 5120: 23.0, 22.2). Of 8192 channels,
+// blocks of 48 to 128 rows lie within 9 % of 64, blocks of 16 up to 18 % above.
 // Sequences of one token also update their carried inputs here (longer ones: the kernel
 // below, after every block has read them).
-template <int TAPS, bool LONG>
+template <int TAPS, bool LONG, bool PAIRS>
 __global__ void __launch_bounds__(128) conv_silu_vec_kernel(
     const __nv_bfloat16* __restrict__ xz, long ldxz, int C, const float* __restrict__ w, const float* __restrict__ b,
     __nv_bfloat16* __restrict__ state, const int* __restrict__ rec_slots, const int* __restrict__ seq_lens,
@@ -381,28 +383,29 @@ __global__ void __launch_bounds__(128) conv_silu_vec_kernel(
   const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
   if (c >= C) return;
   const int t0 = blockIdx.x * rows, t1 = min(t0 + rows, ntok);
-  f2 wr[TAPS][2], br[2], ib[2];                  // channels c, c + 1 and c + 2, c + 3
+  using V = std::conditional_t<PAIRS, f2, float2>;
+  V wr[TAPS][2], br[2], ib[2];                   // channels c, c + 1 and c + 2, c + 3
   {
     __align__(16) float raw[4 * TAPS];           // weight of channel e, tap j: raw[e * TAPS + j]
 #pragma unroll
     for (int e = 0; e < 4 * TAPS; e += 4)
       *reinterpret_cast<float4*>(raw + e) = *reinterpret_cast<const float4*>(w + (size_t)c * TAPS + e);
     const float4 bv = *reinterpret_cast<const float4*>(b + c);
-    br[0] = pk(bv.x, bv.y);
-    br[1] = pk(bv.z, bv.w);
+    br[0] = pair<V>(bv.x, bv.y);
+    br[1] = pair<V>(bv.z, bv.w);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      ib[h] = in_bias != nullptr ? pk(in_bias[c + 2 * h], in_bias[c + 2 * h + 1]) : pk(0.f, 0.f);
+      ib[h] = in_bias != nullptr ? pair<V>(in_bias[c + 2 * h], in_bias[c + 2 * h + 1]) : pair<V>(0.f, 0.f);
 #pragma unroll
-      for (int j = 0; j < TAPS; ++j) wr[j][h] = pk(raw[2 * h * TAPS + j], raw[(2 * h + 1) * TAPS + j]);
+      for (int j = 0; j < TAPS; ++j) wr[j][h] = pair<V>(raw[2 * h * TAPS + j], raw[(2 * h + 1) * TAPS + j]);
     }
   }
-  auto unpack = [](const uint2 v, f2 (&f)[2]) {
-    f[0] = pk(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u));
-    f[1] = pk(__uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+  auto unpack = [](const uint2 v, V (&f)[2]) {
+    f[0] = pair<V>(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u));
+    f[1] = pair<V>(__uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
   };
-  const f2 minus_log2e = pk(-1.4426950408889634f, -1.4426950408889634f), one = pk(1.f, 1.f);
-  f2 win[TAPS][2];                               // win[0 .. TAPS-2]: inputs before the row; win[TAPS-1]: the row's own
+  const V minus_log2e = pair<V>(-1.4426950408889634f, -1.4426950408889634f), one = pair<V>(1.f, 1.f);
+  V win[TAPS][2];                               // win[0 .. TAPS-2]: inputs before the row; win[TAPS-1]: the row's own
   int s = find_seq(qsl, nseq, t0), q0 = 0, q1 = -1;
   constexpr int kAhead = LONG ? 4 : 1, kGroups = 4;      // rows of a copy group; groups on their way
   __shared__ uint2 ring[LONG ? kGroups * kAhead : 1][128];
@@ -428,14 +431,14 @@ __global__ void __launch_bounds__(128) conv_silu_vec_kernel(
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       win[TAPS - 1][h] = add2(win[TAPS - 1][h], ib[h]);
-      f2 acc = br[h];
+      V acc = br[h];
 #pragma unroll
       for (int j = 0; j < TAPS; ++j) acc = fma2(wr[j][h], win[j][h], acc);
       if (act == 0) {  // times 1 / (1 + e^-acc): within |acc| 2^-24 + 2^-21 of it, for the exponent is rounded to one fp32
         float e0, e1;
         un(mul2(acc, minus_log2e), e0, e1);
-        un(add2(pk(ex2(e0), ex2(e1)), one), e0, e1);
-        acc = mul2(acc, pk(rcp(e0), rcp(e1)));
+        un(add2(pair<V>(ex2(e0), ex2(e1)), one), e0, e1);
+        acc = mul2(acc, pair<V>(rcp(e0), rcp(e1)));
       }
       float y0, y1;
       un(acc, y0, y1);
@@ -477,12 +480,12 @@ __global__ void __launch_bounds__(128) conv_silu_vec_kernel(
         for (int j = 0; j < TAPS - 1; ++j) {
           const int src = li - (TAPS - 1) + j;
           const bool own = src >= 0, have = own || (carried && pos0 + src >= 0);
-          f2 f[2];
+          V f[2];
           if (own) unpack(*reinterpret_cast<const uint2*>(xz + (size_t)(q0 + src) * ldxz + c), f);
           else if (have)
             unpack(*reinterpret_cast<const uint2*>(state + ((size_t)rec_slots[s] * (TAPS - 1) + TAPS - 1 + src) * C + c), f);
 #pragma unroll
-          for (int h = 0; h < 2; ++h) win[j][h] = have ? add2(f[h], ib[h]) : pk(0.f, 0.f);
+          for (int h = 0; h < 2; ++h) win[j][h] = have ? add2(f[h], ib[h]) : pair<V>(0.f, 0.f);
         }
       }
       one_row(t, cur);
@@ -816,7 +819,8 @@ GLLM_EXPORT int gllm_seq_conv_silu(const void* xz, long ldxz, int ntok, int nseq
     while (rows > 16 && (int64_t)((ntok + rows - 1) / rows) * across < 8 * b200::num_sms()) rows /= 2;
     dim3 vgrid((ntok + rows - 1) / rows, across);
 #define GLLM_CONV_VEC(TAPS)                                                                                        \
-  (rows >= 16 ? conv_silu_vec_kernel<TAPS, true> : conv_silu_vec_kernel<TAPS, false>)<<<vgrid, 128, 0, st>>>(              \
+  (rows >= 16 ? conv_silu_vec_kernel<TAPS, true, true>                                                            \
+   : rows > 1 ? conv_silu_vec_kernel<TAPS, false, true> : conv_silu_vec_kernel<TAPS, false, false>)<<<vgrid, 128, 0, st>>>(              \
       (const __nv_bfloat16*)xz, ldxz, C, (const float*)w, (const float*)b, (__nv_bfloat16*)state,                  \
       (const int*)rec_slots, (const int*)seq_lens, (const int*)qsl, nseq, ntok, rows, (__nv_bfloat16*)out, act,    \
       (const float*)in_bias)
