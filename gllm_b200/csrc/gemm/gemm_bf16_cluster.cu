@@ -302,25 +302,25 @@ const Slots* slots() {                                   // null: not known
 
 }  // namespace
 
-// The plan with the least modelled time (us): rounds of clusters, each 4.4 + 0.005 per row of A (start, exchange, stores), and the
-// larger of what an SM copies (100 KB per us) and what the memory gives. Fitted to some 9000 timings (20 weights of 512 x 4096 to
-// 57,344 x 8192, 1 to 512 rows, all plans, weights cold, launched back to back). Of clusters of three or five, fewer run at once than
-// the query says (45 of three on an SM each: 5760 x 4096, 128 rows 21.5 us, 16.2 with a plan that leaves two of them free; 26 of five:
-// 3328 x 8192, 512 rows 40.6 / 31.5); 15 of eight, 33 of four and 22 of six do.
+// The plan with the least modelled time (us): rounds of clusters, each 4.4 + 0.005 per row of A (start, exchange, stores), and the larger
+// of what an SM copies (100 KB per us) and what the memory gives. Fitted to some 9000 timings (20 weights of 512 x 4096 to 57,344 x 8192,
+// 1 to 512 rows, all plans, weights cold, launched back to back). Of clusters of three or five, fewer run at once than the query says (45
+// of three on an SM each: 5760 x 4096, 128 rows 21.5 us, 16.2 with a plan that leaves two of them free; 26 of five: 3328 x 8192, 512 rows
+// 40.6 / 31.5); 15 of eight, 33 of four and 22 of six do.
 //
-// Taken instead of the other kernels: over 3456 plain and 770 gated products (weights drawn between 512 and 24,576 rows and 768 and 14,336
-// columns, 3 to 512 rows of A) one takes 0.80 (gated 0.72) of the time that those took on average; 30 plain ones take 5 % more or
-// worse, 1.16 at worst (without the rules (e) to (g) and with the slots as the query says 211, 1.56). Some (rows: weights, before -> now, us): 4: 24,576 x 4096 gated 37.9 -> 35.1; 16: 6144 x 4096 14.6 -> 11.8, 1024 x
-// 3072 7.8 -> 5.8; 32: 4096 x 4096 14.2 -> 10.2; 64: 4096 x 12,288 29 -> 21, 10,240 x 8192 50 -> 31; 128: 2112 x 7168 15.5 -> 13.8;
-// 256: 6144 x 4096 24.3 -> 21.5.
-// Not taken: (a) 592 and more tiles across (heads of 151,936 columns): persistent CTAs with one start lose less (16 rows 49 us, here 63).
-// (b) As wide as the machine or wider, with more than 64 rows (57,344 x 8192 gated, 128 rows: 165, here 171), or gated tiles of 192
-// that fit one round, with more than 32 (24,576 x 4096, 64 rows: 37.3, here 38.2): nothing to cut, and those tiles read A less often. (c) A
-// few rows on few tiles: sixteen parts draw more than eight (768 x 4096, 4 rows 5.7 us, here 6.3). (d) Over 256 rows,
-// except for narrow products with enough K (512 rows, 4096 x 4096: 24.2 -> 20.8 taken; 6144 x 4096 31.0, here 32.7). Plain ones
-// where the other tiles fill the machine in one round: (e) K is not cut here either, up to 32 rows on nearly as many tiles as SMs (16,896 x
-// 832, 32 rows 8.8, here 10.3), or rows that nearly fill tiles of 128 (12,736 x 1856, 128 rows 14.0, here 16.7), or with
-// more than 216 rows more than one round of a short K (10,432 x 2496, 256 rows 17, here 21; 9664 x 9472 64.7 and 55.7); (f) K in four parts there (4608 x 2368, 128 rows 11.5, here 12.6; 3072 x
+// Taken instead of the other kernels: over 3456 plain and 770 gated products (weights drawn between 512 and 24,576 rows and 768 and
+// 14,336 columns, 3 to 512 rows of A) one takes 0.80 (gated 0.72) of the time that those took on average; 30 plain ones take 5 % more or
+// worse, 1.16 at worst (without the rules (e) to (g) and with the slots as the query says 211, 1.56). Some (rows: weights, before -> now,
+// us): 4: 24,576 x 4096 gated 37.9 -> 35.1; 16: 6144 x 4096 14.6 -> 11.8, 1024 x 3072 7.8 -> 5.8; 32: 4096 x 4096 14.2 -> 10.2; 64: 4096
+// x 12,288 29 -> 21, 10,240 x 8192 50 -> 31; 128: 2112 x 7168 15.5 -> 13.8; 256: 6144 x 4096 24.3 -> 21.5. Not taken: (a) 592 and more
+// tiles across (heads of 151,936 columns): persistent CTAs with one start lose less (16 rows 49 us, here 63). (b) As wide as the machine
+// or wider, with more than 64 rows (57,344 x 8192 gated, 128 rows: 165, here 171), or gated tiles of 192 that fit one round, with more
+// than 32 (24,576 x 4096, 64 rows: 37.3, here 38.2): nothing to cut, and those tiles read A less often. (c) A few rows on few tiles:
+// sixteen parts draw more than eight (768 x 4096, 4 rows 5.7 us, here 6.3). (d) Over 256 rows, except for narrow products with enough K
+// (512 rows, 4096 x 4096: 24.2 -> 20.8 taken; 6144 x 4096 31.0, here 32.7). Plain ones where the other tiles fill the machine in one
+// round: (e) K is not cut here either, up to 32 rows on nearly as many tiles as SMs (16,896 x 832, 32 rows 8.8, here 10.3), or rows that
+// nearly fill tiles of 128 (12,736 x 1856, 128 rows 14.0, here 16.7), or with more than 216 rows more than one round of a short K (10,432
+// x 2496, 256 rows 17, here 21; 9664 x 9472 64.7 and 55.7); (f) K in four parts there (4608 x 2368, 128 rows 11.5, here 12.6; 3072 x
 // 8192, 384 rows 25, here 30; with K below 4480 15.9 and 15.3); (g) a short K (11,008 x 960, 128 rows 9.7, here 11.3).
 static bool others_are_faster(int M, int N, int K, int bn, int split, const ClusterPlan& plan, int rounds) {
   const int tiles_n = (N + kCW - 1) / kCW, sms = num_sms(), num_kb = (K + kCK - 1) / kCK, rows = (M + 127) / 128, spare = rows * 128 - M;

@@ -320,7 +320,8 @@ __global__ void __launch_bounds__(kAlignThreads) moe_align_kernel(const RoutePar
   griddep_wait();
   const int valid = p.n_valid != nullptr ? min(p.n_slots, *p.n_valid) : p.n_slots;
   const int part = ONE ? 0 : blockIdx.x, parts = ONE ? 1 : gridDim.x;
-  const int lo = static_cast<int>(static_cast<int64_t>(valid) * part / parts), hi = static_cast<int>(static_cast<int64_t>(valid) * (part + 1) / parts);
+  const int lo = static_cast<int>(static_cast<int64_t>(valid) * part / parts);
+  const int hi = static_cast<int>(static_cast<int64_t>(valid) * (part + 1) / parts);
   const int first = lo + static_cast<int>(threadIdx.x);
   auto experts_of = [&](int i0, int (&e)[kU]) {
 #pragma unroll
