@@ -458,7 +458,8 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ o, int n, cons
 // warp has the loads of 4 x 128 columns in flight, where 4-byte loads of one group at a time were bound by their latency.
 // 6000 tokens x 32 groups of 128: 97 -> 61 us, with the gate from the 2^x and 1/x units instead of expf and a division 51. What bounds
 // it then is the issue slots (73 % of the cycles): two columns to an instruction, and one tree of sums and one root for the warp's
-// four groups, 53 -> 43 (3.4 TB/s; 8192 tokens 70 -> 54; groups of 256, 8192 tokens: 61 -> 54). Where the
+// four groups, 53 -> 43 (3.4 TB/s; 8192 tokens 70 -> 54; groups of 256, 8192 tokens: 61 -> 54). The weights are fetched with the rows:
+// behind the sums, a weight for every column cost one token of 16 groups of 256 2.6 us for 2.2, 8192 tokens 45 for 42. Where the
 // groups do not fill the machine, four in a row only make a warp slower (one token, 32 groups of 128: 3.2 us element-wise, 4.1 with
 // four): one group per warp there.
 template <int NCH, int kRows>
@@ -472,7 +473,7 @@ __global__ void __launch_bounds__(128) gated_group_norm_vec_kernel(
   const int count = (int)min((long)kRows, total - g0);
   int t = (int)(g0 / ngroups), gi = (int)(g0 % ngroups);
   float4 v[kRows][NCH];
-  uint2 gt[kRows][NCH];
+  uint2 gt[kRows][NCH], wt[kRows][NCH];
   int tok[kRows], col[kRows];
 #pragma unroll
   for (int i = 0; i < kRows; ++i) {
@@ -484,6 +485,8 @@ __global__ void __launch_bounds__(128) gated_group_norm_vec_kernel(
       for (int c = 0; c < NCH; ++c) {
         v[i][c] = *reinterpret_cast<const float4*>(o + (size_t)tok[i] * n + col[i] + c * 128);
         gt[i][c] = *reinterpret_cast<const uint2*>(gate + (size_t)tok[i] * ldg + col[i] + c * 128);
+        const int k = col[i] + c * 128;
+        wt[i][c] = *reinterpret_cast<const uint2*>(w + (wlen == kGroup ? lane * 4 + c * 128 : wlen == n ? k : k % wlen));
       }
     }
   }
@@ -517,8 +520,8 @@ __global__ void __launch_bounds__(128) gated_group_norm_vec_kernel(
     const f2 r = pk(ri, ri);
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {
-      const int k = col[i] + c * 128, wc = wlen == kGroup ? lane * 4 + c * 128 : wlen == n ? k : k % wlen;
-      const uint2 wr = *reinterpret_cast<const uint2*>(w + wc);
+      const int k = col[i] + c * 128;
+      const uint2 wr = wt[i][c];
       auto two = [&](float x0, float x1, uint32_t wt, uint32_t g) {
         const float g0 = __uint_as_float(g << 16), g1 = __uint_as_float(g & 0xffff0000u);
         f2 sg = sigmoid_parts2(g0, g1);
