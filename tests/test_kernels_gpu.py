@@ -1321,6 +1321,21 @@ def test_norm_that_no_product_takes(m, k):
     assert torch.equal(Fn.NormedSum(y, res, w, 1e-6).tensor(), normed)
 
 
+@pytest.mark.parametrize("m,k,deferred", [(1, 3072, True), (1, 3080, False), (2, 1024, True), (2, 1032, False), (3, 512, False)])
+def test_rows_whose_norm_is_deferred(m, k, deferred):
+    """Short rows leave their norm to the product behind it, longer ones do not; either way the product and the sum are those of the
+    norm and the product by themselves (fp32 sums in another order: 2^-8 of some normed values)."""
+    from gllm_b200.layers import functional as Fn
+    from gllm_b200.parallel.tp import TPComm
+    torch.manual_seed(k)
+    a, w1, w2 = torch.randn(m, 256, device=_dev()).bfloat16(), torch.randn(k, 256, device=_dev()).bfloat16(), torch.randn(384, k, device=_dev()).bfloat16()
+    res, nw, tpc = torch.randn(m, k, device=_dev()).bfloat16(), (1 + 0.2 * torch.randn(k, device=_dev())).bfloat16(), TPComm()
+    normed, want = Fn.rmsnorm(Fn.linear(a, w1), nw, 1e-6, res.clone())
+    h, got = tpc.row_linear_add_norm(a, w1, res, nw, 1e-6, defer=True)
+    assert isinstance(h, Fn.NormedSum) == deferred
+    assert _rel_err(tpc.col_linear(h, w2), Fn.linear(normed, w2)) < 6e-3 and torch.equal(got, want)
+
+
 @pytest.mark.parametrize("where", ["layer", "layer behind", "attention", "all modules", None])
 def test_hooks_see_tensors_between_layers(where, monkeypatch):
     """A hook between two layers sees the normed input and the residual stream as tensors that are there: the norm is not left to the
