@@ -252,7 +252,7 @@ mla_attn_kernel(const __grid_constant__ CUtensorMap tmap, const MlaParams p) {
 
     for (int i = 0; i < len; ++i, ++it) {
       const int s = it % kMlaStages;
-      if (!guard.gave_up()) guard.wait(&full_bar[s], (it / kMlaStages) & 1);   // given up: the share's tiles are run out, not waited for
+      guard.wait<true>(&full_bar[s], (it / kMlaStages) & 1);   // polled: a wait per tile (256 tokens, 128 heads: 443 us, suspended 451)
       const uint32_t sk = smem_u32(smem + s * kMlaTileBytes);
 
       // S = Q K^T for 16 rows x 16 keys, k = this warp's half of 576; two chains per 8 keys

@@ -1,7 +1,8 @@
 // Bounded mbarrier waits. A wait that never ends would hang the GPU for everyone on it, so after a limit the kernel records
-// that it gave up, every later wait of the CTA ends within a suspension (0.1 ms), the roles leave their loops without issuing copies
-// or products, what is in flight lands and the kernel returns. Its results are wrong then: the record is one word of pinned host
-// memory, which the engine reads before it uses a step's tokens (ops/lib.py) and fails on.
+// that it gave up, every later wait of the CTA ends within a suspension (0.1 ms; polled ones within a microsecond or two), the
+// roles run or leave their loops without issuing copies or products, what is in flight lands and the kernel returns. Its results
+// are wrong then: the record is one word of pinned host memory, which the engine reads before it uses a step's tokens (ops/lib.py)
+// and fails on.
 #pragma once
 
 #include "host_utils.h"

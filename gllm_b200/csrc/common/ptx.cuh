@@ -83,7 +83,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity, ui
 }
 
 // the same, back as soon as the hardware likes: polling wakes up a little sooner, where one wait follows another (prefill attention of 8192
-// tokens over 8192 cached: 4292 us for a block, suspended 4309)
+// tokens over 8192 cached: 4292 us for a block, suspended 4309; latent attention of 256 tokens, 128 heads: 443, suspended 451)
 __device__ __forceinline__ bool mbar_try_wait_soon(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
