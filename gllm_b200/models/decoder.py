@@ -245,8 +245,9 @@ class DecoderLayer(nn.Module):
         when `next_norm_w` is None (last layer of a non-final pipeline stage)."""
         eps = self.spec.rms_eps
         a = self.attn(inp, h, kv_cache, tpc, qkv=qkv)
-        h, residual = tpc.row_linear_add_norm(a, _qw(self.attn.o_w, self.attn.o_ws), residual, self.post_norm_w, eps, self.attn.o_b,
-                                              defer=not self.is_moe and self.mlp.fused_act)
+        known = getattr(tpc, "defers", False)
+        more = {"defer": True} if known and type(self.mlp) is DenseMLP and self.mlp.fused_act else {}
+        h, residual = tpc.row_linear_add_norm(a, _qw(self.attn.o_w, self.attn.o_ws), residual, self.post_norm_w, eps, self.attn.o_b, **more)
         if self.is_moe:
             if next_norm_w is None:
                 return tpc.all_reduce(self.mlp(tpc.materialize(h), tpc)), residual
@@ -254,7 +255,7 @@ class DecoderLayer(nn.Module):
         act = self.mlp.act(h, tpc)
         if next_norm_w is None:
             return tpc.row_linear(act, self.mlp.down_weight()), residual
-        return tpc.row_linear_add_norm(act, self.mlp.down_weight(), residual, next_norm_w, eps, defer=defer)
+        return tpc.row_linear_add_norm(act, self.mlp.down_weight(), residual, next_norm_w, eps, **({"defer": True} if known and defer else {}))
 
 
 def _hooked(module: nn.Module) -> bool:

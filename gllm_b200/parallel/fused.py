@@ -317,7 +317,7 @@ class FusedTPComm(TPComm):
             return sm100.linear_silu_mul(x, w_interleaved)
         return sm100.linear_silu_mul(x, w_interleaved, comm=comm)
 
-    def row_linear_add_norm(self, x, w, residual, norm_w, eps, bias=None, defer=False):
+    def row_linear_add_norm(self, x, w, residual, norm_w, eps, bias=None):
         from gllm_b200.ops import sm100
         if self.small:
             # decode-sized T: best local GEMM for the shape (swap-AB / split-K), then the one-kernel

@@ -30,6 +30,9 @@ class TPComm:
         st = ps.get_state()
         self.tp_size = st.tp_size
         self.tp_rank = st.tp_rank
+        # a deferred norm goes through these: a strategy with one of its own is neither asked for it nor given it
+        self.defers = all(getattr(type(self), n) is getattr(TPComm, n)
+                          for n in ("row_linear_add_norm", "col_linear", "col_linear_silu_mul", "materialize"))
 
     # hooks the runner calls around a forward pass (used by the fused implementation)
     def begin_forward(self, num_tokens: int):

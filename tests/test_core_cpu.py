@@ -828,3 +828,52 @@ def test_deferred_norm_refuses_a_weight_of_another_width(act):
         h = Fn.NormedSum(y, torch.zeros(1, 64).bfloat16(), w, 1e-6)
         with pytest.raises(AssertionError):
             (h.linear_silu_mul if act else h.linear)(torch.zeros(256, k).bfloat16())
+
+
+@pytest.mark.parametrize("what", ["mlp", "strategy", "products"])
+def test_layers_take_a_users_mlp_and_parallel_strategy(what):
+    """A feed-forward of a user's own with `act` and `down_weight`, and a strategy with a `row_linear_add_norm` of its own: a layer calls them
+    as it called its own before norms could be deferred, and hands them tensors."""
+    from types import SimpleNamespace
+    import torch
+    from gllm_b200.models.decoder import CausalLM, ModelSpec
+    from gllm_b200.parallel.tp import TPComm
+    torch.manual_seed(1)
+    spec = ModelSpec(arch="Qwen3ForCausalLM", hidden_size=64, num_layers=2, num_heads=2, num_kv_heads=1, head_dim=32, intermediate_size=128,
+                     vocab_size=32, max_position=16, dtype=torch.float32)
+    model = CausalLM(spec)
+    for p in model.parameters():
+        p.data.normal_(std=0.1)
+    inp, tpc = SimpleNamespace(tokens=torch.tensor([3], dtype=torch.int32)), TPComm()
+    want, _ = model(inp, None, tpc)
+
+    class Mlp(torch.nn.Module):
+        def __init__(self, of):
+            super().__init__()
+            self.of = of
+
+        def act(self, h, tpc):
+            assert isinstance(h, torch.Tensor)
+            return self.of.act(h, tpc)
+
+        def down_weight(self):
+            return self.of.down_weight()
+
+    class Strategy(TPComm):
+        def row_linear_add_norm(self, x, w, residual, norm_w, eps, bias=None):
+            return super().row_linear_add_norm(x, w, residual, norm_w, eps, bias)
+
+    class Products(TPComm):
+        def col_linear(self, x, w, bias=None):
+            assert isinstance(x, torch.Tensor)
+            return super().col_linear(x, w, bias)
+
+    if what == "mlp":
+        for layer in model.layers:
+            layer.mlp = Mlp(layer.mlp)
+    elif what == "strategy":
+        tpc = Strategy()
+    else:
+        tpc = Products()
+        assert not tpc.defers
+    assert torch.equal(model(inp, None, tpc)[0], want)
