@@ -303,11 +303,19 @@ sample_kernel(int shared_by, const T* __restrict__ logits, int64_t ld, int V, co
   const float tp = top_p != nullptr ? top_p[row] : 1.0f;
 
   // ---- pass A: max / argmax ----
+  // A row that draws is read again by the first CTA, out of its L1 if it fits. A cluster's barrier empties that, so such a row is the
+  // first CTA's alone, behind the barrier (64 rows of 128,256 bf16 logits with a temperature 71 us, shared 78; one of
+  // 50,257 27 and 32). Larger rows gain by sharing: one of 262,144 157 us, alone 170.
+  const bool alone = SHARED && k != 1 && static_cast<int64_t>(V) * static_cast<int>(sizeof(T)) <= 262144;
+  if (alone) {
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (part != 0) return;
+  }
   float vmax;
   int imax;
-  R.argmax(V, part, parts, vmax, imax);
+  R.argmax(V, part, alone ? 1 : parts, vmax, imax);
   block_argmax(vmax, imax, S);
-  if constexpr (SHARED) {
+  if (SHARED && !alone) {
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");            // every CTA of the cluster has begun: its memory is there
     if (threadIdx.x == 0)
       asm volatile("st.shared::cluster.v2.b32 [%0], {%1, %2};" ::"r"(cluster_addr(&winners[part], 0)), "r"(__float_as_uint(vmax)),

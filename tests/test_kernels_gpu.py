@@ -546,10 +546,11 @@ def test_sampler_greedy_edges(v, dt):
 
 
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("b,v", [(1, 24575), (1, 24576), (3, 49159), (13, 50001), (14, 50000), (32, 49152), (33, 49156), (69, 49152), (70, 49151)])
+@pytest.mark.parametrize("b,v", [(1, 24575), (1, 24576), (3, 49159), (13, 50001), (14, 50000), (32, 49152), (33, 49156), (69, 49152), (70, 49151), (2, 131072),
+                                 (2, 131073)])
 def test_sampler_rows_shared_by_a_cluster(b, v, dt):
     """Rows whose argmax pass eight, four, two CTAs or one share: ties within and across their parts, an unaligned row, rows that draw
-    beside greedy ones, whose tokens do not depend on how many CTAs share the row."""
+    beside greedy ones (up to 256 KB by one CTA), whose tokens do not depend on how many CTAs share the row."""
     from gllm_b200.ops import sm100
     torch.manual_seed(b + v)
     base = torch.randn(b, v + 3, device=_dev()).to(dt)
